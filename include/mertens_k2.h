@@ -263,14 +263,15 @@ int mb_k2_fast(mb_table *t, int64_t P, const uint64_t *v_int, const uint64_t *v_
 
 /* Grid scan: out_h[p * n_m + i] = K2(v_p + (m0 + i) step) for i < n_m, with step the 64.64
  * fixed-point number step_int + step_frac 2^-64.  Every grid point's phase is exact
- * (frac(y G) = frac(v G) + m frac(step G), 128-bit); sine/cosine and sums in FP64.
- * Replaces the FP64 grid of search/polish.py:50-72 (phi + m dphi mod 2pi) and the grid stages
+ * (frac(y G) = frac(v G) + m frac(step G), 128-bit); sine/cosine and sums in FP64, over the zeros
+ * or, where that is less work, over moments of cells of zeros taken once per block of points (the
+ * same value within FP64 rounding).  Replaces the FP64 grid of search/polish.py:50-72 (phi + m dphi mod 2pi) and the grid stages
  * of search/gpu_mertens_stream.cu:381-505 / path1_eval_fast.cpp:86-101. */
 int mb_grid_scan(mb_table *t, int64_t P, const uint64_t *v_int, const uint64_t *v_frac, double k, double T,
                  uint64_t step_int, uint64_t step_frac, int64_t m0, int64_t n_m, double *out_h);
 
 /* Many small grids: out_h[p * n_m + i] = K2 over the first n_use zeros at v_p + (m0 + i) step,
- * n_m <= 1024, one CTA per base point.  The stage scans of the enumerators' hit polish
+ * n_m <= 1024, as mb_grid_scan.  The stage scans of the enumerators' hit polish
  * (search/gpu_mertens_stream.cu:381-505 ZeroData::polish, search/fast_mertens_enum.cpp:145-276:
  * 256, 512, 2048, 15000 and all zeros at decreasing steps) are calls of this. */
 int mb_hit_scan(mb_table *t, int64_t P, const uint64_t *v_int, const uint64_t *v_frac, double k, int64_t n_use,
@@ -350,9 +351,12 @@ int mb_polish_peaks_exact(mb_table *t, int64_t P, const uint64_t *v_int, const u
 /* mb_polish_peaks_exact under n_weights registered weight vectors at once (outputs n_weights x P,
  * row w for weight_slots[w]; each row equals the single-weight call).  The search drivers' step
  * (search/eval_tech1_600k.py:216-273: compute_peak_AB once, then polish_peaks_with_weights per
- * weight vector): the exact (A, B) of up to 65,535 peaks at a time is written once to a device
- * buffer of at most 4 GiB and at most half of the device's free memory, allocated for the call and
- * freed before it returns, and read by every weight's polish. */
+ * weight vector): each candidate's terms are formed once and summed into moments over cells of zeros
+ * under up to five vectors at a time, and the polishes run on the moments; a peak whose Newton path
+ * amplifies rounding is polished over the zeros instead.  Device workspace of the table, at most
+ * 0.6 GiB, kept between calls.  A grid too wide for the cells (grid_half_width above ~0.1) builds the
+ * exact (A, B) of up to 65,535 peaks at a time in a buffer of at most 4 GiB and at most half of the
+ * device's free memory, allocated for the call and freed before it returns. */
 int mb_polish_peaks_weights(mb_table *t, int64_t P, const uint64_t *v_int, const uint64_t *v_frac,
                             const double *delta, int64_t n_zeros, int n_weights, const int *weight_slots,
                             double grid_half_width, int grid_steps, double *out_h_unpol, double *out_h_pol,

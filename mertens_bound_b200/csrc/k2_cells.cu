@@ -1,0 +1,1084 @@
+// Cell moments (see k2_cells.h), their evaluation on offset grids and the polishes on them.
+//
+// The moment pass is a contraction: for each cell, [peaks x zeros] unit phasors times [zeros x
+// columns] weighted powers.  It runs on the FP64 tensor instruction (mma.m8n8k4.f64).  That
+// instruction's A fragment holds one (row, k) element per lane, so with rows = 8 peaks and k = 4
+// zeros each lane computes the exact phase and the (cos, sin) of its own (peak, zero) pair in
+// registers -- the cosine is its A element of the real product, the sine that of the imaginary
+// product -- and no phasor is ever stored.  The powers (B) come from shared memory, staged once per
+// 64 zeros for the CTA's 64 peaks.
+#include <algorithm>
+#include <cmath>
+
+#include "k2_cells.h"
+#include "k2_common.cuh"
+#include "k2_polish.cuh"
+
+namespace mb {
+namespace {
+
+constexpr int CELL_THREADS = 256;
+constexpr int CELL_TILE = 64;                  // zeros staged at a time
+
+// ------------------------------------------------------------------ phasors
+
+// (cos, sin)(2 pi q / 256) in eight interleaved copies: entry q of copy c sits in the c-th
+// 16-byte bank group, and lane l reads copy l mod 8, so a warp's 32 random entries are read in the
+// four shared-memory cycles of a conflict-free 512-byte access (4.2 cycles measured, 9.4 for one
+// copy of a 2048-entry table).
+constexpr int PH_TAB = 256;
+constexpr int PH_COPIES = 8;
+constexpr int PH_BYTES = PH_TAB * PH_COPIES * (int)sizeof(double2);
+
+MB_DEV void phasor_table_init(double2 *tab, int threads) {
+    for (int i = threadIdx.x; i < PH_TAB; i += threads) {
+        double sn, cs;
+        sincospi((double)i * (2.0 / PH_TAB), &sn, &cs);
+#pragma unroll
+        for (int c = 0; c < PH_COPIES; ++c) tab[i * PH_COPIES + c] = make_double2(cs, sn);
+    }
+}
+
+// cos, sin of the phase word w - 2^55 (units of 2^-64 turn; the caller adds 2^55, half a table step):
+// table entry w >> 56 rotated by d 2^-60 turn, d = ((w mod 2^56) >> 4) - 2^51 exact in FP64
+// (|d| <= 2^51, i.e. at most 0.0123 rad; the dropped bits are 5e-18 rad).  With a = 2 pi 2^-60:
+//   sin(a d)     = d (a - a^3 d^2 / 6 + a^5 d^4 / 120)            (truncation 8.4e-18)
+//   cos(a d) - 1 = d^2 (-a^2 / 2 + a^4 d^2 / 24 - a^6 d^4 / 720)  (truncation 1.3e-20)
+// so the result carries the table's and the last FMA's roundings only.
+MB_DEV void phasor(uint64_t w, const double2 *tab, double &cs, double &sn) {
+    constexpr double a = 6.283185307179586 * 0x1p-60;
+    const double2 T = tab[(uint32_t)(w >> 56) * PH_COPIES + (threadIdx.x & (PH_COPIES - 1))];
+    const uint64_t rem = (w & 0x00FFFFFFFFFFFFFFull) >> 4;
+    const double d = __longlong_as_double((long long)(rem | 0x4330000000000000ull)) - 6755399441055744.0;
+    const double u = d * d;
+    const double s = d * fma(u, fma(u, a * a * a * a * a / 120.0, -a * a * a / 6.0), a);
+    const double m = u * fma(u, fma(u, -a * a * a * a * a * a / 720.0, a * a * a * a / 24.0), -a * a / 2.0);
+    cs = fma(T.x, m, fma(-T.y, s, T.x));
+    sn = fma(T.y, m, fma(T.x, s, T.y));
+}
+
+MB_DEV uint64_t wide(uint32_t a, uint32_t b) {
+    uint64_t r;
+    asm("mul.wide.u32 %0, %1, %2;" : "=l"(r) : "r"(a), "r"(b));
+    return r;
+}
+MB_DEV uint64_t wide_add(uint32_t a, uint32_t b, uint64_t c) {
+    uint64_t r;
+    asm("mad.wide.u32 %0, %1, %2, %3;" : "=l"(r) : "r"(a), "r"(b), "l"(c));
+    return r;
+}
+
+struct ZRec {                   // 32 B
+    uint32_t g0, g1, g2, g3, g4, pad;
+    uint64_t psi;               // arg(c) / 2pi 2^64 + 2^55 (half a table step of phasor())
+};
+
+// floor(frac(v G) 2^64) less at most 7 units of 2^-64 turn (the carries out of the columns below
+// 2^-64), plus psi: columns 4 and 5 of phase128_exact and the high halves of column 3.
+MB_DEV uint64_t phase64(uint32_t v0, uint32_t v1, uint32_t v2, uint32_t v3, const ZRec &z) {
+    const uint64_t h3 = (wide(v0, z.g3) >> 32) + (wide(v1, z.g2) >> 32) + (wide(v2, z.g1) >> 32) + (wide(v3, z.g0) >> 32);
+    const uint32_t top = v1 * z.g4 + v2 * z.g3 + v3 * z.g2;
+    uint64_t acc = wide_add(v0, z.g4, z.psi + h3);
+    acc = wide_add(v1, z.g3, acc);
+    acc = wide_add(v2, z.g2, acc);
+    acc = wide_add(v3, z.g1, acc);
+    return acc + ((uint64_t)top << 32);
+}
+
+MB_DEV void dmma(double (&c)[2], double a, double b) {
+    asm("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1},{%2},{%3},{%0,%1};"
+        : "+d"(c[0]), "+d"(c[1])
+        : "d"(a), "d"(b));
+}
+
+// ------------------------------------------------------------------ cells
+
+struct CellGroups {
+    int64_t a[2], b[2], e0[2];
+    int nc[2];
+};
+
+__global__ void cells_kernel(TabView t, CellGroups g, int n, int64_t half, int *j0, int *j1, int64_t *ctr) {
+    const int c = blockIdx.x * blockDim.x + threadIdx.x;
+    if (c >= n) return;
+    const int q = c < g.nc[0] ? 0 : 1, l = q ? c - g.nc[0] : c;
+    // the first zero of the group at or above an edge (G in units of 2^-16, rounded down)
+    auto first = [&](int64_t edge) {
+        int64_t lo = g.a[q], hi = g.b[q];
+        while (lo < hi) {
+            const int64_t mid = (lo + hi) >> 1;
+            if (((int64_t)t.g4[mid] << 16 | t.g3[mid] >> 16) < edge) lo = mid + 1;
+            else hi = mid;
+        }
+        return lo;
+    };
+    const int64_t e = g.e0[q] + 2 * half * l;
+    j0[c] = (int)(l == 0 ? g.a[q] : first(e));
+    j1[c] = (int)(l == g.nc[q] - 1 ? g.b[q] : first(e + 2 * half));
+    ctr[c] = e + half;
+}
+
+// n chunks of the zeros [0, n_zeros) as cells (the power sums need no centre).  Their lengths grow with
+// the zeros (edges n_zeros (c / n)^1.5): the lowest zeros carry most of the sum, and short chunks there
+// keep the rounding of the running sums down.
+__global__ void chunks_kernel(int64_t n_zeros, int n, int *j0, int *j1) {
+    const int c = blockIdx.x * blockDim.x + threadIdx.x;
+    if (c >= n) return;
+    auto edge = [&](int i) {
+        const double x = (double)i / n;
+        return i == n ? (int)n_zeros : (int)((double)n_zeros * x * sqrt(x));
+    };
+    j0[c] = edge(c);
+    j1[c] = edge(c + 1);
+}
+
+// ------------------------------------------------------------------ moments
+
+enum CellKind : int { CELL_GAUSS = 0, CELL_WEIGHTS = 1, CELL_POWERS = 2 };
+
+// Columns of the power matrix: W series of D1 terms (both products), or the Taylor polish's nine even
+// powers (real product, two tiles) and eight odd powers (imaginary product, one tile).
+template <int KIND, int W, int D1>
+struct CellShape {
+    static constexpr int cols = KIND == CELL_POWERS ? 24 : (W * D1 + 7) / 8 * 8;
+    static constexpr int NT = cols / 8;
+    static constexpr int NTR = KIND == CELL_POWERS ? 2 : NT;      // tiles of the real product
+    static constexpr int I0 = KIND == CELL_POWERS ? 2 : 0;        // first tile of the imaginary one
+    static constexpr int NTI = NT - I0;
+    // row stride in doubles = 4 mod 8: the 4 x 8 B fragment's half warps touch 16 distinct banks
+    static constexpr int S = cols + 4;
+    static constexpr int smem = PH_BYTES + CELL_TILE * (int)sizeof(ZRec) + CELL_TILE * S * 8;
+    static constexpr int frag = 2 * (NTR + NTI);                   // accumulators per lane
+};
+
+// gamma - 2 pi G (at most 4 ulp of gamma): G's leading 53 bits and the rest times 2 pi in two parts, so the
+// error is about 2^-100 G.
+MB_DEV double gamma_excess(double gamma, uint32_t g4, uint32_t g3, uint32_t g2, uint32_t g1) {
+    constexpr double P_HI = 6.283185307179586, P_LO = 2.4492935982947064e-16;       // 2 pi
+    double h, l;
+    two_sum(u32_to_f64(g4), u32_to_f64(g3) * 0x1p-32, h, l);
+    l += fma(u32_to_f64(g2), 0x1p-64, u32_to_f64(g1) * 0x1p-96);
+    const double p = P_HI * h, pe = fma(P_HI, h, -p);
+    return (gamma - p) - (pe + fma(P_HI, l, P_LO * h));
+}
+
+// One item = one cell x CELL_PEAKS / nzw peaks.  Warp w serves peaks 8 (w / nzw) .. + 7 and the
+// 4-zero steps congruent to w mod nzw; with nzw > 1 the warps' sums are added in warp order.
+// Bound: the FP64 pipe, 16 cycles per mma and scheduler, 2 mma per step and 8 columns, beside ~24 for
+// the phasor; measured with its callers (k2_scan.cu, k2_path1.cu).
+template <int KIND, int W, int D1>
+__global__ void __launch_bounds__(CELL_THREADS, 2)
+cell_moments_kernel(TabView t, const uint64_t *vi, const uint64_t *vf, const double *delta, const int *sel, int64_t P,
+                    Cells cells, CellWeights wts, double k, int n_pt, int nzw, int n_items, double *out) {
+    using Sh = CellShape<KIND, W, D1>;
+    extern __shared__ __align__(16) unsigned char smem[];
+    double2 *tab = reinterpret_cast<double2 *>(smem);
+    ZRec *rec = reinterpret_cast<ZRec *>(smem + PH_BYTES);
+    double *E = reinterpret_cast<double *>(smem + PH_BYTES + CELL_TILE * sizeof(ZRec));
+    phasor_table_init(tab, CELL_THREADS);
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int cg = warp / nzw, zw = warp - cg * nzw;
+    const int ppc = CELL_PEAKS / nzw;
+    const double inv_h = 1.0 / ((double)cells.half * 65536.0);     // units of 2^-32
+    const double inv_kappa = 65536.0 / (6.283185307179586 * (double)cells.half);
+    for (int item = blockIdx.x; item < n_items; item += gridDim.x) {
+        const int cell = item / n_pt, pt = item - cell * n_pt;
+        const int64_t pw = (int64_t)pt * ppc + cg * 8;             // the warp's first peak
+        const int64_t p = pw + (lane >> 2);
+        Cand64 v{0, 0};
+        if (p < P) {
+            const int64_t i = sel ? sel[p] : p;
+            v = fold_delta(vi[i], vf[i], delta ? delta[i] : 0.0);
+        }
+        const uint32_t v0 = (uint32_t)v.vf, v1 = (uint32_t)(v.vf >> 32), v2 = (uint32_t)v.vi, v3 = (uint32_t)(v.vi >> 32);
+        double aR[Sh::NTR][2], aI[Sh::NTI][2];
+#pragma unroll
+        for (int i = 0; i < Sh::NTR; ++i) aR[i][0] = aR[i][1] = 0.0;
+#pragma unroll
+        for (int i = 0; i < Sh::NTI; ++i) aI[i][0] = aI[i][1] = 0.0;
+        const int64_t ja = cells.j0[cell], jb = cells.j1[cell];
+        const int64_t ctr = KIND == CELL_POWERS ? 0 : cells.ctr[cell] << 16;
+        for (int64_t tb = ja; tb < jb; tb += CELL_TILE) {
+            const int nt = (int)min((int64_t)CELL_TILE, jb - tb);
+            const int n4 = (nt + 3) & ~3;
+            __syncthreads();
+            // 64 zeros x parts: a weight vector's D1 columns each, or four column groups
+            constexpr int PARTS = KIND == CELL_WEIGHTS ? W : 4;
+            for (int id = threadIdx.x; id < CELL_TILE * PARTS; id += CELL_THREADS) {
+                const int z = id & (CELL_TILE - 1), q = id / CELL_TILE;
+                if (z >= n4) continue;
+                const bool live = z < nt;
+                const int64_t j = tb + (live ? z : 0);
+                const uint32_t g2 = t.g2[j], g3 = t.g3[j], g4 = t.g4[j];
+                if (q == 0) {
+                    ZRec r;
+                    r.g0 = t.g0[j]; r.g1 = t.g1[j]; r.g2 = g2; r.g3 = g3; r.g4 = g4;
+                    r.pad = 0;
+                    r.psi = t.psi[j] + (1ull << 55);
+                    rec[z] = r;
+                }
+                double *row = E + z * Sh::S;
+                const double al = live ? 2.0 * t.alpha[j] : 0.0;
+                if constexpr (KIND == CELL_POWERS) {
+                    const double u = t.gamma[j] * 1.0e-4, u2 = u * u, u4 = u2 * u2, u8 = u4 * u4;
+                    const double wa = al * wts.w[0][j];
+                    if (q == 0) {                               // u^0 .. u^8
+                        double x = wa;
+#pragma unroll
+                        for (int m = 0; m < 5; ++m, x *= u2) row[m] = x;
+                    } else if (q == 1) {                        // u^10 .. u^16, then unused columns
+                        double x = wa * (u8 * u2);
+#pragma unroll
+                        for (int m = 5; m < 9; ++m, x *= u2) row[m] = x;
+#pragma unroll
+                        for (int m = 9; m < 16; ++m) row[m] = 0.0;
+                    } else {                                    // u^1 .. u^7, u^9 .. u^15
+                        double x = wa * (q == 2 ? u : u8 * u);
+#pragma unroll
+                        for (int m = 0; m < 4; ++m, x *= u2) row[16 + (q - 2) * 4 + m] = x;
+                    }
+                } else {
+                    const int64_t df = (int64_t)((uint64_t)g4 << 32 | g3) - ctr;
+                    double x = ((double)df + u32_to_f64(g2) * 0x1p-32) * inv_h;
+                    // the polishes' offsets turn by the table's FP64 gamma, not 2 pi G
+                    if constexpr (KIND == CELL_WEIGHTS) x += gamma_excess(t.gamma[j], g4, g3, g2, t.g1[j]) * inv_kappa;
+                    if constexpr (KIND == CELL_GAUSS) {
+                        constexpr int C4 = D1 / 4;
+                        const double g = t.gamma[j];
+                        const double x2 = x * x, x4 = C4 == 2 ? x2 : x2 * x2;
+                        double e = al * exp(-k * g * g);
+                        if (q & 1) e *= x4;
+                        if (q & 2) e *= x4 * x4;
+#pragma unroll
+                        for (int m = 0; m < C4; ++m, e *= x) row[q * C4 + m] = e;
+                    } else {
+                        double e = al * wts.w[q][j];
+#pragma unroll
+                        for (int m = 0; m < D1; ++m, e *= x) row[q * D1 + m] = e;
+                        if (q == W - 1)
+#pragma unroll
+                            for (int m = W * D1; m < Sh::cols; ++m) row[m] = 0.0;
+                    }
+                }
+            }
+            __syncthreads();
+            if (pw < P) {
+                const int n_step = n4 >> 2;
+#pragma unroll 2
+                for (int st = zw; st < n_step; st += nzw) {
+                    const int z = st * 4 + (lane & 3);
+                    double cs, sn;
+                    phasor(phase64(v0, v1, v2, v3, rec[z]), tab, cs, sn);
+                    const double *b = E + z * Sh::S + (lane >> 2);
+#pragma unroll
+                    for (int i = 0; i < Sh::NT; ++i) {
+                        const double bv = b[i * 8];
+                        if (i < Sh::NTR) dmma(aR[i], cs, bv);
+                        if (i >= Sh::I0) dmma(aI[i - Sh::I0], sn, bv);
+                    }
+                }
+            }
+        }
+        if (nzw > 1) {                     // add the other warps' sums of this peak group, in order
+            double *buf = E + cg * 32 * Sh::frag;
+            for (int w = 1; w < nzw; ++w) {
+                __syncthreads();
+                if (zw == w) {
+#pragma unroll
+                    for (int i = 0; i < 2 * Sh::NTR; ++i) buf[i * 32 + lane] = aR[i >> 1][i & 1];
+#pragma unroll
+                    for (int i = 0; i < 2 * Sh::NTI; ++i) buf[(2 * Sh::NTR + i) * 32 + lane] = aI[i >> 1][i & 1];
+                }
+                __syncthreads();
+                if (zw == 0) {
+#pragma unroll
+                    for (int i = 0; i < 2 * Sh::NTR; ++i) aR[i >> 1][i & 1] += buf[i * 32 + lane];
+#pragma unroll
+                    for (int i = 0; i < 2 * Sh::NTI; ++i) aI[i >> 1][i & 1] += buf[(2 * Sh::NTR + i) * 32 + lane];
+                }
+            }
+        }
+        if (zw == 0 && p < P) {            // C fragment: row = peak, columns 2 (lane mod 4) + {0, 1}
+#pragma unroll
+            for (int i = 0; i < Sh::NT; ++i)
+#pragma unroll
+                for (int e = 0; e < 2; ++e) {
+                    const int col = i * 8 + (lane & 3) * 2 + e;
+                    if constexpr (KIND == CELL_POWERS) {
+                        out[(p * cells.n + cell) * 24 + col] = i < Sh::NTR ? aR[i < Sh::NTR ? i : 0][e]
+                                                                           : aI[i < Sh::NTR ? 0 : i - Sh::I0][e];
+                    } else if (col < W * D1) {
+                        const int w = col / D1, m = col - w * D1;
+                        double *o = out + (((int64_t)w * P + p) * cells.n + cell) * (2 * D1) + m;
+                        o[0] = aR[i < Sh::NTR ? i : 0][e];
+                        o[D1] = aI[i - Sh::I0 >= 0 ? i - Sh::I0 : 0][e];
+                    }
+                }
+        }
+    }
+}
+
+// Resident CTAs of the moment kernels: two per SM.
+int cell_slots(const Table &t, int *slots) {
+    int sms = 148;
+    MB_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, t.device));
+    *slots = 2 * sms;
+    return MB_OK;
+}
+
+template <int KIND, int W, int D1>
+int launch_moments(const Table &t, const Cells &c, const uint64_t *vi, const uint64_t *vf, const double *delta,
+                   const int *sel, int64_t P, const CellWeights &w, double k, int nzw, double *out, cudaStream_t s) {
+    using Sh = CellShape<KIND, W, D1>;
+    static_assert(8 * 32 * Sh::frag * 8 / 2 <= CELL_TILE * Sh::S * 8 || KIND == CELL_WEIGHTS, "reduction buffer");
+    MB_TRY(cell_kernel_attributes());
+    int slots = 296;
+    MB_TRY(cell_slots(t, &slots));
+    const int64_t n_pt = (P + CELL_PEAKS / nzw - 1) / (CELL_PEAKS / nzw);
+    const int64_t items = n_pt * c.n;
+    MB_CHECK_ARG(items < ((int64_t)1 << 31), "cell moments: %lld items", (long long)items);
+    cell_moments_kernel<KIND, W, D1><<<(unsigned)std::min<int64_t>(slots, items), CELL_THREADS, Sh::smem, s>>>(
+        view(t), vi, vf, delta, sel, P, c, w, k, (int)n_pt, nzw, (int)items, out);
+    MB_CUDA(cudaGetLastError());
+    return MB_OK;
+}
+
+// Warps sharing a peak group's zeros: as many as keep the CTA's peak slots full.
+int cell_nzw(int64_t P) {
+    int nzw = 1;
+    while (nzw < 8 && P <= CELL_PEAKS / (2 * nzw)) nzw *= 2;
+    return nzw;
+}
+
+// ------------------------------------------------------------------ offset scans
+
+constexpr int CSCAN_THREADS = 128;
+constexpr int CSCAN_PT = 2;                    // grid points per thread
+constexpr int CSCAN_CELLS = 32;                // cells staged at a time
+
+// Thread: CSCAN_PT points of one base point over all cells; the moments are read as broadcasts.
+template <int D1>
+__global__ void __launch_bounds__(CSCAN_THREADS)
+cell_scan_kernel(Cells cells, const double *M, int NB, int Bp, int64_t n_m, uint64_t si, uint64_t sf, double kstep,
+                 double *out) {
+    extern __shared__ __align__(16) unsigned char smem[];
+    double2 *tab = reinterpret_cast<double2 *>(smem);
+    double2 *mom = reinterpret_cast<double2 *>(smem + PH_BYTES);                  // [cell][D1]: pairs of one row
+    ulonglong2 *dph = reinterpret_cast<ulonglong2 *>(mom + CSCAN_CELLS * D1);     // frac(step G_c): lo, hi
+    phasor_table_init(tab, CSCAN_THREADS);
+    const int64_t pb = blockIdx.y;                               // point p NB + b
+    const int64_t p = pb / NB, b = pb - p * NB;
+    const int np = (int)min((int64_t)Bp, n_m - b * Bp);          // points of this block
+    double e[CSCAN_PT][D1], h[CSCAN_PT];
+    int ml[CSCAN_PT];
+#pragma unroll
+    for (int i = 0; i < CSCAN_PT; ++i) {
+        ml[i] = (int)(blockIdx.x * CSCAN_PT + i) * CSCAN_THREADS + threadIdx.x - Bp / 2;
+        // (kappa d)^n / n! with the sign of i^n: + + - -
+        const double y = kstep * ml[i];
+        double x = 1.0;
+#pragma unroll
+        for (int n = 0; n < D1; ++n) {
+            e[i][n] = (n & 2) ? -x : x;
+            x *= y * (1.0 / (n + 1));
+        }
+        h[i] = 0.0;
+    }
+    for (int cb = 0; cb < cells.n; cb += CSCAN_CELLS) {
+        const int nc = min(CSCAN_CELLS, cells.n - cb);
+        __syncthreads();
+        const double2 *src = reinterpret_cast<const double2 *>(M + (pb * cells.n + cb) * (2 * D1));
+        for (int i = threadIdx.x; i < nc * D1; i += CSCAN_THREADS) mom[i] = src[i];
+        if ((int)threadIdx.x < nc) {
+            const uint64_t g = (uint64_t)cells.ctr[cb + threadIdx.x] << 16;          // G_c 2^32
+            uint64_t hi, lo;
+            phase128_exact((uint32_t)sf, (uint32_t)(sf >> 32), (uint32_t)si, (uint32_t)(si >> 32), 0, 0, 0,
+                           (uint32_t)g, (uint32_t)(g >> 32), hi, lo);
+            dph[threadIdx.x] = make_ulonglong2(lo, hi);
+        }
+        __syncthreads();
+        for (int c = 0; c < nc; ++c) {
+            const double2 *m2 = mom + c * D1;
+            const ulonglong2 d = dph[c];
+            double qr[CSCAN_PT], qi[CSCAN_PT];
+#pragma unroll
+            for (int i = 0; i < CSCAN_PT; ++i) qr[i] = qi[i] = 0.0;
+#pragma unroll
+            for (int n = 0; n < D1; n += 2) {
+                const double2 re = m2[n / 2], im = m2[(D1 + n) / 2];
+#pragma unroll
+                for (int i = 0; i < CSCAN_PT; ++i) {
+                    qr[i] = fma(e[i][n], re.x, fma(-e[i][n + 1], im.y, qr[i]));
+                    qi[i] = fma(e[i][n], im.x, fma(e[i][n + 1], re.y, qi[i]));
+                }
+            }
+#pragma unroll
+            for (int i = 0; i < CSCAN_PT; ++i) {
+                // frac(m step G_c), m the signed offset index (2^-64 turn short at most when negative)
+                const uint64_t ma = (uint64_t)(ml[i] < 0 ? -ml[i] : ml[i]);
+                uint64_t w = ma * d.y + __umul64hi(ma, d.x);
+                if (ml[i] < 0) w = ~w;
+                double cs, sn;
+                phasor(w + (1ull << 55), tab, cs, sn);
+                h[i] = fma(cs, qr[i], fma(-sn, qi[i], h[i]));
+            }
+        }
+    }
+#pragma unroll
+    for (int i = 0; i < CSCAN_PT; ++i) {
+        const int l = ml[i] + Bp / 2;
+        if (l < np) out[p * n_m + b * Bp + l] = h[i];
+    }
+}
+
+template <int D1>
+constexpr int cscan_smem() { return PH_BYTES + CSCAN_CELLS * (D1 * 16 + 16); }
+
+// ------------------------------------------------------------------ polishes on moments
+
+constexpr int CPOL_THREADS = 256;
+
+// The series at one offset: F0 = E Q0 and, with DERIV, F1 = E Q1, F2 = E Q2, where E = e^{2 pi i G_c d} and
+// Q0 = sum M_n (i y)^n / n!, Q1, Q2 its first and second derivative in i y (y = kappa d).
+// The rotation's offset is d + rho, rho the part of the point's delta below 2^-64 that its fixed-point fold
+// dropped (at most 2^-65; in the series it is far below rounding).
+struct CellSeries {
+    double d, rho, e[CELL_D1];
+    MB_DEV CellSeries(double d_, double rho_, double kappa) : d(d_), rho(rho_) {
+        const double y = kappa * d_;
+        double x = 1.0;
+#pragma unroll
+        for (int n = 0; n < CELL_D1; ++n) {
+            e[n] = (n & 2) ? -x : x;
+            x *= y * (1.0 / (n + 1));
+        }
+    }
+    // sum_{n >= s} M_n (i y)^{n - s} / (n - s)!
+    template <int SHIFT>
+    MB_DEV void q(const double *m, double &qr, double &qi) const {
+        qr = qi = 0.0;
+#pragma unroll
+        for (int n = SHIFT; n < CELL_D1; ++n) {
+            const double x = e[n - SHIFT], re = m[n], im = m[CELL_D1 + n];
+            if ((n - SHIFT) & 1) {
+                qr = fma(-x, im, qr);
+                qi = fma(x, re, qi);
+            } else {
+                qr = fma(x, re, qr);
+                qi = fma(x, im, qi);
+            }
+        }
+    }
+    // e^{2 pi i G (d + rho)}: the product's rounding error is carried into the angle
+    MB_DEV void rot(double G, double &cs, double &sn) const {
+        const double p = G * d, pe = fma(G, rho, fma(G, d, -p));
+        sincospi(2.0 * ((p - rint(p)) + pe), &sn, &cs);
+    }
+};
+
+// A peak for the second pass: its output, weight and point index, and Newton's starting offsets.
+struct Redo {
+    int64_t out;
+    int w, point;
+    double start[2];
+};
+
+template <int MODE>
+struct PolishRule;              // Newton's constants and starts in each loop of k2_polish.cuh
+template <>
+struct PolishRule<POLISH_EVAL_FAST> {
+    static constexpr int iters = 6, starts = 1;
+    static constexpr double clamp = 1e-4, tol = 1e-13;
+};
+template <>
+struct PolishRule<POLISH_SINGLE> {
+    static constexpr int iters = 8, starts = 2;
+    static constexpr double clamp = 2e-5, tol = 1e-14;
+};
+template <>
+struct PolishRule<POLISH_TOPK> {
+    static constexpr int iters = 4, starts = 1;
+    static constexpr double clamp = 1e-5, tol = 1e-13;
+};
+
+// Whether a start's h replaces the best so far, in each loop's way.
+template <int MODE>
+MB_DEV bool polish_keep(double h, double best) {
+    return MODE == POLISH_EVAL_FAST ? !(fabs(best) > fabs(h)) : fabs(h) > fabs(best);
+}
+
+template <int MODE>
+__global__ void __launch_bounds__(CPOL_THREADS)
+cell_polish_kernel(Cells cells, const double *M, CellPolishArgs a, const double *delta, Redo *redo, int *n_redo) {
+    using R = PolishRule<MODE>;
+    __shared__ double red[3][CPOL_THREADS / 32];
+    __shared__ double best_v[CPOL_THREADS / 32];
+    __shared__ int best_i[CPOL_THREADS / 32];
+    const int64_t p = blockIdx.x;
+    const int w = blockIdx.y;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const double *m0 = M + ((int64_t)w * a.P + p) * cells.n * (2 * CELL_D1);
+    const double H = (double)cells.half * 0x1p-16, kappa = 6.283185307179586 * H;
+    const int64_t point = a.sel ? a.sel[p] : p;
+    const int64_t o = (int64_t)w * a.out_stride + point;
+    const double fixed = (delta ? delta[point] : 0.0) * 0x1p64, rho = (fixed - rint(fixed)) * 0x1p-64;
+
+    // N sums over the CTA, every thread gets them (warp partials in warp order)
+    auto block_sums = [&](auto &x) {
+        constexpr int N = sizeof(x) / sizeof(double);
+#pragma unroll
+        for (int i = 0; i < N; ++i)
+            for (int s = 16; s > 0; s >>= 1) x[i] += __shfl_xor_sync(0xffffffffu, x[i], s);
+        __syncthreads();
+        if (lane == 0)
+#pragma unroll
+            for (int i = 0; i < N; ++i) red[i][warp] = x[i];
+        __syncthreads();
+#pragma unroll
+        for (int i = 0; i < N; ++i) {
+            x[i] = 0.0;
+#pragma unroll
+            for (int s = 0; s < CPOL_THREADS / 32; ++s) x[i] += red[i][s];
+        }
+    };
+    auto value = [&](double d) {
+        const CellSeries S(d, rho, kappa);
+        double x[1] = {0.0};
+        for (int c = threadIdx.x; c < cells.n; c += CPOL_THREADS) {
+            double cs, sn, qr, qi;
+            S.rot((double)cells.ctr[c] * 0x1p-16, cs, sn);
+            S.q<0>(m0 + (int64_t)c * (2 * CELL_D1), qr, qi);
+            x[0] += cs * qr - sn * qi;
+        }
+        block_sums(x);
+        return x[0];
+    };
+    // h(0), and sqrt(sum gamma^4 |M_c0|^2): 2^-53 |d| times it is the size of the error that rounding
+    // gamma_j d leaves in h'(d)
+    double h0, noise;
+    {
+        double x[2] = {0.0, 0.0};
+        for (int c = threadIdx.x; c < cells.n; c += CPOL_THREADS) {
+            const double *m = m0 + (int64_t)c * (2 * CELL_D1);
+            const double g = 6.283185307179586 * (double)cells.ctr[c] * 0x1p-16, g2 = g * g;
+            x[0] += m[0];
+            x[1] += g2 * g2 * (m[0] * m[0] + m[CELL_D1] * m[CELL_D1]);
+        }
+        block_sums(x);
+        h0 = x[0];
+        noise = 0x1p-53 * sqrt(x[1]);
+    }
+    // Newton on h' = 0 from d (the loop of polish_newton): with g = 2 pi G_c,
+    //   h'  = -(g Im F0 + kappa Im F1),   h'' = -(g^2 Re F0 + 2 g kappa Re F1 + kappa^2 Re F2),
+    // and for the sensitivity the third derivative's leading part.  A step d - h' / h'' multiplies the
+    // error so far by |h' h3 / h''^2| and adds its own sums' error; a clamped step does neither.
+    auto newton = [&](double d, double &sens) {
+        sens = 0.0;
+        for (int it = 0; it < R::iters; ++it) {
+            const CellSeries S(d, rho, kappa);
+            double x[3] = {0.0, 0.0, 0.0};
+            for (int c = threadIdx.x; c < cells.n; c += CPOL_THREADS) {
+                const double *m = m0 + (int64_t)c * (2 * CELL_D1);
+                const double G = (double)cells.ctr[c] * 0x1p-16, g = 6.283185307179586 * G;
+                double cs, sn, q0r, q0i, q1r, q1i, q2r, q2i;
+                S.rot(G, cs, sn);
+                S.q<0>(m, q0r, q0i);
+                S.q<1>(m, q1r, q1i);
+                S.q<2>(m, q2r, q2i);
+                const double ar = g * q0r + kappa * q1r, ai = g * q0i + kappa * q1i;
+                const double br = g * (g * q0r + 2.0 * kappa * q1r) + kappa * kappa * q2r;
+                const double bi = g * (g * q0i + 2.0 * kappa * q1i) + kappa * kappa * q2i;
+                x[0] -= cs * ai + sn * ar;
+                x[1] -= cs * br - sn * bi;
+                x[2] += g * (cs * bi + sn * br);
+            }
+            block_sums(x);
+            if (!(fabs(x[1]) > 1e-12)) break;
+            double step = x[0] / x[1];
+            if (fabs(step) < R::clamp)
+                sens = sens * fabs(step * x[2] / x[1]) + noise * fmax(fabs(d), R::clamp) / fabs(x[1]);
+            step = fmin(fmax(step, -R::clamp), R::clamp);
+            d -= step;
+            if (fabs(step) < R::tol) break;
+        }
+        return d;
+    };
+    // the first index in [0, n) of the largest |h(at(i))| over the cells [0, n_cells) if it exceeds `from`,
+    // else -1: one warp per grid point
+    auto grid_best = [&](int n, int n_cells, double from, auto at) {
+        double bv = from;
+        int bi = -1;
+        for (int i = warp; i < n; i += CPOL_THREADS / 32) {
+            const CellSeries S(at(i), rho, kappa);
+            double x = 0.0;
+            for (int c = lane; c < n_cells; c += 32) {
+                double cs, sn, qr, qi;
+                S.rot((double)cells.ctr[c] * 0x1p-16, cs, sn);
+                S.q<0>(m0 + (int64_t)c * (2 * CELL_D1), qr, qi);
+                x += cs * qr - sn * qi;
+            }
+            for (int s = 16; s > 0; s >>= 1) x += __shfl_xor_sync(0xffffffffu, x, s);
+            if (fabs(x) > bv) {
+                bv = fabs(x);
+                bi = i;
+            }
+        }
+        __syncthreads();
+        if (lane == 0) {
+            best_v[warp] = bv;
+            best_i[warp] = bi;
+        }
+        __syncthreads();
+        bv = from;
+        bi = -1;
+        for (int s = 0; s < CPOL_THREADS / 32; ++s)
+            if (best_i[s] >= 0 && (best_v[s] > bv || (best_v[s] == bv && bi >= 0 && best_i[s] < bi))) {
+                bv = best_v[s];
+                bi = best_i[s];
+            }
+        return bi;
+    };
+
+    double hp = h0, dp = 0.0, start[2] = {0.0, 0.0};
+    int ns = 1;
+    if constexpr (MODE == POLISH_TOPK) {
+        hp = h0 = a.h_unpol[o];                      // the grid stage's
+        start[0] = a.ddy_pol[o];
+    } else if constexpr (MODE == POLISH_EVAL_FAST) {
+        const int steps = a.n_grid;
+        auto at = [&](int i) { return (a.half * (i - steps)) / steps; };
+        const int i = steps > 0 ? grid_best(2 * steps + 1, cells.n_first, fabs(h0), at) : -1;
+        start[0] = i >= 0 ? at(i) : 0.0;
+    } else if (a.n_grid > 0) {
+        const int i = grid_best(a.n_grid, cells.n, -1.0, [&](int i) { return a.grid[i]; });
+        start[1] = i >= 0 ? a.grid[i] : 0.0;
+        ns = 2;
+    }
+    double worst = 0.0;
+    for (int s = 0; s < ns; ++s) {
+        double sens;
+        const double d = newton(start[s], sens);
+        const double h = value(d);
+        if (!(sens <= worst)) worst = sens;
+        if (polish_keep<MODE>(h, hp)) {
+            hp = h;
+            dp = d;
+        }
+    }
+    if (threadIdx.x == 0) {
+        a.h_unpol[o] = h0;
+        a.h_pol[o] = hp;
+        a.ddy_pol[o] = dp;
+        if (!(worst <= POLISH_SENSITIVE * R::clamp)) redo[atomicAdd(n_redo, 1)] = Redo{o, w, (int)point, {start[0], start[1]}};
+    }
+}
+
+// The second pass: the listed peaks' Newton and final value by the loops over the zeros, bit for bit as
+// peak_polish_kernel forms them.  Pass `it` forms the terms of every zero (redo_term_kernel, over the whole
+// GPU) and adds them in that kernel's order (redo_sum_kernel: POLISH_CLUSTER x POLISH_THREADS strided running
+// sums, warp tree, warps and CTA ranks in order); one peak's eight sums of 293 serial additions at 600,000
+// zeros are bound by load latency, so each thread keeps REDO_AHEAD zeros' loads in flight.
+constexpr int REDO_AHEAD = 16;
+
+struct RedoState {
+    double d;
+    int done, pad;
+};
+
+struct RedoBuf {
+    const Redo *list;
+    RedoState *state;           // [2][batch], by the pass's parity
+    double2 *slot;              // [batch][POLISH_CLUSTER]: the ranks' sums
+    double *h_best, *d_best;    // [batch]
+    double2 *ab, *term;         // [batch][n]: (A, B); (value, derivative) of each zero's term
+    int batch;
+};
+
+__global__ void __launch_bounds__(256) redo_ab_kernel(ABExact src, int64_t n, RedoBuf rb) {
+    const int64_t j = (int64_t)blockIdx.x * 256 + threadIdx.x;
+    if (j >= n) return;
+    double A, B;
+    src.at(src.peak(rb.list[blockIdx.y].point), j, A, B);
+    rb.ab[blockIdx.y * n + j] = make_double2(A, B);
+}
+
+// The ranks' totals in rank order.
+MB_DEV double2 redo_total(const RedoBuf &rb, int e) {
+    double2 t = make_double2(0.0, 0.0);
+    for (int r = 0; r < POLISH_CLUSTER; ++r) {
+        t.x += rb.slot[e * POLISH_CLUSTER + r].x;
+        t.y += rb.slot[e * POLISH_CLUSTER + r].y;
+    }
+    return t;
+}
+
+template <int MODE>
+__global__ void __launch_bounds__(256) redo_term_kernel(const double *gamma, int64_t n, RedoBuf rb, int start, int it) {
+    using R = PolishRule<MODE>;
+    const int e = blockIdx.y;
+    RedoState st;
+    if (it == 0) {
+        st = RedoState{rb.list[e].start[start], 0, 0};
+    } else {                                       // the step of the pass before, alike in every CTA
+        st = rb.state[((it - 1) & 1) * rb.batch + e];
+        if (!st.done) {
+            const double2 t = redo_total(rb, e);
+            if (!(fabs(t.y) > 1e-12)) {
+                st.done = 1;
+            } else {
+                double step = t.x / t.y;
+                step = fmin(fmax(step, -R::clamp), R::clamp);
+                st.d -= step;
+                if (fabs(step) < R::tol) st.done = 1;
+            }
+        }
+    }
+    if (blockIdx.x == 0 && threadIdx.x == 0) rb.state[(it & 1) * rb.batch + e] = st;
+    if (st.done && it < R::iters) return;
+    for (int64_t j = (int64_t)blockIdx.x * 256 + threadIdx.x; j < n; j += (int64_t)gridDim.x * 256) {
+        const double2 v = rb.ab[e * n + j];
+        const double g = gamma[j];
+        double sn, cs;
+        sincos(g * st.d, &sn, &cs);
+        const double val = v.x * cs - v.y * sn;
+        const double dval = g * (-v.x * sn - v.y * cs);
+        rb.term[e * n + j] = make_double2(val, dval);
+    }
+}
+
+__global__ void __launch_bounds__(POLISH_THREADS)
+redo_sum_kernel(const double *gamma, int64_t n, CellWeights wts, RedoBuf rb, int it, bool value) {
+    __shared__ double red[POLISH_THREADS / 32];
+    const int e = blockIdx.y, rank = blockIdx.x;
+    if (!value && rb.state[(it & 1) * rb.batch + e].done) return;
+    const double *w = wts.w[rb.list[e].w];
+    const double2 *term = rb.term + e * n;
+    double x = 0.0, y = 0.0;
+    // REDO_AHEAD zeros' loads are issued before the first of their additions (0.46 us per zero otherwise)
+    for (int64_t j0 = (int64_t)rank * POLISH_THREADS + threadIdx.x; j0 < n; j0 += REDO_AHEAD * POLISH_STRIDE) {
+        double2 v[REDO_AHEAD];
+        double wv[REDO_AHEAD], g[REDO_AHEAD];
+#pragma unroll
+        for (int i = 0; i < REDO_AHEAD; ++i) {
+            const int64_t j = j0 + i * POLISH_STRIDE;
+            const bool in = j < n;
+            v[i] = in ? term[j] : make_double2(0.0, 0.0);
+            wv[i] = in ? w[j] : 0.0;
+            g[i] = in ? gamma[j] : 0.0;
+        }
+#pragma unroll
+        for (int i = 0; i < REDO_AHEAD; ++i) {
+            if (j0 + i * POLISH_STRIDE >= n) break;
+            if (value) {
+                x += wv[i] * v[i].x;
+            } else {
+                x += wv[i] * v[i].y;
+                y += wv[i] * (-(g[i] * g[i]) * v[i].x);
+            }
+        }
+    }
+    x = block_sum(x, red);
+    y = block_sum(y, red);
+    if (threadIdx.x == 0) rb.slot[e * POLISH_CLUSTER + rank] = make_double2(x, y);
+}
+
+// The start's h against the best so far; after the last start, the outputs.
+template <int MODE>
+__global__ void redo_keep_kernel(RedoBuf rb, CellPolishArgs a, int m, int start, bool last) {
+    using R = PolishRule<MODE>;
+    const int e = blockIdx.x * blockDim.x + threadIdx.x;
+    if (e >= m) return;
+    const int64_t o = rb.list[e].out;
+    double hb = start == 0 ? a.h_unpol[o] : rb.h_best[e], db = start == 0 ? 0.0 : rb.d_best[e];
+    const double h = redo_total(rb, e).x;
+    if (polish_keep<MODE>(h, hb)) {
+        hb = h;
+        db = rb.state[(R::iters & 1) * rb.batch + e].d;
+    }
+    rb.h_best[e] = hb;
+    rb.d_best[e] = db;
+    if (last) {
+        a.h_pol[o] = hb;
+        a.ddy_pol[o] = db;
+    }
+}
+
+// ------------------------------------------------------------------ Taylor polish, grid stage
+
+constexpr int TAY_THREADS = 128;
+
+// One CTA per peak: the chunks' power sums added in a fixed order (four chunk strides, then those
+// four), then the grid points; ties of |h| go to the smaller index.
+__global__ void __launch_bounds__(TAY_THREADS)
+taylor_grid_kernel(const double *S, int n_chunk, const double *grid, int n_grid, double *h_unpol, double *h_pol,
+                   double *ddy_pol) {
+    __shared__ double part[4][24], mom[24];
+    __shared__ double best_v[TAY_THREADS / 32], best_h[TAY_THREADS / 32];
+    __shared__ int best_i[TAY_THREADS / 32];
+    // (-1)^m/(2m)! and (-1)^m/(2m+1)!
+    constexpr double CC[9] = {1.0, -1.0 / 2, 1.0 / 24, -1.0 / 720, 1.0 / 40320, -1.0 / 3628800,
+                              1.0 / 479001600, -1.0 / 87178291200.0, 1.0 / 20922789888000.0};
+    constexpr double CS[8] = {1.0, -1.0 / 6, 1.0 / 120, -1.0 / 5040, 1.0 / 362880, -1.0 / 39916800,
+                              1.0 / 6227020800.0, -1.0 / 1307674368000.0};
+    const int64_t p = blockIdx.x;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    if (lane < 24) {
+        double x = 0.0;
+        for (int c = warp; c < n_chunk; c += 4) x += S[(p * n_chunk + c) * 24 + lane];
+        part[warp][lane] = x;
+    }
+    __syncthreads();
+    if (threadIdx.x < 24) mom[lane] = (part[0][lane] + part[1][lane]) + (part[2][lane] + part[3][lane]);
+    __syncthreads();
+    double bv = -1.0, hv = 0.0;
+    int bi = n_grid;
+    for (int g = threadIdx.x; g < n_grid; g += TAY_THREADS) {
+        const double z = grid[g] * 1.0e4, z2 = z * z;
+        double hc = 0.0, hs = 0.0, pw = 1.0;
+#pragma unroll
+        for (int m = 0; m < 9; ++m) {
+            hc = fma(mom[m] * CC[m], pw, hc);
+            if (m < 8) hs = fma(mom[16 + m] * CS[m], pw * z, hs);
+            pw *= z2;
+        }
+        const double h = hc - hs;
+        if (fabs(h) > bv) {
+            bv = fabs(h);
+            bi = g;
+            hv = h;
+        }
+    }
+    auto take = [&](double v2, int i2, double h2) {
+        if (v2 > bv || (v2 == bv && i2 < bi)) {
+            bv = v2;
+            bi = i2;
+            hv = h2;
+        }
+    };
+    for (int o = 16; o > 0; o >>= 1) {
+        const double v2 = __shfl_xor_sync(0xffffffffu, bv, o), h2 = __shfl_xor_sync(0xffffffffu, hv, o);
+        take(v2, __shfl_xor_sync(0xffffffffu, bi, o), h2);
+    }
+    if (lane == 0) {
+        best_v[warp] = bv;
+        best_i[warp] = bi;
+        best_h[warp] = hv;
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        for (int w = 1; w < TAY_THREADS / 32; ++w) take(best_v[w], best_i[w], best_h[w]);
+        h_unpol[p] = mom[0];
+        ddy_pol[p] = bi < n_grid ? grid[bi] : 0.0;
+        h_pol[p] = bi < n_grid ? hv : mom[0];
+    }
+}
+
+template <typename K>
+int set_smem(K kern, int bytes) {
+    MB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
+    MB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout,
+                                 (int)cudaSharedmemCarveoutMaxShared));
+    return MB_OK;
+}
+
+}  // namespace
+
+int cell_kernel_attributes() {
+    static void *done_ctx[64] = {};             // the context the attributes were set in
+    int dev = 0;
+    MB_CUDA(cudaGetDevice(&dev));
+    void *ctx = current_context();
+    if (dev >= 0 && dev < 64 && ctx && done_ctx[dev] == ctx) return MB_OK;
+    MB_TRY(set_smem(cell_moments_kernel<CELL_GAUSS, 1, 8>, CellShape<CELL_GAUSS, 1, 8>::smem));
+    MB_TRY(set_smem(cell_moments_kernel<CELL_GAUSS, 1, 16>, CellShape<CELL_GAUSS, 1, 16>::smem));
+    MB_TRY(set_smem(cell_moments_kernel<CELL_WEIGHTS, 1, CELL_D1>, CellShape<CELL_WEIGHTS, 1, CELL_D1>::smem));
+    MB_TRY(set_smem(cell_moments_kernel<CELL_WEIGHTS, 2, CELL_D1>, CellShape<CELL_WEIGHTS, 2, CELL_D1>::smem));
+    MB_TRY(set_smem(cell_moments_kernel<CELL_WEIGHTS, 3, CELL_D1>, CellShape<CELL_WEIGHTS, 3, CELL_D1>::smem));
+    MB_TRY(set_smem(cell_moments_kernel<CELL_WEIGHTS, 4, CELL_D1>, CellShape<CELL_WEIGHTS, 4, CELL_D1>::smem));
+    MB_TRY(set_smem(cell_moments_kernel<CELL_WEIGHTS, 5, CELL_D1>, CellShape<CELL_WEIGHTS, 5, CELL_D1>::smem));
+    MB_TRY(set_smem(cell_moments_kernel<CELL_POWERS, 1, 17>, CellShape<CELL_POWERS, 1, 17>::smem));
+    MB_TRY(set_smem(cell_scan_kernel<8>, cscan_smem<8>()));
+    MB_TRY(set_smem(cell_scan_kernel<16>, cscan_smem<16>()));
+    if (dev >= 0 && dev < 64) done_ctx[dev] = current_context();
+    return MB_OK;
+}
+
+bool plan_cells(const Table &t, int64_t n, int64_t split, double R, int d1, int64_t min_cells, CellPlan &out) {
+    const double two_pi = 6.283185307179586;
+    if (n < 1 || !(R >= 0.0) || !(t.h_gamma[n - 1] < two_pi * 0x1p30)) return false;
+    // half width in units of 2^-16: 2 pi H R <= X
+    const double want = R > 0.0 ? cell_x(d1) / (two_pi * R) * 65536.0 : 1e15;
+    if (!(want >= 2.0)) return false;
+    int64_t half = (int64_t)std::min(want, 1e12);
+    const int64_t lo = (int64_t)std::floor(t.h_gamma[0] / two_pi * 65536.0) - 2;
+    const int64_t hi = (int64_t)std::ceil(t.h_gamma[n - 1] / two_pi * 65536.0) + 2;
+    if (min_cells > 1) half = std::min(half, std::max<int64_t>(2, (hi - lo) / (2 * min_cells)));
+    out.half = half;
+    auto group = [&](int q, int64_t a, int64_t b) {
+        out.a[q] = a;
+        out.b[q] = b;
+        out.e0[q] = std::max<int64_t>(0, (int64_t)std::floor(t.h_gamma[a] / two_pi * 65536.0) - 2);
+        const int64_t e1 = (int64_t)std::ceil(t.h_gamma[b - 1] / two_pi * 65536.0) + 2;
+        const int64_t nc = (e1 - out.e0[q]) / (2 * half) + 1;
+        out.nc[q] = (int)std::min<int64_t>(nc, (int64_t)1 << 30);
+    };
+    if (split > 0 && split < n) {
+        out.groups = 2;
+        group(0, 0, split);
+        group(1, split, n);
+    } else {
+        out.groups = 1;
+        group(0, 0, n);
+        out.nc[1] = 0;
+        out.a[1] = out.b[1] = out.e0[1] = 0;
+    }
+    return (int64_t)out.nc[0] + out.nc[1] < ((int64_t)1 << 28);
+}
+
+size_t cells_bytes(const CellPlan &p) { return ((size_t)p.cells() * 8 + 255) / 256 * 256 + 2 * (((size_t)p.cells() * 4 + 255) / 256 * 256); }
+
+int build_cells(const Table &t, const CellPlan &p, void *buf, Cells &out, cudaStream_t s) {
+    char *q = (char *)buf;
+    const int n = p.cells();
+    int64_t *ctr = carve<int64_t>(q, n);
+    int *j0 = carve<int>(q, n), *j1 = carve<int>(q, n);
+    CellGroups g;
+    for (int i = 0; i < 2; ++i) {
+        g.a[i] = p.a[i];
+        g.b[i] = p.b[i];
+        g.e0[i] = p.e0[i];
+        g.nc[i] = p.nc[i];
+    }
+    cells_kernel<<<(unsigned)((n + 127) / 128), 128, 0, s>>>(view(t), g, n, p.half, j0, j1, ctr);
+    MB_CUDA(cudaGetLastError());
+    out = Cells{n, p.nc[0], p.half, j0, j1, ctr};
+    return MB_OK;
+}
+
+int launch_moments_gauss(const Table &t, const Cells &c, const uint64_t *vi, const uint64_t *vf, int64_t P, double k,
+                         int d1, double *out, cudaStream_t s) {
+    const CellWeights none{};
+    const int nzw = cell_nzw(P);
+    return d1 == 8 ? launch_moments<CELL_GAUSS, 1, 8>(t, c, vi, vf, nullptr, nullptr, P, none, k, nzw, out, s)
+                   : launch_moments<CELL_GAUSS, 1, 16>(t, c, vi, vf, nullptr, nullptr, P, none, k, nzw, out, s);
+}
+
+int launch_moments_weights(const Table &t, const Cells &c, const uint64_t *vi, const uint64_t *vf,
+                           const double *delta, const int *sel, int64_t P, int nw, const CellWeights &w,
+                           double *out, cudaStream_t s) {
+    // one warp per 8 peaks and zero order (nzw = 1) whatever P: a peak's moments keep their bits
+    switch (nw) {
+        case 1: return launch_moments<CELL_WEIGHTS, 1, CELL_D1>(t, c, vi, vf, delta, sel, P, w, 0.0, 1, out, s);
+        case 2: return launch_moments<CELL_WEIGHTS, 2, CELL_D1>(t, c, vi, vf, delta, sel, P, w, 0.0, 1, out, s);
+        case 3: return launch_moments<CELL_WEIGHTS, 3, CELL_D1>(t, c, vi, vf, delta, sel, P, w, 0.0, 1, out, s);
+        case 4: return launch_moments<CELL_WEIGHTS, 4, CELL_D1>(t, c, vi, vf, delta, sel, P, w, 0.0, 1, out, s);
+        default: return launch_moments<CELL_WEIGHTS, 5, CELL_D1>(t, c, vi, vf, delta, sel, P, w, 0.0, 1, out, s);
+    }
+}
+
+// Chunks so that every CTA slot gets about four items, each at least 512 zeros.
+int taylor_chunks(const Table &t, int64_t P, int64_t n, int *n_chunk) {
+    int slots = 296;
+    MB_TRY(cell_slots(t, &slots));
+    const int ppc = CELL_PEAKS / cell_nzw(P);
+    const int64_t n_pt = std::max<int64_t>(1, (P + ppc - 1) / ppc);
+    *n_chunk = (int)std::max<int64_t>(1, std::min<int64_t>((4 * (int64_t)slots + n_pt - 1) / n_pt, n / 512));
+    return MB_OK;
+}
+
+size_t taylor_work_bytes(int64_t P, int n_chunk) {
+    return 2 * ((size_t)n_chunk * 4 + 256) + (size_t)P * n_chunk * 24 * 8 + 256;
+}
+
+int launch_taylor_grid(const Table &t, const uint64_t *vi, const uint64_t *vf, const double *delta, int64_t P,
+                       int64_t n, int n_chunk, const double *w, const double *grid, int n_grid, void *work,
+                       double *h_unpol, double *h_pol, double *ddy_pol, cudaStream_t s) {
+    char *q = (char *)work;
+    int *j0 = carve<int>(q, n_chunk), *j1 = carve<int>(q, n_chunk);
+    double *S = carve<double>(q, (size_t)P * n_chunk * 24);
+    chunks_kernel<<<(unsigned)((n_chunk + 127) / 128), 128, 0, s>>>(n, n_chunk, j0, j1);
+    MB_CUDA(cudaGetLastError());
+    const Cells c{n_chunk, n_chunk, 1, j0, j1, nullptr};
+    const CellWeights cw{{w}};
+    MB_TRY((launch_moments<CELL_POWERS, 1, 17>(t, c, vi, vf, delta, nullptr, P, cw, 0.0, cell_nzw(P), S, s)));
+    taylor_grid_kernel<<<(unsigned)P, TAY_THREADS, 0, s>>>(S, n_chunk, grid, n_grid, h_unpol, h_pol, ddy_pol);
+    MB_CUDA(cudaGetLastError());
+    return MB_OK;
+}
+
+int launch_cell_scan(const Cells &c, int d1, const double *M, int64_t P, int NB, int Bp, int64_t n_m,
+                     uint64_t step_int, uint64_t step_frac, double *out, cudaStream_t s) {
+    MB_TRY(cell_kernel_attributes());
+    const double step = (double)step_int + (double)step_frac * 0x1p-64;
+    const double kstep = 6.283185307179586 * c.H() * step;
+    const dim3 grid((unsigned)((Bp + CSCAN_THREADS * CSCAN_PT - 1) / (CSCAN_THREADS * CSCAN_PT)), (unsigned)(P * NB));
+    if (d1 == 8)
+        cell_scan_kernel<8><<<grid, CSCAN_THREADS, cscan_smem<8>(), s>>>(c, M, NB, Bp, n_m, step_int, step_frac, kstep, out);
+    else
+        cell_scan_kernel<16><<<grid, CSCAN_THREADS, cscan_smem<16>(), s>>>(c, M, NB, Bp, n_m, step_int, step_frac, kstep, out);
+    MB_CUDA(cudaGetLastError());
+    return MB_OK;
+}
+
+// Peaks of one batch of the second pass: their terms take at most 256 MB.
+static int redo_batch(int64_t count, int64_t n) {
+    const int64_t fit = ((int64_t)256 << 20) / (2 * (int64_t)sizeof(double2) * n);
+    return (int)std::max<int64_t>(1, std::min<int64_t>({fit, count, 1024}));
+}
+
+size_t cell_polish_bytes(int64_t P, int nw) { return 256 + ((size_t)P * nw * sizeof(Redo) + 256); }
+
+template <int MODE>
+static int polish_mode(Table &t, const Cells &c, const double *M, CellPolishArgs a, const uint64_t *vi,
+                       const uint64_t *vf, const double *delta, int64_t n, CellWeights w, void *work, cudaStream_t s) {
+    using R = PolishRule<MODE>;
+    char *q = (char *)work;
+    int *d_count = carve<int>(q, 1);
+    Redo *list = carve<Redo>(q, (size_t)a.P * a.nw);
+    MB_CUDA(cudaMemsetAsync(d_count, 0, sizeof(int), s));
+    cell_polish_kernel<MODE><<<dim3((unsigned)a.P, (unsigned)a.nw), CPOL_THREADS, 0, s>>>(c, M, a, delta, list, d_count);
+    MB_CUDA(cudaGetLastError());
+    int count = 0;
+    MB_CUDA(cudaMemcpyAsync(&count, d_count, sizeof(int), cudaMemcpyDeviceToHost, s));
+    MB_CUDA(cudaStreamSynchronize(s));
+    if (count == 0) return MB_OK;
+    RedoBuf rb;
+    rb.batch = redo_batch(count, n);
+    const size_t bn = (size_t)rb.batch * n;
+    MB_TRY(t.redo.ensure((2 * rb.batch * sizeof(RedoState) + 256) + (rb.batch * POLISH_CLUSTER * sizeof(double2) + 256) +
+                         2 * (rb.batch * 8 + 256) + 2 * (bn * sizeof(double2) + 256)));
+    q = (char *)t.redo.p;
+    rb.state = carve<RedoState>(q, 2 * (size_t)rb.batch);
+    rb.slot = carve<double2>(q, (size_t)rb.batch * POLISH_CLUSTER);
+    rb.h_best = carve<double>(q, rb.batch);
+    rb.d_best = carve<double>(q, rb.batch);
+    rb.ab = carve<double2>(q, bn);
+    rb.term = carve<double2>(q, bn);
+    const int ns = MODE == POLISH_SINGLE && a.n_grid == 0 ? 1 : R::starts;
+    const ABExact src{view(t), vi, vf, delta};
+    for (int e0 = 0; e0 < count; e0 += rb.batch) {
+        const unsigned m = (unsigned)std::min(rb.batch, count - e0);
+        rb.list = list + e0;
+        const unsigned nb = (unsigned)((n + 255) / 256);
+        redo_ab_kernel<<<dim3(nb, m), 256, 0, s>>>(src, n, rb);
+        for (int st = 0; st < ns; ++st) {
+            for (int it = 0; it <= R::iters; ++it) {     // the last pass sums h
+                redo_term_kernel<MODE><<<dim3((nb + 1) / 2, m), 256, 0, s>>>(t.d_gamma, n, rb, st, it);
+                redo_sum_kernel<<<dim3(POLISH_CLUSTER, m), POLISH_THREADS, 0, s>>>(t.d_gamma, n, w, rb, it, it == R::iters);
+            }
+            redo_keep_kernel<MODE><<<(m + 127) / 128, 128, 0, s>>>(rb, a, (int)m, st, st == ns - 1);
+        }
+        MB_CUDA(cudaGetLastError());
+    }
+    return MB_OK;
+}
+
+int launch_cell_polish(Table &t, const Cells &c, const double *M, const CellPolishArgs &a, const uint64_t *vi,
+                       const uint64_t *vf, const double *delta, int64_t n, const CellWeights &w, void *work,
+                       cudaStream_t s) {
+    if (a.mode == POLISH_EVAL_FAST) return polish_mode<POLISH_EVAL_FAST>(t, c, M, a, vi, vf, delta, n, w, work, s);
+    if (a.mode == POLISH_SINGLE) return polish_mode<POLISH_SINGLE>(t, c, M, a, vi, vf, delta, n, w, work, s);
+    return polish_mode<POLISH_TOPK>(t, c, M, a, vi, vf, delta, n, w, work, s);
+}
+
+}  // namespace mb

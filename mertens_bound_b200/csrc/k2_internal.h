@@ -76,6 +76,7 @@ struct Table {
     // (which runs on the caller's stream, so it shares no buffer with calls on `stream`).  Calls
     // on one table that use the same buffer must not overlap on the GPU.
     DevBuf io, work, screen;
+    DevBuf redo;                      // the second pass of polishes on cell moments (k2_cells.cu)
     int n_plans = 0;                  // live plans on this table (it cannot be destroyed under them)
 
     int64_t count_below(double T) const;

@@ -10,7 +10,9 @@
 // anchor).  FP64 accumulation, deterministic reduction over zero chunks.
 #include <algorithm>
 #include <cmath>
+#include <vector>
 
+#include "k2_cells.h"
 #include "k2_common.cuh"
 #include "k2_internal.h"
 
@@ -242,6 +244,119 @@ __global__ void scan_reduce_kernel(const double *partial, int P, int n_chunk, in
     h[idx] = s;
 }
 
+// ------------------------------------------------------------------ scans on cell moments
+//
+// Each base point's grid is cut into NB blocks of Bp points; the moments about each block's middle
+// point (64.64, exact) are taken once per zero and evaluated on the block's points (k2_cells.h).
+
+typedef unsigned __int128 u128;
+
+struct ScanPlan {
+    int Bp = 0, NB = 0, d1 = 0;
+    int64_t chunk = 0;         // base points per pass
+    CellPlan cp;
+};
+
+constexpr size_t SCAN_MOMENT_BYTES = (size_t)256 << 20;
+constexpr int64_t SCAN_MAX_POINTS = 65535;                  // block points per pass (a grid dimension)
+
+// Chooses the block count and the series length with the smallest estimated work; false when the direct
+// kernel is the cheaper one (c_old: its warp cycles per 32 (point, zero) pairs): few points per base,
+// or a step so large that a block's cells hold less than a few zeros each.  The estimates are warp cycles
+// of one scheduler: a moment step (32 pairs) ~60 for the phasors + 32 per 8 columns, the staging ~10 per
+// zero and CTA, a point of the evaluation 2 (2 D1 + 14) + 25 per cell.
+bool plan_scan(const Table &t, int64_t P, int64_t n_use, int64_t n_m, uint64_t step_int, uint64_t step_frac,
+               double c_old, int64_t old_points, ScanPlan &best) {
+    if (n_use < 1 || step_int >> 31) return false;
+    const double step = (double)step_int + (double)step_frac * 0x1p-64;
+    double best_cost = c_old / 32.0 * P * old_points * n_use;
+    bool found = false;
+    for (int64_t NB = 1; NB <= n_m; NB = NB < 64 ? 2 * NB : NB + 64) {
+        const int64_t Bp = (n_m + NB - 1) / NB;
+        if (NB > 1 && Bp < 32) break;
+        if (NB > SCAN_MAX_POINTS) break;
+        const int64_t pts = P * NB;
+        int nzw = 1;
+        while (nzw < 8 && pts <= CELL_PEAKS / (2 * nzw)) nzw *= 2;
+        const int ppc = CELL_PEAKS / nzw;
+        const double tiles = (double)((pts + ppc - 1) / ppc);
+        for (int d1 : {8, 16}) {
+            // at least one item per CTA slot where the cells hold 16 zeros or more
+            const int64_t min_cells = std::min<int64_t>(n_use / 16, (int64_t)(296 / tiles));
+            CellPlan cp;
+            if (!plan_cells(t, n_use, 0, (double)((Bp + 1) / 2) * step, d1, min_cells, cp)) continue;
+            const double nc = cp.cells();
+            const double zeros = n_use + 2.0 * nc;
+            const double mom = tiles * zeros * (ppc / 32.0 * (60.0 + 4.0 * d1) + 10.0);
+            const double eval = (double)pts * ((Bp + 255) / 256 * 256) / 32.0 * nc * (2.0 * (2 * d1 + 14) + 25.0);
+            const double bytes = (double)NB * nc * 2 * d1 * 8;
+            if (bytes > (double)SCAN_MOMENT_BYTES) continue;
+            if (mom + eval < best_cost) {
+                best_cost = mom + eval;
+                best.Bp = (int)Bp;
+                best.NB = (int)NB;
+                best.d1 = d1;
+                best.cp = cp;
+                best.chunk = std::max<int64_t>(
+                    1, std::min({P, SCAN_MAX_POINTS / NB, (int64_t)((double)SCAN_MOMENT_BYTES / bytes)}));
+                found = true;
+            }
+        }
+    }
+    return found;
+}
+
+// Whether v + m step stays in [0, 2^64) for m0 <= m <= m0 + n_m (the blocks' span) at every base point, so
+// that each block's middle point is a 64.64 number.
+bool scan_in_range(int64_t P, const uint64_t *vi, const uint64_t *vf, u128 step, int64_t m0, int64_t n_m) {
+    const u128 lo = step * (u128)(m0 < 0 ? -m0 : 0), hi = step * (u128)std::max<int64_t>(0, m0 + n_m);
+    for (int64_t p = 0; p < P; ++p) {
+        const u128 v = (u128)vi[p] << 64 | vf[p];
+        if (v < lo || v + hi < v) return false;
+    }
+    return true;
+}
+
+// The scan of P base points on cell moments, results in out_h (host).
+int scan_cells(Table &t, int64_t P, const uint64_t *v_int, const uint64_t *v_frac, double k, uint64_t step_int,
+               uint64_t step_frac, int64_t m0, int64_t n_m, const ScanPlan &sp, double *out_h) {
+    const u128 step = (u128)step_int << 64 | step_frac;
+    const int64_t per = sp.chunk * sp.NB;
+    const size_t pb = (size_t)per * 8, cb = cells_bytes(sp.cp);
+    MB_TRY(t.io.ensure(2 * (pb + 256) + cb + 256 + (size_t)sp.chunk * n_m * 8 + 256));
+    MB_TRY(t.work.ensure((size_t)per * sp.cp.cells() * 2 * sp.d1 * 8));
+    char *q = (char *)t.io.p;
+    uint64_t *d_v = carve<uint64_t>(q, 2 * per);
+    void *cbuf = carve<char>(q, cb);
+    double *d_h = carve<double>(q, sp.chunk * n_m);
+    double *M = (double *)t.work.p;
+    Cells cells;
+    MB_TRY(build_cells(t, sp.cp, cbuf, cells, t.stream));
+    std::vector<uint64_t> pts(2 * per);
+    for (int64_t p0 = 0; p0 < P; p0 += sp.chunk) {
+        const int64_t np = std::min(sp.chunk, P - p0), nb = np * sp.NB;
+        for (int64_t p = 0; p < np; ++p)
+            for (int64_t b = 0; b < sp.NB; ++b) {
+                const int64_t m = m0 + b * sp.Bp + sp.Bp / 2;
+                const u128 off = step * (u128)(m < 0 ? -m : m);
+                const u128 v = (u128)v_int[p0 + p] << 64 | v_frac[p0 + p];
+                const u128 y = m < 0 ? v - off : v + off;
+                pts[p * sp.NB + b] = (uint64_t)(y >> 64);
+                pts[nb + p * sp.NB + b] = (uint64_t)y;
+            }
+        MB_CUDA(cudaMemcpyAsync(d_v, pts.data(), 2 * (size_t)nb * 8, cudaMemcpyHostToDevice, t.stream));
+        MB_TRY(launch_moments_gauss(t, cells, d_v, d_v + nb, nb, k, sp.d1, M, t.stream));
+        MB_TRY(launch_cell_scan(cells, sp.d1, M, np, sp.NB, sp.Bp, n_m, step_int, step_frac, d_h, t.stream));
+        MB_CUDA(cudaMemcpyAsync(out_h + p0 * n_m, d_h, (size_t)np * n_m * 8, cudaMemcpyDeviceToHost, t.stream));
+    }
+    MB_CUDA(cudaStreamSynchronize(t.stream));
+    return MB_OK;
+}
+
+// Warp cycles of the direct kernels per 32 (point, zero) pairs, from their measured times (25,001 points x
+// 98,624 zeros in 1.36 ms; 256 x 241 points x 600,000 zeros in 33.6 ms).
+constexpr double GRID_CYCLES = 20.0, HIT_CYCLES = 34.0;
+
 }  // namespace
 }  // namespace mb
 
@@ -258,6 +373,11 @@ extern "C" int mb_grid_scan(mb_table *h, int64_t P, const uint64_t *v_int, const
     Table &t = table_of(h);
     MB_TRY(device_guard(t.device));
     const int64_t n_use = t.count_below(T);
+    ScanPlan sp;
+    const int64_t grid_points = (n_m + SCAN_THREADS * SCAN_MPT - 1) / (SCAN_THREADS * SCAN_MPT) * (SCAN_THREADS * SCAN_MPT);
+    if (plan_scan(t, P, n_use, n_m, step_int, step_frac, GRID_CYCLES, grid_points, sp) &&
+        scan_in_range(P, v_int, v_frac, (u128)step_int << 64 | step_frac, m0, (int64_t)sp.NB * sp.Bp))
+        return scan_cells(t, P, v_int, v_frac, k, step_int, step_frac, m0, n_m, sp, out_h);
     const size_t cb = (size_t)P * 8, hb = (size_t)P * n_m * 8;
     int sms = 148;
     MB_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, t.device));
@@ -304,6 +424,10 @@ extern "C" int mb_hit_scan(mb_table *h, int64_t P, const uint64_t *v_int, const 
     Table &t = table_of(h);
     MB_CHECK_ARG(n_use >= 0 && n_use <= t.n, "mb_hit_scan: n_use=%lld of %lld", (long long)n_use, (long long)t.n);
     MB_TRY(device_guard(t.device));
+    ScanPlan sp;
+    if (plan_scan(t, P, n_use, n_m, step_int, step_frac, HIT_CYCLES, (n_m + HIT_MB - 1) / HIT_MB * HIT_MB, sp) &&
+        scan_in_range(P, v_int, v_frac, (u128)step_int << 64 | step_frac, m0, (int64_t)sp.NB * sp.Bp))
+        return scan_cells(t, P, v_int, v_frac, k, step_int, step_frac, m0, n_m, sp, out_h);
     const size_t cb = (size_t)P * 8, hb = (size_t)P * n_m * 8;
     MB_TRY(t.io.ensure(2 * cb + hb + 256));
     char *base = (char *)t.io.p;

@@ -81,6 +81,7 @@ static void free_table(Table &t) {
     t.io.release();
     t.work.release();
     t.screen.release();
+    t.redo.release();
     for (double *w : t.d_weights) cudaFree(w);
     if (t.ev_fork) cudaEventDestroy(t.ev_fork);
     if (t.ev_join) cudaEventDestroy(t.ev_join);
