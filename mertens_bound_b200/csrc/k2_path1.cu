@@ -14,6 +14,7 @@
 #include <numeric>
 #include <vector>
 
+#include "k2_cells.h"
 #include "k2_polish.cuh"
 
 namespace mb {
@@ -113,7 +114,7 @@ int stage_exact(Table &t, int64_t P, const uint64_t *vi, const uint64_t *vf, con
         MB_CUDA(cudaMemcpyAsync(s.delta, delta, P * 8, cudaMemcpyHostToDevice, t.stream));
     else
         MB_CUDA(cudaMemsetAsync(s.delta, 0, P * 8, t.stream));
-    if (n_grid > 0) MB_CUDA(cudaMemcpyAsync(s.grid, grid, n_grid * 8, cudaMemcpyHostToDevice, t.stream));
+    if (n_grid > 0 && grid) MB_CUDA(cudaMemcpyAsync(s.grid, grid, n_grid * 8, cudaMemcpyHostToDevice, t.stream));
     return MB_OK;
 }
 
@@ -125,6 +126,61 @@ int fetch_outputs(cudaStream_t st, int64_t P, const double *hu, const double *hp
     MB_CUDA(cudaStreamSynchronize(st));
     return MB_OK;
 }
+
+// ------------------------------------------------------------------ polishes on cell moments
+
+constexpr size_t POLISH_MOMENT_BYTES = (size_t)256 << 20;
+
+// Plans the cells of a polish whose offsets stay within R of the peaks: true where they hold four zeros or
+// more on average (fewer cells than that make an evaluation on moments cheaper than one over the zeros:
+// ~110 FP64 operations per cell against ~60 per zero and pass).  At least 592 cells (two items per CTA
+// slot) where they hold 64 zeros: few peaks then still fill the GPU; the split depends on the zeros and
+// R alone, so a peak's results do not depend on the others in the call.
+bool plan_polish(const Table &t, int64_t n, int64_t split, double R, CellPlan &cp) {
+    if (n < 1 || !std::isfinite(R)) return false;
+    return plan_cells(t, n, split, R, CELL_D1, std::min<int64_t>(n / 64, 592), cp) &&
+           (int64_t)cp.cells() <= std::max<int64_t>(64, n / 4);
+}
+
+// Polishes the P peaks of stage s (or its P selected ones, a.sel) over the zeros [0, n) under the weight
+// slots, outputs a.h_unpol etc. on the device: per chunk of peaks and up to CELL_MAX_W vectors, one moment
+// pass over the zeros and the polish on the moments.
+int polish_on_cells(Table &t, const ExactStage &s, int64_t P, int64_t n, int n_weights, const int *slots,
+                    const CellPlan &cp, CellPolishArgs a) {
+    const size_t cb = cells_bytes(cp), one = (size_t)cp.cells() * 2 * CELL_D1 * 8;     // per (peak, weight)
+    const int wmax = std::min(n_weights, CELL_MAX_W);
+    const int64_t chunk = std::max<int64_t>(1, std::min<int64_t>(P, (int64_t)(POLISH_MOMENT_BYTES / (one * wmax))));
+    MB_TRY(t.work.ensure((cb + 256) + ((size_t)chunk * wmax * one + 256) + cell_polish_bytes(chunk, wmax)));
+    char *q = (char *)t.work.p;
+    void *cbuf = carve<char>(q, cb);
+    double *M = carve<double>(q, (size_t)chunk * wmax * (one / 8));
+    void *work = q;
+    Cells cells;
+    MB_TRY(build_cells(t, cp, cbuf, cells, t.stream));
+    const CellPolishArgs all = a;
+    for (int64_t p0 = 0; p0 < P; p0 += chunk)
+        for (int w0 = 0; w0 < n_weights; w0 += CELL_MAX_W) {
+            const int64_t np = std::min(chunk, P - p0);
+            const int nw = std::min(n_weights - w0, CELL_MAX_W);
+            CellWeights w{};
+            for (int i = 0; i < nw; ++i) w.w[i] = t.d_weights[slots[w0 + i]];
+            const int *sel = all.sel ? all.sel + p0 : nullptr;
+            const int64_t po = sel ? 0 : p0, o = (int64_t)w0 * all.out_stride + po;
+            MB_TRY(launch_moments_weights(t, cells, s.vi + po, s.vf + po, s.delta + po, sel, np, nw, w, M, t.stream));
+            a.P = np;
+            a.nw = nw;
+            a.sel = sel;
+            a.h_unpol = all.h_unpol + o;
+            a.h_pol = all.h_pol + o;
+            a.ddy_pol = all.ddy_pol + o;
+            MB_TRY(launch_cell_polish(t, cells, M, a, s.vi + po, s.vf + po, s.delta + po, n, w, work, t.stream));
+        }
+    return MB_OK;
+}
+
+// The farthest offset the loops of k2_polish.cuh reach: the grid's, plus every Newton step at its clamp.
+double eval_fast_reach(double half, int steps) { return (steps > 0 ? std::fabs(half) : 0.0) + 6 * 1e-4; }
+double single_reach(double hw, int steps) { return (steps > 0 ? std::fabs(hw) : 0.0) + 8 * 2e-5; }
 
 }  // namespace
 }  // namespace mb
@@ -286,6 +342,12 @@ extern "C" int mb_polish_single_exact(mb_table *h, int64_t P, const uint64_t *v_
     const std::vector<double> grid = linspace_grid(grid_hw, grid_steps);
     ExactStage s;
     MB_TRY(stage_exact(t, P, v_int, v_frac, delta, grid.data(), (int64_t)grid.size(), 0, s));
+    CellPlan cp;
+    if (plan_polish(t, n_zeros, 0, single_reach(grid_hw, grid_steps), cp)) {
+        MB_TRY(polish_on_cells(t, s, P, n_zeros, 1, &weight_slot, cp,
+                               CellPolishArgs{POLISH_SINGLE, P, 1, P, s.grid, (int)grid.size(), 0.0, nullptr, s.hu, s.hp, s.dp}));
+        return fetch_outputs(t.stream, P, s.hu, s.hp, s.dp, out_h_unpol, out_h_pol, out_ddy_pol);
+    }
     PolishArgs a{n_zeros, t.d_gamma, t.d_weights[weight_slot], s.grid, (int)grid.size(), 0.0, nullptr, s.hu, s.hp, s.dp};
     peak_polish_kernel<ABExact, POLISH_SINGLE><<<(unsigned)(P * POLISH_CLUSTER), POLISH_THREADS, 0, t.stream>>>(
         ABExact{view(t), s.vi, s.vf, s.delta}, a);
@@ -308,6 +370,13 @@ extern "C" int mb_polish_peaks_exact(mb_table *h, int64_t P, const uint64_t *v_i
     MB_TRY(device_guard(t.device));
     ExactStage s;
     MB_TRY(stage_exact(t, P, v_int, v_frac, delta, nullptr, 0, 0, s));
+    CellPlan cp;
+    if (plan_polish(t, n_zeros, 4096, eval_fast_reach(grid_half_width, grid_steps), cp)) {
+        MB_TRY(polish_on_cells(t, s, P, n_zeros, 1, &weight_slot, cp,
+                               CellPolishArgs{POLISH_EVAL_FAST, P, 1, P, nullptr, grid_steps, grid_half_width, nullptr,
+                                              s.hu, s.hp, s.dp}));
+        return fetch_outputs(t.stream, P, s.hu, s.hp, s.dp, out_h_unpol, out_h_pol, out_ddy_pol);
+    }
     PolishArgs a{n_zeros, t.d_gamma, t.d_weights[weight_slot], nullptr, grid_steps, grid_half_width, nullptr,
                  s.hu, s.hp, s.dp};
     peak_polish_kernel<ABExact, POLISH_EVAL_FAST><<<(unsigned)(P * POLISH_CLUSTER), POLISH_THREADS, 0, t.stream>>>(
@@ -344,6 +413,16 @@ extern "C" int mb_polish_peaks_weights(mb_table *h, int64_t P, const uint64_t *v
     }
     MB_TRY(device_guard(t.device));
     ExactStage s;
+    CellPlan cp;
+    if (plan_polish(t, n_zeros, 4096, eval_fast_reach(grid_half_width, grid_steps), cp)) {
+        const size_t ob = (size_t)n_weights * P;
+        MB_TRY(stage_exact(t, P, v_int, v_frac, delta, nullptr, (int64_t)(3 * ob), 0, s));
+        double *hu = s.grid, *hp = hu + ob, *dp = hp + ob;       // outputs in the stage's grid array
+        MB_TRY(polish_on_cells(t, s, P, n_zeros, n_weights, weight_slots, cp,
+                               CellPolishArgs{POLISH_EVAL_FAST, P, n_weights, P, nullptr, grid_steps, grid_half_width,
+                                              nullptr, hu, hp, dp}));
+        return fetch_outputs(t.stream, (int64_t)ob, hu, hp, dp, out_h_unpol, out_h_pol, out_ddy_pol);
+    }
     MB_TRY(stage_exact(t, P, v_int, v_frac, delta, nullptr, 0, 0, s));
     // the matrices take at most AB_BUDGET bytes and at most half of the device's free memory
     size_t free_b = 0, total_b = 0;
@@ -409,13 +488,26 @@ extern "C" int mb_fast_polish_exact(mb_table *h, int64_t P, const uint64_t *v_in
     MB_TRY(stage_exact(t, P, v_int, v_frac, delta, ddy_grid, n_grid, nsel, s));
     const ABExact src{view(t), s.vi, s.vf, s.delta};
     const double *d_w = t.d_weights[weight_slot];
-    MomentArgs m{n_zeros, t.d_gamma, d_w, s.grid, (int)n_grid, s.hu, s.hp, s.dp};
-    taylor_moments_kernel<ABExact><<<(unsigned)(P * POLISH_CLUSTER), POLISH_THREADS, 0, t.stream>>>(src, m);
-    MB_CUDA(cudaGetLastError());
+    int n_chunk = 1;
+    MB_TRY(taylor_chunks(t, P, n_zeros, &n_chunk));
+    const int64_t pc = std::max<int64_t>(
+        1, std::min<int64_t>(P, (int64_t)(POLISH_MOMENT_BYTES / taylor_work_bytes(1, n_chunk))));
+    MB_TRY(t.work.ensure(taylor_work_bytes(pc, n_chunk)));
+    for (int64_t p0 = 0; p0 < P; p0 += pc)
+        MB_TRY(launch_taylor_grid(t, s.vi + p0, s.vf + p0, s.delta + p0, std::min(pc, P - p0), n_zeros, n_chunk, d_w,
+                                  s.grid, (int)n_grid, t.work.p, s.hu + p0, s.hp + p0, s.dp + p0, t.stream));
     MB_TRY(fetch_outputs(t.stream, P, s.hu, s.hp, s.dp, out_h_unpol, out_h_pol, out_ddy_pol));
     if (nsel == 0) return MB_OK;
     const std::vector<int> sel = top_indices(out_h_pol, P, nsel);
     MB_CUDA(cudaMemcpyAsync(s.sel, sel.data(), nsel * sizeof(int), cudaMemcpyHostToDevice, t.stream));
+    double reach = 4 * 1e-5;
+    for (int64_t i = 0; i < n_grid; ++i) reach = std::max(reach, std::fabs(ddy_grid[i]) + 4 * 1e-5);
+    CellPlan cp;
+    if (plan_polish(t, n_zeros, 0, reach, cp)) {
+        MB_TRY(polish_on_cells(t, s, nsel, n_zeros, 1, &weight_slot, cp,
+                               CellPolishArgs{POLISH_TOPK, nsel, 1, P, nullptr, 0, 0.0, s.sel, s.hu, s.hp, s.dp}));
+        return fetch_outputs(t.stream, P, s.hu, s.hp, s.dp, out_h_unpol, out_h_pol, out_ddy_pol);
+    }
     PolishArgs a{n_zeros, t.d_gamma, d_w, nullptr, 0, 0.0, s.sel, s.hu, s.hp, s.dp};
     peak_polish_kernel<ABExact, POLISH_TOPK><<<(unsigned)(nsel * POLISH_CLUSTER), POLISH_THREADS, 0, t.stream>>>(src, a);
     MB_CUDA(cudaGetLastError());
