@@ -20,6 +20,8 @@
 //            upper ends with __dadd_ru.  Also an upper bound of sum 2 w |c| (certify_K2's absS).
 #include <algorithm>
 #include <cmath>
+#include <cstring>
+#include <vector>
 
 #include "k2_common.cuh"
 #include "k2_internal.h"
@@ -176,6 +178,32 @@ constexpr int CERT_THREADS = 256;
 template <bool GRAD>
 __host__ __device__ constexpr int cert_sums() { return GRAD ? 7 : 3; }
 
+// Upper ends and abs_hi round up, lower ends down.
+__host__ __device__ constexpr bool cert_up(int q) { return q == 1 || q == 2 || q == 4 || q == 6; }
+
+// The CTA's directed-rounding sums, in thread 0's acc: the warps' shuffle trees, then the warps in order.
+template <int NS>
+MB_DEV void cert_block_sum(double (&acc)[NS], double (*red)[NS]) {
+    for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+        for (int q = 0; q < NS; ++q) {
+            const double x = __shfl_xor_sync(0xffffffffu, acc[q], o);
+            acc[q] = cert_up(q) ? __dadd_ru(acc[q], x) : __dadd_rd(acc[q], x);
+        }
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    if (lane == 0)
+#pragma unroll
+        for (int q = 0; q < NS; ++q) red[warp][q] = acc[q];
+    __syncthreads();
+    if (threadIdx.x == 0)
+#pragma unroll
+        for (int q = 0; q < NS; ++q) {
+            double v = 0.0;
+            for (int w = 0; w < CERT_THREADS / 32; ++w) v = cert_up(q) ? __dadd_ru(v, red[w][q]) : __dadd_rd(v, red[w][q]);
+            acc[q] = v;
+        }
+}
+
 // grid (zero blocks, candidates); partial[(blockIdx.x * P + p) * NS + s] with s = K2 lo, K2 hi,
 // abs_hi[, dd lo, dd hi, dk lo, dk hi]: lower ends summed with __dadd_rd, upper ends with __dadd_ru.
 template <bool GRAD>
@@ -201,48 +229,38 @@ k2_certified_kernel(TabView tv, const uint64_t *vi, const uint64_t *vf, const do
             acc[6] = __dadd_ru(acc[6], ct.dk.hi);
         }
     }
-    // lower ends (even indices except abs_hi at 2) round down, the others up
-    auto up = [](int q) { return q == 1 || q == 2 || q == 4 || q == 6; };
-    for (int o = 16; o > 0; o >>= 1) {
-#pragma unroll
-        for (int q = 0; q < NS; ++q) {
-            const double x = __shfl_xor_sync(0xffffffffu, acc[q], o);
-            acc[q] = up(q) ? __dadd_ru(acc[q], x) : __dadd_rd(acc[q], x);
-        }
-    }
     __shared__ double red[CERT_THREADS / 32][NS];
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    if (lane == 0)
-#pragma unroll
-        for (int q = 0; q < NS; ++q) red[warp][q] = acc[q];
-    __syncthreads();
+    cert_block_sum<NS>(acc, red);
     if (threadIdx.x == 0) {
         double *o = partial + ((int64_t)blockIdx.x * P + p) * NS;
 #pragma unroll
-        for (int q = 0; q < NS; ++q) {
-            double v = 0.0;
-            for (int w = 0; w < CERT_THREADS / 32; ++w) v = up(q) ? __dadd_ru(v, red[w][q]) : __dadd_rd(v, red[w][q]);
-            o[q] = v;
-        }
+        for (int q = 0; q < NS; ++q) o[q] = acc[q];
     }
 }
 
-// out[s * P + p] for the NS sums of candidate p (the same order as the partials).
+// out[s * P + p] for the NS sums of candidate p (the same order as the partials).  One CTA per candidate:
+// a strided directed-rounding sum per thread, then the warps' shuffle trees and the warps in order.  (One
+// thread per candidate spent 118 of the 176 us of the 2.3 M-zero, one-candidate interval here: 3,552
+// dependent loads.  Now 5 us.)
 template <bool GRAD>
-__global__ void certified_reduce_kernel(const double *partial, int64_t P, int nblk, double *out) {
+__global__ void __launch_bounds__(CERT_THREADS)
+certified_reduce_kernel(const double *partial, int64_t P, int nblk, double *out) {
     constexpr int NS = cert_sums<GRAD>();
-    int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (p >= P) return;
+    __shared__ double red[CERT_THREADS / 32][NS];
+    const int64_t p = blockIdx.x;
+    double acc[NS];
 #pragma unroll
-    for (int q = 0; q < NS; ++q) {
-        const bool up = q == 1 || q == 2 || q == 4 || q == 6;
-        double v = 0.0;
-        for (int b = 0; b < nblk; ++b) {
+    for (int q = 0; q < NS; ++q) acc[q] = 0.0;
+    for (int b = threadIdx.x; b < nblk; b += CERT_THREADS)
+#pragma unroll
+        for (int q = 0; q < NS; ++q) {
             const double x = partial[((int64_t)b * P + p) * NS + q];
-            v = up ? __dadd_ru(v, x) : __dadd_rd(v, x);
+            acc[q] = cert_up(q) ? __dadd_ru(acc[q], x) : __dadd_rd(acc[q], x);
         }
-        out[q * P + p] = v;
-    }
+    cert_block_sum<NS>(acc, red);
+    if (threadIdx.x == 0)
+#pragma unroll
+        for (int q = 0; q < NS; ++q) out[q * P + p] = acc[q];
 }
 
 // out (device, NS x P): rows K2 lo, K2 hi, abs_hi [, dd lo, dd hi, dk lo, dk hi].
@@ -260,17 +278,16 @@ int launch_certified(Table &t, const uint64_t *d_vi, const uint64_t *d_vf, const
     MB_TRY(t.work.ensure((size_t)nblk * P * ns * sizeof(double)));
     double *partial = (double *)t.work.p;
     dim3 grid((unsigned)nblk, (unsigned)P);
-    const unsigned rgrid = (unsigned)((P + 255) / 256);
     if (grad) {
         k2_certified_kernel<true><<<grid, CERT_THREADS, 0, s>>>(view(t), d_vi, d_vf, d_vrad, P, j0, j1, k_lo, k_hi,
                                                                 d_term_rad, partial);
         MB_CUDA(cudaGetLastError());
-        certified_reduce_kernel<true><<<rgrid, 256, 0, s>>>(partial, P, (int)nblk, d_out);
+        certified_reduce_kernel<true><<<(unsigned)P, CERT_THREADS, 0, s>>>(partial, P, (int)nblk, d_out);
     } else {
         k2_certified_kernel<false><<<grid, CERT_THREADS, 0, s>>>(view(t), d_vi, d_vf, d_vrad, P, j0, j1, k_lo, k_hi,
                                                                  d_term_rad, partial);
         MB_CUDA(cudaGetLastError());
-        certified_reduce_kernel<false><<<rgrid, 256, 0, s>>>(partial, P, (int)nblk, d_out);
+        certified_reduce_kernel<false><<<(unsigned)P, CERT_THREADS, 0, s>>>(partial, P, (int)nblk, d_out);
     }
     MB_CUDA(cudaGetLastError());
     return MB_OK;
@@ -316,9 +333,12 @@ int certified_call(const char *who, mb_table *h, int64_t P, const uint64_t *v_in
     if (term_rad && rb) MB_CUDA(cudaMemcpyAsync(d_rad, term_rad, rb, cudaMemcpyHostToDevice, t.stream));
     MB_TRY(launch_certified(t, d_vi, d_vf, v_rad ? d_vrad : nullptr, P, j0, j1, k_lo, k_hi, d_rad, grad, d_out,
                             t.stream));
-    for (int r = 0; r < ns; ++r)
-        if (out_rows[r]) MB_CUDA(cudaMemcpyAsync(out_rows[r], d_out + r * P, cb, cudaMemcpyDeviceToHost, t.stream));
+    // one copy for all rows (each small pageable copy costs several microseconds)
+    std::vector<double> rows((size_t)ns * P);
+    MB_CUDA(cudaMemcpyAsync(rows.data(), d_out, ns * cb, cudaMemcpyDeviceToHost, t.stream));
     MB_CUDA(cudaStreamSynchronize(t.stream));
+    for (int r = 0; r < ns; ++r)
+        if (out_rows[r]) std::memcpy(out_rows[r], rows.data() + (size_t)r * P, cb);
     return MB_OK;
 }
 
