@@ -406,16 +406,18 @@ k2_tiers_kernel(TabView t, CandView c, const FastItem *items, int n_items, int n
     }
 }
 
-// Eight lanes per candidate, four candidates per warp: lane 4r + q sums the chunks r, r + 8, ...
-// of candidate 4w + q, so the four lanes of one chunk read 96 consecutive bytes; a fixed shuffle
-// tree then adds the eight lanes (deterministic: the order depends only on the chunk count).
-constexpr int REDUCE_LANES = 8;
-__global__ void fast_reduce_kernel(const FastGroup *groups, int n_groups, const double *partial,
-                                   int64_t P, double *val, double *dd, double *dk) {
-    const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    const int lane = threadIdx.x & 31;
-    const int r = lane >> 2;
-    const int64_t p = (t >> 5) * 4 + (lane & 3);
+// REDUCE_CANDS candidates per CTA, REDUCE_LANES chunk lanes each: lane r of candidate q sums the chunks
+// r, r + REDUCE_LANES, ... (the eight lanes of one chunk read 192 consecutive bytes), then the lanes are
+// added pairwise through shared memory (deterministic: the order depends only on the chunk count).
+// Latency bound: a thousand candidates have ~460 chunks, so eight lanes per candidate took 31-49 us there
+// (15 rounds of loads); 32 lanes take 16 us, and 4,096 x 286 chunks 10 instead of 20 us.
+constexpr int REDUCE_LANES = 32, REDUCE_CANDS = 8;
+__global__ void __launch_bounds__(REDUCE_LANES *REDUCE_CANDS)
+fast_reduce_kernel(const FastGroup *groups, int n_groups, const double *partial, int64_t P, double *val, double *dd,
+                   double *dk) {
+    __shared__ double red[3][REDUCE_LANES][REDUCE_CANDS];
+    const int q = threadIdx.x & (REDUCE_CANDS - 1), r = threadIdx.x / REDUCE_CANDS;
+    const int64_t p = (int64_t)blockIdx.x * REDUCE_CANDS + q;
     const bool live = p < P;
     double s0 = 0, s1 = 0, s2 = 0;
     if (live) {
@@ -436,27 +438,36 @@ __global__ void fast_reduce_kernel(const FastGroup *groups, int n_groups, const 
 #pragma unroll
             for (int u = 0; u < 4; ++u)
 #pragma unroll
-                for (int q = 0; q < 3; ++q) x[u][q] = o[u * REDUCE_LANES * stride + q];
+                for (int i = 0; i < 3; ++i) x[u][i] = o[u * REDUCE_LANES * stride + i];
             s0 += (x[0][0] + x[1][0]) + (x[2][0] + x[3][0]);
             s1 += (x[0][1] + x[1][1]) + (x[2][1] + x[3][1]);
             s2 += (x[0][2] + x[1][2]) + (x[2][2] + x[3][2]);
         }
-        for (; ch < gr.n_chunks; ch += REDUCE_LANES, o += REDUCE_LANES * stride) {
-            s0 += o[0]; s1 += o[1]; s2 += o[2];
-        }
+        double x[3][3];
+#pragma unroll
+        for (int u = 0; u < 3; ++u)
+#pragma unroll
+            for (int i = 0; i < 3; ++i) x[u][i] = ch + u * REDUCE_LANES < gr.n_chunks ? o[u * REDUCE_LANES * stride + i] : 0.0;
+        s0 += (x[0][0] + x[1][0]) + x[2][0];
+        s1 += (x[0][1] + x[1][1]) + x[2][1];
+        s2 += (x[0][2] + x[1][2]) + x[2][2];
     }
-    for (int off = 16; off >= 4; off >>= 1) {
-        s0 += __shfl_xor_sync(0xffffffffu, s0, off);
-        s1 += __shfl_xor_sync(0xffffffffu, s1, off);
-        s2 += __shfl_xor_sync(0xffffffffu, s2, off);
+    red[0][r][q] = s0;
+    red[1][r][q] = s1;
+    red[2][r][q] = s2;
+    for (int h = REDUCE_LANES / 2; h > 0; h >>= 1) {
+        __syncthreads();
+        if (r < h)
+#pragma unroll
+            for (int i = 0; i < 3; ++i) red[i][r][q] += red[i][r + h][q];
     }
     if (live && r == 0) {
-        val[p] = s0;
-        dd[p] = s1;
-        dk[p] = s2;
+        val[p] = red[0][0][q];
+        dd[p] = red[1][0][q];
+        dk[p] = red[2][0][q];
     }
 }
-static unsigned reduce_blocks(int64_t P) { return (unsigned)(((P + 3) / 4 * 32 + 255) / 256); }
+static unsigned reduce_blocks(int64_t P) { return (unsigned)((P + REDUCE_CANDS - 1) / REDUCE_CANDS); }
 
 static int launch_light(const TabView &tv, const FastPlanDev &pd, CandView c, cudaStream_t s) {
     if (pd.n_light == 0) return MB_OK;
@@ -557,7 +568,7 @@ int launch_fast(const Table &t, const FastPlanDev &pd, CandView c, double *d_val
         if (ev) MB_CUDA(cudaEventRecord(ev->light0, s));
         MB_TRY(launch_tiers_one(tv, pd, c, s));
         if (ev) MB_CUDA(cudaEventRecord(ev->light1, s));
-        fast_reduce_kernel<<<reduce_blocks(c.P), 256, 0, s>>>(pd.groups, pd.n_groups, pd.partial, c.P,
+        fast_reduce_kernel<<<reduce_blocks(c.P), REDUCE_LANES * REDUCE_CANDS, 0, s>>>(pd.groups, pd.n_groups, pd.partial, c.P,
                                                                          d_val, d_dd, d_dk);
         MB_CUDA(cudaGetLastError());
         return MB_OK;
@@ -587,7 +598,7 @@ int launch_fast(const Table &t, const FastPlanDev &pd, CandView c, double *d_val
         if (ev) MB_CUDA(cudaEventRecord(ev->light1, s));
     }
     if (fork) MB_CUDA(cudaStreamWaitEvent(s, t.ev_join, 0));
-    fast_reduce_kernel<<<reduce_blocks(c.P), 256, 0, s>>>(pd.groups, pd.n_groups, pd.partial, c.P,
+    fast_reduce_kernel<<<reduce_blocks(c.P), REDUCE_LANES * REDUCE_CANDS, 0, s>>>(pd.groups, pd.n_groups, pd.partial, c.P,
                                                                      d_val, d_dd, d_dk);
     MB_CUDA(cudaGetLastError());
     return MB_OK;
