@@ -277,6 +277,17 @@ int mb_grid_scan(mb_table *t, int64_t P, const uint64_t *v_int, const uint64_t *
 int mb_hit_scan(mb_table *t, int64_t P, const uint64_t *v_int, const uint64_t *v_frac, double k, int64_t n_use,
                 uint64_t step_int, uint64_t step_frac, int64_t m0, int64_t n_m, double *out_h);
 
+/* The enumerators' staged hit polish (search/gpu_mertens_stream.cu:381-505 ZeroData::polish,
+ * search/fast_mertens_enum.cpp:145-276) for P hits: stage s scans the m_half[s] points on either side
+ * of the hit (of the stage before's best point where recentre[s]) at the 64.64 step steps[2s] +
+ * steps[2s+1] 2^-64 over the first min(zeros[s], n) zeros, as mb_hit_scan, and moves the hit's offset to the
+ * first point of largest |h|; out_h takes that h where keep_h[s]; a hit goes on to the next stage if
+ * |h| >= threshold[s] (-inf keeps all).  out_dy: the last offset, out_stage: the last stage run.
+ * 2 m_half[s] + 1 <= 1024. */
+int mb_hit_polish(mb_table *t, int64_t P, const uint64_t *v_int, const uint64_t *v_frac, double k, int n_stages,
+                  const int64_t *zeros, const int64_t *m_half, const uint64_t *steps, const int *recentre,
+                  const int *keep_h, const double *threshold, double *out_h, double *out_dy, int64_t *out_stage);
+
 /* Staged leaf screen of the lattice enumerators: for each leaf v_p (64.64) and m = -3..3,
  * S_m = sum_j 2|c_j| e^{-k gamma_j^2} cos(2 pi frac((v_p + m step) G_j) + arg c_j) over the first
  * stage_end[s] zeros; a leaf passes stage s if max_m |S_m| >= threshold[s] and is a hit if it

@@ -64,6 +64,7 @@ SIGNATURES: dict[str, tuple] = {
     "mb_k2_certified_grad_range": (i32, [vp, i64, vp, vp, vp, f64, f64, i64, i64, vp, vp, vp]),
     "mb_grid_scan": (i32, [vp, i64, vp, vp, f64, f64, C.c_uint64, C.c_uint64, i64, i64, vp]),
     "mb_hit_scan": (i32, [vp, i64, vp, vp, f64, i64, C.c_uint64, C.c_uint64, i64, i64, vp]),
+    "mb_hit_polish": (i32, [vp, i64, vp, vp, f64, i32, vp, vp, vp, vp, vp, vp, vp, vp, vp]),
     "mb_exact_AB": (i32, [vp, i64, vp, vp, vp, i64, vp, vp]),
     "mb_polish_single_peak": (i32, [i64, i64, i64, vp, vp, vp, vp, f64, i32, vp, vp, vp]),
     "mb_fast_polish_batch": (i32, [i64, i64, vp, vp, vp, vp, vp, i64, i32, vp, vp, vp]),

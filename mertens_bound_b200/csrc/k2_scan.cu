@@ -317,9 +317,11 @@ bool scan_in_range(int64_t P, const uint64_t *vi, const uint64_t *vf, u128 step,
     return true;
 }
 
-// The scan of P base points on cell moments, results in out_h (host).
+// The scan of P base points on cell moments; take(p0, np, d_h) queues what is done with the results of the
+// base points [p0, p0 + np) (device, np x n_m) on t.stream.
+template <typename Take>
 int scan_cells(Table &t, int64_t P, const uint64_t *v_int, const uint64_t *v_frac, double k, uint64_t step_int,
-               uint64_t step_frac, int64_t m0, int64_t n_m, const ScanPlan &sp, double *out_h) {
+               uint64_t step_frac, int64_t m0, int64_t n_m, const ScanPlan &sp, Take take) {
     const u128 step = (u128)step_int << 64 | step_frac;
     const int64_t per = sp.chunk * sp.NB;
     const size_t pb = (size_t)per * 8, cb = cells_bytes(sp.cp);
@@ -347,10 +349,47 @@ int scan_cells(Table &t, int64_t P, const uint64_t *v_int, const uint64_t *v_fra
         MB_CUDA(cudaMemcpyAsync(d_v, pts.data(), 2 * (size_t)nb * 8, cudaMemcpyHostToDevice, t.stream));
         MB_TRY(launch_moments_gauss(t, cells, d_v, d_v + nb, nb, k, sp.d1, M, t.stream));
         MB_TRY(launch_cell_scan(cells, sp.d1, M, np, sp.NB, sp.Bp, n_m, step_int, step_frac, d_h, t.stream));
-        MB_CUDA(cudaMemcpyAsync(out_h + p0 * n_m, d_h, (size_t)np * n_m * 8, cudaMemcpyDeviceToHost, t.stream));
+        MB_TRY(take(p0, np, (const double *)d_h));
     }
-    MB_CUDA(cudaStreamSynchronize(t.stream));
     return MB_OK;
+}
+
+// The first point of largest |h| of each base point's grid.
+struct HitBest {
+    double h;
+    int64_t m;
+};
+__global__ void __launch_bounds__(128) hit_best_kernel(const double *h, int n_m, HitBest *best) {
+    __shared__ double sv[4];
+    __shared__ int si[4];
+    const double *row = h + (int64_t)blockIdx.x * n_m;
+    double bv = -1.0;
+    int bi = n_m;
+    for (int m = threadIdx.x; m < n_m; m += 128)
+        if (fabs(row[m]) > bv) {
+            bv = fabs(row[m]);
+            bi = m;
+        }
+    auto take = [&](double v, int i) {
+        if (v > bv || (v == bv && i < bi)) {
+            bv = v;
+            bi = i;
+        }
+    };
+    for (int o = 16; o > 0; o >>= 1) {
+        const double v = __shfl_xor_sync(0xffffffffu, bv, o);
+        take(v, __shfl_xor_sync(0xffffffffu, bi, o));
+    }
+    if ((threadIdx.x & 31) == 0) {
+        sv[threadIdx.x >> 5] = bv;
+        si[threadIdx.x >> 5] = bi;
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        for (int w = 1; w < 4; ++w) take(sv[w], si[w]);
+        if (bi >= n_m) bi = 0;
+        best[blockIdx.x] = HitBest{row[bi], bi};
+    }
 }
 
 // Warp cycles of the direct kernels per 32 (point, zero) pairs, from their measured times (25,001 points x
@@ -361,6 +400,17 @@ constexpr double GRID_CYCLES = 20.0, HIT_CYCLES = 34.0;
 }  // namespace mb
 
 using namespace mb;
+
+// Copies a scan's results to the host.
+struct ToHost {
+    double *out;
+    int64_t n_m;
+    cudaStream_t s;
+    int operator()(int64_t p0, int64_t np, const double *d_h) const {
+        MB_CUDA(cudaMemcpyAsync(out + p0 * n_m, d_h, (size_t)np * n_m * 8, cudaMemcpyDeviceToHost, s));
+        return MB_OK;
+    }
+};
 
 extern "C" int mb_grid_scan(mb_table *h, int64_t P, const uint64_t *v_int, const uint64_t *v_frac, double k,
                             double T, uint64_t step_int, uint64_t step_frac, int64_t m0, int64_t n_m, double *out_h) {
@@ -377,7 +427,11 @@ extern "C" int mb_grid_scan(mb_table *h, int64_t P, const uint64_t *v_int, const
     const int64_t grid_points = (n_m + SCAN_THREADS * SCAN_MPT - 1) / (SCAN_THREADS * SCAN_MPT) * (SCAN_THREADS * SCAN_MPT);
     if (plan_scan(t, P, n_use, n_m, step_int, step_frac, GRID_CYCLES, grid_points, sp) &&
         scan_in_range(P, v_int, v_frac, (u128)step_int << 64 | step_frac, m0, (int64_t)sp.NB * sp.Bp))
-        return scan_cells(t, P, v_int, v_frac, k, step_int, step_frac, m0, n_m, sp, out_h);
+        {
+        MB_TRY(scan_cells(t, P, v_int, v_frac, k, step_int, step_frac, m0, n_m, sp, ToHost{out_h, n_m, t.stream}));
+        MB_CUDA(cudaStreamSynchronize(t.stream));
+        return MB_OK;
+    }
     const size_t cb = (size_t)P * 8, hb = (size_t)P * n_m * 8;
     int sms = 148;
     MB_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, t.device));
@@ -412,22 +466,14 @@ extern "C" int mb_grid_scan(mb_table *h, int64_t P, const uint64_t *v_int, const
     return MB_OK;
 }
 
-extern "C" int mb_hit_scan(mb_table *h, int64_t P, const uint64_t *v_int, const uint64_t *v_frac, double k,
-                           int64_t n_use, uint64_t step_int, uint64_t step_frac, int64_t m0, int64_t n_m,
-                           double *out_h) {
-    MB_CHECK_ARG(h && v_int && v_frac && out_h, "mb_hit_scan: null argument");
-    MB_CHECK_ARG(P >= 0 && P <= (1 << 24), "mb_hit_scan: P=%lld", (long long)P);
-    MB_CHECK_ARG(n_m >= 1 && n_m <= HIT_MAX_M, "mb_hit_scan: n_m=%lld (1..%d)", (long long)n_m, HIT_MAX_M);
-    MB_CHECK_ARG(m0 > -((int64_t)1 << 31) && m0 + n_m < ((int64_t)1 << 31), "mb_hit_scan: grid indices exceed 2^31");
-    MB_CHECK_ARG(std::isfinite(k) && k >= 0.0, "mb_hit_scan: k=%g", k);
-    if (P == 0) return MB_OK;
-    Table &t = table_of(h);
-    MB_CHECK_ARG(n_use >= 0 && n_use <= t.n, "mb_hit_scan: n_use=%lld of %lld", (long long)n_use, (long long)t.n);
-    MB_TRY(device_guard(t.device));
+// The scan of mb_hit_scan by whichever way is the cheaper, its results handed to take (see scan_cells).
+template <typename Take>
+static int hit_scan(Table &t, int64_t P, const uint64_t *v_int, const uint64_t *v_frac, double k, int64_t n_use,
+                    uint64_t step_int, uint64_t step_frac, int64_t m0, int64_t n_m, Take take) {
     ScanPlan sp;
     if (plan_scan(t, P, n_use, n_m, step_int, step_frac, HIT_CYCLES, (n_m + HIT_MB - 1) / HIT_MB * HIT_MB, sp) &&
         scan_in_range(P, v_int, v_frac, (u128)step_int << 64 | step_frac, m0, (int64_t)sp.NB * sp.Bp))
-        return scan_cells(t, P, v_int, v_frac, k, step_int, step_frac, m0, n_m, sp, out_h);
+        return scan_cells(t, P, v_int, v_frac, k, step_int, step_frac, m0, n_m, sp, take);
     const size_t cb = (size_t)P * 8, hb = (size_t)P * n_m * 8;
     MB_TRY(t.io.ensure(2 * cb + hb + 256));
     char *base = (char *)t.io.p;
@@ -450,7 +496,82 @@ extern "C" int mb_hit_scan(mb_table *h, int64_t P, const uint64_t *v_int, const 
     MB_CUDA(cudaGetLastError());
     hit_reduce_kernel<<<(unsigned)((P * n_m + 255) / 256), 256, 0, t.stream>>>(partial, P, n_split, (int)n_m, d_h);
     MB_CUDA(cudaGetLastError());
-    MB_CUDA(cudaMemcpyAsync(out_h, d_h, hb, cudaMemcpyDeviceToHost, t.stream));
+    return take((int64_t)0, P, (const double *)d_h);
+}
+
+extern "C" int mb_hit_scan(mb_table *h, int64_t P, const uint64_t *v_int, const uint64_t *v_frac, double k,
+                           int64_t n_use, uint64_t step_int, uint64_t step_frac, int64_t m0, int64_t n_m,
+                           double *out_h) {
+    MB_CHECK_ARG(h && v_int && v_frac && out_h, "mb_hit_scan: null argument");
+    MB_CHECK_ARG(P >= 0 && P <= (1 << 24), "mb_hit_scan: P=%lld", (long long)P);
+    MB_CHECK_ARG(n_m >= 1 && n_m <= HIT_MAX_M, "mb_hit_scan: n_m=%lld (1..%d)", (long long)n_m, HIT_MAX_M);
+    MB_CHECK_ARG(m0 > -((int64_t)1 << 31) && m0 + n_m < ((int64_t)1 << 31), "mb_hit_scan: grid indices exceed 2^31");
+    MB_CHECK_ARG(std::isfinite(k) && k >= 0.0, "mb_hit_scan: k=%g", k);
+    if (P == 0) return MB_OK;
+    Table &t = table_of(h);
+    MB_CHECK_ARG(n_use >= 0 && n_use <= t.n, "mb_hit_scan: n_use=%lld of %lld", (long long)n_use, (long long)t.n);
+    MB_TRY(device_guard(t.device));
+    MB_TRY(hit_scan(t, P, v_int, v_frac, k, n_use, step_int, step_frac, m0, n_m, ToHost{out_h, n_m, t.stream}));
     MB_CUDA(cudaStreamSynchronize(t.stream));
+    return MB_OK;
+}
+
+extern "C" int mb_hit_polish(mb_table *h, int64_t P, const uint64_t *v_int, const uint64_t *v_frac, double k,
+                             int n_stages, const int64_t *zeros, const int64_t *m_half, const uint64_t *steps,
+                             const int *recentre, const int *keep_h, const double *threshold, double *out_h,
+                             double *out_dy, int64_t *out_stage) {
+    const char *who = "mb_hit_polish";
+    MB_CHECK_ARG(h && zeros && m_half && steps && recentre && keep_h && threshold, "%s: null argument", who);
+    MB_CHECK_ARG(P >= 0 && P <= (1 << 24), "%s: P=%lld", who, (long long)P);
+    MB_CHECK_ARG(n_stages >= 1 && n_stages <= 64, "%s: n_stages=%d", who, n_stages);
+    MB_CHECK_ARG(std::isfinite(k) && k >= 0.0, "%s: k=%g", who, k);
+    Table &t = table_of(h);
+    for (int s = 0; s < n_stages; ++s)
+        MB_CHECK_ARG(zeros[s] >= 0 && m_half[s] >= 0 && 2 * m_half[s] + 1 <= HIT_MAX_M, "%s: stage %d", who, s);
+    if (P == 0) return MB_OK;
+    MB_CHECK_ARG(v_int && v_frac && out_h && out_dy && out_stage, "%s: null array", who);
+    MB_TRY(device_guard(t.device));
+    typedef __int128 i128;
+    std::vector<i128> centre(P, 0);
+    std::vector<int64_t> alive(P);
+    for (int64_t p = 0; p < P; ++p) {
+        alive[p] = p;
+        out_h[p] = out_dy[p] = 0.0;
+        out_stage[p] = 0;
+    }
+    std::vector<uint64_t> vi(P), vf(P);
+    std::vector<HitBest> best(P);
+    MB_TRY(t.redo.ensure((size_t)P * sizeof(HitBest)));
+    HitBest *d_best = (HitBest *)t.redo.p;
+    for (int s = 0; s < n_stages && !alive.empty(); ++s) {
+        const int64_t na = (int64_t)alive.size(), n_m = 2 * m_half[s] + 1;
+        for (int64_t i = 0; i < na; ++i) {
+            u128 v = (u128)v_int[alive[i]] << 64 | v_frac[alive[i]];
+            if (recentre[s]) v += (u128)centre[alive[i]];
+            vi[i] = (uint64_t)(v >> 64);
+            vf[i] = (uint64_t)v;
+        }
+        auto take = [&](int64_t p0, int64_t np, const double *d_h) {
+            hit_best_kernel<<<(unsigned)np, 128, 0, t.stream>>>(d_h, (int)n_m, d_best + p0);
+            MB_CUDA(cudaGetLastError());
+            return MB_OK;
+        };
+        MB_TRY(hit_scan(t, na, vi.data(), vf.data(), k, std::min(zeros[s], t.n), steps[2 * s], steps[2 * s + 1],
+                        -m_half[s], n_m, take));
+        MB_CUDA(cudaMemcpyAsync(best.data(), d_best, (size_t)na * sizeof(HitBest), cudaMemcpyDeviceToHost, t.stream));
+        MB_CUDA(cudaStreamSynchronize(t.stream));
+        const i128 step = (i128)((u128)steps[2 * s] << 64 | steps[2 * s + 1]);
+        int64_t kept = 0;
+        for (int64_t i = 0; i < na; ++i) {
+            const int64_t p = alive[i];
+            const i128 c = (recentre[s] ? centre[p] : 0) + (i128)(best[i].m - m_half[s]) * step;
+            out_stage[p] = s;
+            if (keep_h[s]) out_h[p] = best[i].h;
+            centre[p] = c;
+            out_dy[p] = (double)c * 0x1p-64;
+            if (std::fabs(best[i].h) >= threshold[s]) alive[kept++] = p;
+        }
+        alive.resize(kept);
+    }
     return MB_OK;
 }

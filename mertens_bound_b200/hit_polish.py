@@ -12,8 +12,8 @@ FP64 grid scans of h(y) = sum_j two_astar_j cos(theta_j + gamma_j dy), two_astar
   3      15000   m in [-320, 320]      2.5e-6   stage-2 best     (moves the centre only)
   4      all     m in [-120, 120]      5e-7     stage-3 best     returns (h, dy)
 
-Here each stage is one mb_hit_scan call over all hits still alive (one CTA per hit), with
-exact phases at every grid point; hits are x = floor(y 2^30) as in the reference
+Here the stages are one mb_hit_polish call over all hits (each stage a scan of those still alive, the
+best points found on the device); hits are x = floor(y 2^30) as in the reference
 (gpu_mertens_stream.cu:711) or 64.64 points.
 """
 from __future__ import annotations
@@ -60,48 +60,25 @@ def points_from_x(x) -> np.ndarray:
     return out
 
 
-def _scan(table, pts_fixed, k, n_use, step_fixed, m_half):
-    P = len(pts_fixed)
-    vi = np.array([p >> 64 for p in pts_fixed], dtype=np.uint64)
-    vf = np.array([p & MASK64 for p in pts_fixed], dtype=np.uint64)
-    n_m = 2 * m_half + 1
-    h = np.empty((P, n_m))
-    check(lib().mb_hit_scan(table.handle, P, ptr(vi), ptr(vf), float(k), int(n_use), step_fixed >> 64,
-                            step_fixed & MASK64, -m_half, n_m, ptr(h)))
-    return h
-
-
 def polish_hits(table: k2.ZeroTable, points: np.ndarray, k: float = 3e-9, thresholds=None) -> HitResult:
     """Run the staged polish for every hit (points: (n, 2) u64 v_int, v_frac)."""
     thr = [s[4] for s in STAGES[:3]] if thresholds is None else list(thresholds)
     n = len(points)
-    base = [(int(points[i, 0]) << 64) | int(points[i, 1]) for i in range(n)]
-    centre = [0] * n                       # fixed-point offset of the current centre
-    best_h = np.zeros(n)
-    best_dy = np.zeros(n)
-    stage = np.zeros(n, dtype=np.int64)
-    alive = np.arange(n)
-    for s, (K, m_half, step, recentre, _) in enumerate(STAGES):
-        if len(alive) == 0:
-            break
-        n_use = table.n if K is None else min(K, table.n)
-        sf = _fixed(step)
-        pts = [(base[i] + (centre[i] if recentre else 0)) & ((1 << 128) - 1) for i in alive]
-        h = _scan(table, pts, k, n_use, sf, m_half)
-        j = np.argmax(np.abs(h), axis=1)                       # first maximum, like the reference
-        hb = h[np.arange(len(alive)), j]
-        for idx, i in enumerate(alive):
-            off = (int(j[idx]) - m_half) * sf
-            c = (centre[i] if recentre else 0) + off
-            stage[i] = s
-            if s != 3:                                         # stage 3 only moves the centre
-                best_h[i] = hb[idx]
-            centre[i] = c
-            best_dy[i] = float(Fraction(c, 1 << 64))
-        if s < 3 and thr[s] is not None:
-            keep = np.abs(hb) >= thr[s]
-            alive = alive[keep]
-    return HitResult(best_h, best_dy, stage)
+    res = HitResult(np.zeros(n), np.zeros(n), np.zeros(n, dtype=np.int64))
+    if n == 0:
+        return res
+    pts = np.ascontiguousarray(points, dtype=np.uint64)
+    vi, vf = np.ascontiguousarray(pts[:, 0]), np.ascontiguousarray(pts[:, 1])
+    zeros = np.array([table.n if s[0] is None else s[0] for s in STAGES], dtype=np.int64)
+    m_half = np.array([s[1] for s in STAGES], dtype=np.int64)
+    steps = np.array([divmod(_fixed(s[2]), 1 << 64) for s in STAGES], dtype=np.uint64)
+    recentre = np.array([s[3] for s in STAGES], dtype=np.int32)
+    keep_h = np.array([i != 3 for i in range(len(STAGES))], dtype=np.int32)   # stage 3 only moves the centre
+    limit = np.array([-np.inf if t is None else t for t in (thr[:3] + [None] * len(STAGES))[:len(STAGES)]])
+    check(lib().mb_hit_polish(table.handle, n, ptr(vi), ptr(vf), float(k), len(STAGES), ptr(zeros), ptr(m_half),
+                              ptr(steps), ptr(recentre), ptr(keep_h), ptr(limit), ptr(res.h), ptr(res.dy),
+                              ptr(res.stage)))
+    return res
 
 
 # Leaf screens: (zeros at the end of each stage, thresholds) of the reference's proxies.
