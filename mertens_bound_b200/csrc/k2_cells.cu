@@ -18,7 +18,6 @@ namespace mb {
 namespace {
 
 constexpr int CELL_THREADS = 256;
-constexpr int CELL_TILE = 64;                  // zeros staged at a time
 
 // ------------------------------------------------------------------ phasors
 
@@ -39,17 +38,18 @@ MB_DEV void phasor_table_init(double2 *tab, int threads) {
     }
 }
 
-// cos, sin of the phase word w - 2^55 (units of 2^-64 turn; the caller adds 2^55, half a table step):
-// table entry w >> 56 rotated by d 2^-60 turn, d = ((w mod 2^56) >> 4) - 2^51 exact in FP64
-// (|d| <= 2^51, i.e. at most 0.0123 rad; the dropped bits are 5e-18 rad).  With a = 2 pi 2^-60:
+// cos, sin of the phase word w - 2^51 in units of 2^-60 turn (the top four bits of w are ignored; the caller
+// adds 2^51, half a table step): table entry bits [52, 60) of w rotated by d 2^-60 turn,
+// d = (w mod 2^52) - 2^51 exact in FP64 (at most 0.0123 rad).  With a = 2 pi 2^-60:
 //   sin(a d)     = d (a - a^3 d^2 / 6 + a^5 d^4 / 120)            (truncation 8.4e-18)
 //   cos(a d) - 1 = d^2 (-a^2 / 2 + a^4 d^2 / 24 - a^6 d^4 / 720)  (truncation 1.3e-20)
-// so the result carries the table's and the last FMA's roundings only.
-MB_DEV void phasor(uint64_t w, const double2 *tab, double &cs, double &sn) {
+// so the result carries the table's and the last FMA's roundings only.  copy: the lane's copy of the table.
+MB_DEV void phasor(uint64_t w, const double2 *copy, double &cs, double &sn) {
     constexpr double a = 6.283185307179586 * 0x1p-60;
-    const double2 T = tab[(uint32_t)(w >> 56) * PH_COPIES + (threadIdx.x & (PH_COPIES - 1))];
-    const uint64_t rem = (w & 0x00FFFFFFFFFFFFFFull) >> 4;
-    const double d = __longlong_as_double((long long)(rem | 0x4330000000000000ull)) - 6755399441055744.0;
+    const uint32_t hi = (uint32_t)(w >> 32);
+    const double2 T = *reinterpret_cast<const double2 *>(reinterpret_cast<const char *>(copy) +
+                                                         ((hi >> 13) & (uint32_t)((PH_TAB - 1) * PH_COPIES * 16)));
+    const double d = __hiloint2double((int)((hi & 0xFFFFFu) | 0x43300000u), (int)(uint32_t)w) - 6755399441055744.0;
     const double u = d * d;
     const double s = d * fma(u, fma(u, a * a * a * a * a / 120.0, -a * a * a / 6.0), a);
     const double m = u * fma(u, fma(u, -a * a * a * a * a * a / 720.0, a * a * a * a / 24.0), -a * a / 2.0);
@@ -68,14 +68,27 @@ MB_DEV uint64_t wide_add(uint32_t a, uint32_t b, uint64_t c) {
     return r;
 }
 
+// A zero for the phase in units of 2^-60 turn: the limbs of G 2^124 (G 2^128 shifted down four bits, so the
+// phase's fraction is where phasor() wants it), and arg(c) / 2pi 2^60 + 2^51 (half a table step).
 struct ZRec {                   // 32 B
     uint32_t g0, g1, g2, g3, g4, pad;
-    uint64_t psi;               // arg(c) / 2pi 2^64 + 2^55 (half a table step of phasor())
+    uint64_t psi;
 };
+MB_DEV ZRec zrec(uint32_t g0, uint32_t g1, uint32_t g2, uint32_t g3, uint32_t g4, uint64_t psi) {
+    ZRec r;
+    r.g0 = __funnelshift_r(g0, g1, 4);
+    r.g1 = __funnelshift_r(g1, g2, 4);
+    r.g2 = __funnelshift_r(g2, g3, 4);
+    r.g3 = __funnelshift_r(g3, g4, 4);
+    r.g4 = g4 >> 4;
+    r.pad = 0;
+    r.psi = (psi >> 4) + (1ull << 51);
+    return r;
+}
 
-// floor(frac(v G) 2^64) less at most 7 units of 2^-64 turn (the carries out of the columns below
-// 2^-64), plus psi: columns 4 and 5 of phase128_exact and the high halves of column 3.
-MB_DEV uint64_t phase64(uint32_t v0, uint32_t v1, uint32_t v2, uint32_t v3, const ZRec &z) {
+// floor(frac(v G) 2^60) less at most 7 units of 2^-60 turn (4e-17 rad: the carries out of the columns below),
+// plus psi: columns 4 and 5 of phase128_exact and the high halves of column 3.
+MB_DEV uint64_t phase60(uint32_t v0, uint32_t v1, uint32_t v2, uint32_t v3, const ZRec &z) {
     const uint64_t h3 = (wide(v0, z.g3) >> 32) + (wide(v1, z.g2) >> 32) + (wide(v2, z.g1) >> 32) + (wide(v3, z.g0) >> 32);
     const uint32_t top = v1 * z.g4 + v2 * z.g3 + v3 * z.g2;
     uint64_t acc = wide_add(v0, z.g4, z.psi + h3);
@@ -98,24 +111,35 @@ struct CellGroups {
     int nc[2];
 };
 
-__global__ void cells_kernel(TabView t, CellGroups g, int n, int64_t half, int *j0, int *j1, int64_t *ctr) {
-    const int c = blockIdx.x * blockDim.x + threadIdx.x;
-    if (c >= n) return;
-    const int q = c < g.nc[0] ? 0 : 1, l = q ? c - g.nc[0] : c;
-    // the first zero of the group at or above an edge (G in units of 2^-16, rounded down)
-    auto first = [&](int64_t edge) {
-        int64_t lo = g.a[q], hi = g.b[q];
-        while (lo < hi) {
-            const int64_t mid = (lo + hi) >> 1;
-            if (((int64_t)t.g4[mid] << 16 | t.g3[mid] >> 16) < edge) lo = mid + 1;
-            else hi = mid;
+// One warp per cell edge: a 32-way search of the group's zeros (four or five loads deep instead of the ~20
+// of a binary search: 17 -> 5 us on 600,000 zeros).  Edge i of a group ends its cell i - 1 and starts cell i.
+__global__ void cells_kernel(TabView t, CellGroups g, int64_t half, int *j0, int *j1, int64_t *ctr) {
+    const int lane = threadIdx.x & 31;
+    const int w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    const int q = w <= g.nc[0] ? 0 : 1, i = q ? w - g.nc[0] - 1 : w;      // nc + 1 edges each
+    if (i > g.nc[q] || (q && g.nc[1] == 0)) return;
+    const int64_t edge = g.e0[q] + 2 * half * i;
+    // the first zero of the group at or above the edge (G in units of 2^-16, rounded down)
+    int64_t lo = g.a[q], hi = g.b[q];
+    if (i == 0) hi = lo;
+    else if (i == g.nc[q]) lo = hi;
+    while (lo < hi) {
+        // 32 probes split [lo, hi) in 33 parts: the zeros below the edge are a prefix of the probes
+        const int64_t m = lo + (hi - lo) * (lane + 1) / 33;
+        const bool below = m < hi && ((int64_t)t.g4[m] << 16 | t.g3[m] >> 16) < edge;
+        const int n = __popc(__ballot_sync(0xffffffffu, below));
+        const int64_t nlo = n == 0 ? lo : lo + (hi - lo) * n / 33 + 1;
+        hi = n == 32 ? hi : lo + (hi - lo) * (n + 1) / 33;
+        lo = nlo;
+    }
+    if (lane == 0) {
+        const int c = q ? g.nc[0] + i : i;
+        if (i < g.nc[q]) {
+            j0[c] = (int)lo;
+            ctr[c] = edge + half;
         }
-        return lo;
-    };
-    const int64_t e = g.e0[q] + 2 * half * l;
-    j0[c] = (int)(l == 0 ? g.a[q] : first(e));
-    j1[c] = (int)(l == g.nc[q] - 1 ? g.b[q] : first(e + 2 * half));
-    ctr[c] = e + half;
+        if (i > 0) j1[c - 1] = (int)lo;
+    }
 }
 
 // n chunks of the zeros [0, n_zeros) as cells (the power sums need no centre).  Their lengths grow with
@@ -147,7 +171,12 @@ struct CellShape {
     static constexpr int NTI = NT - I0;
     // row stride in doubles = 4 mod 8: the 4 x 8 B fragment's half warps touch 16 distinct banks
     static constexpr int S = cols + 4;
-    static constexpr int smem = PH_BYTES + CELL_TILE * (int)sizeof(ZRec) + CELL_TILE * S * 8;
+    // a tile is TILE zeros x PARTS threads: a weight vector's D1 columns each, or four column groups
+    static constexpr int PARTS = KIND == CELL_WEIGHTS ? W : 4;
+    static constexpr int TILE = KIND == CELL_WEIGHTS && W == 5 ? 48 : 64;
+    static_assert(TILE * PARTS <= CELL_THREADS, "one (zero, part) per thread");
+    static constexpr int ctas = KIND == CELL_WEIGHTS ? 2 : 3;       // resident per SM
+    static constexpr int smem = PH_BYTES + 2 * TILE * ((int)sizeof(ZRec) + S * 8);
     static constexpr int frag = 2 * (NTR + NTI);                   // accumulators per lane
 };
 
@@ -162,167 +191,213 @@ MB_DEV double gamma_excess(double gamma, uint32_t g4, uint32_t g3, uint32_t g2, 
     return (gamma - p) - (pe + fma(P_HI, l, P_LO * h));
 }
 
+// One tile of an item: the zeros [tb, min(tb + TILE, jb)) of a cell for one group of peaks.
+struct CellTile {
+    int item, cell, pt;
+    uint32_t tb, jb;
+};
+
 // One item = one cell x CELL_PEAKS / nzw peaks.  Warp w serves peaks 8 (w / nzw) .. + 7 and the
 // 4-zero steps congruent to w mod nzw; with nzw > 1 the warps' sums are added in warp order.
 // Bound: the FP64 pipe, 16 cycles per mma and scheduler, 2 mma per step and 8 columns, beside ~24 for
-// the phasor; measured with its callers (k2_scan.cu, k2_path1.cu).
+// the phasor (60 instructions).  The next tile's zeros are loaded before the current one is summed and
+// staged after it, into the other half of a double buffer, across items too: one barrier per tile.
 template <int KIND, int W, int D1>
-__global__ void __launch_bounds__(CELL_THREADS, 2)
+__global__ void __launch_bounds__(CELL_THREADS, (CellShape<KIND, W, D1>::ctas))
 cell_moments_kernel(TabView t, const uint64_t *vi, const uint64_t *vf, const double *delta, const int *sel, int64_t P,
                     Cells cells, CellWeights wts, double k, int n_pt, int nzw, int n_items, double *out) {
     using Sh = CellShape<KIND, W, D1>;
+    constexpr int TILE = Sh::TILE;
     extern __shared__ __align__(16) unsigned char smem[];
     double2 *tab = reinterpret_cast<double2 *>(smem);
-    ZRec *rec = reinterpret_cast<ZRec *>(smem + PH_BYTES);
-    double *E = reinterpret_cast<double *>(smem + PH_BYTES + CELL_TILE * sizeof(ZRec));
-    phasor_table_init(tab, CELL_THREADS);
+    ZRec *rec_ = reinterpret_cast<ZRec *>(smem + PH_BYTES);                          // [2][TILE]
+    double *E_ = reinterpret_cast<double *>(smem + PH_BYTES + 2 * TILE * sizeof(ZRec));   // [2][TILE][S]
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int cg = warp / nzw, zw = warp - cg * nzw;
     const int ppc = CELL_PEAKS / nzw;
     const double inv_h = 1.0 / ((double)cells.half * 65536.0);     // units of 2^-32
     const double inv_kappa = 65536.0 / (6.283185307179586 * (double)cells.half);
-    for (int item = blockIdx.x; item < n_items; item += gridDim.x) {
-        const int cell = item / n_pt, pt = item - cell * n_pt;
-        const int64_t pw = (int64_t)pt * ppc + cg * 8;             // the warp's first peak
+    // this thread's part of a tile: zero sz, weight vector or column group sq
+    const int sq = threadIdx.x / TILE, sz = threadIdx.x - sq * TILE;
+    const double2 *copy = tab + (lane & (PH_COPIES - 1));
+    const double *sw = wts.w[0];
+    if constexpr (KIND == CELL_WEIGHTS) {
+#pragma unroll
+        for (int i = 1; i < W; ++i)
+            if (sq == i) sw = wts.w[i];
+    }
+    auto open = [&](int item) {
+        CellTile x;
+        x.item = item;
+        x.cell = item / n_pt;
+        x.pt = item - x.cell * n_pt;
+        x.tb = (uint32_t)cells.j0[x.cell];
+        x.jb = (uint32_t)cells.j1[x.cell];
+        return x;
+    };
+    // the zero's data in registers, then its record and columns into buffer b
+    uint32_t g0, g1, g2, g3, g4;
+    uint64_t psi;
+    double al, gam, wv;
+    auto fetch = [&](const CellTile &x) {
+        const int nt = (int)(x.jb - x.tb);
+        if (sq >= Sh::PARTS || sz >= min(TILE, (nt + 3) & ~3)) return;
+        const int64_t j = (int64_t)x.tb + (sz < nt ? sz : 0);
+        g1 = t.g1[j]; g2 = t.g2[j]; g3 = t.g3[j]; g4 = t.g4[j];
+        if (sq == 0) {
+            g0 = t.g0[j];
+            psi = t.psi[j];
+        }
+        al = sz < nt ? 2.0 * t.alpha[j] : 0.0;
+        gam = t.gamma[j];
+        if constexpr (KIND != CELL_GAUSS) wv = sw[j];
+    };
+    auto stage = [&](const CellTile &x, int b) {
+        const int nt = (int)(x.jb - x.tb);
+        if (sq >= Sh::PARTS || sz >= min(TILE, (nt + 3) & ~3)) return;
+        if (sq == 0) {
+            rec_[b * TILE + sz] = zrec(g0, g1, g2, g3, g4, psi);
+        }
+        double *row = E_ + (b * TILE + sz) * Sh::S;
+        if constexpr (KIND == CELL_POWERS) {
+            const double u = gam * 1.0e-4, u2 = u * u, u4 = u2 * u2, u8 = u4 * u4;
+            const double wa = al * wv;
+            if (sq == 0) {                               // u^0 .. u^8
+                double e = wa;
+#pragma unroll
+                for (int m = 0; m < 5; ++m, e *= u2) row[m] = e;
+            } else if (sq == 1) {                        // u^10 .. u^16, then unused columns
+                double e = wa * (u8 * u2);
+#pragma unroll
+                for (int m = 5; m < 9; ++m, e *= u2) row[m] = e;
+#pragma unroll
+                for (int m = 9; m < 16; ++m) row[m] = 0.0;
+            } else {                                     // u^1 .. u^7, u^9 .. u^15
+                double e = wa * (sq == 2 ? u : u8 * u);
+#pragma unroll
+                for (int m = 0; m < 4; ++m, e *= u2) row[16 + (sq - 2) * 4 + m] = e;
+            }
+        } else {
+            const int64_t df = (int64_t)((uint64_t)g4 << 32 | g3) - (cells.ctr[x.cell] << 16);
+            double y = ((double)df + u32_to_f64(g2) * 0x1p-32) * inv_h;
+            // the polishes' offsets turn by the table's FP64 gamma, not 2 pi G
+            if constexpr (KIND == CELL_WEIGHTS) y += gamma_excess(gam, g4, g3, g2, g1) * inv_kappa;
+            if constexpr (KIND == CELL_GAUSS) {
+                constexpr int C4 = D1 / 4;
+                const double y2 = y * y, y4 = C4 == 2 ? y2 : y2 * y2;
+                double e = al * exp(-k * gam * gam);
+                if (sq & 1) e *= y4;
+                if (sq & 2) e *= y4 * y4;
+#pragma unroll
+                for (int m = 0; m < C4; ++m, e *= y) row[sq * C4 + m] = e;
+            } else {
+                double e = al * wv;
+#pragma unroll
+                for (int m = 0; m < D1; ++m, e *= y) row[sq * D1 + m] = e;
+                if (sq == W - 1)
+#pragma unroll
+                    for (int m = W * D1; m < Sh::cols; ++m) row[m] = 0.0;
+            }
+        }
+    };
+
+    CellTile cur = open(blockIdx.x);                 // the grid is at most n_items CTAs
+    fetch(cur);
+    phasor_table_init(tab, CELL_THREADS);
+    stage(cur, 0);
+    __syncthreads();
+    uint32_t v0 = 0, v1 = 0, v2 = 0, v3 = 0;
+    double aR[Sh::NTR][2], aI[Sh::NTI][2];
+    bool first = true;
+    for (int b = 0;; b ^= 1) {
+        CellTile nxt = cur;
+        nxt.tb += TILE;
+        const bool last = nxt.tb >= cur.jb;          // the item's last tile (an empty cell has one)
+        if (last) {
+            nxt.item += gridDim.x;
+            if (nxt.item < n_items) nxt = open(nxt.item);
+        }
+        const bool more = nxt.item < n_items;
+        if (more) fetch(nxt);
+        const int64_t pw = (int64_t)cur.pt * ppc + cg * 8;             // the warp's first peak
         const int64_t p = pw + (lane >> 2);
-        Cand64 v{0, 0};
-        if (p < P) {
-            const int64_t i = sel ? sel[p] : p;
-            v = fold_delta(vi[i], vf[i], delta ? delta[i] : 0.0);
-        }
-        const uint32_t v0 = (uint32_t)v.vf, v1 = (uint32_t)(v.vf >> 32), v2 = (uint32_t)v.vi, v3 = (uint32_t)(v.vi >> 32);
-        double aR[Sh::NTR][2], aI[Sh::NTI][2];
-#pragma unroll
-        for (int i = 0; i < Sh::NTR; ++i) aR[i][0] = aR[i][1] = 0.0;
-#pragma unroll
-        for (int i = 0; i < Sh::NTI; ++i) aI[i][0] = aI[i][1] = 0.0;
-        const int64_t ja = cells.j0[cell], jb = cells.j1[cell];
-        const int64_t ctr = KIND == CELL_POWERS ? 0 : cells.ctr[cell] << 16;
-        for (int64_t tb = ja; tb < jb; tb += CELL_TILE) {
-            const int nt = (int)min((int64_t)CELL_TILE, jb - tb);
-            const int n4 = (nt + 3) & ~3;
-            __syncthreads();
-            // 64 zeros x parts: a weight vector's D1 columns each, or four column groups
-            constexpr int PARTS = KIND == CELL_WEIGHTS ? W : 4;
-            for (int id = threadIdx.x; id < CELL_TILE * PARTS; id += CELL_THREADS) {
-                const int z = id & (CELL_TILE - 1), q = id / CELL_TILE;
-                if (z >= n4) continue;
-                const bool live = z < nt;
-                const int64_t j = tb + (live ? z : 0);
-                const uint32_t g2 = t.g2[j], g3 = t.g3[j], g4 = t.g4[j];
-                if (q == 0) {
-                    ZRec r;
-                    r.g0 = t.g0[j]; r.g1 = t.g1[j]; r.g2 = g2; r.g3 = g3; r.g4 = g4;
-                    r.pad = 0;
-                    r.psi = t.psi[j] + (1ull << 55);
-                    rec[z] = r;
-                }
-                double *row = E + z * Sh::S;
-                const double al = live ? 2.0 * t.alpha[j] : 0.0;
-                if constexpr (KIND == CELL_POWERS) {
-                    const double u = t.gamma[j] * 1.0e-4, u2 = u * u, u4 = u2 * u2, u8 = u4 * u4;
-                    const double wa = al * wts.w[0][j];
-                    if (q == 0) {                               // u^0 .. u^8
-                        double x = wa;
-#pragma unroll
-                        for (int m = 0; m < 5; ++m, x *= u2) row[m] = x;
-                    } else if (q == 1) {                        // u^10 .. u^16, then unused columns
-                        double x = wa * (u8 * u2);
-#pragma unroll
-                        for (int m = 5; m < 9; ++m, x *= u2) row[m] = x;
-#pragma unroll
-                        for (int m = 9; m < 16; ++m) row[m] = 0.0;
-                    } else {                                    // u^1 .. u^7, u^9 .. u^15
-                        double x = wa * (q == 2 ? u : u8 * u);
-#pragma unroll
-                        for (int m = 0; m < 4; ++m, x *= u2) row[16 + (q - 2) * 4 + m] = x;
-                    }
-                } else {
-                    const int64_t df = (int64_t)((uint64_t)g4 << 32 | g3) - ctr;
-                    double x = ((double)df + u32_to_f64(g2) * 0x1p-32) * inv_h;
-                    // the polishes' offsets turn by the table's FP64 gamma, not 2 pi G
-                    if constexpr (KIND == CELL_WEIGHTS) x += gamma_excess(t.gamma[j], g4, g3, g2, t.g1[j]) * inv_kappa;
-                    if constexpr (KIND == CELL_GAUSS) {
-                        constexpr int C4 = D1 / 4;
-                        const double g = t.gamma[j];
-                        const double x2 = x * x, x4 = C4 == 2 ? x2 : x2 * x2;
-                        double e = al * exp(-k * g * g);
-                        if (q & 1) e *= x4;
-                        if (q & 2) e *= x4 * x4;
-#pragma unroll
-                        for (int m = 0; m < C4; ++m, e *= x) row[q * C4 + m] = e;
-                    } else {
-                        double e = al * wts.w[q][j];
-#pragma unroll
-                        for (int m = 0; m < D1; ++m, e *= x) row[q * D1 + m] = e;
-                        if (q == W - 1)
-#pragma unroll
-                            for (int m = W * D1; m < Sh::cols; ++m) row[m] = 0.0;
-                    }
-                }
+        if (first) {
+            Cand64 v{0, 0};
+            if (p < P) {
+                const int64_t i = sel ? sel[p] : p;
+                v = fold_delta(vi[i], vf[i], delta ? delta[i] : 0.0);
             }
-            __syncthreads();
-            if (pw < P) {
-                const int n_step = n4 >> 2;
+            v0 = (uint32_t)v.vf; v1 = (uint32_t)(v.vf >> 32); v2 = (uint32_t)v.vi; v3 = (uint32_t)(v.vi >> 32);
+#pragma unroll
+            for (int i = 0; i < Sh::NTR; ++i) aR[i][0] = aR[i][1] = 0.0;
+#pragma unroll
+            for (int i = 0; i < Sh::NTI; ++i) aI[i][0] = aI[i][1] = 0.0;
+        }
+        if (pw < P) {
+            const int n_step = (min(TILE, (int)(cur.jb - cur.tb)) + 3) >> 2;
+            const ZRec *rp = rec_ + b * TILE + zw * 4 + (lane & 3);
+            const double *bp = E_ + (b * TILE + zw * 4 + (lane & 3)) * Sh::S + (lane >> 2);
+            const int dr = nzw * 4, de = dr * Sh::S;
 #pragma unroll 2
-                for (int st = zw; st < n_step; st += nzw) {
-                    const int z = st * 4 + (lane & 3);
-                    double cs, sn;
-                    phasor(phase64(v0, v1, v2, v3, rec[z]), tab, cs, sn);
-                    const double *b = E + z * Sh::S + (lane >> 2);
+            for (int st = zw; st < n_step; st += nzw, rp += dr, bp += de) {
+                double cs, sn;
+                phasor(phase60(v0, v1, v2, v3, *rp), copy, cs, sn);
 #pragma unroll
-                    for (int i = 0; i < Sh::NT; ++i) {
-                        const double bv = b[i * 8];
-                        if (i < Sh::NTR) dmma(aR[i], cs, bv);
-                        if (i >= Sh::I0) dmma(aI[i - Sh::I0], sn, bv);
-                    }
+                for (int i = 0; i < Sh::NT; ++i) {
+                    const double bv = bp[i * 8];
+                    if (i < Sh::NTR) dmma(aR[i], cs, bv);
+                    if (i >= Sh::I0) dmma(aI[i - Sh::I0], sn, bv);
                 }
             }
         }
-        if (nzw > 1) {                     // add the other warps' sums of this peak group, in order
-            double *buf = E + cg * 32 * Sh::frag;
-            for (int w = 1; w < nzw; ++w) {
-                __syncthreads();
-                if (zw == w) {
+        if (last) {
+            if (nzw > 1) {                     // add the other warps' sums of this peak group, in order
+                double *buf = E_ + b * TILE * Sh::S + cg * 32 * Sh::frag;
+                for (int w = 1; w < nzw; ++w) {
+                    __syncthreads();
+                    if (zw == w) {
 #pragma unroll
-                    for (int i = 0; i < 2 * Sh::NTR; ++i) buf[i * 32 + lane] = aR[i >> 1][i & 1];
+                        for (int i = 0; i < 2 * Sh::NTR; ++i) buf[i * 32 + lane] = aR[i >> 1][i & 1];
 #pragma unroll
-                    for (int i = 0; i < 2 * Sh::NTI; ++i) buf[(2 * Sh::NTR + i) * 32 + lane] = aI[i >> 1][i & 1];
-                }
-                __syncthreads();
-                if (zw == 0) {
+                        for (int i = 0; i < 2 * Sh::NTI; ++i) buf[(2 * Sh::NTR + i) * 32 + lane] = aI[i >> 1][i & 1];
+                    }
+                    __syncthreads();
+                    if (zw == 0) {
 #pragma unroll
-                    for (int i = 0; i < 2 * Sh::NTR; ++i) aR[i >> 1][i & 1] += buf[i * 32 + lane];
+                        for (int i = 0; i < 2 * Sh::NTR; ++i) aR[i >> 1][i & 1] += buf[i * 32 + lane];
 #pragma unroll
-                    for (int i = 0; i < 2 * Sh::NTI; ++i) aI[i >> 1][i & 1] += buf[(2 * Sh::NTR + i) * 32 + lane];
-                }
-            }
-        }
-        if (zw == 0 && p < P) {            // C fragment: row = peak, columns 2 (lane mod 4) + {0, 1}
-#pragma unroll
-            for (int i = 0; i < Sh::NT; ++i)
-#pragma unroll
-                for (int e = 0; e < 2; ++e) {
-                    const int col = i * 8 + (lane & 3) * 2 + e;
-                    if constexpr (KIND == CELL_POWERS) {
-                        out[(p * cells.n + cell) * 24 + col] = i < Sh::NTR ? aR[i < Sh::NTR ? i : 0][e]
-                                                                           : aI[i < Sh::NTR ? 0 : i - Sh::I0][e];
-                    } else if (col < W * D1) {
-                        const int w = col / D1, m = col - w * D1;
-                        double *o = out + (((int64_t)w * P + p) * cells.n + cell) * (2 * D1) + m;
-                        o[0] = aR[i < Sh::NTR ? i : 0][e];
-                        o[D1] = aI[i - Sh::I0 >= 0 ? i - Sh::I0 : 0][e];
+                        for (int i = 0; i < 2 * Sh::NTI; ++i) aI[i >> 1][i & 1] += buf[(2 * Sh::NTR + i) * 32 + lane];
                     }
                 }
+            }
+            if (zw == 0 && p < P) {            // C fragment: row = peak, columns 2 (lane mod 4) + {0, 1}
+#pragma unroll
+                for (int i = 0; i < Sh::NT; ++i)
+#pragma unroll
+                    for (int e = 0; e < 2; ++e) {
+                        const int col = i * 8 + (lane & 3) * 2 + e;
+                        if constexpr (KIND == CELL_POWERS) {
+                            out[(p * cells.n + cur.cell) * 24 + col] = i < Sh::NTR ? aR[i < Sh::NTR ? i : 0][e]
+                                                                                   : aI[i < Sh::NTR ? 0 : i - Sh::I0][e];
+                        } else if (col < W * D1) {
+                            const int w = col / D1, m = col - w * D1;
+                            double *o = out + (((int64_t)w * P + p) * cells.n + cur.cell) * (2 * D1) + m;
+                            o[0] = aR[i < Sh::NTR ? i : 0][e];
+                            o[D1] = aI[i - Sh::I0 >= 0 ? i - Sh::I0 : 0][e];
+                        }
+                    }
+            }
         }
+        if (!more) break;
+        stage(nxt, b ^ 1);
+        __syncthreads();
+        cur = nxt;
+        first = last;
     }
 }
 
-// Resident CTAs of the moment kernels: two per SM.
-int cell_slots(const Table &t, int *slots) {
-    int sms = 148;
-    MB_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, t.device));
-    *slots = 2 * sms;
+int sm_count(const Table &t, int *sms) {
+    MB_CUDA(cudaDeviceGetAttribute(sms, cudaDevAttrMultiProcessorCount, t.device));
     return MB_OK;
 }
 
@@ -330,10 +405,11 @@ template <int KIND, int W, int D1>
 int launch_moments(const Table &t, const Cells &c, const uint64_t *vi, const uint64_t *vf, const double *delta,
                    const int *sel, int64_t P, const CellWeights &w, double k, int nzw, double *out, cudaStream_t s) {
     using Sh = CellShape<KIND, W, D1>;
-    static_assert(8 * 32 * Sh::frag * 8 / 2 <= CELL_TILE * Sh::S * 8 || KIND == CELL_WEIGHTS, "reduction buffer");
+    static_assert(4 * 32 * Sh::frag <= Sh::TILE * Sh::S || KIND == CELL_WEIGHTS, "reduction buffer");
     MB_TRY(cell_kernel_attributes());
-    int slots = 296;
-    MB_TRY(cell_slots(t, &slots));
+    int sms = 148;
+    MB_TRY(sm_count(t, &sms));
+    const int64_t slots = (int64_t)Sh::ctas * sms;
     const int64_t n_pt = (P + CELL_PEAKS / nzw - 1) / (CELL_PEAKS / nzw);
     const int64_t items = n_pt * c.n;
     MB_CHECK_ARG(items < ((int64_t)1 << 31), "cell moments: %lld items", (long long)items);
@@ -352,11 +428,16 @@ int cell_nzw(int64_t P) {
 
 // ------------------------------------------------------------------ offset scans
 
-constexpr int CSCAN_THREADS = 128;
+constexpr int CSCAN_PTS = 256;                 // grid points per CTA
 constexpr int CSCAN_PT = 2;                    // grid points per thread
+constexpr int CSCAN_LANES = CSCAN_PTS / CSCAN_PT;
+constexpr int CSCAN_SPLIT = 2;                 // thread groups sharing the cells
+constexpr int CSCAN_THREADS = CSCAN_LANES * CSCAN_SPLIT;
 constexpr int CSCAN_CELLS = 32;                // cells staged at a time
 
-// Thread: CSCAN_PT points of one base point over all cells; the moments are read as broadcasts.
+// Thread: CSCAN_PT points of one base point over every CSCAN_SPLIT-th cell; the moments are read as
+// broadcasts.  With a few hundred CTAs the cells' dependent chains are exposed, hence the split (its sums are
+// added in order) and the four products of each point summed apart.
 template <int D1>
 __global__ void __launch_bounds__(CSCAN_THREADS)
 cell_scan_kernel(Cells cells, const double *M, int NB, int Bp, int64_t n_m, uint64_t si, uint64_t sf, double kstep,
@@ -365,7 +446,9 @@ cell_scan_kernel(Cells cells, const double *M, int NB, int Bp, int64_t n_m, uint
     double2 *tab = reinterpret_cast<double2 *>(smem);
     double2 *mom = reinterpret_cast<double2 *>(smem + PH_BYTES);                  // [cell][D1]: pairs of one row
     ulonglong2 *dph = reinterpret_cast<ulonglong2 *>(mom + CSCAN_CELLS * D1);     // frac(step G_c): lo, hi
+    const double2 *copy = tab + (threadIdx.x & (PH_COPIES - 1));
     phasor_table_init(tab, CSCAN_THREADS);
+    const int part = threadIdx.x / CSCAN_LANES, tl = threadIdx.x - part * CSCAN_LANES;
     const int64_t pb = blockIdx.y;                               // point p NB + b
     const int64_t p = pb / NB, b = pb - p * NB;
     const int np = (int)min((int64_t)Bp, n_m - b * Bp);          // points of this block
@@ -373,7 +456,7 @@ cell_scan_kernel(Cells cells, const double *M, int NB, int Bp, int64_t n_m, uint
     int ml[CSCAN_PT];
 #pragma unroll
     for (int i = 0; i < CSCAN_PT; ++i) {
-        ml[i] = (int)(blockIdx.x * CSCAN_PT + i) * CSCAN_THREADS + threadIdx.x - Bp / 2;
+        ml[i] = (int)(blockIdx.x * CSCAN_PT + i) * CSCAN_LANES + tl - Bp / 2;
         // (kappa d)^n / n! with the sign of i^n: + + - -
         const double y = kstep * ml[i];
         double x = 1.0;
@@ -397,33 +480,50 @@ cell_scan_kernel(Cells cells, const double *M, int NB, int Bp, int64_t n_m, uint
             dph[threadIdx.x] = make_ulonglong2(lo, hi);
         }
         __syncthreads();
-        for (int c = 0; c < nc; ++c) {
+        for (int c = part; c < nc; c += CSCAN_SPLIT) {
             const double2 *m2 = mom + c * D1;
             const ulonglong2 d = dph[c];
-            double qr[CSCAN_PT], qi[CSCAN_PT];
+            double cs[CSCAN_PT], sn[CSCAN_PT];
 #pragma unroll
-            for (int i = 0; i < CSCAN_PT; ++i) qr[i] = qi[i] = 0.0;
+            for (int i = 0; i < CSCAN_PT; ++i) {
+                // frac(m step G_c) to 2^-64 turn, m the signed offset index of less than 2^31
+                const uint32_t ma = (uint32_t)(ml[i] < 0 ? -ml[i] : ml[i]);
+                uint64_t w = wide(ma, (uint32_t)d.y) + ((uint64_t)(ma * (uint32_t)(d.y >> 32)) << 32) +
+                             (wide(ma, (uint32_t)(d.x >> 32)) >> 32);
+                if (ml[i] < 0) w = ~w;
+                phasor((w >> 4) + (1ull << 51), copy, cs[i], sn[i]);
+            }
+            double rr[CSCAN_PT], ri[CSCAN_PT], ir[CSCAN_PT], ii[CSCAN_PT];
+#pragma unroll
+            for (int i = 0; i < CSCAN_PT; ++i) rr[i] = ri[i] = ir[i] = ii[i] = 0.0;
 #pragma unroll
             for (int n = 0; n < D1; n += 2) {
                 const double2 re = m2[n / 2], im = m2[(D1 + n) / 2];
 #pragma unroll
                 for (int i = 0; i < CSCAN_PT; ++i) {
-                    qr[i] = fma(e[i][n], re.x, fma(-e[i][n + 1], im.y, qr[i]));
-                    qi[i] = fma(e[i][n], im.x, fma(e[i][n + 1], re.y, qi[i]));
+                    rr[i] = fma(e[i][n], re.x, rr[i]);
+                    ri[i] = fma(e[i][n + 1], im.y, ri[i]);
+                    ir[i] = fma(e[i][n], im.x, ir[i]);
+                    ii[i] = fma(e[i][n + 1], re.y, ii[i]);
                 }
             }
 #pragma unroll
-            for (int i = 0; i < CSCAN_PT; ++i) {
-                // frac(m step G_c), m the signed offset index (2^-64 turn short at most when negative)
-                const uint64_t ma = (uint64_t)(ml[i] < 0 ? -ml[i] : ml[i]);
-                uint64_t w = ma * d.y + __umul64hi(ma, d.x);
-                if (ml[i] < 0) w = ~w;
-                double cs, sn;
-                phasor(w + (1ull << 55), tab, cs, sn);
-                h[i] = fma(cs, qr[i], fma(-sn, qi[i], h[i]));
-            }
+            for (int i = 0; i < CSCAN_PT; ++i) h[i] += fma(cs[i], rr[i] - ri[i], -sn[i] * (ir[i] + ii[i]));
         }
     }
+    // the other parts' sums, in order (they take the moments' place)
+    double *other = reinterpret_cast<double *>(mom);
+    for (int q = 1; q < CSCAN_SPLIT; ++q) {
+        __syncthreads();
+        if (part == q)
+#pragma unroll
+            for (int i = 0; i < CSCAN_PT; ++i) other[i * CSCAN_LANES + tl] = h[i];
+        __syncthreads();
+        if (part == 0)
+#pragma unroll
+            for (int i = 0; i < CSCAN_PT; ++i) h[i] += other[i * CSCAN_LANES + tl];
+    }
+    if (part > 0) return;
 #pragma unroll
     for (int i = 0; i < CSCAN_PT; ++i) {
         const int l = ml[i] + Bp / 2;
@@ -432,7 +532,10 @@ cell_scan_kernel(Cells cells, const double *M, int NB, int Bp, int64_t n_m, uint
 }
 
 template <int D1>
-constexpr int cscan_smem() { return PH_BYTES + CSCAN_CELLS * (D1 * 16 + 16); }
+constexpr int cscan_smem() {
+    static_assert(CSCAN_CELLS * D1 * 16 >= CSCAN_PTS * 8, "the parts' sums fit the moments' place");
+    return PH_BYTES + CSCAN_CELLS * (D1 * 16 + 16);
+}
 
 // ------------------------------------------------------------------ polishes on moments
 
@@ -949,7 +1052,7 @@ int build_cells(const Table &t, const CellPlan &p, void *buf, Cells &out, cudaSt
         g.e0[i] = p.e0[i];
         g.nc[i] = p.nc[i];
     }
-    cells_kernel<<<(unsigned)((n + 127) / 128), 128, 0, s>>>(view(t), g, n, p.half, j0, j1, ctr);
+    cells_kernel<<<(unsigned)((n + 2 + 3) / 4), 128, 0, s>>>(view(t), g, p.half, j0, j1, ctr);
     MB_CUDA(cudaGetLastError());
     out = Cells{n, p.nc[0], p.half, j0, j1, ctr};
     return MB_OK;
@@ -976,13 +1079,14 @@ int launch_moments_weights(const Table &t, const Cells &c, const uint64_t *vi, c
     }
 }
 
-// Chunks so that every CTA slot gets about four items, each at least 512 zeros.
+// Chunks so that every CTA slot gets about eight items, each at least 256 zeros on average.
 int taylor_chunks(const Table &t, int64_t P, int64_t n, int *n_chunk) {
-    int slots = 296;
-    MB_TRY(cell_slots(t, &slots));
+    int slots = 148;
+    MB_TRY(sm_count(t, &slots));
+    slots *= CellShape<CELL_POWERS, 1, 17>::ctas;
     const int ppc = CELL_PEAKS / cell_nzw(P);
     const int64_t n_pt = std::max<int64_t>(1, (P + ppc - 1) / ppc);
-    *n_chunk = (int)std::max<int64_t>(1, std::min<int64_t>((4 * (int64_t)slots + n_pt - 1) / n_pt, n / 512));
+    *n_chunk = (int)std::max<int64_t>(1, std::min<int64_t>((8 * (int64_t)slots + n_pt - 1) / n_pt, n / 256));
     return MB_OK;
 }
 
@@ -1011,7 +1115,7 @@ int launch_cell_scan(const Cells &c, int d1, const double *M, int64_t P, int NB,
     MB_TRY(cell_kernel_attributes());
     const double step = (double)step_int + (double)step_frac * 0x1p-64;
     const double kstep = 6.283185307179586 * c.H() * step;
-    const dim3 grid((unsigned)((Bp + CSCAN_THREADS * CSCAN_PT - 1) / (CSCAN_THREADS * CSCAN_PT)), (unsigned)(P * NB));
+    const dim3 grid((unsigned)((Bp + CSCAN_PTS - 1) / CSCAN_PTS), (unsigned)(P * NB));
     if (d1 == 8)
         cell_scan_kernel<8><<<grid, CSCAN_THREADS, cscan_smem<8>(), s>>>(c, M, NB, Bp, n_m, step_int, step_frac, kstep, out);
     else

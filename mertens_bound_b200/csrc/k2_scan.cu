@@ -263,8 +263,8 @@ constexpr int64_t SCAN_MAX_POINTS = 65535;                  // block points per 
 // Chooses the block count and the series length with the smallest estimated work; false when the direct
 // kernel is the cheaper one (c_old: its warp cycles per 32 (point, zero) pairs): few points per base,
 // or a step so large that a block's cells hold less than a few zeros each.  The estimates are warp cycles
-// of one scheduler: a moment step (32 pairs) ~60 for the phasors + 32 per 8 columns, the staging ~10 per
-// zero and CTA, a point of the evaluation 2 (2 D1 + 14) + 25 per cell.
+// of one scheduler: a moment step (32 pairs) ~120 for the phasors + 20 per mma, the staging ~20 per zero and
+// CTA, 32 points of the evaluation 3.6 per FP64 operation, 2 D1 + 15 of them per cell.
 bool plan_scan(const Table &t, int64_t P, int64_t n_use, int64_t n_m, uint64_t step_int, uint64_t step_frac,
                double c_old, int64_t old_points, ScanPlan &best) {
     if (n_use < 1 || step_int >> 31) return false;
@@ -287,8 +287,11 @@ bool plan_scan(const Table &t, int64_t P, int64_t n_use, int64_t n_m, uint64_t s
             if (!plan_cells(t, n_use, 0, (double)((Bp + 1) / 2) * step, d1, min_cells, cp)) continue;
             const double nc = cp.cells();
             const double zeros = n_use + 2.0 * nc;
-            const double mom = tiles * zeros * (ppc / 32.0 * (60.0 + 4.0 * d1) + 10.0);
-            const double eval = (double)pts * ((Bp + 255) / 256 * 256) / 32.0 * nc * (2.0 * (2 * d1 + 14) + 25.0);
+            // one moment item per SM keeps it busy; however few they are, a scan CTA (256 points) takes the
+            // latency of its cells, three CTAs to an SM
+            const double mom = tiles * zeros * (ppc / 32.0 * (120.0 + 5.0 * d1) + 20.0) / std::min(1.0, nc * tiles / 148.0);
+            const double ctas = (double)pts * ((Bp + 255) / 256);
+            const double eval = nc * (2 * d1 + 15) * std::max(ctas * 8.0 * 3.6, 592.0 * 8.0 * std::ceil(ctas / 444.0));
             const double bytes = (double)NB * nc * 2 * d1 * 8;
             if (bytes > (double)SCAN_MOMENT_BYTES) continue;
             if (mom + eval < best_cost) {
