@@ -308,9 +308,7 @@ int mb_screen(mb_table *t, int64_t P, const uint64_t *v_int, const uint64_t *v_f
  * d_v_frac hold P leaves; stage_end and threshold are host arrays as above.  Hits go to d_hits /
  * d_hit_scores (device, at most max_hits, in arbitrary order) and their total to *d_n_hits (device;
  * above max_hits the kept subset is arbitrary); d_scores (device, nullable, P x n_stages) as
- * out_scores.  The zero records are staged in a buffer of the table that only mb_screen_dev uses,
- * so other calls on the table (on its own stream) cannot disturb a screen in flight; two
- * mb_screen_dev calls on one table that overlap on the GPU (different streams) race on it. */
+ * out_scores.  The screen keeps nothing in the table: calls on different streams may overlap. */
 int mb_screen_dev(mb_table *t, int64_t P, const uint64_t *d_v_int, const uint64_t *d_v_frac, double k,
                   uint64_t step_int, uint64_t step_frac, int n_stages, const int64_t *stage_end,
                   const float *threshold, int64_t max_hits, int64_t *d_hits, float *d_hit_scores,

@@ -16,8 +16,10 @@
 #include <algorithm>
 #include <cmath>
 #include <numeric>
+#include <type_traits>
 #include <vector>
 
+#include "k2_fast.h"
 #include "k2_light.cuh"
 
 namespace mb {
@@ -27,13 +29,21 @@ constexpr int SCREEN_THREADS = 256;
 constexpr int SCREEN_MAX_ZEROS = 1024;
 constexpr int SCREEN_MAX_STAGES = 8;
 
-struct __align__(16) ZScreen {   // 80 B
+// A zero's record: the light phase's limbs (light_phase32_fused where every screened zero has gamma below
+// FUSED_PHASE_GAMMA, light_phase32 otherwise) and a cos(2 pi m D), a sin(2 pi m D), m = 1..3, with
+// a = 2|c| e^{-k gamma^2} and D = frac(step G).
+struct __align__(16) ZScreenF {   // 64 B
+    uint32_t b0, b1, psi32;
+    float a;
+    double b0s, c1s, gh;
+    float cm[3], sm[3];
+};
+struct __align__(16) ZScreenS {   // 80 B
     uint32_t b0, b1, gi, psi32;
     double b0s, c1s, gis, b1s;
-    float a;                      // 2|c| e^{-k gamma^2}
-    float cm[3], sm[3];           // a cos(2 pi m D), a sin(2 pi m D), m = 1..3, D = frac(step G)
-    float pad;
+    float a, cm[3], sm[3], pad;
 };
+static_assert(sizeof(ZScreenF) == 64 && sizeof(ZScreenS) == 80, "screen records");
 
 struct ScreenArgs {
     int n_stages;
@@ -41,91 +51,219 @@ struct ScreenArgs {
     float thr[SCREEN_MAX_STAGES];
 };
 
-__global__ void screen_prep_kernel(TabView t, int n, double k, uint64_t step_int, uint64_t step_frac, ZScreen *out) {
-    const int j = blockIdx.x * blockDim.x + threadIdx.x;
-    if (j >= n) return;
-    ZScreen r;
-    const uint32_t c1 = t.g1[j], b0 = t.g2[j], b1 = t.g3[j], gi = t.g4[j];
+struct ScreenOut {
+    int64_t max_hits;
+    unsigned long long *count;
+    int64_t *hit_idx;
+    float *hit_score, *scores;
+};
+
+MB_DEV void screen_limbs(const TabView &t, int j, ZScreenF &r) {
+    const uint32_t b0 = t.g2[j], b1 = t.g3[j];
+    r.b0 = b0;
+    r.b1 = b1;
+    r.psi32 = (uint32_t)((t.psi[j] + 0x80000000ull) >> 32) + 1u;
+    r.b0s = u32_to_f64(b0) * TWO_M32;
+    r.c1s = u32_to_f64(t.g1[j]) * TWO_M32;
+    r.gh = fma(u32_to_f64(t.g4[j]), 4294967296.0, u32_to_f64(b1));
+}
+MB_DEV void screen_limbs(const TabView &t, int j, ZScreenS &r) {
+    const uint32_t b0 = t.g2[j], b1 = t.g3[j], gi = t.g4[j];
     r.b0 = b0;
     r.b1 = b1;
     r.gi = gi;
     r.psi32 = (uint32_t)((t.psi[j] + 0x80000000ull) >> 32) + 2u;
     r.b0s = u32_to_f64(b0) * TWO_M32;
-    r.c1s = u32_to_f64(c1) * TWO_M32;
+    r.c1s = u32_to_f64(t.g1[j]) * TWO_M32;
     r.gis = u32_to_f64(gi) * TWO_M32;
     r.b1s = u32_to_f64(b1) * TWO_M32;
-    const double g = t.gamma[j];
-    const double a = 2.0 * t.alpha[j] * exp(-k * g * g);
-    r.a = (float)a;
-    uint64_t hi, lo;
-    phase128_exact((uint32_t)step_frac, (uint32_t)(step_frac >> 32), (uint32_t)step_int, (uint32_t)(step_int >> 32),
-                   t.g0[j], c1, b0, b1, gi, hi, lo);
-    const double D = s64_turns_to_f64(hi);      // frac(step G) in [-1/2, 1/2)
-#pragma unroll
-    for (int m = 1; m <= 3; ++m) {
-        double s, c;
-        sincospi(2.0 * m * D, &s, &c);
-        r.cm[m - 1] = (float)(a * c);
-        r.sm[m - 1] = (float)(a * s);
-    }
     r.pad = 0.f;
-    out[j] = r;
+}
+MB_DEV int32_t screen_phase(const CandRegs &c, const ZScreenF &z) {
+    return (int32_t)light_phase32_fused(c, z.b0, z.b1, z.b0s, z.c1s, z.gh, z.psi32);
+}
+MB_DEV int32_t screen_phase(const CandRegs &c, const ZScreenS &z) {
+    return (int32_t)light_phase32(c, z.b0, z.b1, z.gi, z.b0s, z.c1s, z.gis, z.b1s, z.psi32);
 }
 
-__global__ void __launch_bounds__(SCREEN_THREADS) screen_kernel(const ZScreen *zs, int n_zeros, CandView c,
-                                                                ScreenArgs sa, int64_t max_hits,
-                                                                unsigned long long *count, int64_t *hit_idx,
-                                                                float *hit_score, float *scores) {
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    ZScreen *tile = reinterpret_cast<ZScreen *>(smem_raw);
-    {
-        const int4 *src = reinterpret_cast<const int4 *>(zs);
-        int4 *dst = reinterpret_cast<int4 *>(tile);
-        const int words = n_zeros * (int)(sizeof(ZScreen) / sizeof(int4));
-        for (int i = threadIdx.x; i < words; i += SCREEN_THREADS) dst[i] = src[i];
+// The seven sums of a leaf by parity: S_0 = e[0], S_{+-m} = e[m] -+ o[m - 1]
+// (cos(theta + m D) = cos theta cos m D - sin theta sin m D), so a term is seven FMAs.
+struct ScreenSums {
+    float e[4], o[3];
+    MB_DEV void clear() {
+        e[0] = e[1] = e[2] = e[3] = o[0] = o[1] = o[2] = 0.f;
     }
-    __syncthreads();
-    const int64_t p = (int64_t)blockIdx.x * SCREEN_THREADS + threadIdx.x;
-    const bool valid = p < c.P;
-    const CandRegs cr = cand_regs(c, p, valid);
-    float S[7];
+    template <class Z>
+    MB_DEV void add(const CandRegs &c, const Z &z) {
+        const float th = (float)screen_phase(c, z) * 1.4629180792671596e-09f;   // 2pi 2^-32
+        const float sn = __sinf(th), cs = __cosf(th);
+        e[0] = fmaf(z.a, cs, e[0]);
 #pragma unroll
-    for (int m = 0; m < 7; ++m) S[m] = 0.f;
-    float sc[SCREEN_MAX_STAGES];
-    bool alive = valid;
-    int reached = 0;
-    int j = 0;
-    for (int s = 0; s < sa.n_stages; ++s) {
-        if (!__any_sync(0xffffffffu, alive)) break;
-        const int end = sa.stage_end[s];
-        for (; j < end; ++j) {
-            const ZScreen z = tile[j];
-            const int32_t u = (int32_t)light_phase32(cr, z.b0, z.b1, z.gi, z.b0s, z.c1s, z.gis, z.b1s, z.psi32);
-            const float th = (float)u * 1.4629180792671596e-09f;   // 2pi 2^-32
-            const float sn = __sinf(th), cs = __cosf(th);
-            S[3] = fmaf(z.a, cs, S[3]);
-#pragma unroll
-            for (int m = 1; m <= 3; ++m) {
-                const float x = cs * z.cm[m - 1], y = sn * z.sm[m - 1];
-                S[3 + m] += x - y;
-                S[3 - m] += x + y;
-            }
+        for (int m = 0; m < 3; ++m) {
+            e[m + 1] = fmaf(z.cm[m], cs, e[m + 1]);
+            o[m] = fmaf(z.sm[m], sn, o[m]);
         }
-        float best = 0.f;
-#pragma unroll
-        for (int m = 0; m < 7; ++m) best = fmaxf(best, fabsf(S[m]));
-        sc[s] = best;
-        if (alive) reached = s + 1;
-        alive = alive && best >= sa.thr[s];
     }
-    if (!valid) return;
-    if (scores)
-        for (int s = 0; s < sa.n_stages; ++s) scores[p * sa.n_stages + s] = s < reached ? sc[s] : -1.0f;
-    if (alive && reached == sa.n_stages) {
-        const unsigned long long h = atomicAdd(count, 1ull);
-        if ((int64_t)h < max_hits) {
-            hit_idx[h] = p;
-            for (int s = 0; s < sa.n_stages; ++s) hit_score[h * sa.n_stages + s] = sc[s];
+    MB_DEV float best() const {
+        float b = fabsf(e[0]);
+#pragma unroll
+        for (int m = 0; m < 3; ++m) b = fmaxf(b, fmaxf(fabsf(e[m + 1] - o[m]), fabsf(e[m + 1] + o[m])));
+        return b;
+    }
+};
+
+// One CTA slot each: an equal share of the leaves, in tiles of LPT x 256.  The first stage runs LPT leaves per thread, so that a
+// zero's record (four 16-byte broadcasts) serves LPT terms: with one leaf per thread those reads were half of the
+// time (2^20 leaves: 155 us; now 78).  Survivors are listed in shared memory with their sums, and the later
+// stages run over the list: a leaf per thread while a quarter of the tile or more is alive, eight lanes
+// per leaf below that, so a few survivors neither hold whole warps nor run a long serial loop.
+template <int LPT, class Z>
+__global__ void __launch_bounds__(SCREEN_THREADS, LPT == 1 ? 4 : 2)
+screen_kernel(TabView t, int n_zeros, double k, uint64_t step_int, uint64_t step_frac, CandView c, ScreenArgs sa,
+              ScreenOut out) {
+    constexpr int LEAVES = LPT * SCREEN_THREADS;
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    Z *zs = reinterpret_cast<Z *>(smem_raw);
+    float *sums = reinterpret_cast<float *>(smem_raw + (size_t)n_zeros * sizeof(Z));     // [7][LEAVES]
+    float *sc = sums + 7 * LEAVES;                                                        // [n_stages][LEAVES]
+    uint16_t *list = reinterpret_cast<uint16_t *>(sc + sa.n_stages * LEAVES);             // [2][LEAVES]
+    __shared__ int n_list[2];
+    for (int j = threadIdx.x; j < n_zeros; j += SCREEN_THREADS) {
+        Z r;
+        screen_limbs(t, j, r);
+        const double g = t.gamma[j];
+        const double a = 2.0 * t.alpha[j] * exp(-k * g * g);
+        r.a = (float)a;
+        uint64_t hi, lo;
+        phase128_exact((uint32_t)step_frac, (uint32_t)(step_frac >> 32), (uint32_t)step_int, (uint32_t)(step_int >> 32),
+                       t.g0[j], t.g1[j], t.g2[j], t.g3[j], t.g4[j], hi, lo);
+        const double D = s64_turns_to_f64(hi);      // frac(step G) in [-1/2, 1/2)
+#pragma unroll
+        for (int m = 1; m <= 3; ++m) {
+            double s, co;
+            sincospi(2.0 * m * D, &s, &co);
+            r.cm[m - 1] = (float)(a * co);
+            r.sm[m - 1] = (float)(a * s);
+        }
+        zs[j] = r;
+    }
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    // this CTA's share of the leaves (whole warps of them), tile by tile
+    const int64_t warps = (c.P + 31) / 32;
+    const int64_t p_end = min(c.P, warps * (blockIdx.x + 1) / gridDim.x * 32);
+    for (int64_t p0 = warps * blockIdx.x / gridDim.x * 32; p0 < p_end; p0 += LEAVES) {
+        const int n_leaves = (int)min((int64_t)LEAVES, p_end - p0);
+        // leaf l's stage result: its score, and the next list or the hit buffers if it survives
+        auto finish = [&](int l, int s, const ScreenSums &x) {
+            const float b = x.best();
+            sc[s * LEAVES + l] = b;
+            if (out.scores) out.scores[(p0 + l) * sa.n_stages + s] = b;
+            if (!(b >= sa.thr[s])) return;
+            if (s + 1 < sa.n_stages) {
+                const int q = atomicAdd(&n_list[s & 1], 1);
+                list[(s & 1) * LEAVES + q] = (uint16_t)l;
+#pragma unroll
+                for (int m = 0; m < 4; ++m) sums[m * LEAVES + l] = x.e[m];
+#pragma unroll
+                for (int m = 0; m < 3; ++m) sums[(4 + m) * LEAVES + l] = x.o[m];
+            } else {
+                const unsigned long long h = atomicAdd(out.count, 1ull);
+                if ((int64_t)h < out.max_hits) {
+                    out.hit_idx[h] = p0 + l;
+                    for (int i = 0; i < sa.n_stages; ++i) out.hit_score[h * sa.n_stages + i] = sc[i * LEAVES + l];
+                }
+            }
+        };
+        auto resume = [&](int l, ScreenSums &x) {
+#pragma unroll
+            for (int m = 0; m < 4; ++m) x.e[m] = sums[m * LEAVES + l];
+#pragma unroll
+            for (int m = 0; m < 3; ++m) x.o[m] = sums[(4 + m) * LEAVES + l];
+        };
+        __syncthreads();                             // the records; the tile before is done with the lists
+        if (threadIdx.x < 2) n_list[threadIdx.x] = 0;
+        __syncthreads();
+        // the first stage with L leaves per thread
+        auto first = [&](auto per) {
+            constexpr int L = decltype(per)::value;
+            CandRegs cr[L];
+            ScreenSums x[L];
+#pragma unroll
+            for (int i = 0; i < L; ++i) {
+                const int l = i * SCREEN_THREADS + threadIdx.x;
+                cr[i] = cand_regs(c, p0 + l, l < n_leaves);
+                x[i].clear();
+            }
+            for (int j = 0; j < sa.stage_end[0]; ++j) {
+                const Z z = zs[j];
+#pragma unroll
+                for (int i = 0; i < L; ++i) x[i].add(cr[i], z);
+            }
+#pragma unroll
+            for (int i = 0; i < L; ++i) {
+                const int l = i * SCREEN_THREADS + threadIdx.x;
+                if (l >= n_leaves) continue;
+                if (out.scores)
+                    for (int s = 1; s < sa.n_stages; ++s) out.scores[(p0 + l) * sa.n_stages + s] = -1.0f;
+                finish(l, 0, x[i]);
+            }
+        };
+        if constexpr (LPT == 1) {
+            first(std::integral_constant<int, 1>());
+        } else {                                     // a last, smaller tile takes fewer per thread
+            static_assert(LPT == 4, "one or four leaves per thread");
+            if (n_leaves > 3 * SCREEN_THREADS) first(std::integral_constant<int, 4>());
+            else if (n_leaves > 2 * SCREEN_THREADS) first(std::integral_constant<int, 3>());
+            else if (n_leaves > SCREEN_THREADS) first(std::integral_constant<int, 2>());
+            else first(std::integral_constant<int, 1>());
+        }
+        for (int s = 1; s < sa.n_stages; ++s) {
+            __syncthreads();                         // the list of stage s - 1 is complete
+            const int n = n_list[(s - 1) & 1];
+            if (n == 0) break;
+            const uint16_t *in = list + ((s - 1) & 1) * LEAVES;
+            const int j0 = sa.stage_end[s - 1], j1 = sa.stage_end[s];
+            if (s > 1) {                             // its other half was stage s - 2's
+                __syncthreads();
+                if (threadIdx.x == 0) n_list[s & 1] = 0;
+                __syncthreads();
+            }
+            if (4 * n >= LEAVES) {
+                for (int q = threadIdx.x; q < n; q += SCREEN_THREADS) {
+                    const int l = in[q];
+                    const CandRegs cr = cand_regs(c, p0 + l, true);
+                    ScreenSums x;
+                    resume(l, x);
+                    for (int j = j0; j < j1; ++j) x.add(cr, zs[j]);
+                    finish(l, s, x);
+                }
+            } else {
+                for (int q0 = warp * 4; q0 < n; q0 += SCREEN_THREADS / 8) {
+                    const int q = q0 + (lane >> 3);
+                    const bool live = q < n;
+                    const int l = in[live ? q : q0];
+                    const CandRegs cr = cand_regs(c, p0 + l, true);
+                    ScreenSums x;
+                    x.clear();
+                    for (int j = j0 + (lane & 7); j < j1; j += 8) x.add(cr, zs[j]);
+#pragma unroll
+                    for (int o = 4; o > 0; o >>= 1) {
+#pragma unroll
+                        for (int m = 0; m < 4; ++m) x.e[m] += __shfl_xor_sync(0xffffffffu, x.e[m], o);
+#pragma unroll
+                        for (int m = 0; m < 3; ++m) x.o[m] += __shfl_xor_sync(0xffffffffu, x.o[m], o);
+                    }
+                    if (live && (lane & 7) == 0) {
+                        ScreenSums y;
+                        resume(l, y);
+#pragma unroll
+                        for (int m = 0; m < 4; ++m) y.e[m] += x.e[m];
+#pragma unroll
+                        for (int m = 0; m < 3; ++m) y.o[m] += x.o[m];
+                        finish(l, s, y);
+                    }
+                }
+            }
         }
     }
 }
@@ -151,22 +289,39 @@ int screen_args(const Table &t, int n_stages, const int64_t *stage_end, const fl
     return MB_OK;
 }
 
-// Zero records into d_z, the count reset, and the screen over P device leaves, all on st.
-int launch_screen(Table &t, int64_t P, const uint64_t *d_vi, const uint64_t *d_vf, double k, uint64_t step_int,
-                  uint64_t step_frac, const ScreenArgs &sa, ZScreen *d_z, int64_t max_hits,
-                  unsigned long long *d_count, int64_t *d_hits, float *d_hsc, float *d_sc, cudaStream_t st) {
+template <int LPT, class Z>
+int launch_screen_as(const Table &t, CandView c, double k, uint64_t step_int, uint64_t step_frac, const ScreenArgs &sa,
+                     const ScreenOut &out, int sms, cudaStream_t st) {
+    constexpr int LEAVES = LPT * SCREEN_THREADS;
     const int nz = sa.stage_end[sa.n_stages - 1];
-    MB_CUDA(cudaMemsetAsync(d_count, 0, 8, st));
-    screen_prep_kernel<<<(nz + 127) / 128, 128, 0, st>>>(view(t), nz, k, step_int, step_frac, d_z);
-    MB_CUDA(cudaGetLastError());
-    const size_t smem = (size_t)nz * sizeof(ZScreen);
-    MB_CUDA(cudaFuncSetAttribute(screen_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)(SCREEN_MAX_ZEROS * sizeof(ZScreen))));
-    const unsigned blocks = (unsigned)((P + SCREEN_THREADS - 1) / SCREEN_THREADS);
-    screen_kernel<<<blocks, SCREEN_THREADS, smem, st>>>(d_z, nz, CandView{d_vi, d_vf, nullptr, P}, sa, max_hits,
-                                                       d_count, d_hits, d_hsc, d_sc);
+    const auto bytes = [](int zeros, int stages) {
+        return (size_t)zeros * sizeof(Z) + (size_t)LEAVES * (7 + stages) * 4 + 2 * LEAVES * sizeof(uint16_t);
+    };
+    MB_CUDA(cudaFuncSetAttribute(screen_kernel<LPT, Z>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)bytes(SCREEN_MAX_ZEROS, SCREEN_MAX_STAGES)));
+    const int64_t tiles = (c.P + LEAVES - 1) / LEAVES;
+    const unsigned grid = (unsigned)std::min<int64_t>(tiles, (int64_t)sms * (LPT == 1 ? 4 : 2));
+    screen_kernel<LPT, Z><<<grid, SCREEN_THREADS, bytes(nz, sa.n_stages), st>>>(view(t), nz, k, step_int, step_frac, c,
+                                                                              sa, out);
     MB_CUDA(cudaGetLastError());
     return MB_OK;
+}
+
+// The count reset and the screen over P device leaves, on st.  Four leaves per thread where that still gives
+// every SM a CTA.
+int launch_screen(const Table &t, int64_t P, const uint64_t *d_vi, const uint64_t *d_vf, double k, uint64_t step_int,
+                  uint64_t step_frac, const ScreenArgs &sa, const ScreenOut &out, cudaStream_t st) {
+    MB_CUDA(cudaMemsetAsync(out.count, 0, 8, st));
+    int sms = 148;
+    MB_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, t.device));
+    const CandView c{d_vi, d_vf, nullptr, P};
+    const bool fused = t.h_gamma[sa.stage_end[sa.n_stages - 1] - 1] < FUSED_PHASE_GAMMA;
+    const bool four = P >= (int64_t)sms * 4 * SCREEN_THREADS;
+    if (fused)
+        return four ? launch_screen_as<4, ZScreenF>(t, c, k, step_int, step_frac, sa, out, sms, st)
+                    : launch_screen_as<1, ZScreenF>(t, c, k, step_int, step_frac, sa, out, sms, st);
+    return four ? launch_screen_as<4, ZScreenS>(t, c, k, step_int, step_frac, sa, out, sms, st)
+                : launch_screen_as<1, ZScreenS>(t, c, k, step_int, step_frac, sa, out, sms, st);
 }
 
 }  // namespace
@@ -187,15 +342,13 @@ extern "C" int mb_screen(mb_table *h, int64_t P, const uint64_t *v_int, const ui
     *n_hits = 0;
     if (P == 0) return MB_OK;
     MB_TRY(device_guard(t.device));
-    const int nz = sa.stage_end[n_stages - 1];
     const size_t cand = (size_t)P * 8;
     const size_t sc_bytes = out_scores ? (size_t)P * n_stages * 4 : 0;
-    const size_t need = 2 * (cand + 256) + (nz * sizeof(ZScreen) + 256) + 256 + ((size_t)max_hits * 8 + 256) +
+    const size_t need = 2 * (cand + 256) + 256 + ((size_t)max_hits * 8 + 256) +
                         ((size_t)max_hits * n_stages * 4 + 256) + (sc_bytes + 256);
     MB_TRY(t.io.ensure(need));
     char *q = (char *)t.io.p;
     uint64_t *d_vi = carve<uint64_t>(q, P), *d_vf = carve<uint64_t>(q, P);
-    ZScreen *d_z = carve<ZScreen>(q, nz);
     unsigned long long *d_count = carve<unsigned long long>(q, 1);
     int64_t *d_hits = carve<int64_t>(q, max_hits);
     float *d_hsc = carve<float>(q, (size_t)max_hits * n_stages);
@@ -203,8 +356,8 @@ extern "C" int mb_screen(mb_table *h, int64_t P, const uint64_t *v_int, const ui
     cudaStream_t st = t.stream;
     MB_CUDA(cudaMemcpyAsync(d_vi, v_int, cand, cudaMemcpyHostToDevice, st));
     MB_CUDA(cudaMemcpyAsync(d_vf, v_frac, cand, cudaMemcpyHostToDevice, st));
-    MB_TRY(launch_screen(t, P, d_vi, d_vf, k, step_int, step_frac, sa, d_z, max_hits, d_count, d_hits, d_hsc,
-                         d_sc, st));
+    MB_TRY(launch_screen(t, P, d_vi, d_vf, k, step_int, step_frac, sa, ScreenOut{max_hits, d_count, d_hits, d_hsc, d_sc},
+                         st));
     unsigned long long total = 0;
     MB_CUDA(cudaMemcpyAsync(&total, d_count, 8, cudaMemcpyDeviceToHost, st));
     if (out_scores) MB_CUDA(cudaMemcpyAsync(out_scores, d_sc, sc_bytes, cudaMemcpyDeviceToHost, st));
@@ -249,9 +402,6 @@ extern "C" int mb_screen_dev(mb_table *h, int64_t P, const uint64_t *d_v_int, co
         MB_CUDA(cudaMemsetAsync(d_n_hits, 0, 8, st));
         return MB_OK;
     }
-    const int nz = sa.stage_end[n_stages - 1];
-    MB_TRY(t.screen.ensure(nz * sizeof(ZScreen)));
-    MB_TRY(launch_screen(t, P, d_v_int, d_v_frac, k, step_int, step_frac, sa, (ZScreen *)t.screen.p, max_hits,
-                         d_n_hits, d_hits, d_hit_scores, d_scores, st));
-    return MB_OK;
+    return launch_screen(t, P, d_v_int, d_v_frac, k, step_int, step_frac, sa,
+                         ScreenOut{max_hits, d_n_hits, d_hits, d_hit_scores, d_scores}, st);
 }
