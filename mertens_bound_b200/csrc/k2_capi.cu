@@ -1,6 +1,7 @@
 // C-ABI entry points: argument checks, host<->device staging, kernel dispatch.
 #include <cmath>
 #include <cstring>
+#include <vector>
 
 #include "k2_internal.h"
 
@@ -26,6 +27,14 @@ int stage_candidates(Table &t, int64_t P, const uint64_t *v_int, const uint64_t 
     s.vf = (uint64_t *)(base + cand);
     s.delta = (double *)(base + 2 * cand);
     s.out = (void *)(base + ((3 * cand + 255) & ~(size_t)255));
+    if (P <= 4096) {             // one copy instead of three (each small pageable copy costs microseconds)
+        std::vector<char> h(3 * cand, 0);
+        std::memcpy(h.data(), v_int, cand);
+        std::memcpy(h.data() + cand, v_frac, cand);
+        if (delta) std::memcpy(h.data() + 2 * cand, delta, cand);
+        MB_CUDA(cudaMemcpyAsync(s.vi, h.data(), 3 * cand, cudaMemcpyHostToDevice, t.stream));
+        return MB_OK;
+    }
     MB_CUDA(cudaMemcpyAsync(s.vi, v_int, cand, cudaMemcpyHostToDevice, t.stream));
     MB_CUDA(cudaMemcpyAsync(s.vf, v_frac, cand, cudaMemcpyHostToDevice, t.stream));
     if (delta)
@@ -86,6 +95,15 @@ extern "C" int mb_k2_plain(mb_table *h, int64_t P, const uint64_t *v_int, const 
     double *d_out = (double *)s.out;
     MB_TRY(launch_plain(t, CandView{s.vi, s.vf, s.delta, P}, t.count_below(T), k, d_out, d_out + P,
                         d_out + 2 * P, t.stream));
+    if (P <= 4096) {             // one copy instead of three
+        std::vector<double> h(3 * (size_t)P);
+        MB_CUDA(cudaMemcpyAsync(h.data(), d_out, 3 * (size_t)P * 8, cudaMemcpyDeviceToHost, t.stream));
+        MB_CUDA(cudaStreamSynchronize(t.stream));
+        std::memcpy(out_val, h.data(), P * 8);
+        if (out_dd) std::memcpy(out_dd, h.data() + P, P * 8);
+        if (out_dk) std::memcpy(out_dk, h.data() + 2 * P, P * 8);
+        return MB_OK;
+    }
     MB_CUDA(cudaMemcpyAsync(out_val, d_out, P * 8, cudaMemcpyDeviceToHost, t.stream));
     if (out_dd) MB_CUDA(cudaMemcpyAsync(out_dd, d_out + P, P * 8, cudaMemcpyDeviceToHost, t.stream));
     if (out_dk) MB_CUDA(cudaMemcpyAsync(out_dk, d_out + 2 * P, P * 8, cudaMemcpyDeviceToHost, t.stream));

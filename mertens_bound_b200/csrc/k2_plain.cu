@@ -2,7 +2,7 @@
 //
 // Plain method: the phase frac(v G) is reduced exactly with 32x32->64 integer multiplies
 // on 32-bit limbs (search/path1_eval_fast.cpp:41-46 does the same product with u128),
-// sine/cosine in FP64 from the half-angle polynomials, FP64 accumulation, warp-shuffle
+// sine/cosine in FP64 from a table and short polynomials (k2_phasor.cuh), FP64 accumulation, warp-shuffle
 // reduction inside the CTA and a deterministic FP64 reduction across zero chunks.
 #include <algorithm>
 #include <cmath>
@@ -10,6 +10,7 @@
 
 #include "k2_common.cuh"
 #include "k2_internal.h"
+#include "k2_phasor.cuh"
 
 namespace mb {
 
@@ -57,39 +58,14 @@ struct PlainShape {
     int cands_per_cta() const { return (PLAIN_THREADS / 32 / nzw) * (32 >> lpc_log2) * cpt; }
 };
 
-// sin/cos(2 pi hi 2^-64) of the exact 64-bit phase word: the nearest of PLAIN_TAB table angles
-// (the top 11 bits of hi + 2^52) and the remainder r = ((hi + 2^52) mod 2^53 - 2^52) 2^-64 turn,
-// exact in FP64 (|r| <= 2^-12), rotated by
-//   cos(2 pi r) - 1 = r^2 (-2 pi^2 + r^2 2 pi^4 / 3)     (truncation 1.8e-20)
-//   sin(2 pi r)     = r (2 pi - r^2 4 pi^3 / 3)           (truncation 7.1e-17)
-// so the result is within ~4e-16 of the exact values (table entries rounded once, four FMA
-// roundings).  11 FP64 operations and one shared-memory load instead of a 21-operation
-// polynomial pair on the full turn.
-constexpr int PLAIN_TAB = 2048;
-MB_DEV void sincos_phase64_tab(uint64_t hi, const double2 *tab, double &sn, double &cs) {
-    const uint64_t h = hi + (1ull << 52);
-    const int q = (int)(h >> 53);
-    const int32_t rh = (int32_t)((uint32_t)(h >> 32) & 0x1FFFFFu) - (1 << 20);
-    const double r = fma(s32_to_f64(rh), 2.3283064365386963e-10, u32_to_f64((uint32_t)h) * 5.421010862427522e-20);
-    const double u = r * r;
-    const double s = r * fma(u, -41.341702240399755, 6.283185307179586);
-    const double cm1 = u * fma(u, 64.93939402266829, -19.739208802178716);
-    const double2 T = tab[q];
-    cs = fma(T.x, cm1, fma(-T.y, s, T.x));
-    sn = fma(T.y, cm1, fma(T.x, s, T.y));
-}
-
 template <int CPT>
 __global__ void __launch_bounds__(PLAIN_THREADS)
 k2_plain_kernel(TabView t, CandView c, int64_t n_use, int64_t chunk, double k, int lpc_log2,
                 int nzw, double *partial) {
     __shared__ ZRecPlain tile[PLAIN_TILE];
-    __shared__ double2 s_tab[PLAIN_TAB];       // (cos, sin)(2 pi i / PLAIN_TAB); the first tile's
-    for (int i = threadIdx.x; i < PLAIN_TAB; i += PLAIN_THREADS) {   // barrier publishes it
-        double sn, cs;
-        sincospi((double)i * (2.0 / PLAIN_TAB), &sn, &cs);
-        s_tab[i] = make_double2(cs, sn);
-    }
+    __shared__ double2 s_tab[PH_TAB * PH_COPIES];
+    phasor_table_init(s_tab, PLAIN_THREADS);   // the first tile's barrier publishes it
+    const double2 *copy = s_tab + (threadIdx.x & (PH_COPIES - 1));
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int lpc = 1 << lpc_log2;
     const int cgroup = warp / nzw, zw = warp - cgroup * nzw;
@@ -139,7 +115,7 @@ k2_plain_kernel(TabView t, CandView c, int64_t n_use, int64_t chunk, double k, i
                 uint64_t hi, lo;
                 phase128_exact(v0[i], v1[i], v2[i], v3[i], r.g0, r.g1, r.g2, r.g3, r.g4, hi, lo);
                 double s, co;
-                sincos_phase64_tab(hi, s_tab, s, co);
+                phasor((hi >> 4) + (1ull << 51), copy, co, s);
                 double wre = fma(r.wcr, co, -r.wci * s);
                 double wim = fma(r.wcr, s, r.wci * co);
                 sv[i] += wre;
@@ -190,27 +166,60 @@ k2_plain_kernel(TabView t, CandView c, int64_t n_use, int64_t chunk, double k, i
     }
 }
 
-// Sum the per-chunk partials in chunk order (deterministic) and apply the factors 2, -2, -2.
-__global__ void reduce_partials_kernel(const double *partial, int64_t P, int n_chunk, double *val,
-                                       double *dd, double *dk) {
-    int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (p >= P) return;
+// Sum the per-chunk partials (deterministic) and apply the factors 2, -2, -2: eight candidates per CTA, 32
+// chunk lanes each, the lanes then added pairwise.  (One thread per candidate adding 40 chunks took 12 us of
+// a 64-candidate call; now 3.)
+constexpr int PRED_LANES = 32, PRED_CANDS = 8;
+__global__ void __launch_bounds__(PRED_LANES *PRED_CANDS)
+reduce_partials_kernel(const double *partial, int64_t P, int n_chunk, double *val, double *dd, double *dk) {
+    __shared__ double red[3][PRED_LANES][PRED_CANDS];
+    const int q = threadIdx.x & (PRED_CANDS - 1), r = threadIdx.x / PRED_CANDS;
+    const int64_t p = (int64_t)blockIdx.x * PRED_CANDS + q;
     double a = 0, b = 0, e = 0;
-    for (int ch = 0; ch < n_chunk; ++ch) {
-        const double *o = partial + ((int64_t)ch * P + p) * 3;
-        a += o[0]; b += o[1]; e += o[2];
+    if (p < P)
+#pragma unroll 4
+        for (int ch = r; ch < n_chunk; ch += PRED_LANES) {
+            const double *o = partial + ((int64_t)ch * P + p) * 3;
+            a += o[0]; b += o[1]; e += o[2];
+        }
+    red[0][r][q] = a;
+    red[1][r][q] = b;
+    red[2][r][q] = e;
+    for (int h = PRED_LANES / 2; h > 0; h >>= 1) {
+        __syncthreads();
+        if (r < h)
+#pragma unroll
+            for (int i = 0; i < 3; ++i) red[i][r][q] += red[i][r + h][q];
     }
-    if (val) val[p] = 2.0 * a;
-    if (dd) dd[p] = -2.0 * b;
-    if (dk) dk[p] = -2.0 * e;
+    if (p < P && r == 0) {
+        if (val) val[p] = 2.0 * red[0][0][q];
+        if (dd) dd[p] = -2.0 * red[1][0][q];
+        if (dk) dk[p] = -2.0 * red[2][0][q];
+    }
 }
+static unsigned pred_blocks(int64_t P) { return (unsigned)((P + PRED_CANDS - 1) / PRED_CANDS); }
 
 static PlainShape plain_shape(int64_t P) {
     if (P >= 2048) return {2, 0, 1};
-    if (P >= 256) return {1, 0, 1};
+    // four lanes per candidate, 64 candidates per CTA: the same rate as one lane each and 256 per CTA (252 G
+    // terms/s on 466,659 zeros) with a quarter of the padding (300 candidates: 1,026 -> 592 us)
     if (P >= 64) return {1, 2, 1};
     if (P >= 8) return {1, 5, 1};
     return {1, 5, 8};
+}
+
+// Zero chunks of a launch: about eight CTAs per SM in all, a chunk whole tiles -- or, where the zeros are
+// too few for that, quarter tiles, so that a small call still spreads over the SMs (64 candidates x 10,000
+// zeros: 40 -> 157 CTAs).  At most max_chunks (0: no limit).
+struct PlainChunks {
+    int64_t chunk, n;
+};
+static PlainChunks plain_chunks(int64_t n_ctile, int64_t n_use, int sms, int64_t max_chunks) {
+    int64_t want = std::max<int64_t>(1, ((int64_t)sms * 8 + n_ctile - 1) / n_ctile);
+    if (max_chunks > 0) want = std::min(want, max_chunks);
+    const int64_t unit = n_use >= want * PLAIN_TILE ? PLAIN_TILE : PLAIN_TILE / 4;
+    const int64_t chunk = std::max<int64_t>(1, ((n_use + want - 1) / want + unit - 1) / unit) * unit;
+    return {chunk, std::max<int64_t>(1, (n_use + chunk - 1) / chunk)};
 }
 
 static int sm_count(int device) {
@@ -261,14 +270,9 @@ int launch_plain(Table &t, CandView c, int64_t n_use, double k, double *d_val, d
     PlainShape sh = plain_shape(c.P);
     int64_t cta_c = sh.cands_per_cta();
     int64_t n_ctile = (c.P + cta_c - 1) / cta_c;
-    int64_t target = (int64_t)sm_count(t.device) * 8;          // ~4 waves of 2 CTAs/SM
-    int64_t n_chunk = std::max<int64_t>(1, (target + n_ctile - 1) / n_ctile);
-    int64_t max_chunks = std::max<int64_t>(1, (n_use + PLAIN_TILE - 1) / PLAIN_TILE);
-    n_chunk = std::min(n_chunk, max_chunks);
-    int64_t chunk = (n_use + n_chunk - 1) / n_chunk;
-    chunk = ((chunk + PLAIN_TILE - 1) / PLAIN_TILE) * PLAIN_TILE;
-    if (chunk == 0) chunk = PLAIN_TILE;
-    n_chunk = std::max<int64_t>(1, (n_use + chunk - 1) / chunk);
+    const PlainChunks pc = plain_chunks(n_ctile, n_use, sm_count(t.device), 0);
+    const int64_t chunk = pc.chunk;
+    int64_t n_chunk = pc.n;
     size_t need = (size_t)n_chunk * c.P * 3 * sizeof(double);
     double *partial = d_partial_override;
     if (partial) {
@@ -291,7 +295,7 @@ int launch_plain(Table &t, CandView c, int64_t n_use, double k, double *d_val, d
             k2_plain_kernel<1><<<grid, PLAIN_THREADS, 0, s>>>(view(t), c, n_use, chunk, k, sh.lpc_log2, sh.nzw, partial);
         MB_CUDA(cudaGetLastError());
     }
-    reduce_partials_kernel<<<(unsigned)((c.P + 255) / 256), 256, 0, s>>>(partial, c.P, (int)n_chunk, d_val, d_dd, d_dk);
+    reduce_partials_kernel<<<pred_blocks(c.P), PRED_LANES * PRED_CANDS, 0, s>>>(partial, c.P, (int)n_chunk, d_val, d_dd, d_dk);
     MB_CUDA(cudaGetLastError());
     return MB_OK;
 }
@@ -389,12 +393,9 @@ extern "C" int mb_k2_plain_noalloc_dev(const uint32_t *d_g, const double *d_gamm
     PlainShape sh = plain_shape(P);
     int64_t cta_c = sh.cands_per_cta();
     int64_t n_ctile = (P + cta_c - 1) / cta_c;
-    int64_t n_chunk = std::max<int64_t>(1, ((int64_t)sm_count(dev) * 8 + n_ctile - 1) / n_ctile);
-    n_chunk = std::min(n_chunk, std::max<int64_t>(1, (n_use + PLAIN_TILE - 1) / PLAIN_TILE));
-    n_chunk = std::min(n_chunk, NOALLOC_PARTIAL_DOUBLES / (3 * P));      // fits the fixed array
-    int64_t chunk = std::max<int64_t>(1, (n_use + n_chunk - 1) / n_chunk);
-    chunk = ((chunk + PLAIN_TILE - 1) / PLAIN_TILE) * PLAIN_TILE;
-    n_chunk = std::max<int64_t>(1, (n_use + chunk - 1) / chunk);
+    const PlainChunks pc = plain_chunks(n_ctile, n_use, sm_count(dev), NOALLOC_PARTIAL_DOUBLES / (3 * P));   // fits the array
+    const int64_t chunk = pc.chunk;
+    int64_t n_chunk = pc.n;
     if (n_use == 0) {
         // nothing to sum: clear the one chunk the reduction reads
         MB_CUDA(cudaMemsetAsync(partial, 0, (size_t)P * 3 * sizeof(double), s));
@@ -407,7 +408,7 @@ extern "C" int mb_k2_plain_noalloc_dev(const uint32_t *d_g, const double *d_gamm
             k2_plain_kernel<1><<<grid, PLAIN_THREADS, 0, s>>>(tv, c, n_use, chunk, k, sh.lpc_log2, sh.nzw, partial);
         MB_CUDA(cudaGetLastError());
     }
-    reduce_partials_kernel<<<(unsigned)((P + 255) / 256), 256, 0, s>>>(partial, P, (int)n_chunk, d_val, d_dd, d_dk);
+    reduce_partials_kernel<<<pred_blocks(P), PRED_LANES * PRED_CANDS, 0, s>>>(partial, P, (int)n_chunk, d_val, d_dd, d_dk);
     MB_CUDA(cudaGetLastError());
     return MB_OK;
 }
