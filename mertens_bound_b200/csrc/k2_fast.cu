@@ -2,8 +2,8 @@
 //
 // Each group (k, T, a range of candidates) splits its zeros [0, n_T) at a boundary n_h chosen
 // from an a-priori error bound (host, k2_plan.cu):
-//   heavy tier  j <  n_h : 64-bit phase (3 IMAD.lo + 4 DFMA + 4 FFMA, error ~2^-48 turn), sin/cos
-//                          from a 2048-entry table rotated by short FP64 polynomials, FP64
+//   heavy tier  j <  n_h : 64-bit phase (3 IMAD.lo + 4 DFMA, error ~2^-48 turn), sin/cos
+//                          from a 256-entry table rotated by short FP64 polynomials, FP64
 //                          accumulation.                                  -> k2_heavy_kernel
 //   light tier  j >= n_h : 32-bit phase (3 IMAD.lo + 4 DFMA in two chains; 2 IMAD.lo + 3 DFMA
 //                          when every zero has gamma < 3.29e6, light_phase32_fused), MUFU sin/cos
@@ -30,6 +30,7 @@
 #include "k2_fast.h"
 #include "k2_internal.h"
 #include "k2_light.cuh"
+#include "k2_phasor.cuh"
 
 namespace mb {
 
@@ -48,13 +49,13 @@ struct __align__(16) ZLightF {  // 48 B: the light record of light_phase32_fused
     float b, d;                  // b = -a gamma, d = -a gamma^2
 };
 
-struct __align__(16) ZHeavy {   // 96 B
-    uint32_t b0, b1, gi, psi_hi; // psi_hi = top 32 bits of arg(c)/2pi 2^64, plus 2^20 (half a table step)
-    double b0s, c1s, gis, b1s;   // limb 2^-32
-    float c0f, c1f, b0f, b1f;    // limb 2^-64 (FP32: these products need 2^-18 relative)
-    float psi_lo, pad0;          // low 32 bits of arg(c)/2pi 2^64, times 2^-32
+struct __align__(16) ZHeavy {   // 80 B
+    uint32_t b0, b1, gi, psi_hi; // psi_hi = top 32 bits of arg(c)/2pi 2^64, plus 2^23 (half a table step)
+    double B0, C1, B1, GI;       // b0, c1, b1, gI and the limb below each, 2^-32 (rounded to 53 bits)
+    double psi_lo;               // low 32 bits of arg(c)/2pi 2^64, times 2^-32
     double a, b, d;
 };
+static_assert(sizeof(ZHeavy) == 80, "heavy record");
 
 constexpr int FAST_THREADS = 256;
 constexpr int LIGHT_TILE = 256;
@@ -120,32 +121,31 @@ MB_DEV void light_tile(const void *tile_v, int nt, int zl, int ZL, const CandReg
     flush();
 }
 
-// sin/cos(2 pi (q/2048 + r)) for |r| <= 2^-12 turn: the table entry (cos, sin)(2 pi q/2048)
-// rotated by r: sin(2 pi r) = r (2pi - (2pi)^3 r^2 / 6) (truncation 7e-17) and
-// cos(2 pi r) - 1 = C r^2 with C the minimax constant on |r| <= 2^-12 (-(2pi)^2/2 + 3.2e-6:
-// error 3.96e-14, computed with mpmath), so the cosine costs one product.
-constexpr int HEAVY_TAB = 2048;
-constexpr int HEAVY_TAB_BYTES = HEAVY_TAB * (int)sizeof(double2);
-MB_DEV void sincos_rotate(double2 T, double r, double &sn, double &cs) {
-    const double u = r * r;
-    const double s = r * fma(u, -41.341702240399755, 6.283185307179586);     // sin(2 pi r)
-    const double cm1 = u * -19.739205595594533;                            // cos(2 pi r) - 1
-    cs = fma(T.x, cm1, fma(-T.y, s, T.x));
-    sn = fma(T.y, cm1, fma(T.x, s, T.y));
+// The heavy tier's (cos, sin) table is k2_phasor.cuh's: 256 entries in eight interleaved copies, read without
+// bank conflicts.  (One copy of 2048 entries cost 9.4 shared-memory cycles per warp and term, more than the
+// term's 17 FP64 operations take on their pipe; this one costs 4.2 and two more operations.)  An entry is
+// rotated by d 2^-49 turn, |d| <= 2^40 (0.0123 rad); with a = 2 pi 2^-49:
+//   sin(a d)     = d (a - a^3 d^2 / 6 + a^5 d^4 / 120)    (truncation 8.4e-18)
+//   cos(a d) - 1 = d^2 (-a^2 / 2 + a^4 d^2 / 24)          (truncation 4.7e-15)
+constexpr int HEAVY_TAB_BYTES = PH_BYTES;
+MB_DEV void sincos_rotate(double2 T, double d, double &sn, double &cs) {
+    constexpr double a = 6.283185307179586 * 0x1p-49;
+    const double u = d * d;
+    const double s = d * fma(u, fma(u, a * a * a * a * a / 120.0, -a * a * a / 6.0), a);
+    const double m = u * fma(u, a * a * a * a / 24.0, -a * a / 2.0);
+    cs = fma(T.x, m, fma(-T.y, s, T.x));
+    sn = fma(T.y, m, fma(T.x, s, T.y));
 }
 
 // The heavy tier's shared memory: the staged tile / reduction buffer, then the (cos, sin) table
 // (dynamic shared memory: 24 KB + 32 KB is above the 48 KB static limit).
 constexpr int HEAVY_DSMEM = FAST_SMEM + HEAVY_TAB_BYTES;
 
-MB_DEV double2 *heavy_table_init(unsigned char *dsm) {
+// Fills the table; returns this lane's copy.
+MB_DEV const double2 *heavy_table_init(unsigned char *dsm) {
     double2 *tab = reinterpret_cast<double2 *>(dsm + FAST_SMEM);
-    for (int i = threadIdx.x; i < HEAVY_TAB; i += FAST_THREADS) {
-        double sn, cs;
-        sincospi((double)i * (2.0 / HEAVY_TAB), &sn, &cs);
-        tab[i] = make_double2(cs, sn);
-    }
-    return tab;
+    phasor_table_init(tab, FAST_THREADS);
+    return tab + (threadIdx.x & (PH_COPIES - 1));
 }
 
 // 1.5 2^35: a sum x in [0, 2^34) units of 2^-32 turn added to it rounds to a multiple of 2^-17
@@ -153,32 +153,31 @@ MB_DEV double2 *heavy_table_init(unsigned char *dsm) {
 constexpr double HEAVY_MAGIC = 51539607552.0;
 
 // The heavy term's phase in units of 2^-32 turn, T = L + F mod 2^32 with
-//   L = a1 b0 + a0 b1 + d1 gI + psi_hi (+ 2^20)     exact mod 2^32 (IMAD.lo)
-//   F = (a0 b0 + a1 c1 + d0 gI + d1 b1) 2^-32       < 2^34, two FP64 chains, one on HEAVY_MAGIC
-//     + (a1 c0 + a0 c1 + d1 b0 + d0 b1) 2^-64 + psi_lo   < 5, FP32
-// (error <= 2^-16 unit = 2^-48 turn).  The bits of HEAVY_MAGIC + F plus L 2^17 (one 64-bit
-// integer multiply-add) are T 2^17: bits [38, 49) are the table index q, bits [0, 38) the offset
-// R, and r = R 2^-49 - 2^-12 turn is exact as (2^52 + R) 2^-49 - (8 + 2^-12).
+//   L = a1 b0 + a0 b1 + d1 gI + psi_hi (+ 2^23)     exact mod 2^32 (IMAD.lo)
+//   F = a0 B0 + a1 C1 + d1 B1 + d0 GI + psi_lo      < 2^34, two FP64 chains, one on HEAVY_MAGIC,
+// B0 = (b0 + c1 2^-32) 2^-32 and so on: each of v's limbs meets G's next two limbs in one product, whose
+// 53-bit rounding is 2^-22 unit (error of T <= 2^-16 unit = 2^-48 turn).  The bits of HEAVY_MAGIC + F plus
+// L 2^17 (one 64-bit integer multiply-add) are T 2^17: bits [41, 49) are the table index q, bits [0, 41) the
+// offset R, and d = R - 2^40 in units of 2^-49 turn is exact as (2^52 + R) - (2^52 + 2^40).
 template <int CPT>
 MB_DEV void heavy_tile(const ZHeavy *tile, int nt, int zl, int ZL, const CandRegs (&cr)[CPT],
-                       double (&acc)[CPT][3], const double2 *tab) {
+                       double (&acc)[CPT][3], const double2 *copy) {
     for (int jj = zl; jj < nt; jj += ZL) {
         const ZHeavy z = tile[jj];
 #pragma unroll
         for (int i = 0; i < CPT; ++i) {
             const uint32_t L = cr[i].a1 * z.b0 + cr[i].a0 * z.b1 + cr[i].d1 * z.gi + z.psi_hi;
-            const float low = fmaf(__uint2float_rn(cr[i].a1), z.c0f, fmaf(__uint2float_rn(cr[i].a0), z.c1f,
-                              fmaf(__uint2float_rn(cr[i].d1), z.b0f,
-                              fmaf(__uint2float_rn(cr[i].d0), z.b1f, z.psi_lo))));
-            const double p1 = fma(cr[i].A0, z.b0s, fma(cr[i].A1, z.c1s, (double)low));
-            const double p2 = fma(cr[i].D0, z.gis, fma(cr[i].D1, z.b1s, HEAVY_MAGIC));
+            const double p1 = fma(cr[i].A0, z.B0, fma(cr[i].A1, z.C1, z.psi_lo));
+            const double p2 = fma(cr[i].D0, z.GI, fma(cr[i].D1, z.B1, HEAVY_MAGIC));
             const unsigned long long w =
                 (unsigned long long)L * 131072ull + (unsigned long long)__double_as_longlong(p1 + p2);
             const uint32_t wh = (uint32_t)(w >> 32);
-            const double r = fma(__hiloint2double((int)((wh & 0x3Fu) | 0x43300000u), (int)(uint32_t)w),
-                                 1.7763568394002505e-15, -8.000244140625);        // 2^-49, 8 + 2^-12
+            const double d = __hiloint2double((int)((wh & 0x1FFu) | 0x43300000u), (int)(uint32_t)w) - 4504699138998272.0;
+            // entry q of the lane's copy, 128 bytes apart
+            const double2 T = *reinterpret_cast<const double2 *>(reinterpret_cast<const char *>(copy) +
+                                                                 ((wh >> 2) & (uint32_t)((PH_TAB - 1) * PH_COPIES * 16)));
             double sn, cs;
-            sincos_rotate(tab[(wh >> 6) & (HEAVY_TAB - 1)], r, sn, cs);
+            sincos_rotate(T, d, sn, cs);
             acc[i][0] = fma(z.a, cs, acc[i][0]);
             acc[i][1] = fma(z.b, sn, acc[i][1]);
             acc[i][2] = fma(z.d, cs, acc[i][2]);
@@ -225,18 +224,13 @@ MB_DEV void stage_heavy(const TabView &t, int64_t j, double k, const double *w, 
     double a = 2.0 * t.alpha[j] * (w ? w[j] : exp(-k * g * g));
     uint32_t c0 = t.g0[j], c1 = t.g1[j], b0 = t.g2[j], b1 = t.g3[j], gi = t.g4[j];
     r.b0 = b0; r.b1 = b1; r.gi = gi;
-    r.b0s = u32_to_f64(b0) * TWO_M32;
-    r.c1s = u32_to_f64(c1) * TWO_M32;
-    r.gis = u32_to_f64(gi) * TWO_M32;
-    r.b1s = u32_to_f64(b1) * TWO_M32;
-    r.c0f = (float)(u32_to_f64(c0) * TWO_M64);
-    r.c1f = (float)(u32_to_f64(c1) * TWO_M64);
-    r.b0f = (float)(u32_to_f64(b0) * TWO_M64);
-    r.b1f = (float)(u32_to_f64(b1) * TWO_M64);
+    r.B0 = fma(u32_to_f64(c1), TWO_M64, u32_to_f64(b0) * TWO_M32);
+    r.C1 = fma(u32_to_f64(c0), TWO_M64, u32_to_f64(c1) * TWO_M32);
+    r.B1 = fma(u32_to_f64(b0), TWO_M64, u32_to_f64(b1) * TWO_M32);
+    r.GI = fma(u32_to_f64(b1), TWO_M64, u32_to_f64(gi) * TWO_M32);
     const uint64_t ps = t.psi[j];
-    r.psi_hi = (uint32_t)(ps >> 32) + (1u << 20);
-    r.psi_lo = (float)(u32_to_f64((uint32_t)ps) * TWO_M32);
-    r.pad0 = 0.f;
+    r.psi_hi = (uint32_t)(ps >> 32) + (1u << 23);
+    r.psi_lo = u32_to_f64((uint32_t)ps) * TWO_M32;
     r.a = a;
     r.b = -a * g;
     r.d = -a * g * g;
@@ -304,7 +298,7 @@ MB_DEV void light_item(const FastItem &it, const FastGroup &gr, const TabView &t
 
 template <int CPT>
 MB_DEV void heavy_item(const FastItem &it, const FastGroup &gr, const TabView &t, const CandView &c,
-                       double *partial, unsigned char *smem, const double2 *tab) {
+                       double *partial, unsigned char *smem, const double2 *copy) {
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int nzw = it.nzw;
     const int cgroup = warp / nzw, zw = warp - cgroup * nzw;
@@ -322,7 +316,7 @@ MB_DEV void heavy_item(const FastItem &it, const FastGroup &gr, const TabView &t
         int64_t j = tb + threadIdx.x;
         if (threadIdx.x < HEAVY_TILE && j < it.z1) stage_heavy(t, j, gr.k, gr.w, tile[threadIdx.x]);
         __syncthreads();
-        heavy_tile<CPT>(tile, (int)min((int64_t)HEAVY_TILE, it.z1 - tb), zw, nzw, cr, res, tab);
+        heavy_tile<CPT>(tile, (int)min((int64_t)HEAVY_TILE, it.z1 - tb), zw, nzw, cr, res, copy);
     }
     finish_item<CPT>(it, gr, res, warp, lane, zw, cbase, cend, partial, smem);
 }
@@ -334,7 +328,7 @@ k2_heavy_kernel(TabView t, CandView c, const FastItem *items, int n_items, const
                 int *counter, double *partial) {
     extern __shared__ __align__(16) unsigned char smem[];
     __shared__ int s_item;
-    const double2 *s_tab = heavy_table_init(smem);
+    const double2 *copy = heavy_table_init(smem);
     for (;;) {
         __syncthreads();
         if (threadIdx.x == 0) s_item = atomicAdd(counter, 1);
@@ -342,7 +336,7 @@ k2_heavy_kernel(TabView t, CandView c, const FastItem *items, int n_items, const
         const int idx = s_item;
         if (idx >= n_items) break;
         const FastItem it = items[idx];
-        heavy_item<HEAVY_CPT>(it, groups[it.group], t, c, partial, smem, s_tab);
+        heavy_item<HEAVY_CPT>(it, groups[it.group], t, c, partial, smem, copy);
     }
 }
 
@@ -370,7 +364,7 @@ k2_tiers_kernel(TabView t, CandView c, const FastItem *items, int n_items, int n
                 int *counter, double *partial) {
     extern __shared__ __align__(16) unsigned char smem[];
     __shared__ int s_item, s_queue;
-    const double2 *s_tab = heavy_table_init(smem);
+    const double2 *copy = heavy_table_init(smem);
     if (threadIdx.x == 0 && n_first > 0) {
         unsigned smid;
         asm volatile("mov.u32 %0, %%smid;" : "=r"(smid));
@@ -400,7 +394,7 @@ k2_tiers_kernel(TabView t, CandView c, const FastItem *items, int n_items, int n
         if (idx >= n_items) break;
         const FastItem it = items[idx];
         if (it.tier == 0)
-            heavy_item<HEAVY_CPT>(it, groups[it.group], t, c, partial, smem, s_tab);
+            heavy_item<HEAVY_CPT>(it, groups[it.group], t, c, partial, smem, copy);
         else
             light_item<CPT, FUSED>(it, groups[it.group], t, c, partial, smem);
     }
