@@ -164,7 +164,7 @@ void replan_tiers(mb_plan *p) {
 
 // Work items.  Heavy items (FP64 tier) use HEAVY_CPT candidates per thread and are pulled by
 // the persistent heavy kernel (two CTAs per SM); light items use the plan's light_cpt and run
-// one CTA each.  Chunk sizes aim at ~4 heavy items and ~18 light items per SM.
+// one CTA each.  Chunk sizes aim at ~4 heavy items per SM and ~5 light items per CTA slot.
 int build_items(mb_plan *p, int sms) {
     p->groups.clear();
     p->items.clear();
@@ -174,14 +174,21 @@ int build_items(mb_plan *p, int sms) {
     auto he = [&](int g) { return std::min(p->n_heavy[g], p->z_end); };
     auto lb = [&](int g) { return std::max(p->n_heavy[g], p->z_begin); };
     auto le = [&](int g) { return std::min(p->n_eval[g], p->z_end); };
-    double Wh = 0, Wl = 0;
+    auto light_tile = [&](int g) { return (int64_t)(8 / p->shape_nzw[g]) * 32 * p->light_cpt; };
+    double Wh = 0, Ul = 0;
     for (int g = 0; g < p->n_groups; ++g) {
         Wh += (double)p->counts[g] * std::max<int64_t>(0, he(g) - hb(g));
-        Wl += (double)p->counts[g] * std::max<int64_t>(0, le(g) - lb(g));
+        Ul += (double)((p->counts[g] + light_tile(g) - 1) / light_tile(g)) * std::max<int64_t>(0, le(g) - lb(g));
     }
-    // ~4 heavy items per SM (two per heavy CTA) and ~18 light items per SM (several waves)
+    // ~4 heavy items per SM (two per heavy CTA)
     const double target_h = std::max(p->chunk_scale * Wh / (4.0 * sms), 1.0);
-    const double target_l = std::max(p->chunk_scale * Wl / (18.0 * sms), 1.0);
+    // Light chunks, largest first: four fifths of a group's zeros in chunks of a third, the rest in chunks of a
+    // twelfth of Ul, the zeros that fall to one light CTA slot.  Chunks of a fixed size or more left a
+    // thousand candidates' 156 chunks of 2,048 zeros (and 296 of 512) to 296 slots: the last ended 29%
+    // after the average one (1,001 x 600,000: 739 -> 641 us).  Other splits (a half in halves, and so on down to
+    // twentieths; six levels' worth of sizes) were within 2%.
+    const int slots = sms * (p->light_cpt == 2 ? 4 : (p->light_cpt == 3 ? 3 : 2));
+    Ul = p->chunk_scale * Ul / slots;
     std::vector<FastItem> heavy, light;
     int64_t c0 = 0, pbase = 0;
     for (int g = 0; g < p->n_groups; ++g) {
@@ -193,27 +200,25 @@ int build_items(mb_plan *p, int sms) {
         gr.pbase = pbase;
         const int nzw = p->shape_nzw[g];
         const int64_t CTh = (int64_t)(8 / nzw) * 32 * HEAVY_CPT;
-        const int64_t CTl = (int64_t)(8 / nzw) * 32 * p->light_cpt;
-        int64_t hz = p->heavy_chunk[g], lz = p->light_chunk[g];
-        // chunk = target terms / tile candidates, rounded to whole tiles (at least 1 heavy tile of
-        // 128 zeros and 8 light tiles of 256: finer heavy items balance the persistent kernel,
-        // coarser light items cost less per term -- both measured)
+        const int64_t CTl = light_tile(g);
+        int64_t hz = p->heavy_chunk[g];
+        const int64_t lz = p->light_chunk[g];
+        // chunk = target terms / tile candidates, rounded to whole tiles (at least one heavy tile of 128 zeros:
+        // finer heavy items balance the persistent kernel)
         if (hz <= 0)
             hz = std::max<int64_t>(128, ((int64_t)(target_h / std::min<int64_t>(CTh, std::max<int64_t>(gr.nc, 1))) + 64) / 128 * 128);
-        // the last light chunks of a group are a quarter of the size, about one round of CTA slots
-        // in all (this group's share of it), so the light items' last wave -- they run largest
-        // first -- ends in small items instead of leaving SMs idle behind full-size ones
-        int64_t small_lz = 0, small_from = le(g);
-        if (lz <= 0) {
-            lz = std::max<int64_t>(2048, ((int64_t)(target_l / std::min<int64_t>(CTl, std::max<int64_t>(gr.nc, 1))) + 128) / 256 * 256);
-            const int per_sm = p->light_cpt == 2 ? 4 : (p->light_cpt == 3 ? 3 : 2);
-            const double wg = (double)gr.nc * std::max<int64_t>(0, le(g) - lb(g));
-            const int64_t n_tiles = std::max<int64_t>(1, (gr.nc + CTl - 1) / CTl);
-            const int64_t items = (int64_t)std::ceil((double)sms * per_sm * (Wl > 0 ? wg / Wl : 0.0));
-            small_lz = std::max<int64_t>(256, lz / 4 / 256 * 256);
-            const int64_t span = ((items + n_tiles - 1) / n_tiles) * small_lz;
-            if (span > 0 && le(g) - lb(g) > 2 * span) small_from = le(g) - span;
-        }
+        // light chunk ends: whole flush windows of every warp (32 nzw zeros from the group's first light zero),
+        // so the FP32 sums are the same whatever the sizes
+        const int64_t unit = 32 * nzw, L = std::max<int64_t>(0, le(g) - lb(g));
+        auto windows = [&](double zeros) { return std::max<int64_t>(1, (int64_t)(zeros / unit + 0.5)) * unit; };
+        struct Level {
+            int64_t end, size;
+        };
+        const Level fixed[1] = {{le(g), lz}};
+        const Level guided[2] = {{lb(g) + std::min(L, windows(0.8 * L)), std::max<int64_t>(windows(Ul / 3), 128)},
+                                 {le(g), std::max<int64_t>(windows(Ul / 12), 128)}};
+        const Level *levels = lz > 0 ? fixed : guided;
+        const int n_levels = lz > 0 ? 1 : 2;
         int ch = 0;
         auto emit = [&](int64_t z0, int64_t z1, int tier, int64_t CT, int cpt, std::vector<FastItem> &dst) {
             for (int64_t ct = 0; ct * CT < gr.nc; ++ct) {
@@ -233,10 +238,10 @@ int build_items(mb_plan *p, int sms) {
         };
         for (int64_t z = hb(g); z < he(g); z += hz)
             emit(z, std::min(z + hz, he(g)), 0, CTh, HEAVY_CPT, heavy);
-        for (int64_t z = lb(g); z < small_from; z += lz)
-            emit(z, std::min(z + lz, small_from), 1, CTl, p->light_cpt, light);
-        for (int64_t z = small_from; z < le(g); z += small_lz)
-            emit(z, std::min(z + small_lz, le(g)), 1, CTl, p->light_cpt, light);
+        int64_t z = lb(g);
+        for (int v = 0; v < n_levels; ++v)
+            for (; z < levels[v].end; z += levels[v].size)
+                emit(z, std::min(z + levels[v].size, le(g)), 1, CTl, p->light_cpt, light);
         gr.n_chunks = ch;
         p->zero_terms += (double)gr.nc * (std::max<int64_t>(0, he(g) - hb(g)) + std::max<int64_t>(0, le(g) - lb(g)));
         pbase += (int64_t)gr.n_chunks * gr.nc * 3;
