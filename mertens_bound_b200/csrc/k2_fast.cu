@@ -321,6 +321,41 @@ MB_DEV void heavy_item(const FastItem &it, const FastGroup &gr, const TabView &t
     finish_item<CPT>(it, gr, res, warp, lane, zw, cbase, cend, partial, smem);
 }
 
+// A heavy item of at most 32 candidates (tiles of 128 would leave most lanes idle): one candidate per lane,
+// the lanes left over and the warps split the zeros.  clog: log2 of the candidate lanes, a power of two.
+// Kept out of line: inlined it costs the large items' loop registers (24 bytes of spills).
+static __device__ __noinline__ void heavy_item_small(const FastItem &it, const FastGroup &gr, const TabView &t, const CandView &c,
+                             double *partial, unsigned char *smem, const double2 *copy) {
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int clog = it.nc <= 1 ? 0 : 32 - __clz(it.nc - 1);
+    const int cl = lane & ((1 << clog) - 1), zsplit = 32 >> clog;
+    const bool live = cl < it.nc;
+    CandRegs cr[1] = {cand_regs(c, it.c0 + cl, live)};
+    ZHeavy *tile = reinterpret_cast<ZHeavy *>(smem);
+    double res[1][3] = {{0.0, 0.0, 0.0}};
+    for (int64_t tb = it.z0; tb < it.z1; tb += HEAVY_TILE) {
+        __syncthreads();
+        const int64_t j = tb + threadIdx.x;
+        if (threadIdx.x < HEAVY_TILE && j < it.z1) stage_heavy(t, j, gr.k, gr.w, tile[threadIdx.x]);
+        __syncthreads();
+        heavy_tile<1>(tile, (int)min((int64_t)HEAVY_TILE, it.z1 - tb), warp * zsplit + (lane >> clog),
+                      zsplit * (FAST_THREADS / 32), cr, res, copy);
+    }
+    double *red = reinterpret_cast<double *>(smem);      // [warp][candidate][3]
+    __syncthreads();
+#pragma unroll
+    for (int q = 0; q < 3; ++q) {
+        for (int o = 16; o >= 1 << clog; o >>= 1) res[0][q] += __shfl_xor_sync(0xffffffffu, res[0][q], o);
+        if (lane < 1 << clog) red[(warp * 32 + lane) * 3 + q] = res[0][q];
+    }
+    __syncthreads();
+    for (int i = threadIdx.x; i < it.nc * 3; i += FAST_THREADS) {
+        double x = 0.0;
+        for (int w = 0; w < FAST_THREADS / 32; ++w) x += red[w * 96 + i];
+        partial[it.pbase + (it.c0 - gr.c0) * 3 + i] = x;
+    }
+}
+
 // Heavy tier: persistent, items pulled from an atomic counter (largest first).  At most 128
 // registers per thread: two CTAs per SM.
 __global__ void __launch_bounds__(FAST_THREADS, 2)
@@ -329,15 +364,20 @@ k2_heavy_kernel(TabView t, CandView c, const FastItem *items, int n_items, const
     extern __shared__ __align__(16) unsigned char smem[];
     __shared__ int s_item;
     const double2 *copy = heavy_table_init(smem);
-    for (;;) {
-        __syncthreads();
-        if (threadIdx.x == 0) s_item = atomicAdd(counter, 1);
-        __syncthreads();
-        const int idx = s_item;
-        if (idx >= n_items) break;
+    const bool queue = gridDim.x < n_items;      // else a CTA per item: no queue (and no counter to reset)
+    do {
+        int idx = blockIdx.x;
+        if (queue) {
+            __syncthreads();
+            if (threadIdx.x == 0) s_item = atomicAdd(counter, 1);
+            __syncthreads();
+            idx = s_item;
+            if (idx >= n_items) break;
+        }
         const FastItem it = items[idx];
-        heavy_item<HEAVY_CPT>(it, groups[it.group], t, c, partial, smem, copy);
-    }
+        if (it.cpt == 1) heavy_item_small(it, groups[it.group], t, c, partial, smem, copy);
+        else heavy_item<HEAVY_CPT>(it, groups[it.group], t, c, partial, smem, copy);
+    } while (queue);
 }
 
 // Light tier: one CTA per item.  MINB sets the register budget (65536 / (256 MINB)).
@@ -393,7 +433,9 @@ k2_tiers_kernel(TabView t, CandView c, const FastItem *items, int n_items, int n
         const int idx = s_item;
         if (idx >= n_items) break;
         const FastItem it = items[idx];
-        if (it.tier == 0)
+        if (it.tier == 0 && it.cpt == 1)
+            heavy_item_small(it, groups[it.group], t, c, partial, smem, copy);
+        else if (it.tier == 0)
             heavy_item<HEAVY_CPT>(it, groups[it.group], t, c, partial, smem, copy);
         else
             light_item<CPT, FUSED>(it, groups[it.group], t, c, partial, smem);
@@ -578,7 +620,7 @@ int launch_fast(const Table &t, const FastPlanDev &pd, CandView c, double *d_val
             MB_CUDA(cudaEventRecord(t.ev_fork, s));
             MB_CUDA(cudaStreamWaitEvent(t.side, t.ev_fork, 0));
         }
-        MB_CUDA(cudaMemsetAsync(pd.counter, 0, sizeof(int), hs));
+        if ((int)pd.heavy_grid < pd.n_heavy) MB_CUDA(cudaMemsetAsync(pd.counter, 0, sizeof(int), hs));
         if (ev) MB_CUDA(cudaEventRecord(ev->heavy0, hs));
         k2_heavy_kernel<<<pd.heavy_grid, FAST_THREADS, HEAVY_DSMEM, hs>>>(tv, c, pd.items, pd.n_heavy, pd.groups,
                                                                           pd.counter, pd.partial);

@@ -25,12 +25,13 @@ struct FastItem {
     int nc;            // candidates in this tile
     int group;
     int tier;          // 0 heavy (FP64), 1 light (FP32 + MUFU)
-    int cpt;           // candidates per thread: 1, 2 or 4
+    int cpt;           // candidates per thread; 1 in the heavy tier: heavy_item_small
     int nzw;           // warps splitting the zeros of one candidate set: 1..8
     int pad;
 };
 
 constexpr int HEAVY_CPT = 4;     // candidates per thread in the heavy kernel
+constexpr int HEAVY_SMALL = 32;  // groups of at most this many candidates: one per lane, zeros split over the rest
 constexpr int TIERS_COUNTERS = 2 + 256;   // item counters of one launch: two queues + per-SM arrivals
 
 // Device side of a plan: items[0, n_heavy) are heavy-tier items (pulled by the persistent

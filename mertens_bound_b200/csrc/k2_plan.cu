@@ -82,8 +82,6 @@ void free_io(mb_plan *p) {
     if (p->graph) cudaGraphExecDestroy(p->graph);
     p->graph = nullptr;
     cudaFree(p->d_vi);
-    cudaFree(p->d_vf);
-    cudaFree(p->d_delta);
     cudaFree(p->d_out);
     if (p->h_pinned) cudaFreeHost(p->h_pinned);
     p->d_vi = p->d_vf = nullptr;
@@ -236,8 +234,11 @@ int build_items(mb_plan *p, int sms) {
             }
             ++ch;
         };
+        const bool small = gr.nc <= HEAVY_SMALL;
+        // a few candidates' items are short: half a tile each where whole ones would leave SMs idle
+        if (small && p->heavy_chunk[g] <= 0 && he(g) - hb(g) < 128 * (int64_t)sms) hz = 64;
         for (int64_t z = hb(g); z < he(g); z += hz)
-            emit(z, std::min(z + hz, he(g)), 0, CTh, HEAVY_CPT, heavy);
+            emit(z, std::min(z + hz, he(g)), 0, small ? HEAVY_SMALL : CTh, small ? 1 : HEAVY_CPT, heavy);
         int64_t z = lb(g);
         for (int v = 0; v < n_levels; ++v)
             for (; z < levels[v].end; z += levels[v].size)
@@ -333,18 +334,17 @@ int plan_run_timed(mb_plan *p, int tiers, const uint64_t *vi, const uint64_t *vf
 int ensure_io(mb_plan *p) {
     if (p->d_out) return MB_OK;
     size_t P = (size_t)std::max<int64_t>(p->P, 1);
-    MB_CUDA(cudaMalloc(&p->d_vi, P * 8));
-    MB_CUDA(cudaMalloc(&p->d_vf, P * 8));
-    MB_CUDA(cudaMalloc(&p->d_delta, P * 8));
+    // candidates as in the pinned staging buffer, so one copy brings them all
+    MB_CUDA(cudaMalloc(&p->d_vi, 3 * P * 8));
+    p->d_vf = p->d_vi + P;
+    p->d_delta = (double *)(p->d_vi + 2 * P);
     MB_CUDA(cudaMalloc(&p->d_out, 3 * P * 8));
     MB_CUDA(cudaHostAlloc(&p->h_pinned, 6 * P * 8, cudaHostAllocDefault));
     // capture: H2D of the candidates, the kernels, D2H of the results
     cudaStream_t s = p->table->stream;
     char *h = (char *)p->h_pinned;
     MB_CUDA(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
-    cudaMemcpyAsync(p->d_vi, h, P * 8, cudaMemcpyHostToDevice, s);
-    cudaMemcpyAsync(p->d_vf, h + P * 8, P * 8, cudaMemcpyHostToDevice, s);
-    cudaMemcpyAsync(p->d_delta, h + 2 * P * 8, P * 8, cudaMemcpyHostToDevice, s);
+    cudaMemcpyAsync(p->d_vi, h, 3 * P * 8, cudaMemcpyHostToDevice, s);
     int st = plan_run_dev(p, p->d_vi, p->d_vf, p->d_delta, p->d_out, p->d_out + P, p->d_out + 2 * P, s);
     cudaMemcpyAsync(h + 3 * P * 8, p->d_out, 3 * P * 8, cudaMemcpyDeviceToHost, s);
     cudaGraph_t g = nullptr;
