@@ -136,9 +136,11 @@ struct CellShape {
     static constexpr int NTI = NT - I0;
     // row stride in doubles = 4 mod 8: the 4 x 8 B fragment's half warps touch 16 distinct banks
     static constexpr int S = cols + 4;
-    // a tile is TILE zeros x PARTS threads: a weight vector's D1 columns each, or four column groups
-    static constexpr int PARTS = KIND == CELL_WEIGHTS ? W : 4;
-    static constexpr int TILE = KIND == CELL_WEIGHTS && W == 5 ? 48 : 64;
+    // a tile is TILE zeros x PARTS threads: a weight vector's D1 columns each, or two or four column groups
+    // (two with 128 zeros where that leaves shared memory for three CTAs: the zeros' weights are then formed
+    // twice instead of four times, 642 -> 602 us at 256 peaks x 600,000 zeros)
+    static constexpr int PARTS = KIND == CELL_WEIGHTS ? W : (KIND == CELL_GAUSS && D1 == 8 ? 2 : 4);
+    static constexpr int TILE = KIND == CELL_WEIGHTS ? (W == 5 ? 48 : 64) : CELL_THREADS / PARTS;
     static_assert(TILE * PARTS <= CELL_THREADS, "one (zero, part) per thread");
     static constexpr int ctas = KIND == CELL_WEIGHTS ? 2 : 3;       // resident per SM
     static constexpr int smem = PH_BYTES + 2 * TILE * ((int)sizeof(ZRec) + S * 8);
@@ -248,13 +250,15 @@ cell_moments_kernel(TabView t, const uint64_t *vi, const uint64_t *vf, const dou
             // the polishes' offsets turn by the table's FP64 gamma, not 2 pi G
             if constexpr (KIND == CELL_WEIGHTS) y += gamma_excess(gam, g4, g3, g2, g1) * inv_kappa;
             if constexpr (KIND == CELL_GAUSS) {
-                constexpr int C4 = D1 / 4;
-                const double y2 = y * y, y4 = C4 == 2 ? y2 : y2 * y2;
-                double e = al * exp(-k * gam * gam);
-                if (sq & 1) e *= y4;
-                if (sq & 2) e *= y4 * y4;
+                constexpr int C = D1 / Sh::PARTS;          // columns of a group, a power of two
+                double step = y;                               // y^C
 #pragma unroll
-                for (int m = 0; m < C4; ++m, e *= y) row[sq * C4 + m] = e;
+                for (int m = 1; m < C; m *= 2) step *= step;
+                double e = al * exp(-k * gam * gam);
+                if (sq & 1) e *= step;
+                if (sq & 2) e *= step * step;
+#pragma unroll
+                for (int m = 0; m < C; ++m, e *= y) row[sq * C + m] = e;
             } else {
                 double e = al * wv;
 #pragma unroll
