@@ -329,13 +329,15 @@ int certified_call(const char *who, mb_table *h, int64_t P, const uint64_t *v_in
     uint64_t *d_vi = (uint64_t *)base, *d_vf = (uint64_t *)(base + cb);
     double *d_vrad = (double *)(base + 2 * cb), *d_out = (double *)(base + 3 * cb);
     double *d_rad = term_rad ? (double *)(base + (3 + ns) * cb) : nullptr;
-    MB_CUDA(cudaMemcpyAsync(d_vi, v_int, cb, cudaMemcpyHostToDevice, t.stream));
-    MB_CUDA(cudaMemcpyAsync(d_vf, v_frac, cb, cudaMemcpyHostToDevice, t.stream));
-    if (v_rad) MB_CUDA(cudaMemcpyAsync(d_vrad, v_rad, cb, cudaMemcpyHostToDevice, t.stream));
+    // one copy for the candidates, one for all result rows (each small pageable copy costs microseconds)
+    std::vector<char> in((v_rad ? 3 : 2) * cb);
+    std::memcpy(in.data(), v_int, cb);
+    std::memcpy(in.data() + cb, v_frac, cb);
+    if (v_rad) std::memcpy(in.data() + 2 * cb, v_rad, cb);
+    MB_CUDA(cudaMemcpyAsync(d_vi, in.data(), in.size(), cudaMemcpyHostToDevice, t.stream));
     if (term_rad && rb) MB_CUDA(cudaMemcpyAsync(d_rad, term_rad, rb, cudaMemcpyHostToDevice, t.stream));
     MB_TRY(launch_certified(t, d_vi, d_vf, v_rad ? d_vrad : nullptr, P, j0, j1, k_lo, k_hi, d_rad, grad, d_out,
                             t.stream));
-    // one copy for all rows (each small pageable copy costs several microseconds)
     std::vector<double> rows((size_t)ns * P);
     MB_CUDA(cudaMemcpyAsync(rows.data(), d_out, ns * cb, cudaMemcpyDeviceToHost, t.stream));
     MB_CUDA(cudaStreamSynchronize(t.stream));

@@ -11,6 +11,7 @@
 // P x N matrices, so they are bound by the phase and sincos work, not by 16 B/term of HBM traffic.
 #include <algorithm>
 #include <cmath>
+#include <cstring>
 #include <numeric>
 #include <vector>
 
@@ -108,18 +109,38 @@ int stage_exact(Table &t, int64_t P, const uint64_t *vi, const uint64_t *vf, con
     s.dp = carve<double>(p, P);
     s.grid = carve<double>(p, n_grid);
     s.sel = carve<int>(p, top);
-    MB_CUDA(cudaMemcpyAsync(s.vi, vi, P * 8, cudaMemcpyHostToDevice, t.stream));
-    MB_CUDA(cudaMemcpyAsync(s.vf, vf, P * 8, cudaMemcpyHostToDevice, t.stream));
-    if (delta)
-        MB_CUDA(cudaMemcpyAsync(s.delta, delta, P * 8, cudaMemcpyHostToDevice, t.stream));
-    else
-        MB_CUDA(cudaMemsetAsync(s.delta, 0, P * 8, t.stream));
+    if (P <= 4096) {             // one copy for the three arrays (each small pageable copy costs microseconds)
+        const size_t step = (size_t)(s.vf - s.vi);
+        std::vector<uint64_t> h(3 * step, 0);
+        std::memcpy(h.data(), vi, P * 8);
+        std::memcpy(h.data() + step, vf, P * 8);
+        if (delta) std::memcpy(h.data() + 2 * step, delta, P * 8);
+        MB_CUDA(cudaMemcpyAsync(s.vi, h.data(), 3 * step * 8, cudaMemcpyHostToDevice, t.stream));
+    } else {
+        MB_CUDA(cudaMemcpyAsync(s.vi, vi, P * 8, cudaMemcpyHostToDevice, t.stream));
+        MB_CUDA(cudaMemcpyAsync(s.vf, vf, P * 8, cudaMemcpyHostToDevice, t.stream));
+        if (delta)
+            MB_CUDA(cudaMemcpyAsync(s.delta, delta, P * 8, cudaMemcpyHostToDevice, t.stream));
+        else
+            MB_CUDA(cudaMemsetAsync(s.delta, 0, P * 8, t.stream));
+    }
     if (n_grid > 0 && grid) MB_CUDA(cudaMemcpyAsync(s.grid, grid, n_grid * 8, cudaMemcpyHostToDevice, t.stream));
     return MB_OK;
 }
 
+// The three output arrays of P values, one copy where they lie together.
 int fetch_outputs(cudaStream_t st, int64_t P, const double *hu, const double *hp, const double *dp, double *out_hu,
                   double *out_hp, double *out_dp) {
+    const int64_t step = hp - hu;
+    if (P <= 65536 && step >= P && step <= P + 32 && dp - hp == step) {
+        std::vector<double> h(2 * step + P);
+        MB_CUDA(cudaMemcpyAsync(h.data(), hu, h.size() * 8, cudaMemcpyDeviceToHost, st));
+        MB_CUDA(cudaStreamSynchronize(st));
+        std::memcpy(out_hu, h.data(), P * 8);
+        std::memcpy(out_hp, h.data() + step, P * 8);
+        std::memcpy(out_dp, h.data() + 2 * step, P * 8);
+        return MB_OK;
+    }
     MB_CUDA(cudaMemcpyAsync(out_hu, hu, P * 8, cudaMemcpyDeviceToHost, st));
     MB_CUDA(cudaMemcpyAsync(out_hp, hp, P * 8, cudaMemcpyDeviceToHost, st));
     MB_CUDA(cudaMemcpyAsync(out_dp, dp, P * 8, cudaMemcpyDeviceToHost, st));
@@ -496,8 +517,9 @@ extern "C" int mb_fast_polish_exact(mb_table *h, int64_t P, const uint64_t *v_in
     for (int64_t p0 = 0; p0 < P; p0 += pc)
         MB_TRY(launch_taylor_grid(t, s.vi + p0, s.vf + p0, s.delta + p0, std::min(pc, P - p0), n_zeros, n_chunk, d_w,
                                   s.grid, (int)n_grid, t.work.p, s.hu + p0, s.hp + p0, s.dp + p0, t.stream));
-    MB_TRY(fetch_outputs(t.stream, P, s.hu, s.hp, s.dp, out_h_unpol, out_h_pol, out_ddy_pol));
-    if (nsel == 0) return MB_OK;
+    if (nsel == 0) return fetch_outputs(t.stream, P, s.hu, s.hp, s.dp, out_h_unpol, out_h_pol, out_ddy_pol);
+    MB_CUDA(cudaMemcpyAsync(out_h_pol, s.hp, P * 8, cudaMemcpyDeviceToHost, t.stream));
+    MB_CUDA(cudaStreamSynchronize(t.stream));
     const std::vector<int> sel = top_indices(out_h_pol, P, nsel);
     MB_CUDA(cudaMemcpyAsync(s.sel, sel.data(), nsel * sizeof(int), cudaMemcpyHostToDevice, t.stream));
     double reach = 4 * 1e-5;
