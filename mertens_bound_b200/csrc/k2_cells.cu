@@ -142,7 +142,12 @@ struct CellShape {
     static constexpr int PARTS = KIND == CELL_WEIGHTS ? W : (KIND == CELL_GAUSS && D1 == 8 ? 2 : 4);
     static constexpr int TILE = KIND == CELL_WEIGHTS ? (W == 5 ? 48 : 64) : CELL_THREADS / PARTS;
     static_assert(TILE * PARTS <= CELL_THREADS, "one (zero, part) per thread");
-    static constexpr int ctas = KIND == CELL_WEIGHTS ? 2 : 3;       // resident per SM
+    // peaks per lane: two halve the reads of a zero's record and columns (a 16-term grid scan call
+    // 178 -> 167 us, a Taylor polish of 1,024 peaks 605 -> 577).  One where the accumulators leave no
+    // registers (weights), and with 8 terms, where three CTAs to an SM gain more (614 us, two peaks 630)
+    static constexpr int MP = KIND == CELL_WEIGHTS || D1 == 8 ? 1 : 2;
+    static constexpr int peaks = 64 * MP;                            // of one CTA
+    static constexpr int ctas = MP == 1 && KIND != CELL_WEIGHTS ? 3 : 2;             // resident per SM
     static constexpr int smem = PH_BYTES + 2 * TILE * ((int)sizeof(ZRec) + S * 8);
     static constexpr int frag = 2 * (NTR + NTI);                   // accumulators per lane
 };
@@ -164,7 +169,7 @@ struct CellTile {
     uint32_t tb, jb;
 };
 
-// One item = one cell x CELL_PEAKS / nzw peaks.  Warp w serves peaks 8 (w / nzw) .. + 7 and the
+// One item = one cell x Sh::peaks / nzw peaks.  Warp w serves 8 MP peaks from 8 MP (w / nzw) and the
 // 4-zero steps congruent to w mod nzw; with nzw > 1 the warps' sums are added in warp order.
 // Bound: the FP64 pipe, 16 cycles per mma and scheduler, 2 mma per step and 8 columns, beside ~24 for
 // the phasor (60 instructions).  The next tile's zeros are loaded before the current one is summed and
@@ -181,7 +186,8 @@ cell_moments_kernel(TabView t, const uint64_t *vi, const uint64_t *vf, const dou
     double *E_ = reinterpret_cast<double *>(smem + PH_BYTES + 2 * TILE * sizeof(ZRec));   // [2][TILE][S]
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int cg = warp / nzw, zw = warp - cg * nzw;
-    const int ppc = CELL_PEAKS / nzw;
+    constexpr int MP = Sh::MP;
+    const int ppc = Sh::peaks / nzw;
     const double inv_h = 1.0 / ((double)cells.half * 65536.0);     // units of 2^-32
     const double inv_kappa = 65536.0 / (6.283185307179586 * (double)cells.half);
     // this thread's part of a tile: zero sz, weight vector or column group sq
@@ -275,8 +281,8 @@ cell_moments_kernel(TabView t, const uint64_t *vi, const uint64_t *vf, const dou
     phasor_table_init(tab, CELL_THREADS);
     stage(cur, 0);
     __syncthreads();
-    uint32_t v0 = 0, v1 = 0, v2 = 0, v3 = 0;
-    double aR[Sh::NTR][2], aI[Sh::NTI][2];
+    Cand64 v[MP];
+    double aR[MP][Sh::NTR][2], aI[MP][Sh::NTI][2];
     bool first = true;
     for (int b = 0;; b ^= 1) {
         CellTile nxt = cur;
@@ -288,19 +294,21 @@ cell_moments_kernel(TabView t, const uint64_t *vi, const uint64_t *vf, const dou
         }
         const bool more = nxt.item < n_items;
         if (more) fetch(nxt);
-        const int64_t pw = (int64_t)cur.pt * ppc + cg * 8;             // the warp's first peak
-        const int64_t p = pw + (lane >> 2);
+        const int64_t pw = (int64_t)cur.pt * ppc + cg * 8 * MP;        // the warp's first peak
+        const int64_t p0 = pw + (lane >> 2);                           // this lane's peaks: p0 + 8 m
         if (first) {
-            Cand64 v{0, 0};
-            if (p < P) {
-                const int64_t i = sel ? sel[p] : p;
-                v = fold_delta(vi[i], vf[i], delta ? delta[i] : 0.0);
+#pragma unroll
+            for (int m = 0; m < MP; ++m) {
+                v[m] = Cand64{0, 0};
+                if (p0 + 8 * m < P) {
+                    const int64_t i = sel ? sel[p0 + 8 * m] : p0 + 8 * m;
+                    v[m] = fold_delta(vi[i], vf[i], delta ? delta[i] : 0.0);
+                }
+#pragma unroll
+                for (int i = 0; i < Sh::NTR; ++i) aR[m][i][0] = aR[m][i][1] = 0.0;
+#pragma unroll
+                for (int i = 0; i < Sh::NTI; ++i) aI[m][i][0] = aI[m][i][1] = 0.0;
             }
-            v0 = (uint32_t)v.vf; v1 = (uint32_t)(v.vf >> 32); v2 = (uint32_t)v.vi; v3 = (uint32_t)(v.vi >> 32);
-#pragma unroll
-            for (int i = 0; i < Sh::NTR; ++i) aR[i][0] = aR[i][1] = 0.0;
-#pragma unroll
-            for (int i = 0; i < Sh::NTI; ++i) aI[i][0] = aI[i][1] = 0.0;
         }
         if (pw < P) {
             const int n_step = (min(TILE, (int)(cur.jb - cur.tb)) + 3) >> 2;
@@ -309,50 +317,60 @@ cell_moments_kernel(TabView t, const uint64_t *vi, const uint64_t *vf, const dou
             const int dr = nzw * 4, de = dr * Sh::S;
 #pragma unroll 2
             for (int st = zw; st < n_step; st += nzw, rp += dr, bp += de) {
-                double cs, sn;
-                phasor(phase60(v0, v1, v2, v3, *rp), copy, cs, sn);
+                const ZRec z = *rp;
+                double cs[MP], sn[MP];
+#pragma unroll
+                for (int m = 0; m < MP; ++m)
+                    phasor(phase60((uint32_t)v[m].vf, (uint32_t)(v[m].vf >> 32), (uint32_t)v[m].vi,
+                                   (uint32_t)(v[m].vi >> 32), z), copy, cs[m], sn[m]);
 #pragma unroll
                 for (int i = 0; i < Sh::NT; ++i) {
                     const double bv = bp[i * 8];
-                    if (i < Sh::NTR) dmma(aR[i], cs, bv);
-                    if (i >= Sh::I0) dmma(aI[i - Sh::I0], sn, bv);
+#pragma unroll
+                    for (int m = 0; m < MP; ++m) {
+                        if (i < Sh::NTR) dmma(aR[m][i], cs[m], bv);
+                        if (i >= Sh::I0) dmma(aI[m][i - Sh::I0], sn[m], bv);
+                    }
                 }
             }
         }
         if (last) {
             if (nzw > 1) {                     // add the other warps' sums of this peak group, in order
-                double *buf = E_ + b * TILE * Sh::S + cg * 32 * Sh::frag;
+                double *buf = E_ + cg * 32 * MP * Sh::frag;      // both halves: the next tile is staged later
+                auto each = [&](auto f) {
+#pragma unroll
+                    for (int m = 0; m < MP; ++m) {
+#pragma unroll
+                        for (int i = 0; i < 2 * Sh::NTR; ++i) f(m * Sh::frag + i, aR[m][i >> 1][i & 1]);
+#pragma unroll
+                        for (int i = 0; i < 2 * Sh::NTI; ++i) f(m * Sh::frag + 2 * Sh::NTR + i, aI[m][i >> 1][i & 1]);
+                    }
+                };
                 for (int w = 1; w < nzw; ++w) {
                     __syncthreads();
-                    if (zw == w) {
-#pragma unroll
-                        for (int i = 0; i < 2 * Sh::NTR; ++i) buf[i * 32 + lane] = aR[i >> 1][i & 1];
-#pragma unroll
-                        for (int i = 0; i < 2 * Sh::NTI; ++i) buf[(2 * Sh::NTR + i) * 32 + lane] = aI[i >> 1][i & 1];
-                    }
+                    if (zw == w) each([&](int i, double &x) { buf[i * 32 + lane] = x; });
                     __syncthreads();
-                    if (zw == 0) {
-#pragma unroll
-                        for (int i = 0; i < 2 * Sh::NTR; ++i) aR[i >> 1][i & 1] += buf[i * 32 + lane];
-#pragma unroll
-                        for (int i = 0; i < 2 * Sh::NTI; ++i) aI[i >> 1][i & 1] += buf[(2 * Sh::NTR + i) * 32 + lane];
-                    }
+                    if (zw == 0) each([&](int i, double &x) { x += buf[i * 32 + lane]; });
                 }
             }
-            if (zw == 0 && p < P) {            // C fragment: row = peak, columns 2 (lane mod 4) + {0, 1}
+            // C fragment: row = peak, columns 2 (lane mod 4) + {0, 1}
+#pragma unroll
+            for (int m = 0; m < MP; ++m) {
+                const int64_t p = p0 + 8 * m;
+                if (zw > 0 || p >= P) continue;
 #pragma unroll
                 for (int i = 0; i < Sh::NT; ++i)
 #pragma unroll
                     for (int e = 0; e < 2; ++e) {
                         const int col = i * 8 + (lane & 3) * 2 + e;
                         if constexpr (KIND == CELL_POWERS) {
-                            out[(p * cells.n + cur.cell) * 24 + col] = i < Sh::NTR ? aR[i < Sh::NTR ? i : 0][e]
-                                                                                   : aI[i < Sh::NTR ? 0 : i - Sh::I0][e];
+                            out[(p * cells.n + cur.cell) * 24 + col] = i < Sh::NTR ? aR[m][i < Sh::NTR ? i : 0][e]
+                                                                                   : aI[m][i < Sh::NTR ? 0 : i - Sh::I0][e];
                         } else if (col < W * D1) {
-                            const int w = col / D1, m = col - w * D1;
-                            double *o = out + (((int64_t)w * P + p) * cells.n + cur.cell) * (2 * D1) + m;
-                            o[0] = aR[i < Sh::NTR ? i : 0][e];
-                            o[D1] = aI[i - Sh::I0 >= 0 ? i - Sh::I0 : 0][e];
+                            const int w = col / D1, n = col - w * D1;
+                            double *o = out + (((int64_t)w * P + p) * cells.n + cur.cell) * (2 * D1) + n;
+                            o[0] = aR[m][i < Sh::NTR ? i : 0][e];
+                            o[D1] = aI[m][i - Sh::I0 >= 0 ? i - Sh::I0 : 0][e];
                         }
                     }
             }
@@ -374,25 +392,18 @@ template <int KIND, int W, int D1>
 int launch_moments(const Table &t, const Cells &c, const uint64_t *vi, const uint64_t *vf, const double *delta,
                    const int *sel, int64_t P, const CellWeights &w, double k, int nzw, double *out, cudaStream_t s) {
     using Sh = CellShape<KIND, W, D1>;
-    static_assert(4 * 32 * Sh::frag <= Sh::TILE * Sh::S || KIND == CELL_WEIGHTS, "reduction buffer");
+    static_assert(4 * 32 * Sh::MP * Sh::frag <= 2 * Sh::TILE * Sh::S || KIND == CELL_WEIGHTS, "reduction buffer");
     MB_TRY(cell_kernel_attributes());
     int sms = 148;
     MB_TRY(sm_count(t, &sms));
     const int64_t slots = (int64_t)Sh::ctas * sms;
-    const int64_t n_pt = (P + CELL_PEAKS / nzw - 1) / (CELL_PEAKS / nzw);
+    const int64_t n_pt = (P + Sh::peaks / nzw - 1) / (Sh::peaks / nzw);
     const int64_t items = n_pt * c.n;
     MB_CHECK_ARG(items < ((int64_t)1 << 31), "cell moments: %lld items", (long long)items);
     cell_moments_kernel<KIND, W, D1><<<(unsigned)std::min<int64_t>(slots, items), CELL_THREADS, Sh::smem, s>>>(
         view(t), vi, vf, delta, sel, P, c, w, k, (int)n_pt, nzw, (int)items, out);
     MB_CUDA(cudaGetLastError());
     return MB_OK;
-}
-
-// Warps sharing a peak group's zeros: as many as keep the CTA's peak slots full.
-int cell_nzw(int64_t P) {
-    int nzw = 1;
-    while (nzw < 8 && P <= CELL_PEAKS / (2 * nzw)) nzw *= 2;
-    return nzw;
 }
 
 // ------------------------------------------------------------------ offset scans
@@ -955,6 +966,20 @@ int set_smem(K kern, int bytes) {
 
 }  // namespace
 
+// Warps sharing a peak group's zeros in the scans and power sums: as many as keep the CTA's peak slots full,
+// and two at least with 16 peaks a warp, unless there are peaks for eight full CTAs (fewer, larger items would
+// not balance).
+static int cell_nzw(int64_t P, int peaks) {
+    int nzw = peaks == 128 && P < 8 * peaks ? 2 : 1;
+    while (nzw < 8 && P <= peaks / (2 * nzw)) nzw *= 2;
+    return nzw;
+}
+
+int cell_peaks(int64_t P, int d1) {
+    const int peaks = d1 == 8 ? CellShape<CELL_GAUSS, 1, 8>::peaks : CellShape<CELL_GAUSS, 1, 16>::peaks;
+    return peaks / cell_nzw(P, peaks);
+}
+
 int cell_kernel_attributes() {
     static void *done_ctx[64] = {};             // the context the attributes were set in
     int dev = 0;
@@ -1030,9 +1055,10 @@ int build_cells(const Table &t, const CellPlan &p, void *buf, Cells &out, cudaSt
 int launch_moments_gauss(const Table &t, const Cells &c, const uint64_t *vi, const uint64_t *vf, int64_t P, double k,
                          int d1, double *out, cudaStream_t s) {
     const CellWeights none{};
-    const int nzw = cell_nzw(P);
-    return d1 == 8 ? launch_moments<CELL_GAUSS, 1, 8>(t, c, vi, vf, nullptr, nullptr, P, none, k, nzw, out, s)
-                   : launch_moments<CELL_GAUSS, 1, 16>(t, c, vi, vf, nullptr, nullptr, P, none, k, nzw, out, s);
+    return d1 == 8 ? launch_moments<CELL_GAUSS, 1, 8>(t, c, vi, vf, nullptr, nullptr, P, none, k,
+                                                      cell_nzw(P, CellShape<CELL_GAUSS, 1, 8>::peaks), out, s)
+                   : launch_moments<CELL_GAUSS, 1, 16>(t, c, vi, vf, nullptr, nullptr, P, none, k,
+                                                       cell_nzw(P, CellShape<CELL_GAUSS, 1, 16>::peaks), out, s);
 }
 
 int launch_moments_weights(const Table &t, const Cells &c, const uint64_t *vi, const uint64_t *vf,
@@ -1052,8 +1078,9 @@ int launch_moments_weights(const Table &t, const Cells &c, const uint64_t *vi, c
 int taylor_chunks(const Table &t, int64_t P, int64_t n, int *n_chunk) {
     int slots = 148;
     MB_TRY(sm_count(t, &slots));
-    slots *= CellShape<CELL_POWERS, 1, 17>::ctas;
-    const int ppc = CELL_PEAKS / cell_nzw(P);
+    using Sh = CellShape<CELL_POWERS, 1, 17>;
+    slots *= Sh::ctas;
+    const int ppc = Sh::peaks / cell_nzw(P, Sh::peaks);
     const int64_t n_pt = std::max<int64_t>(1, (P + ppc - 1) / ppc);
     *n_chunk = (int)std::max<int64_t>(1, std::min<int64_t>((8 * (int64_t)slots + n_pt - 1) / n_pt, n / 256));
     return MB_OK;
@@ -1073,7 +1100,8 @@ int launch_taylor_grid(const Table &t, const uint64_t *vi, const uint64_t *vf, c
     MB_CUDA(cudaGetLastError());
     const Cells c{n_chunk, n_chunk, 1, j0, j1, nullptr};
     const CellWeights cw{{w}};
-    MB_TRY((launch_moments<CELL_POWERS, 1, 17>(t, c, vi, vf, delta, nullptr, P, cw, 0.0, cell_nzw(P), S, s)));
+    MB_TRY((launch_moments<CELL_POWERS, 1, 17>(t, c, vi, vf, delta, nullptr, P, cw, 0.0,
+                                              cell_nzw(P, CellShape<CELL_POWERS, 1, 17>::peaks), S, s)));
     taylor_grid_kernel<<<(unsigned)P, TAY_THREADS, 0, s>>>(S, n_chunk, grid, n_grid, h_unpol, h_pol, ddy_pol);
     MB_CUDA(cudaGetLastError());
     return MB_OK;

@@ -21,7 +21,7 @@ namespace mb {
 // (largest over the cell; the mean of |x|^D1 over a cell is 1 / (D1 + 1)).
 constexpr double cell_x(int d1) { return d1 == 8 ? 0.05 : (d1 == 11 ? 0.2 : 0.68); }
 
-constexpr int CELL_PEAKS = 64;          // peaks of one CTA (8 per warp)
+int cell_peaks(int64_t P, int d1);      // points of one CTA of launch_moments_gauss
 constexpr int CELL_MAX_W = 5;           // weight vectors of one moment pass
 constexpr int CELL_D1 = 11;             // series terms of the polish paths
 

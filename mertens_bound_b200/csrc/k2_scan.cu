@@ -276,11 +276,9 @@ bool plan_scan(const Table &t, int64_t P, int64_t n_use, int64_t n_m, uint64_t s
         if (NB > 1 && Bp < 32) break;
         if (NB > SCAN_MAX_POINTS) break;
         const int64_t pts = P * NB;
-        int nzw = 1;
-        while (nzw < 8 && pts <= CELL_PEAKS / (2 * nzw)) nzw *= 2;
-        const int ppc = CELL_PEAKS / nzw;
-        const double tiles = (double)((pts + ppc - 1) / ppc);
         for (int d1 : {8, 16}) {
+            const int ppc = cell_peaks(pts, d1);
+            const double tiles = (double)((pts + ppc - 1) / ppc);
             // at least one item per CTA slot where the cells hold 16 zeros or more
             const int64_t min_cells = std::min<int64_t>(n_use / 16, (int64_t)(296 / tiles));
             CellPlan cp;
