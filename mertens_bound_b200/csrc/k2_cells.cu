@@ -336,7 +336,7 @@ cell_moments_kernel(TabView t, const uint64_t *vi, const uint64_t *vf, const dou
         }
         if (last) {
             if (nzw > 1) {                     // add the other warps' sums of this peak group, in order
-                double *buf = E_ + cg * 32 * MP * Sh::frag;      // both halves: the next tile is staged later
+                double *buf = E_ + cg * 32 * MP * Sh::frag;      // spans both halves of the tile buffer
                 auto each = [&](auto f) {
 #pragma unroll
                     for (int m = 0; m < MP; ++m) {
@@ -352,6 +352,7 @@ cell_moments_kernel(TabView t, const uint64_t *vi, const uint64_t *vf, const dou
                     __syncthreads();
                     if (zw == 0) each([&](int i, double &x) { x += buf[i * 32 + lane]; });
                 }
+                __syncthreads();               // all read before the next tile is staged there
             }
             // C fragment: row = peak, columns 2 (lane mod 4) + {0, 1}
 #pragma unroll
