@@ -65,11 +65,10 @@ MB_DEV void iv_sincos(const Ival &x, Ival &s, Ival &c) {
     c = {__dsub_rd(q.lo, rc), __dadd_ru(q.hi, rc)};
 }
 
-MB_DEV Ival iv_neg(const Ival &a) { return {-a.hi, -a.lo}; }
-
 // point * interval
 MB_DEV Ival iv_scale(double a, const Ival &b) {
-    return a >= 0.0 ? Ival{__dmul_rd(a, b.lo), __dmul_ru(a, b.hi)} : Ival{__dmul_rd(a, b.hi), __dmul_ru(a, b.lo)};
+    const bool neg = __double2hiint(a) < 0;
+    return {__dmul_rd(a, neg ? b.hi : b.lo), __dmul_ru(a, neg ? b.lo : b.hi)};
 }
 
 // non-negative interval w times interval a
@@ -81,13 +80,46 @@ MB_DEV Ival iv_wmul(const Ival &w, const Ival &a) {
 
 // Enclosure of exp(-y) for y in [ylo, yhi], 0 <= ylo <= yhi.
 MB_DEV Ival iv_exp_neg(double ylo, double yhi) {
-    const double e_small = exp(-yhi), e_big = exp(-ylo);
+    const double e_big = exp(-ylo);
+    // a narrow y: exp(-yhi) >= exp(-ylo) (1 - d), below it by at most d^2 / 2 < 2^-57 relative, and
+    // (1 - 2^-51)(1 - d) >= 1 - (2^-51 + d): one exponential for both ends
+    const double d = __dsub_ru(yhi, ylo);
+    if (d < 0x1p-28 && e_big > 1e-300)
+        return {__fma_rd(-e_big, __dadd_ru(d, 0x1p-51), e_big), __dmul_ru(e_big, 1.0 + 0x1p-51)};
+    const double e_small = exp(-yhi);
     const double tiny = 4.0 * 4.9406564584124654e-324;     // absolute slack in the subnormal range
     double lo = __dmul_rd(e_small, 1.0 - 4.440892098500626e-16);
     double hi = __dmul_ru(e_big, 1.0 + 4.440892098500626e-16);
     if (e_small < 2.2250738585072014e-308) lo = fmax(0.0, __dsub_rd(lo, tiny));
     if (e_big < 2.2250738585072014e-308) hi = __dadd_ru(hi, tiny);
     return {lo, hi};
+}
+
+// One zero's data; rad: its term's own radius.
+struct CertZero {
+    uint32_t g0, g1, g2, g3, g4;
+    double gamma, cr, ci, rad;
+};
+
+MB_DEV CertZero cert_zero(const TabView &tv, int64_t j, const double *term_rad, int64_t jr) {
+    return {tv.g0[j], tv.g1[j], tv.g2[j], tv.g3[j], tv.g4[j], tv.gamma[j], tv.cre[j], tv.cim[j],
+            term_rad ? term_rad[jr] : 0.0};
+}
+
+// What a zero's terms share over the candidates: gamma and the weight enclosed, |c| rounded up.
+struct CertWeight {
+    double glo, ghi, cabs;
+    Ival w;
+};
+
+// k lies in [k_lo, k_hi].
+MB_DEV CertWeight cert_weight(const CertZero &z, double k_lo, double k_hi) {
+    CertWeight x;
+    x.glo = __dmul_rd(z.gamma, 1.0 - 8.881784197001252e-16);
+    x.ghi = __dmul_ru(z.gamma, 1.0 + 8.881784197001252e-16);
+    x.w = iv_exp_neg(__dmul_rd(__dmul_rd(k_lo, x.glo), x.glo), __dmul_ru(__dmul_ru(k_hi, x.ghi), x.ghi));
+    x.cabs = __dsqrt_ru(__fma_ru(z.cr, z.cr, __dmul_ru(z.ci, z.ci)));
+    return x;
 }
 
 struct CertTerm {
@@ -99,19 +131,18 @@ struct CertTerm {
 // -2 x for an interval x (exact)
 MB_DEV Ival iv_m2(const Ival &x) { return {-2.0 * x.hi, -2.0 * x.lo}; }
 
-// Term j; k lies in [k_lo, k_hi]; term_rad (nullable) is the per-term radius at index jr.  With
-// GRAD the term's derivatives in v (= delta) and k are enclosed too:
+// One zero's term for one candidate.  With GRAD its derivatives in v (= delta) and k are enclosed too:
 //   d/dv 2 w Re(c e^{i gamma v}) = -2 w gamma Im(c e^{i gamma v}) = -2 w gamma (Re c sin + Im c cos),
 //   d/dk 2 w Re(c e^{i gamma v}) = -2 w gamma^2 Re(c e^{i gamma v}),
 // from the same sine/cosine and weight intervals and gamma in [gamma_lo, gamma_hi]; a radius rho
 // of c e^{i gamma v} (|c| gamma_hi v_rad + term_rad) widens them by 2 w_hi gamma_hi rho and
 // 2 w_hi gamma_hi^2 rho (each derivative in v brings one more factor gamma).
-template <bool GRAD>
-MB_DEV CertTerm cert_term(const TabView &tv, int64_t j, uint64_t vi, uint64_t vf, double k_lo, double k_hi,
-                          double v_rad, const double *term_rad, int64_t jr) {
+// weight() gives the zero's CertWeight; it is called behind the sines, whose registers it can then take.
+template <bool GRAD, class Weight>
+MB_DEV CertTerm cert_term(const CertZero &z, Weight weight, uint64_t vi, uint64_t vf, double v_rad) {
     uint64_t hi, lo;
-    phase128_exact((uint32_t)vf, (uint32_t)(vf >> 32), (uint32_t)vi, (uint32_t)(vi >> 32), tv.g0[j], tv.g1[j],
-                   tv.g2[j], tv.g3[j], tv.g4[j], hi, lo);
+    phase128_exact((uint32_t)vf, (uint32_t)(vf >> 32), (uint32_t)vi, (uint32_t)(vi >> 32), z.g0, z.g1, z.g2, z.g3,
+                   z.g4, hi, lo);
     const int q = (int)(hi >> 62);
     const uint64_t m = hi & ((1ull << 62) - 1);
     const double two_m62 = 2.168404344971009e-19;
@@ -121,36 +152,25 @@ MB_DEV CertTerm cert_term(const TabView &tv, int64_t j, uint64_t vi, uint64_t vf
         r = {__dsub_rd(1.0, r.hi), __dsub_ru(1.0, r.lo)};
         swap = true;
     }
-    const Ival x{__dmul_rd(CERT_PIO2_LO, r.lo), __dmul_ru(CERT_PIO2_HI, r.hi)};
     Ival s, c;
-    iv_sincos(x, s, c);
-    if (swap) {
-        Ival t = s;
-        s = c;
-        c = t;
-    }
-    // rotate by q quarter turns: q=0 (s,c) 1 (c,-s) 2 (-s,-c) 3 (-c,s)
-    Ival S, Cc;
-    switch (q) {
-        case 0: S = s; Cc = c; break;
-        case 1: S = c; Cc = iv_neg(s); break;
-        case 2: S = iv_neg(s); Cc = iv_neg(c); break;
-        default: S = iv_neg(c); Cc = s; break;
-    }
-    const double cr = tv.cre[j], ci = tv.cim[j];
-    const Ival a1 = iv_scale(cr, Cc), a2 = iv_scale(ci, S);
-    const Ival A{__dsub_rd(a1.lo, a2.hi), __dsub_ru(a1.hi, a2.lo)};
-    const double g = tv.gamma[j];
-    const double glo = __dmul_rd(g, 1.0 - 8.881784197001252e-16), ghi = __dmul_ru(g, 1.0 + 8.881784197001252e-16);
-    const double ylo = __dmul_rd(__dmul_rd(k_lo, glo), glo), yhi = __dmul_ru(__dmul_ru(k_hi, ghi), ghi);
-    const Ival w = iv_exp_neg(ylo, yhi);
+    iv_sincos(Ival{__dmul_rd(CERT_PIO2_LO, r.lo), __dmul_ru(CERT_PIO2_HI, r.hi)}, s, c);
+    // c e^{i theta} over the octant's s and c: the quadrant's signs (q = 0: cos, sin = c, s; 1: -s, c;
+    // 2: -c, -s; 3: s, -c) and its exchange go into the point coefficients
+    const double cr = z.cr, ci = z.ci;
+    const bool nc = q == 1 || q == 2, ns = q >= 2;                 // cos and sin negated
+    const bool ex = swap != ((q & 1) != 0);
+    const double rc = nc ? -cr : cr, rs = ns ? ci : -ci;           // Re = rc cos' + rs sin'
+    const Ival a1 = iv_scale(ex ? rc : rs, s), a2 = iv_scale(ex ? rs : rc, c);
+    const Ival A{__dadd_rd(a1.lo, a2.lo), __dadd_ru(a1.hi, a2.hi)};
+    const CertWeight x = weight();
+    const Ival &w = x.w;
+    const double glo = x.glo, ghi = x.ghi, cabs = x.cabs;
     Ival t = iv_wmul(w, A);
     t.lo *= 2.0;
     t.hi *= 2.0;
-    const double cabs = __dsqrt_ru(__fma_ru(cr, cr, __dmul_ru(ci, ci)));
     double rad = 0.0;
     if (v_rad > 0.0) rad = __dmul_ru(__dmul_ru(cabs, ghi), v_rad);
-    if (term_rad) rad = __dadd_ru(rad, term_rad[jr]);
+    if (z.rad != 0.0) rad = __dadd_ru(rad, z.rad);
     double wr = 0.0;
     if (rad > 0.0) {
         wr = __dmul_ru(2.0 * w.hi, rad);
@@ -159,8 +179,9 @@ MB_DEV CertTerm cert_term(const TabView &tv, int64_t j, uint64_t vi, uint64_t vf
     }
     CertTerm out{t, __dmul_ru(2.0 * w.hi, cabs), {0.0, 0.0}, {0.0, 0.0}};
     if constexpr (GRAD) {
-        const Ival b1 = iv_scale(cr, S), b2 = iv_scale(ci, Cc);
-        const Ival B{__dadd_rd(b1.lo, b2.lo), __dadd_ru(b1.hi, b2.hi)};     // Im(c e^{i theta})
+        const double ic = nc ? -ci : ci, is = ns ? -cr : cr;       // Im = ic cos' + is sin'
+        const Ival b1 = iv_scale(ex ? ic : is, s), b2 = iv_scale(ex ? is : ic, c);
+        const Ival B{__dadd_rd(b1.lo, b2.lo), __dadd_ru(b1.hi, b2.hi)};
         const Ival wg{__dmul_rd(w.lo, glo), __dmul_ru(w.hi, ghi)};          // w gamma >= 0
         const Ival wg2{__dmul_rd(wg.lo, glo), __dmul_ru(wg.hi, ghi)};      // w gamma^2 >= 0
         out.dd = iv_m2(iv_wmul(wg, B));
@@ -206,37 +227,68 @@ MB_DEV void cert_block_sum(double (&acc)[NS], double (*red)[NS]) {
         }
 }
 
-// grid (zero blocks, candidates); partial[(blockIdx.x * P + p) * NS + s] with s = K2 lo, K2 hi,
+// Bound: instruction issue and, with one candidate, the latency of its nine loads per zero: a zero's data are
+// loaded one zero ahead, which takes the registers of a fourth CTA per SM and is still the better side (kernel
+// 49 -> 44 us for one candidate over 2.3 M zeros).  C candidates share a zero's loads, weight and |c|.
+// grid (zero blocks, candidate tiles); partial[(blockIdx.x * P + p) * NS + s] with s = K2 lo, K2 hi,
 // abs_hi[, dd lo, dd hi, dk lo, dk hi]: lower ends summed with __dadd_rd, upper ends with __dadd_ru.
-template <bool GRAD>
-__global__ void __launch_bounds__(CERT_THREADS)
+template <bool GRAD, int C>
+__global__ void __launch_bounds__(CERT_THREADS, C == 1 ? 3 : 2)
 k2_certified_kernel(TabView tv, const uint64_t *vi, const uint64_t *vf, const double *v_rad, int64_t P, int64_t j0,
                     int64_t j1, double k_lo, double k_hi, const double *term_rad, double *partial) {
     constexpr int NS = cert_sums<GRAD>();
-    const int64_t p = blockIdx.y;
-    const uint64_t a = vi[p], b = vf[p];
-    const double vr = v_rad ? v_rad[p] : 0.0;
-    double acc[NS];
+    const int64_t p0 = (int64_t)blockIdx.y * C;
+    const int live = (int)min((int64_t)C, P - p0);
+    uint64_t a[C], b[C];
+    double acc[C][NS];
 #pragma unroll
-    for (int q = 0; q < NS; ++q) acc[q] = 0.0;
-    for (int64_t jr = (int64_t)blockIdx.x * CERT_THREADS + threadIdx.x; j0 + jr < j1; jr += (int64_t)gridDim.x * CERT_THREADS) {
-        CertTerm ct = cert_term<GRAD>(tv, j0 + jr, a, b, k_lo, k_hi, vr, term_rad, jr);
-        acc[0] = __dadd_rd(acc[0], ct.t.lo);
-        acc[1] = __dadd_ru(acc[1], ct.t.hi);
-        acc[2] = __dadd_ru(acc[2], ct.abs_hi);
-        if constexpr (GRAD) {
-            acc[3] = __dadd_rd(acc[3], ct.dd.lo);
-            acc[4] = __dadd_ru(acc[4], ct.dd.hi);
-            acc[5] = __dadd_rd(acc[5], ct.dk.lo);
-            acc[6] = __dadd_ru(acc[6], ct.dk.hi);
+    for (int i = 0; i < C; ++i) {
+        const int64_t p = p0 + min(i, live - 1);
+        a[i] = vi[p];
+        b[i] = vf[p];
+#pragma unroll
+        for (int q = 0; q < NS; ++q) acc[i][q] = 0.0;
+    }
+    const int64_t stride = (int64_t)gridDim.x * CERT_THREADS;
+    int64_t jr = (int64_t)blockIdx.x * CERT_THREADS + threadIdx.x;
+    CertZero nxt;
+    if (j0 + jr < j1) nxt = cert_zero(tv, j0 + jr, term_rad, jr);
+    while (j0 + jr < j1) {
+        const CertZero z = nxt;
+        jr += stride;
+        if (j0 + jr < j1) nxt = cert_zero(tv, j0 + jr, term_rad, jr);
+        CertWeight x;
+        if constexpr (C > 1) x = cert_weight(z, k_lo, k_hi);
+        const auto weight = [&] {
+            if constexpr (C > 1) return x;
+            else return cert_weight(z, k_lo, k_hi);
+        };
+#pragma unroll
+        for (int i = 0; i < C; ++i) {
+            if (i >= live) break;
+            const CertTerm ct = cert_term<GRAD>(z, weight, a[i], b[i], v_rad ? v_rad[p0 + i] : 0.0);
+            acc[i][0] = __dadd_rd(acc[i][0], ct.t.lo);
+            acc[i][1] = __dadd_ru(acc[i][1], ct.t.hi);
+            acc[i][2] = __dadd_ru(acc[i][2], ct.abs_hi);
+            if constexpr (GRAD) {
+                acc[i][3] = __dadd_rd(acc[i][3], ct.dd.lo);
+                acc[i][4] = __dadd_ru(acc[i][4], ct.dd.hi);
+                acc[i][5] = __dadd_rd(acc[i][5], ct.dk.lo);
+                acc[i][6] = __dadd_ru(acc[i][6], ct.dk.hi);
+            }
         }
     }
     __shared__ double red[CERT_THREADS / 32][NS];
-    cert_block_sum<NS>(acc, red);
-    if (threadIdx.x == 0) {
-        double *o = partial + ((int64_t)blockIdx.x * P + p) * NS;
 #pragma unroll
-        for (int q = 0; q < NS; ++q) o[q] = acc[q];
+    for (int i = 0; i < C; ++i) {
+        if (i >= live) break;
+        if (i > 0) __syncthreads();                  // thread 0 has read the sums before
+        cert_block_sum<NS>(acc[i], red);
+        if (threadIdx.x == 0) {
+            double *o = partial + ((int64_t)blockIdx.x * P + p0 + i) * NS;
+#pragma unroll
+            for (int q = 0; q < NS; ++q) o[q] = acc[i][q];
+        }
     }
 }
 
@@ -273,26 +325,29 @@ int launch_certified(Table &t, const uint64_t *d_vi, const uint64_t *d_vf, const
     const int64_t n_use = std::max<int64_t>(0, j1 - j0);
     int sms = 148;
     MB_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, t.device));
-    int64_t want = std::max<int64_t>(1, ((int64_t)sms * 8 + P - 1) / P);
-    int64_t nblk = std::max<int64_t>(1, std::min(want, (n_use + CERT_THREADS - 1) / CERT_THREADS));
+    // four candidates per thread share a third of the work (24 x 400,000: 185 -> 138 us, 4 x 1,000,000: 101 -> 88).
+    // 12 CTAs per SM (four rounds of three): longer chains of directed sums would widen the intervals.
+    const int C = P >= 4 ? 4 : 1;
+    const int64_t n_tile = (P + C - 1) / C;
+    const int64_t want = std::max<int64_t>(1, ((int64_t)sms * 12 + n_tile - 1) / n_tile);
+    const int64_t nblk = std::max<int64_t>(1, std::min(want, (n_use + CERT_THREADS - 1) / CERT_THREADS));
     MB_CHECK_ARG(P <= 65535, "certified: P=%lld exceeds 65535 candidates per call", (long long)P);
     const int ns = grad ? cert_sums<true>() : cert_sums<false>();
     MB_TRY(t.work.ensure((size_t)nblk * P * ns * sizeof(double)));
     double *partial = (double *)t.work.p;
-    dim3 grid((unsigned)nblk, (unsigned)P);
-    if (grad) {
-        k2_certified_kernel<true><<<grid, CERT_THREADS, 0, s>>>(view(t), d_vi, d_vf, d_vrad, P, j0, j1, k_lo, k_hi,
-                                                                d_term_rad, partial);
+    const dim3 grid((unsigned)nblk, (unsigned)n_tile);
+    auto launch = [&](auto kernel, auto reduce) -> int {
+        kernel<<<grid, CERT_THREADS, 0, s>>>(view(t), d_vi, d_vf, d_vrad, P, j0, j1, k_lo, k_hi, d_term_rad, partial);
         MB_CUDA(cudaGetLastError());
-        certified_reduce_kernel<true><<<(unsigned)P, CERT_THREADS, 0, s>>>(partial, P, (int)nblk, d_out);
-    } else {
-        k2_certified_kernel<false><<<grid, CERT_THREADS, 0, s>>>(view(t), d_vi, d_vf, d_vrad, P, j0, j1, k_lo, k_hi,
-                                                                 d_term_rad, partial);
+        reduce<<<(unsigned)P, CERT_THREADS, 0, s>>>(partial, P, (int)nblk, d_out);
         MB_CUDA(cudaGetLastError());
-        certified_reduce_kernel<false><<<(unsigned)P, CERT_THREADS, 0, s>>>(partial, P, (int)nblk, d_out);
-    }
-    MB_CUDA(cudaGetLastError());
-    return MB_OK;
+        return MB_OK;
+    };
+    if (grad)
+        return C == 1 ? launch(k2_certified_kernel<true, 1>, certified_reduce_kernel<true>)
+                      : launch(k2_certified_kernel<true, 4>, certified_reduce_kernel<true>);
+    return C == 1 ? launch(k2_certified_kernel<false, 1>, certified_reduce_kernel<false>)
+                  : launch(k2_certified_kernel<false, 4>, certified_reduce_kernel<false>);
 }
 
 }  // namespace mb

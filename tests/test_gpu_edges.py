@@ -1,6 +1,6 @@
 """Kernel variants at the sizes where their rules change over: four leaves per thread in the screen (and
 its split records above gamma = 3.29e6), the plain kernel's tile widths, the heavy tier's groups of at most 32
-candidates, 16-term scans over one and two peak groups per warp, and the hit polish's early exits.
+candidates, the certified kernel's tiles of four candidates, 16-term scans over one and two peak groups per warp, and the hit polish's early exits.
 Tolerances are those of the general tests of each path: 2e-5 for a screen score (MUFU and FP32 sums), 2e-13 for
 the plain kernel and 3e-13 for a scan against it, a plan's own bounds for the tiers."""
 import math
@@ -151,3 +151,32 @@ def test_hit_polish_exits(gpu, n, P):
         h, dy = zerodata_polish(top[i].view(np.int64), two_astar, data.gamma, thresholds=tuple(thr))
         assert abs(r.h[i] - h) < 1e-11 * max(1.0, abs(h))
         assert abs(r.dy[i] - dy) < 1e-12
+
+
+@pytest.mark.parametrize("P", [1, 3, 4, 5, 9])
+@pytest.mark.parametrize("n", [1, 257, 3000])
+def test_certified_candidate_tiles(table, small_table, oracle, P, n):
+    """Every interval holds the oracle's value; a radius per candidate widens its own interval alone."""
+    cd = synth.make_candidates(P, seed=P + n)
+    T = float(small_table.gamma[n])
+    ohi, olo = oracle.k2(cd, small_table, 3e-9, n)
+    lo, hi, ab = k2.k2_certified(table, cd, 3e-9, T)
+    dlo, dhi = k2.k2_certified_grad(table, cd, 3e-9, T)
+    rad = np.zeros(P)
+    rad[P - 1] = 1e-9
+    rlo, rhi, _ = k2.k2_certified(table, cd, 3e-9, T, v_rad=rad)
+    # the FP64 oracle value and each end round by less than an ulp of the sum of amplitudes
+    slack = 4e-16 * ab
+    assert np.all(lo - slack <= ohi[:, 0]) and np.all(ohi[:, 0] <= hi + slack)
+    assert np.all(hi - lo < 1e-13)
+    assert np.array_equal(dlo[0], lo) and np.array_equal(dhi[0], hi)
+    for row in (1, 2):
+        eps = 4e-16 * np.abs(ohi[:, row])
+        assert np.all(dlo[row] - eps <= ohi[:, row]) and np.all(ohi[:, row] <= dhi[row] + eps)
+    wlo, whi = k2.k2_certified_grad(table, cd, 3e-9, T, k_hi=4e-9)           # a wide k: two exponentials
+    mid = oracle.k2(cd, small_table, 3.5e-9, n)[0]
+    for row in range(3):
+        eps = 4e-16 * np.maximum(np.abs(mid[:, row]), ab)
+        assert np.all(wlo[row] - eps <= mid[:, row]) and np.all(mid[:, row] <= whi[row] + eps)
+    assert np.array_equal(rlo[:-1], lo[:-1]) and np.array_equal(rhi[:-1], hi[:-1])
+    assert rlo[-1] < lo[-1] and rhi[-1] > hi[-1]
