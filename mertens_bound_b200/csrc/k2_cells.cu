@@ -758,11 +758,12 @@ cell_polish_kernel(Cells cells, const double *M, CellPolishArgs a, const double 
 }
 
 // The second pass: the listed peaks' Newton and final value by the loops over the zeros, bit for bit as
-// peak_polish_kernel forms them.  Pass `it` forms the terms of every zero (redo_term_kernel, over the whole
-// GPU) and adds them in that kernel's order (redo_sum_kernel: POLISH_CLUSTER x POLISH_THREADS strided running
-// sums, warp tree, warps and CTA ranks in order); one peak's eight sums of 293 serial additions at 600,000
-// zeros are bound by load latency, so each thread keeps REDO_AHEAD zeros' loads in flight.
-constexpr int REDO_AHEAD = 16;
+// peak_polish_kernel forms them: POLISH_STRIDE running sums over zeros POLISH_STRIDE apart, warp trees, warps
+// and CTA ranks in order.  One CTA per (32 of those sums, peak): eight warps form the terms of REDO_ROWS zeros
+// of each sum at a time, a ninth adds the rows before in order.  Bound: instruction issue (an FP64 sincos
+// per zero); with the terms written out by one kernel and added by a second one, a pass over seven peaks and
+// 600,000 zeros took 33 + 31 us (memory traffic, then load latency), now 34.
+constexpr int REDO_ROWS = 16, REDO_THREADS = 288, REDO_GROUPS = (int)(POLISH_STRIDE / 32);
 
 struct RedoState {
     double d;
@@ -772,9 +773,9 @@ struct RedoState {
 struct RedoBuf {
     const Redo *list;
     RedoState *state;           // [2][batch], by the pass's parity
-    double2 *slot;              // [batch][POLISH_CLUSTER]: the ranks' sums
+    double2 *slot;              // [batch][REDO_GROUPS]: the warp sums
     double *h_best, *d_best;    // [batch]
-    double2 *ab, *term;         // [batch][n]: (A, B); (value, derivative) of each zero's term
+    double2 *ab;                // [batch][n]: (A, B)
     int batch;
 };
 
@@ -786,95 +787,123 @@ __global__ void __launch_bounds__(256) redo_ab_kernel(ABExact src, int64_t n, Re
     rb.ab[blockIdx.y * n + j] = make_double2(A, B);
 }
 
-// The ranks' totals in rank order.
+// The totals: a rank's warp sums in order (one lane each), then the ranks in order; every lane gets them.
 MB_DEV double2 redo_total(const RedoBuf &rb, int e) {
-    double2 t = make_double2(0.0, 0.0);
+    constexpr int W = REDO_GROUPS / POLISH_CLUSTER;
+    const int rank = threadIdx.x & (POLISH_CLUSTER - 1);
+    double2 x = make_double2(0.0, 0.0), t = x;
+    for (int i = 0; i < W; ++i) {
+        const double2 v = rb.slot[e * REDO_GROUPS + rank * W + i];
+        x.x += v.x;
+        x.y += v.y;
+    }
     for (int r = 0; r < POLISH_CLUSTER; ++r) {
-        t.x += rb.slot[e * POLISH_CLUSTER + r].x;
-        t.y += rb.slot[e * POLISH_CLUSTER + r].y;
+        t.x += __shfl_sync(0xffffffffu, x.x, r);
+        t.y += __shfl_sync(0xffffffffu, x.y, r);
     }
     return t;
 }
 
+// Pass `it` of a start's Newton loop; it == iters sums h itself.
 template <int MODE>
-__global__ void __launch_bounds__(256) redo_term_kernel(const double *gamma, int64_t n, RedoBuf rb, int start, int it) {
+__global__ void __launch_bounds__(REDO_THREADS, 4)
+redo_pass_kernel(const double *gamma, int64_t n, CellWeights wts, RedoBuf rb, int start, int it) {
     using R = PolishRule<MODE>;
-    const int e = blockIdx.y;
-    RedoState st;
-    if (it == 0) {
-        st = RedoState{rb.list[e].start[start], 0, 0};
-    } else {                                       // the step of the pass before, alike in every CTA
-        st = rb.state[((it - 1) & 1) * rb.batch + e];
-        if (!st.done) {
+    constexpr int PER = REDO_ROWS / 8;                 // rows of one warp
+    __shared__ double s_d[2][REDO_ROWS][32], s_dd[2][REDO_ROWS][32], s_w[2][REDO_ROWS][32];
+    __shared__ RedoState s_state;
+    const int e = blockIdx.y, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    if (warp == 0) {                                   // the step of the pass before, alike in every CTA
+        RedoState st;
+        if (it == 0) {
+            st = RedoState{rb.list[e].start[start], 0, 0};
+        } else {
+            st = rb.state[((it - 1) & 1) * rb.batch + e];
             const double2 t = redo_total(rb, e);
-            if (!(fabs(t.y) > 1e-12)) {
-                st.done = 1;
-            } else {
-                double step = t.x / t.y;
-                step = fmin(fmax(step, -R::clamp), R::clamp);
-                st.d -= step;
-                if (fabs(step) < R::tol) st.done = 1;
+            if (!st.done) {
+                if (!(fabs(t.y) > 1e-12)) {
+                    st.done = 1;
+                } else {
+                    double step = t.x / t.y;
+                    step = fmin(fmax(step, -R::clamp), R::clamp);
+                    st.d -= step;
+                    if (fabs(step) < R::tol) st.done = 1;
+                }
             }
         }
+        if (lane == 0) {
+            s_state = st;
+            if (blockIdx.x == 0) rb.state[(it & 1) * rb.batch + e] = st;
+        }
     }
-    if (blockIdx.x == 0 && threadIdx.x == 0) rb.state[(it & 1) * rb.batch + e] = st;
-    if (st.done && it < R::iters) return;
-    for (int64_t j = (int64_t)blockIdx.x * 256 + threadIdx.x; j < n; j += (int64_t)gridDim.x * 256) {
-        const double2 v = rb.ab[e * n + j];
-        const double g = gamma[j];
-        double sn, cs;
-        sincos(g * st.d, &sn, &cs);
-        const double val = v.x * cs - v.y * sn;
-        const double dval = g * (-v.x * sn - v.y * cs);
-        rb.term[e * n + j] = make_double2(val, dval);
-    }
-}
-
-__global__ void __launch_bounds__(POLISH_THREADS)
-redo_sum_kernel(const double *gamma, int64_t n, CellWeights wts, RedoBuf rb, int it, bool value) {
-    __shared__ double red[POLISH_THREADS / 32];
-    const int e = blockIdx.y, rank = blockIdx.x;
-    if (!value && rb.state[(it & 1) * rb.batch + e].done) return;
+    __syncthreads();
+    const double d = s_state.d;
+    const bool value = it == R::iters;
+    if (s_state.done && !value) return;
     const double *w = wts.w[rb.list[e].w];
-    const double2 *term = rb.term + e * n;
-    double x = 0.0, y = 0.0;
-    // REDO_AHEAD zeros' loads are issued before the first of their additions (0.46 us per zero otherwise)
-    for (int64_t j0 = (int64_t)rank * POLISH_THREADS + threadIdx.x; j0 < n; j0 += REDO_AHEAD * POLISH_STRIDE) {
-        double2 v[REDO_AHEAD];
-        double wv[REDO_AHEAD], g[REDO_AHEAD];
+    const double2 *ab = rb.ab + (int64_t)e * n;
+    const int64_t j0 = (int64_t)blockIdx.x * 32 + lane;             // this lane's sum: zeros j0 + i POLISH_STRIDE
+    const int64_t first = n - (int64_t)blockIdx.x * 32;
+    const int n_batch = first > 0 ? (int)((first + REDO_ROWS * POLISH_STRIDE - 1) / (REDO_ROWS * POLISH_STRIDE)) : 0;
+    double2 v[PER];
+    double g[PER], wv[PER], x = 0.0, y = 0.0;
+    auto fetch = [&](int b) {                          // a row past the end adds 0
 #pragma unroll
-        for (int i = 0; i < REDO_AHEAD; ++i) {
-            const int64_t j = j0 + i * POLISH_STRIDE;
+        for (int i = 0; i < PER; ++i) {
+            const int64_t j = j0 + ((int64_t)b * REDO_ROWS + warp * PER + i) * POLISH_STRIDE;
             const bool in = j < n;
-            v[i] = in ? term[j] : make_double2(0.0, 0.0);
-            wv[i] = in ? w[j] : 0.0;
+            v[i] = in ? ab[j] : make_double2(0.0, 0.0);
             g[i] = in ? gamma[j] : 0.0;
+            wv[i] = in ? w[j] : 0.0;
         }
+    };
+    if (warp < 8 && n_batch > 0) fetch(0);
+    for (int b = 0; b <= n_batch; ++b) {
+        if (warp < 8) {
+            if (b < n_batch) {
 #pragma unroll
-        for (int i = 0; i < REDO_AHEAD; ++i) {
-            if (j0 + i * POLISH_STRIDE >= n) break;
-            if (value) {
-                x += wv[i] * v[i].x;
-            } else {
-                x += wv[i] * v[i].y;
-                y += wv[i] * (-(g[i] * g[i]) * v[i].x);
+                for (int i = 0; i < PER; ++i) {
+                    double sn, cs;
+                    sincos(g[i] * d, &sn, &cs);
+                    const double val = v[i].x * cs - v[i].y * sn;
+                    const double dval = g[i] * (-v[i].x * sn - v[i].y * cs);
+                    const int r = warp * PER + i;
+                    s_d[b & 1][r][lane] = value ? val : dval;
+                    s_dd[b & 1][r][lane] = -(g[i] * g[i]) * val;
+                    s_w[b & 1][r][lane] = wv[i];
+                }
+                if (b + 1 < n_batch) fetch(b + 1);
+            }
+        } else if (b > 0) {
+            const int c = (b - 1) & 1;
+#pragma unroll
+            for (int r = 0; r < REDO_ROWS; ++r) {
+                const double u = s_w[c][r][lane];
+                x += u * s_d[c][r][lane];
+                if (!value) y += u * s_dd[c][r][lane];
             }
         }
+        __syncthreads();
     }
-    x = block_sum(x, red);
-    y = block_sum(y, red);
-    if (threadIdx.x == 0) rb.slot[e * POLISH_CLUSTER + rank] = make_double2(x, y);
+    if (warp == 8) {
+        for (int o = 16; o > 0; o >>= 1) {
+            x += __shfl_xor_sync(0xffffffffu, x, o);
+            y += __shfl_xor_sync(0xffffffffu, y, o);
+        }
+        if (lane == 0) rb.slot[e * REDO_GROUPS + blockIdx.x] = make_double2(x, y);
+    }
 }
 
 // The start's h against the best so far; after the last start, the outputs.
 template <int MODE>
 __global__ void redo_keep_kernel(RedoBuf rb, CellPolishArgs a, int m, int start, bool last) {
     using R = PolishRule<MODE>;
-    const int e = blockIdx.x * blockDim.x + threadIdx.x;
+    const int e = blockIdx.x;                          // a warp each
     if (e >= m) return;
     const int64_t o = rb.list[e].out;
     double hb = start == 0 ? a.h_unpol[o] : rb.h_best[e], db = start == 0 ? 0.0 : rb.d_best[e];
     const double h = redo_total(rb, e).x;
+    if (threadIdx.x > 0) return;
     if (polish_keep<MODE>(h, hb)) {
         hb = h;
         db = rb.state[(R::iters & 1) * rb.batch + e].d;
@@ -1122,9 +1151,9 @@ int launch_cell_scan(const Cells &c, int d1, const double *M, int64_t P, int NB,
     return MB_OK;
 }
 
-// Peaks of one batch of the second pass: their terms take at most 256 MB.
+// Peaks of one batch of the second pass: their A and B take at most 256 MB.
 static int redo_batch(int64_t count, int64_t n) {
-    const int64_t fit = ((int64_t)256 << 20) / (2 * (int64_t)sizeof(double2) * n);
+    const int64_t fit = ((int64_t)256 << 20) / ((int64_t)sizeof(double2) * n);
     return (int)std::max<int64_t>(1, std::min<int64_t>({fit, count, 1024}));
 }
 
@@ -1147,15 +1176,14 @@ static int polish_mode(Table &t, const Cells &c, const double *M, CellPolishArgs
     RedoBuf rb;
     rb.batch = redo_batch(count, n);
     const size_t bn = (size_t)rb.batch * n;
-    MB_TRY(t.redo.ensure((2 * rb.batch * sizeof(RedoState) + 256) + (rb.batch * POLISH_CLUSTER * sizeof(double2) + 256) +
-                         2 * (rb.batch * 8 + 256) + 2 * (bn * sizeof(double2) + 256)));
+    MB_TRY(t.redo.ensure((2 * rb.batch * sizeof(RedoState) + 256) + (rb.batch * REDO_GROUPS * sizeof(double2) + 256) +
+                         2 * (rb.batch * 8 + 256) + (bn * sizeof(double2) + 256)));
     q = (char *)t.redo.p;
     rb.state = carve<RedoState>(q, 2 * (size_t)rb.batch);
-    rb.slot = carve<double2>(q, (size_t)rb.batch * POLISH_CLUSTER);
+    rb.slot = carve<double2>(q, (size_t)rb.batch * REDO_GROUPS);
     rb.h_best = carve<double>(q, rb.batch);
     rb.d_best = carve<double>(q, rb.batch);
     rb.ab = carve<double2>(q, bn);
-    rb.term = carve<double2>(q, bn);
     const int ns = MODE == POLISH_SINGLE && a.n_grid == 0 ? 1 : R::starts;
     const ABExact src{view(t), vi, vf, delta};
     for (int e0 = 0; e0 < count; e0 += rb.batch) {
@@ -1164,11 +1192,9 @@ static int polish_mode(Table &t, const Cells &c, const double *M, CellPolishArgs
         const unsigned nb = (unsigned)((n + 255) / 256);
         redo_ab_kernel<<<dim3(nb, m), 256, 0, s>>>(src, n, rb);
         for (int st = 0; st < ns; ++st) {
-            for (int it = 0; it <= R::iters; ++it) {     // the last pass sums h
-                redo_term_kernel<MODE><<<dim3((nb + 1) / 2, m), 256, 0, s>>>(t.d_gamma, n, rb, st, it);
-                redo_sum_kernel<<<dim3(POLISH_CLUSTER, m), POLISH_THREADS, 0, s>>>(t.d_gamma, n, w, rb, it, it == R::iters);
-            }
-            redo_keep_kernel<MODE><<<(m + 127) / 128, 128, 0, s>>>(rb, a, (int)m, st, st == ns - 1);
+            for (int it = 0; it <= R::iters; ++it)       // the last pass sums h
+                redo_pass_kernel<MODE><<<dim3(REDO_GROUPS, m), REDO_THREADS, 0, s>>>(t.d_gamma, n, w, rb, st, it);
+            redo_keep_kernel<MODE><<<m, 32, 0, s>>>(rb, a, (int)m, st, st == ns - 1);
         }
         MB_CUDA(cudaGetLastError());
     }
