@@ -45,19 +45,18 @@ WORKLOAD = ("search_scoring: all 466,659 synthetic zeros below T0=3e5, 4,096 can
 # `bench.py --profile-case search` (dram__bytes_read.sum + dram__bytes_write.sum), and the
 # executed thread instructions per zero-term of each kernel from the same capture
 # (smsp__inst_executed.sum x 32 / zero-terms): the issue-slot side figure beside the pipe roofline.
-LIGHT_DRAM_BYTES = {2: 16468736, 3: 16439040, 4: 16414976}
-HEAVY_DRAM_BYTES = 2827264
-TIERS_DRAM_BYTES = 19178240          # k2_tiers_kernel<4> (both tiers in one launch)
-LIGHT_INST_PER_TERM = {2: 19.32, 3: 19.86, 4: 16.54}
-HEAVY_INST_PER_TERM = 39.39
+LIGHT_DRAM_BYTES = {2: 16468736, 3: 16439040, 4: 16438784}
+HEAVY_DRAM_BYTES = 2891008
+TIERS_DRAM_BYTES = 27556096          # k2_tiers_kernel<4> (both tiers in one launch)
+LIGHT_INST_PER_TERM = {2: 19.32, 3: 19.86, 4: 16.56}
+HEAVY_INST_PER_TERM = 34.93
 # Algorithmic operations per zero-term on each tier's binding pipe:
 #   light tier, XU (MUFU) pipe: one sine and one cosine of the reduced phase;
-#   heavy tier, FP64 pipe: 4 DFMA for the 2^-64-turn phase products, 1 add onto the rounding
-#   constant, 1 FMA for the exact table remainder, 8 for the table sine/cosine (r^2, the sine
-#   polynomial and product, the cosine product, two 2-FMA rotations) and 3 FMA accumulations of
-#   K2, dK2/ddelta, dK2/dk.
+#   heavy tier, FP64 pipe: 4 DFMA for the phase's limb-pair products, 1 add of the two chains, 1
+#   subtraction for the exact table remainder, 10 for the table sine/cosine (its square, 3 for the sine,
+#   2 for the cosine less 1, two 2-FMA rotations) and 3 FMA accumulations of K2, dK2/ddelta, dK2/dk.
 LIGHT_MUFU_PER_TERM = 2
-HEAVY_FP64_PER_TERM = 17
+HEAVY_FP64_PER_TERM = 19
 REF_SAMPLE_CANDS = 64
 REF_TIMED_BUDGET_S = 200.0   # the reference arm's timed steps, at most (a bounded sample per step)
 

@@ -2,10 +2,9 @@
 K2 kernels, fitted here from the mathematics (Chebyshev interpolation in mpmath at 60
 digits, coefficients rounded to the target type).  Run: python gen_poly.py > poly_coeffs.h
 
-All polynomials are in the *turn* variable (angle = 2 pi t or pi t) so the kernels never
+All polynomials are in the *turn* variable (angle = 2 pi t) so the kernels never
 multiply the exactly reduced phase by an inexact 2 pi before the polynomial.
 
-  HALF_S(u), HALF_C(u):  sin(pi t) = t * HALF_S(t^2),  cos(pi t) = HALF_C(t^2),  |t| <= 1/2
   QUAD_S(u), QUAD_C(u):  sin(2 pi r) = r * QUAD_S(r^2), cos(2 pi r) = QUAD_C(r^2), |r| <= 1/8
   F32_S(u),  F32_C(u):   the same quarter-turn pair in binary32, |r| <= 1/8
 """
@@ -53,8 +52,6 @@ def main():
            "// Ascending powers of u = t^2; see gen_poly.py for the meaning of each set.",
            "#pragma once"]
     sets = [
-        ("HALF_S", lambda u: mp.sin(mp.pi * mp.sqrt(u)) / mp.sqrt(u) if u > 0 else mp.pi, mp.mpf(0), mp.mpf(1) / 4, 8, "double", f64),
-        ("HALF_C", lambda u: mp.cos(mp.pi * mp.sqrt(u)), mp.mpf(0), mp.mpf(1) / 4, 9, "double", f64),
         ("QUAD_S", lambda u: mp.sin(2 * mp.pi * mp.sqrt(u)) / mp.sqrt(u) if u > 0 else 2 * mp.pi, mp.mpf(0), mp.mpf(1) / 64, 5, "double", f64),
         ("QUAD_C", lambda u: mp.cos(2 * mp.pi * mp.sqrt(u)), mp.mpf(0), mp.mpf(1) / 64, 5, "double", f64),
         ("F32_S", lambda u: mp.sin(2 * mp.pi * mp.sqrt(u)) / mp.sqrt(u) if u > 0 else 2 * mp.pi, mp.mpf(0), mp.mpf(1) / 64, 3, "float", f32),
@@ -84,7 +81,7 @@ def certified_sets():
     """Taylor coefficients of sin x / x and cos x in u = x^2 as outward-rounded intervals
     (exact rationals (-1)^k/(2k+1)! and (-1)^k/(2k)!), and an enclosure of pi/2, for the
     directed-rounding interval kernel.  Used on 0 <= x <= pi/4 with the Lagrange remainder
-    x^19/19! (sine, 9 terms) and x^20/20! (cosine, 10 terms) added separately."""
+    x^19/19! (sine, 9 terms) and x^20/20! (cosine, 10 terms) added by the kernel."""
     import math
     from fractions import Fraction
     s = [Fraction((-1) ** k, math.factorial(2 * k + 1)) for k in range(9)]
@@ -102,8 +99,6 @@ def certified_sets():
         _, hi = outward(q + Fraction(1, int(den)))
     out.append(f"#define CERT_PIO2_LO {lo!r}")
     out.append(f"#define CERT_PIO2_HI {hi!r}")
-    out.append(f"#define CERT_REM_S {outward(Fraction(1, math.factorial(19)))[1]!r}   // 1/19! rounded up")
-    out.append(f"#define CERT_REM_C {outward(Fraction(1, math.factorial(20)))[1]!r}   // 1/20! rounded up")
     return out
 
 

@@ -159,22 +159,6 @@ MB_DEV double s64_turns_to_f64(uint64_t w) {
 
 // ---------------------------------------------------------------- trig in turns
 
-// sin(2 pi t), cos(2 pi t) for |t| <= 1/2 (FP64), by the half-angle pair
-// s = sin(pi t), c = cos(pi t): sin(2 pi t) = 2 s c, cos(2 pi t) = 1 - 2 s^2.
-// No quadrant selection, so no integer work; ~21 FP64 operations.
-MB_DEV void sincos_turns_half(double t, double &s2, double &c2) {
-    double u = t * t;
-    double ps = HALF_S[8];
-#pragma unroll
-    for (int i = 7; i >= 0; --i) ps = fma(ps, u, HALF_S[i]);
-    double pc = HALF_C[9];
-#pragma unroll
-    for (int i = 8; i >= 0; --i) pc = fma(pc, u, HALF_C[i]);
-    double s = t * ps;
-    s2 = 2.0 * s * pc;
-    c2 = fma(-2.0 * s, s, 1.0);
-}
-
 // 1.5 2^52: adding it rounds a double of magnitude < 2^51 to an integer held in the low
 // mantissa word.
 constexpr double MB_MAGIC = 6755399441055744.0;
