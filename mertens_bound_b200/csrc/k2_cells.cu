@@ -10,6 +10,8 @@
 #include <algorithm>
 #include <cmath>
 
+#include <cuda_pipeline.h>
+
 #include "k2_cells.h"
 #include "k2_common.cuh"
 #include "k2_phasor.cuh"
@@ -412,23 +414,23 @@ int launch_moments(const Table &t, const Cells &c, const uint64_t *vi, const uin
 constexpr int CSCAN_PTS = 256;                 // grid points per CTA
 constexpr int CSCAN_PT = 2;                    // grid points per thread
 constexpr int CSCAN_LANES = CSCAN_PTS / CSCAN_PT;
-constexpr int CSCAN_SPLIT = 2;                 // thread groups sharing the cells
-constexpr int CSCAN_THREADS = CSCAN_LANES * CSCAN_SPLIT;
 constexpr int CSCAN_CELLS = 32;                // cells staged at a time
 
-// Thread: CSCAN_PT points of one base point over every CSCAN_SPLIT-th cell; the moments are read as
+// Thread: CSCAN_PT points of one base point over every SPLIT-th cell; the moments are read as
 // broadcasts.  With a few hundred CTAs the cells' dependent chains are exposed, hence the split (its sums are
-// added in order) and the four products of each point summed apart.
-template <int D1>
-__global__ void __launch_bounds__(CSCAN_THREADS)
+// added in order) and the four products of each point summed apart.  The next CSCAN_CELLS cells' moments are
+// copied while the current ones are evaluated.
+template <int D1, int SPLIT>
+__global__ void __launch_bounds__(CSCAN_LANES *SPLIT)
 cell_scan_kernel(Cells cells, const double *M, int NB, int Bp, int64_t n_m, uint64_t si, uint64_t sf, double kstep,
                  double *out) {
+    constexpr int THREADS = CSCAN_LANES * SPLIT;
     extern __shared__ __align__(16) unsigned char smem[];
     double2 *tab = reinterpret_cast<double2 *>(smem);
-    double2 *mom = reinterpret_cast<double2 *>(smem + PH_BYTES);                  // [cell][D1]: pairs of one row
-    ulonglong2 *dph = reinterpret_cast<ulonglong2 *>(mom + CSCAN_CELLS * D1);     // frac(step G_c): lo, hi
+    double2 *mom_ = reinterpret_cast<double2 *>(smem + PH_BYTES);                 // [2][cell][D1]: pairs of one row
+    ulonglong2 *dph_ = reinterpret_cast<ulonglong2 *>(mom_ + 2 * CSCAN_CELLS * D1);     // [2][cell] frac(step G_c): lo, hi
     const double2 *copy = tab + (threadIdx.x & (PH_COPIES - 1));
-    phasor_table_init(tab, CSCAN_THREADS);
+    phasor_table_init(tab, THREADS);
     const int part = threadIdx.x / CSCAN_LANES, tl = threadIdx.x - part * CSCAN_LANES;
     const int64_t pb = blockIdx.y;                               // point p NB + b
     const int64_t p = pb / NB, b = pb - p * NB;
@@ -448,20 +450,34 @@ cell_scan_kernel(Cells cells, const double *M, int NB, int Bp, int64_t n_m, uint
         }
         h[i] = 0.0;
     }
-    for (int cb = 0; cb < cells.n; cb += CSCAN_CELLS) {
+    // cells [cb, cb + CSCAN_CELLS): their moments on the way into half k of the buffer, this thread's centre
+    auto fetch = [&](int cb, int k) -> int64_t {
         const int nc = min(CSCAN_CELLS, cells.n - cb);
-        __syncthreads();
         const double2 *src = reinterpret_cast<const double2 *>(M + (pb * cells.n + cb) * (2 * D1));
-        for (int i = threadIdx.x; i < nc * D1; i += CSCAN_THREADS) mom[i] = src[i];
-        if ((int)threadIdx.x < nc) {
-            const uint64_t g = (uint64_t)cells.ctr[cb + threadIdx.x] << 16;          // G_c 2^32
+        for (int i = threadIdx.x; i < nc * D1; i += THREADS)
+            __pipeline_memcpy_async(mom_ + k * CSCAN_CELLS * D1 + i, src + i, sizeof(double2));
+        __pipeline_commit();
+        return (int)threadIdx.x < nc ? cells.ctr[cb + threadIdx.x] : 0;
+    };
+    auto landed = [&](int64_t ctr, int k) {
+        if (threadIdx.x < CSCAN_CELLS) {
+            const uint64_t g = (uint64_t)ctr << 16;                                  // G_c 2^32
             uint64_t hi, lo;
             phase128_exact((uint32_t)sf, (uint32_t)(sf >> 32), (uint32_t)si, (uint32_t)(si >> 32), 0, 0, 0,
                            (uint32_t)g, (uint32_t)(g >> 32), hi, lo);
-            dph[threadIdx.x] = make_ulonglong2(lo, hi);
+            dph_[k * CSCAN_CELLS + threadIdx.x] = make_ulonglong2(lo, hi);
         }
+        __pipeline_wait_prior(0);
         __syncthreads();
-        for (int c = part; c < nc; c += CSCAN_SPLIT) {
+    };
+    if (cells.n > 0) landed(fetch(0, 0), 0);
+    for (int cb = 0, k = 0; cb < cells.n; cb += CSCAN_CELLS, k ^= 1) {
+        const int nc = min(CSCAN_CELLS, cells.n - cb);
+        const bool more = cb + CSCAN_CELLS < cells.n;
+        const int64_t ctr = more ? fetch(cb + CSCAN_CELLS, k ^ 1) : 0;
+        const double2 *mom = mom_ + k * CSCAN_CELLS * D1;
+        const ulonglong2 *dph = dph_ + k * CSCAN_CELLS;
+        for (int c = part; c < nc; c += SPLIT) {
             const double2 *m2 = mom + c * D1;
             const ulonglong2 d = dph[c];
             double cs[CSCAN_PT], sn[CSCAN_PT];
@@ -491,10 +507,11 @@ cell_scan_kernel(Cells cells, const double *M, int NB, int Bp, int64_t n_m, uint
 #pragma unroll
             for (int i = 0; i < CSCAN_PT; ++i) h[i] += fma(cs[i], rr[i] - ri[i], -sn[i] * (ir[i] + ii[i]));
         }
+        if (more) landed(ctr, k ^ 1);
     }
     // the other parts' sums, in order (they take the moments' place)
-    double *other = reinterpret_cast<double *>(mom);
-    for (int q = 1; q < CSCAN_SPLIT; ++q) {
+    double *other = reinterpret_cast<double *>(mom_);
+    for (int q = 1; q < SPLIT; ++q) {
         __syncthreads();
         if (part == q)
 #pragma unroll
@@ -515,7 +532,7 @@ cell_scan_kernel(Cells cells, const double *M, int NB, int Bp, int64_t n_m, uint
 template <int D1>
 constexpr int cscan_smem() {
     static_assert(CSCAN_CELLS * D1 * 16 >= CSCAN_PTS * 8, "the parts' sums fit the moments' place");
-    return PH_BYTES + CSCAN_CELLS * (D1 * 16 + 16);
+    return PH_BYTES + 2 * CSCAN_CELLS * (D1 * 16 + 16);
 }
 
 // ------------------------------------------------------------------ polishes on moments
@@ -1024,8 +1041,10 @@ int cell_kernel_attributes() {
     MB_TRY(set_smem(cell_moments_kernel<CELL_WEIGHTS, 4, CELL_D1>, CellShape<CELL_WEIGHTS, 4, CELL_D1>::smem));
     MB_TRY(set_smem(cell_moments_kernel<CELL_WEIGHTS, 5, CELL_D1>, CellShape<CELL_WEIGHTS, 5, CELL_D1>::smem));
     MB_TRY(set_smem(cell_moments_kernel<CELL_POWERS, 1, 17>, CellShape<CELL_POWERS, 1, 17>::smem));
-    MB_TRY(set_smem(cell_scan_kernel<8>, cscan_smem<8>()));
-    MB_TRY(set_smem(cell_scan_kernel<16>, cscan_smem<16>()));
+    MB_TRY(set_smem(cell_scan_kernel<8, 2>, cscan_smem<8>()));
+    MB_TRY(set_smem(cell_scan_kernel<16, 2>, cscan_smem<16>()));
+    MB_TRY(set_smem(cell_scan_kernel<8, 4>, cscan_smem<8>()));
+    MB_TRY(set_smem(cell_scan_kernel<16, 4>, cscan_smem<16>()));
     if (dev >= 0 && dev < 64) done_ctx[dev] = current_context();
     return MB_OK;
 }
@@ -1137,16 +1156,23 @@ int launch_taylor_grid(const Table &t, const uint64_t *vi, const uint64_t *vf, c
     return MB_OK;
 }
 
-int launch_cell_scan(const Cells &c, int d1, const double *M, int64_t P, int NB, int Bp, int64_t n_m,
+int launch_cell_scan(const Table &t, const Cells &c, int d1, const double *M, int64_t P, int NB, int Bp, int64_t n_m,
                      uint64_t step_int, uint64_t step_frac, double *out, cudaStream_t s) {
     MB_TRY(cell_kernel_attributes());
     const double step = (double)step_int + (double)step_frac * 0x1p-64;
     const double kstep = 6.283185307179586 * c.H() * step;
     const dim3 grid((unsigned)((Bp + CSCAN_PTS - 1) / CSCAN_PTS), (unsigned)(P * NB));
+    // cells split four ways where at most one CTA falls to an SM (2 warps per scheduler otherwise)
+    int sms = 148;
+    MB_TRY(sm_count(t, &sms));
+    const bool four = (int64_t)grid.x * grid.y <= sms;
+    auto launch = [&](auto kernel, int split, int bytes) {
+        kernel<<<grid, CSCAN_LANES * split, bytes, s>>>(c, M, NB, Bp, n_m, step_int, step_frac, kstep, out);
+    };
     if (d1 == 8)
-        cell_scan_kernel<8><<<grid, CSCAN_THREADS, cscan_smem<8>(), s>>>(c, M, NB, Bp, n_m, step_int, step_frac, kstep, out);
+        four ? launch(cell_scan_kernel<8, 4>, 4, cscan_smem<8>()) : launch(cell_scan_kernel<8, 2>, 2, cscan_smem<8>());
     else
-        cell_scan_kernel<16><<<grid, CSCAN_THREADS, cscan_smem<16>(), s>>>(c, M, NB, Bp, n_m, step_int, step_frac, kstep, out);
+        four ? launch(cell_scan_kernel<16, 4>, 4, cscan_smem<16>()) : launch(cell_scan_kernel<16, 2>, 2, cscan_smem<16>());
     MB_CUDA(cudaGetLastError());
     return MB_OK;
 }

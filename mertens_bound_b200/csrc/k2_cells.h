@@ -80,7 +80,7 @@ int launch_taylor_grid(const Table &t, const uint64_t *vi, const uint64_t *vf, c
 
 // out[p n_m + b Bp + i] = h at the offset (i - Bp / 2) step of point p NB + b, i < Bp, b < NB
 // (Bp NB >= n_m; the moments are those of the P NB points).
-int launch_cell_scan(const Cells &c, int d1, const double *M, int64_t P, int NB, int Bp, int64_t n_m,
+int launch_cell_scan(const Table &t, const Cells &c, int d1, const double *M, int64_t P, int NB, int Bp, int64_t n_m,
                      uint64_t step_int, uint64_t step_frac, double *out, cudaStream_t s);
 
 // Polishes of P peaks under nw weights from their moments (CELL_D1 terms): the three loops of

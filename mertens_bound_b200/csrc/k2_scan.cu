@@ -349,7 +349,7 @@ int scan_cells(Table &t, int64_t P, const uint64_t *v_int, const uint64_t *v_fra
             }
         MB_CUDA(cudaMemcpyAsync(d_v, pts.data(), 2 * (size_t)nb * 8, cudaMemcpyHostToDevice, t.stream));
         MB_TRY(launch_moments_gauss(t, cells, d_v, d_v + nb, nb, k, sp.d1, M, t.stream));
-        MB_TRY(launch_cell_scan(cells, sp.d1, M, np, sp.NB, sp.Bp, n_m, step_int, step_frac, d_h, t.stream));
+        MB_TRY(launch_cell_scan(t, cells, sp.d1, M, np, sp.NB, sp.Bp, n_m, step_int, step_frac, d_h, t.stream));
         MB_TRY(take(p0, np, (const double *)d_h));
     }
     return MB_OK;
