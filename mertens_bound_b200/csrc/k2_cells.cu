@@ -411,14 +411,15 @@ int launch_moments(const Table &t, const Cells &c, const uint64_t *vi, const uin
 
 // ------------------------------------------------------------------ offset scans
 
-constexpr int CSCAN_PTS = 256;                 // grid points per CTA
-constexpr int CSCAN_PT = 2;                    // grid points per thread
-constexpr int CSCAN_LANES = CSCAN_PTS / CSCAN_PT;
+constexpr int CSCAN_PT = 2;                    // pairs of offsets +-m step per thread
+constexpr int CSCAN_LANES = CSCAN_PAIRS / CSCAN_PT;
 constexpr int CSCAN_CELLS = 32;                // cells staged at a time
 
-// Thread: CSCAN_PT points of one base point over every SPLIT-th cell; the moments are read as
-// broadcasts.  With a few hundred CTAs the cells' dependent chains are exposed, hence the split (its sums are
-// added in order) and the four products of each point summed apart.  The next CSCAN_CELLS cells' moments are
+// Thread: CSCAN_PT pairs of offsets +-m step of one block over every SPLIT-th cell.  The offset's sign changes
+// only the signs of the odd terms and of the rotation's sine, so the pair costs one rotation and one series
+// (256 x 241 points over 235 cells 60 -> 36 us; a scan call of 25,001 points 158 -> 143).  The moments are read
+// as broadcasts.  With a few hundred CTAs the cells' dependent chains are exposed, hence the split (its sums are
+// added in order) and the four products of each pair summed apart.  The next CSCAN_CELLS cells' moments are
 // copied while the current ones are evaluated.
 template <int D1, int SPLIT>
 __global__ void __launch_bounds__(CSCAN_LANES *SPLIT)
@@ -435,11 +436,11 @@ cell_scan_kernel(Cells cells, const double *M, int NB, int Bp, int64_t n_m, uint
     const int64_t pb = blockIdx.y;                               // point p NB + b
     const int64_t p = pb / NB, b = pb - p * NB;
     const int np = (int)min((int64_t)Bp, n_m - b * Bp);          // points of this block
-    double e[CSCAN_PT][D1], h[CSCAN_PT];
-    int ml[CSCAN_PT];
+    double e[CSCAN_PT][D1], h[CSCAN_PT][2];                      // h at +m and -m
+    uint32_t ml[CSCAN_PT];
 #pragma unroll
     for (int i = 0; i < CSCAN_PT; ++i) {
-        ml[i] = (int)(blockIdx.x * CSCAN_PT + i) * CSCAN_LANES + tl - Bp / 2;
+        ml[i] = (blockIdx.x * CSCAN_PT + i) * CSCAN_LANES + tl;
         // (kappa d)^n / n! with the sign of i^n: + + - -
         const double y = kstep * ml[i];
         double x = 1.0;
@@ -448,7 +449,7 @@ cell_scan_kernel(Cells cells, const double *M, int NB, int Bp, int64_t n_m, uint
             e[i][n] = (n & 2) ? -x : x;
             x *= y * (1.0 / (n + 1));
         }
-        h[i] = 0.0;
+        h[i][0] = h[i][1] = 0.0;
     }
     // cells [cb, cb + CSCAN_CELLS): their moments on the way into half k of the buffer, this thread's centre
     auto fetch = [&](int cb, int k) -> int64_t {
@@ -483,11 +484,9 @@ cell_scan_kernel(Cells cells, const double *M, int NB, int Bp, int64_t n_m, uint
             double cs[CSCAN_PT], sn[CSCAN_PT];
 #pragma unroll
             for (int i = 0; i < CSCAN_PT; ++i) {
-                // frac(m step G_c) to 2^-64 turn, m the signed offset index of less than 2^31
-                const uint32_t ma = (uint32_t)(ml[i] < 0 ? -ml[i] : ml[i]);
-                uint64_t w = wide(ma, (uint32_t)d.y) + ((uint64_t)(ma * (uint32_t)(d.y >> 32)) << 32) +
-                             (wide(ma, (uint32_t)(d.x >> 32)) >> 32);
-                if (ml[i] < 0) w = ~w;
+                // frac(m step G_c) to 2^-64 turn
+                const uint64_t w = wide(ml[i], (uint32_t)d.y) + ((uint64_t)(ml[i] * (uint32_t)(d.y >> 32)) << 32) +
+                                   (wide(ml[i], (uint32_t)(d.x >> 32)) >> 32);
                 phasor((w >> 4) + (1ull << 51), copy, cs[i], sn[i]);
             }
             double rr[CSCAN_PT], ri[CSCAN_PT], ir[CSCAN_PT], ii[CSCAN_PT];
@@ -505,7 +504,10 @@ cell_scan_kernel(Cells cells, const double *M, int NB, int Bp, int64_t n_m, uint
                 }
             }
 #pragma unroll
-            for (int i = 0; i < CSCAN_PT; ++i) h[i] += fma(cs[i], rr[i] - ri[i], -sn[i] * (ir[i] + ii[i]));
+            for (int i = 0; i < CSCAN_PT; ++i) {
+                h[i][0] += fma(cs[i], rr[i] - ri[i], -sn[i] * (ir[i] + ii[i]));
+                h[i][1] += fma(cs[i], rr[i] + ri[i], sn[i] * (ir[i] - ii[i]));
+            }
         }
         if (more) landed(ctr, k ^ 1);
     }
@@ -515,23 +517,24 @@ cell_scan_kernel(Cells cells, const double *M, int NB, int Bp, int64_t n_m, uint
         __syncthreads();
         if (part == q)
 #pragma unroll
-            for (int i = 0; i < CSCAN_PT; ++i) other[i * CSCAN_LANES + tl] = h[i];
+            for (int i = 0; i < 2 * CSCAN_PT; ++i) other[i * CSCAN_LANES + tl] = h[i >> 1][i & 1];
         __syncthreads();
         if (part == 0)
 #pragma unroll
-            for (int i = 0; i < CSCAN_PT; ++i) h[i] += other[i * CSCAN_LANES + tl];
+            for (int i = 0; i < 2 * CSCAN_PT; ++i) h[i >> 1][i & 1] += other[i * CSCAN_LANES + tl];
     }
     if (part > 0) return;
 #pragma unroll
     for (int i = 0; i < CSCAN_PT; ++i) {
-        const int l = ml[i] + Bp / 2;
-        if (l < np) out[p * n_m + b * Bp + l] = h[i];
+        const int l = Bp / 2 + (int)ml[i], r = Bp / 2 - (int)ml[i];
+        if (l < np) out[p * n_m + b * Bp + l] = h[i][0];
+        if (ml[i] > 0 && r >= 0 && r < np) out[p * n_m + b * Bp + r] = h[i][1];
     }
 }
 
 template <int D1>
 constexpr int cscan_smem() {
-    static_assert(CSCAN_CELLS * D1 * 16 >= CSCAN_PTS * 8, "the parts' sums fit the moments' place");
+    static_assert(2 * CSCAN_CELLS * D1 * 16 >= 2 * CSCAN_PAIRS * 8, "the parts' sums fit the moments' place");
     return PH_BYTES + 2 * CSCAN_CELLS * (D1 * 16 + 16);
 }
 
@@ -1041,10 +1044,10 @@ int cell_kernel_attributes() {
     MB_TRY(set_smem(cell_moments_kernel<CELL_WEIGHTS, 4, CELL_D1>, CellShape<CELL_WEIGHTS, 4, CELL_D1>::smem));
     MB_TRY(set_smem(cell_moments_kernel<CELL_WEIGHTS, 5, CELL_D1>, CellShape<CELL_WEIGHTS, 5, CELL_D1>::smem));
     MB_TRY(set_smem(cell_moments_kernel<CELL_POWERS, 1, 17>, CellShape<CELL_POWERS, 1, 17>::smem));
-    MB_TRY(set_smem(cell_scan_kernel<8, 2>, cscan_smem<8>()));
-    MB_TRY(set_smem(cell_scan_kernel<16, 2>, cscan_smem<16>()));
     MB_TRY(set_smem(cell_scan_kernel<8, 4>, cscan_smem<8>()));
     MB_TRY(set_smem(cell_scan_kernel<16, 4>, cscan_smem<16>()));
+    MB_TRY(set_smem(cell_scan_kernel<8, 8>, cscan_smem<8>()));
+    MB_TRY(set_smem(cell_scan_kernel<16, 8>, cscan_smem<16>()));
     if (dev >= 0 && dev < 64) done_ctx[dev] = current_context();
     return MB_OK;
 }
@@ -1161,18 +1164,18 @@ int launch_cell_scan(const Table &t, const Cells &c, int d1, const double *M, in
     MB_TRY(cell_kernel_attributes());
     const double step = (double)step_int + (double)step_frac * 0x1p-64;
     const double kstep = 6.283185307179586 * c.H() * step;
-    const dim3 grid((unsigned)((Bp + CSCAN_PTS - 1) / CSCAN_PTS), (unsigned)(P * NB));
-    // cells split four ways where at most one CTA falls to an SM (2 warps per scheduler otherwise)
+    const dim3 grid((unsigned)cell_scan_ctas(Bp), (unsigned)(P * NB));
+    // cells split eight ways where at most one CTA falls to an SM (2 warps per scheduler otherwise)
     int sms = 148;
     MB_TRY(sm_count(t, &sms));
-    const bool four = (int64_t)grid.x * grid.y <= sms;
+    const bool eight = (int64_t)grid.x * grid.y <= sms;
     auto launch = [&](auto kernel, int split, int bytes) {
         kernel<<<grid, CSCAN_LANES * split, bytes, s>>>(c, M, NB, Bp, n_m, step_int, step_frac, kstep, out);
     };
     if (d1 == 8)
-        four ? launch(cell_scan_kernel<8, 4>, 4, cscan_smem<8>()) : launch(cell_scan_kernel<8, 2>, 2, cscan_smem<8>());
+        eight ? launch(cell_scan_kernel<8, 8>, 8, cscan_smem<8>()) : launch(cell_scan_kernel<8, 4>, 4, cscan_smem<8>());
     else
-        four ? launch(cell_scan_kernel<16, 4>, 4, cscan_smem<16>()) : launch(cell_scan_kernel<16, 2>, 2, cscan_smem<16>());
+        eight ? launch(cell_scan_kernel<16, 8>, 8, cscan_smem<16>()) : launch(cell_scan_kernel<16, 4>, 4, cscan_smem<16>());
     MB_CUDA(cudaGetLastError());
     return MB_OK;
 }

@@ -78,6 +78,10 @@ int launch_taylor_grid(const Table &t, const uint64_t *vi, const uint64_t *vf, c
                        int64_t n, int n_chunk, const double *w, const double *grid, int n_grid, void *work,
                        double *h_unpol, double *h_pol, double *ddy_pol, cudaStream_t s);
 
+// Offset pairs +-m step of one evaluation CTA, and the CTAs of a block of Bp points (pairs 0 .. Bp / 2).
+constexpr int CSCAN_PAIRS = 128;
+inline int64_t cell_scan_ctas(int64_t Bp) { return (Bp / 2 + CSCAN_PAIRS) / CSCAN_PAIRS; }
+
 // out[p n_m + b Bp + i] = h at the offset (i - Bp / 2) step of point p NB + b, i < Bp, b < NB
 // (Bp NB >= n_m; the moments are those of the P NB points).
 int launch_cell_scan(const Table &t, const Cells &c, int d1, const double *M, int64_t P, int NB, int Bp, int64_t n_m,

@@ -288,8 +288,8 @@ bool plan_scan(const Table &t, int64_t P, int64_t n_use, int64_t n_m, uint64_t s
             // one moment item per SM keeps it busy; however few they are, a scan CTA (256 points) takes the
             // latency of its cells, three CTAs to an SM
             const double mom = tiles * zeros * (ppc / 32.0 * (120.0 + 5.0 * d1) + 20.0) / std::min(1.0, nc * tiles / 148.0);
-            const double ctas = (double)pts * ((Bp + 255) / 256);
-            const double eval = nc * (2 * d1 + 15) * std::max(ctas * 8.0 * 3.6, 592.0 * 8.0 * std::ceil(ctas / 444.0));
+            const double ctas = (double)pts * cell_scan_ctas(Bp);
+            const double eval = nc * (2 * d1 + 15) * std::max(ctas * 8.0 * 1.8, 592.0 * 4.0 * std::ceil(ctas / 444.0));
             const double bytes = (double)NB * nc * 2 * d1 * 8;
             if (bytes > (double)SCAN_MOMENT_BYTES) continue;
             if (mom + eval < best_cost) {
