@@ -180,3 +180,19 @@ def test_certified_candidate_tiles(table, small_table, oracle, P, n):
         assert np.all(wlo[row] - eps <= mid[:, row]) and np.all(mid[:, row] <= whi[row] + eps)
     assert np.array_equal(rlo[:-1], lo[:-1]) and np.array_equal(rhi[:-1], hi[:-1])
     assert rlo[-1] < lo[-1] and rhi[-1] > hi[-1]
+
+
+@pytest.mark.parametrize("half", [0.045, 0.055, 0.08])
+def test_polish_cells_around_shared_memory(gpu, half):
+    """About 1,060, 1,290 and 1,880 cells: the polish's moments fit shared memory (1,200 cells) or do not.  The
+    matrix form's offsets agree to 1e-12 and h to 3e-11 (an offset of 1e-14 times |h'| < 3e3)."""
+    from mertens_bound_b200 import compat, path1
+    data = synth.make_table(9000, seed=81)
+    c = synth.make_candidates(5, seed=95)
+    w = np.exp(-3e-9 * data.gamma ** 2)
+    with k2.ZeroTable.from_data(data) as t:
+        got = path1.polish_peaks_exact(t, c, t.add_weights(w), None, half, 40)
+        A, B = path1.compute_exact_AB(t, c)
+    want = compat.polish_peaks_with_weights(A, B, data.gamma, w, half, 40)
+    for g, x, tol in zip(got, want, (3e-13, 3e-11, 1e-12)):
+        np.testing.assert_allclose(g, x, rtol=0, atol=tol)
