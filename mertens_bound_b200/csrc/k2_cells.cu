@@ -6,7 +6,7 @@
 // zeros each lane computes the exact phase and the (cos, sin) of its own (peak, zero) pair in
 // registers -- the cosine is its A element of the real product, the sine that of the imaginary
 // product -- and no phasor is ever stored.  The powers (B) come from shared memory, staged once per
-// 64 zeros for the CTA's 64 peaks.
+// tile of zeros for the CTA's 64 or 128 peaks.
 #include <algorithm>
 #include <cmath>
 
