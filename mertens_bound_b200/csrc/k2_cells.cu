@@ -411,36 +411,34 @@ int launch_moments(const Table &t, const Cells &c, const uint64_t *vi, const uin
 
 // ------------------------------------------------------------------ offset scans
 
-constexpr int CSCAN_PT = 2;                    // pairs of offsets +-m step per thread
-constexpr int CSCAN_LANES = CSCAN_PAIRS / CSCAN_PT;
 constexpr int CSCAN_CELLS = 32;                // cells staged at a time
 
-// Thread: CSCAN_PT pairs of offsets +-m step of one block over every SPLIT-th cell.  The offset's sign changes
+// Thread: PT pairs of offsets +-m step of one block over every SPLIT-th cell.  The offset's sign changes
 // only the signs of the odd terms and of the rotation's sine, so the pair costs one rotation and one series
 // (256 x 241 points over 235 cells 60 -> 36 us; a scan call of 25,001 points 158 -> 143).  The moments are read
 // as broadcasts.  With a few hundred CTAs the cells' dependent chains are exposed, hence the split (its sums are
 // added in order) and the four products of each pair summed apart.  The next CSCAN_CELLS cells' moments are
 // copied while the current ones are evaluated.
-template <int D1, int SPLIT>
-__global__ void __launch_bounds__(CSCAN_LANES *SPLIT)
+template <int D1, int SPLIT, int PT, int LANES>
+__global__ void __launch_bounds__(LANES *SPLIT)
 cell_scan_kernel(Cells cells, const double *M, int NB, int Bp, int64_t n_m, uint64_t si, uint64_t sf, double kstep,
                  double *out) {
-    constexpr int THREADS = CSCAN_LANES * SPLIT;
+    constexpr int THREADS = LANES * SPLIT;
     extern __shared__ __align__(16) unsigned char smem[];
     double2 *tab = reinterpret_cast<double2 *>(smem);
     double2 *mom_ = reinterpret_cast<double2 *>(smem + PH_BYTES);                 // [2][cell][D1]: pairs of one row
     ulonglong2 *dph_ = reinterpret_cast<ulonglong2 *>(mom_ + 2 * CSCAN_CELLS * D1);     // [2][cell] frac(step G_c): lo, hi
     const double2 *copy = tab + (threadIdx.x & (PH_COPIES - 1));
     phasor_table_init(tab, THREADS);
-    const int part = threadIdx.x / CSCAN_LANES, tl = threadIdx.x - part * CSCAN_LANES;
+    const int part = threadIdx.x / LANES, tl = threadIdx.x - part * LANES;
     const int64_t pb = blockIdx.y;                               // point p NB + b
     const int64_t p = pb / NB, b = pb - p * NB;
     const int np = (int)min((int64_t)Bp, n_m - b * Bp);          // points of this block
-    double e[CSCAN_PT][D1], h[CSCAN_PT][2];                      // h at +m and -m
-    uint32_t ml[CSCAN_PT];
+    double e[PT][D1], h[PT][2];                      // h at +m and -m
+    uint32_t ml[PT];
 #pragma unroll
-    for (int i = 0; i < CSCAN_PT; ++i) {
-        ml[i] = (blockIdx.x * CSCAN_PT + i) * CSCAN_LANES + tl;
+    for (int i = 0; i < PT; ++i) {
+        ml[i] = (blockIdx.x * PT + i) * LANES + tl;
         // (kappa d)^n / n! with the sign of i^n: + + - -
         const double y = kstep * ml[i];
         double x = 1.0;
@@ -481,22 +479,22 @@ cell_scan_kernel(Cells cells, const double *M, int NB, int Bp, int64_t n_m, uint
         for (int c = part; c < nc; c += SPLIT) {
             const double2 *m2 = mom + c * D1;
             const ulonglong2 d = dph[c];
-            double cs[CSCAN_PT], sn[CSCAN_PT];
+            double cs[PT], sn[PT];
 #pragma unroll
-            for (int i = 0; i < CSCAN_PT; ++i) {
+            for (int i = 0; i < PT; ++i) {
                 // frac(m step G_c) to 2^-64 turn
                 const uint64_t w = wide(ml[i], (uint32_t)d.y) + ((uint64_t)(ml[i] * (uint32_t)(d.y >> 32)) << 32) +
                                    (wide(ml[i], (uint32_t)(d.x >> 32)) >> 32);
                 phasor((w >> 4) + (1ull << 51), copy, cs[i], sn[i]);
             }
-            double rr[CSCAN_PT], ri[CSCAN_PT], ir[CSCAN_PT], ii[CSCAN_PT];
+            double rr[PT], ri[PT], ir[PT], ii[PT];
 #pragma unroll
-            for (int i = 0; i < CSCAN_PT; ++i) rr[i] = ri[i] = ir[i] = ii[i] = 0.0;
+            for (int i = 0; i < PT; ++i) rr[i] = ri[i] = ir[i] = ii[i] = 0.0;
 #pragma unroll
             for (int n = 0; n < D1; n += 2) {
                 const double2 re = m2[n / 2], im = m2[(D1 + n) / 2];
 #pragma unroll
-                for (int i = 0; i < CSCAN_PT; ++i) {
+                for (int i = 0; i < PT; ++i) {
                     rr[i] = fma(e[i][n], re.x, rr[i]);
                     ri[i] = fma(e[i][n + 1], im.y, ri[i]);
                     ir[i] = fma(e[i][n], im.x, ir[i]);
@@ -504,7 +502,7 @@ cell_scan_kernel(Cells cells, const double *M, int NB, int Bp, int64_t n_m, uint
                 }
             }
 #pragma unroll
-            for (int i = 0; i < CSCAN_PT; ++i) {
+            for (int i = 0; i < PT; ++i) {
                 h[i][0] += fma(cs[i], rr[i] - ri[i], -sn[i] * (ir[i] + ii[i]));
                 h[i][1] += fma(cs[i], rr[i] + ri[i], sn[i] * (ir[i] - ii[i]));
             }
@@ -517,15 +515,15 @@ cell_scan_kernel(Cells cells, const double *M, int NB, int Bp, int64_t n_m, uint
         __syncthreads();
         if (part == q)
 #pragma unroll
-            for (int i = 0; i < 2 * CSCAN_PT; ++i) other[i * CSCAN_LANES + tl] = h[i >> 1][i & 1];
+            for (int i = 0; i < 2 * PT; ++i) other[i * LANES + tl] = h[i >> 1][i & 1];
         __syncthreads();
         if (part == 0)
 #pragma unroll
-            for (int i = 0; i < 2 * CSCAN_PT; ++i) h[i >> 1][i & 1] += other[i * CSCAN_LANES + tl];
+            for (int i = 0; i < 2 * PT; ++i) h[i >> 1][i & 1] += other[i * LANES + tl];
     }
     if (part > 0) return;
 #pragma unroll
-    for (int i = 0; i < CSCAN_PT; ++i) {
+    for (int i = 0; i < PT; ++i) {
         const int l = Bp / 2 + (int)ml[i], r = Bp / 2 - (int)ml[i];
         if (l < np) out[p * n_m + b * Bp + l] = h[i][0];
         if (ml[i] > 0 && r >= 0 && r < np) out[p * n_m + b * Bp + r] = h[i][1];
@@ -1059,10 +1057,12 @@ int cell_kernel_attributes() {
     MB_TRY(set_smem(cell_moments_kernel<CELL_WEIGHTS, 4, CELL_D1>, CellShape<CELL_WEIGHTS, 4, CELL_D1>::smem));
     MB_TRY(set_smem(cell_moments_kernel<CELL_WEIGHTS, 5, CELL_D1>, CellShape<CELL_WEIGHTS, 5, CELL_D1>::smem));
     MB_TRY(set_smem(cell_moments_kernel<CELL_POWERS, 1, 17>, CellShape<CELL_POWERS, 1, 17>::smem));
-    MB_TRY(set_smem(cell_scan_kernel<8, 4>, cscan_smem<8>()));
-    MB_TRY(set_smem(cell_scan_kernel<16, 4>, cscan_smem<16>()));
-    MB_TRY(set_smem(cell_scan_kernel<8, 8>, cscan_smem<8>()));
-    MB_TRY(set_smem(cell_scan_kernel<16, 8>, cscan_smem<16>()));
+    MB_TRY(set_smem(cell_scan_kernel<8, 16, 1, 32>, cscan_smem<8>()));
+    MB_TRY(set_smem(cell_scan_kernel<16, 16, 1, 32>, cscan_smem<16>()));
+    MB_TRY(set_smem(cell_scan_kernel<8, 4, 2, 64>, cscan_smem<8>()));
+    MB_TRY(set_smem(cell_scan_kernel<16, 4, 2, 64>, cscan_smem<16>()));
+    MB_TRY(set_smem(cell_scan_kernel<8, 8, 2, 64>, cscan_smem<8>()));
+    MB_TRY(set_smem(cell_scan_kernel<16, 8, 2, 64>, cscan_smem<16>()));
     if (dev >= 0 && dev < 64) done_ctx[dev] = current_context();
     return MB_OK;
 }
@@ -1179,18 +1179,24 @@ int launch_cell_scan(const Table &t, const Cells &c, int d1, const double *M, in
     MB_TRY(cell_kernel_attributes());
     const double step = (double)step_int + (double)step_frac * 0x1p-64;
     const double kstep = 6.283185307179586 * c.H() * step;
-    const dim3 grid((unsigned)cell_scan_ctas(Bp), (unsigned)(P * NB));
-    // cells split eight ways where at most one CTA falls to an SM (2 warps per scheduler otherwise)
     int sms = 148;
     MB_TRY(sm_count(t, &sms));
-    const bool eight = (int64_t)grid.x * grid.y <= sms;
-    auto launch = [&](auto kernel, int split, int bytes) {
-        kernel<<<grid, CSCAN_LANES * split, bytes, s>>>(c, M, NB, Bp, n_m, step_int, step_frac, kstep, out);
+    auto launch = [&](auto kernel, int pairs, int threads, int bytes) {
+        const dim3 grid((unsigned)((Bp / 2 + pairs) / pairs), (unsigned)(P * NB));
+        kernel<<<grid, threads, bytes, s>>>(c, M, NB, Bp, n_m, step_int, step_frac, kstep, out);
+    };
+    auto form = [&](auto few, auto one, auto many, int bytes) {
+        const int64_t ctas = cell_scan_ctas(Bp) * P * NB;
+        // a CTA per SM at most: the cells split eight ways (2 warps per scheduler otherwise); at most a quarter of
+        // the SMs: 32 pairs a CTA instead of 128 (a scan of 801 points over 98,624 zeros 114 -> 93 us, 5,001: 119 -> 106)
+        if (4 * ctas <= sms) launch(few, 32, 512, bytes);
+        else if (ctas <= sms) launch(one, CSCAN_PAIRS, 512, bytes);
+        else launch(many, CSCAN_PAIRS, 256, bytes);
     };
     if (d1 == 8)
-        eight ? launch(cell_scan_kernel<8, 8>, 8, cscan_smem<8>()) : launch(cell_scan_kernel<8, 4>, 4, cscan_smem<8>());
+        form(cell_scan_kernel<8, 16, 1, 32>, cell_scan_kernel<8, 8, 2, 64>, cell_scan_kernel<8, 4, 2, 64>, cscan_smem<8>());
     else
-        eight ? launch(cell_scan_kernel<16, 8>, 8, cscan_smem<16>()) : launch(cell_scan_kernel<16, 4>, 4, cscan_smem<16>());
+        form(cell_scan_kernel<16, 16, 1, 32>, cell_scan_kernel<16, 8, 2, 64>, cell_scan_kernel<16, 4, 2, 64>, cscan_smem<16>());
     MB_CUDA(cudaGetLastError());
     return MB_OK;
 }
