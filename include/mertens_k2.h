@@ -373,6 +373,9 @@ int mb_polish_peaks_weights(mb_table *t, int64_t P, const uint64_t *v_int, const
 int mb_fast_polish_exact(mb_table *t, int64_t P, const uint64_t *v_int, const uint64_t *v_frac,
                          const double *delta, int64_t n_zeros, int weight_slot, const double *ddy_grid,
                          int64_t n_grid, int top, double *out_h_unpol, double *out_h_pol, double *out_ddy_pol);
+/* The (peak, weight) pairs that the table's last such call polished over the zeros after their cell
+ * moments, because their Newton path amplifies rounding (0 where it used no moments). */
+int mb_table_polish_redone(const mb_table *t, int64_t *n_out);
 
 /* ---- compatibility with the reference's libpath1_eval.so ---------------------------------
  * Same names, signatures and host-array contracts as search/path1_eval_fast.cpp:15 and :58, so

@@ -805,8 +805,10 @@ struct RedoState {
 
 struct RedoBuf {
     const Redo *list;
-    RedoState *state;           // [2][batch], by the pass's parity
-    double2 *slot;              // [batch][REDO_GROUPS]: the warp sums
+    // A pass reads what the pass before wrote while other CTAs of its peak already write theirs, so both are
+    // kept by the pass's parity.
+    RedoState *state;           // [2][batch]
+    double2 *slot;              // [2][batch][REDO_GROUPS]: the warp sums
     double *h_best, *d_best;    // [batch]
     double2 *ab;                // [batch][n]: (A, B)
     int batch;
@@ -820,13 +822,19 @@ __global__ void __launch_bounds__(256) redo_ab_kernel(ABExact src, int64_t n, Re
     rb.ab[blockIdx.y * n + j] = make_double2(A, B);
 }
 
-// The totals: a rank's warp sums in order (one lane each), then the ranks in order; every lane gets them.
-MB_DEV double2 redo_total(const RedoBuf &rb, int e) {
+MB_DEV double2 *redo_slots(const RedoBuf &rb, int it, int e) {
+    return rb.slot + ((int64_t)(it & 1) * rb.batch + e) * REDO_GROUPS;
+}
+
+// The totals of pass `it`: a rank's warp sums in order (one lane each), then the ranks in order; every lane
+// gets them.
+MB_DEV double2 redo_total(const RedoBuf &rb, int it, int e) {
     constexpr int W = REDO_GROUPS / POLISH_CLUSTER;
+    const double2 *slot = redo_slots(rb, it, e);
     const int rank = threadIdx.x & (POLISH_CLUSTER - 1);
     double2 x = make_double2(0.0, 0.0), t = x;
     for (int i = 0; i < W; ++i) {
-        const double2 v = rb.slot[e * REDO_GROUPS + rank * W + i];
+        const double2 v = slot[rank * W + i];
         x.x += v.x;
         x.y += v.y;
     }
@@ -852,7 +860,7 @@ redo_pass_kernel(const double *gamma, int64_t n, CellWeights wts, RedoBuf rb, in
             st = RedoState{rb.list[e].start[start], 0, 0};
         } else {
             st = rb.state[((it - 1) & 1) * rb.batch + e];
-            const double2 t = redo_total(rb, e);
+            const double2 t = redo_total(rb, it - 1, e);
             if (!st.done) {
                 if (!(fabs(t.y) > 1e-12)) {
                     st.done = 1;
@@ -923,7 +931,7 @@ redo_pass_kernel(const double *gamma, int64_t n, CellWeights wts, RedoBuf rb, in
             x += __shfl_xor_sync(0xffffffffu, x, o);
             y += __shfl_xor_sync(0xffffffffu, y, o);
         }
-        if (lane == 0) rb.slot[e * REDO_GROUPS + blockIdx.x] = make_double2(x, y);
+        if (lane == 0) redo_slots(rb, it, e)[blockIdx.x] = make_double2(x, y);
     }
 }
 
@@ -935,7 +943,7 @@ __global__ void redo_keep_kernel(RedoBuf rb, CellPolishArgs a, int m, int start,
     if (e >= m) return;
     const int64_t o = rb.list[e].out;
     double hb = start == 0 ? a.h_unpol[o] : rb.h_best[e], db = start == 0 ? 0.0 : rb.d_best[e];
-    const double h = redo_total(rb, e).x;
+    const double h = redo_total(rb, R::iters, e).x;
     if (threadIdx.x > 0) return;
     if (polish_keep<MODE>(h, hb)) {
         hb = h;
@@ -1231,14 +1239,15 @@ static int polish_mode(Table &t, const Cells &c, const double *M, CellPolishArgs
     MB_CUDA(cudaMemcpyAsync(&count, d_count, sizeof(int), cudaMemcpyDeviceToHost, s));
     MB_CUDA(cudaStreamSynchronize(s));
     if (count == 0) return MB_OK;
+    t.polish_redone += count;
     RedoBuf rb;
     rb.batch = redo_batch(count, n);
     const size_t bn = (size_t)rb.batch * n;
-    MB_TRY(t.redo.ensure((2 * rb.batch * sizeof(RedoState) + 256) + (rb.batch * REDO_GROUPS * sizeof(double2) + 256) +
+    MB_TRY(t.redo.ensure((2 * rb.batch * sizeof(RedoState) + 256) + (2 * rb.batch * REDO_GROUPS * sizeof(double2) + 256) +
                          2 * (rb.batch * 8 + 256) + (bn * sizeof(double2) + 256)));
     q = (char *)t.redo.p;
     rb.state = carve<RedoState>(q, 2 * (size_t)rb.batch);
-    rb.slot = carve<double2>(q, (size_t)rb.batch * REDO_GROUPS);
+    rb.slot = carve<double2>(q, 2 * (size_t)rb.batch * REDO_GROUPS);
     rb.h_best = carve<double>(q, rb.batch);
     rb.d_best = carve<double>(q, rb.batch);
     rb.ab = carve<double2>(q, bn);

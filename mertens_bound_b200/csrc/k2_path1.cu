@@ -100,6 +100,7 @@ int stage_exact(Table &t, int64_t P, const uint64_t *vi, const uint64_t *vf, con
                 const double *grid, int64_t n_grid, int top, ExactStage &s) {
     const size_t need = 6 * ((size_t)P * 8 + 256) + ((size_t)n_grid * 8 + 256) + ((size_t)top * 4 + 256) + 256;
     MB_TRY(t.io.ensure(need));
+    t.polish_redone = 0;
     char *p = (char *)t.io.p;
     s.vi = carve<uint64_t>(p, P);
     s.vf = carve<uint64_t>(p, P);
@@ -486,6 +487,12 @@ extern "C" int mb_polish_peaks_weights(mb_table *h, int64_t P, const uint64_t *v
         set_error("%s: %s", who, cudaGetErrorString(e));
         return MB_ERR_CUDA;
     }
+    return MB_OK;
+}
+
+extern "C" int mb_table_polish_redone(const mb_table *h, int64_t *n_out) {
+    MB_CHECK_ARG(h && n_out, "mb_table_polish_redone: null argument");
+    *n_out = table_of(const_cast<mb_table *>(h)).polish_redone;
     return MB_OK;
 }
 
