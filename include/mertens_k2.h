@@ -282,7 +282,7 @@ int mb_hit_scan(mb_table *t, int64_t P, const uint64_t *v_int, const uint64_t *v
  * of the hit (of the stage before's best point where recentre[s]) at the 64.64 step steps[2s] +
  * steps[2s+1] 2^-64 over the first min(zeros[s], n) zeros, as mb_hit_scan, and moves the hit's offset to the
  * first point of largest |h|; out_h takes that h where keep_h[s]; a hit goes on to the next stage if
- * |h| >= threshold[s] (-inf keeps all).  out_dy: the last offset, out_stage: the last stage run.
+ * |h| >= threshold[s] (-inf keeps all, a NaN |h| too).  out_dy: the last offset, out_stage: the last stage run.
  * 2 m_half[s] + 1 <= 1024. */
 int mb_hit_polish(mb_table *t, int64_t P, const uint64_t *v_int, const uint64_t *v_frac, double k, int n_stages,
                   const int64_t *zeros, const int64_t *m_half, const uint64_t *steps, const int *recentre,

@@ -355,30 +355,34 @@ int scan_cells(Table &t, int64_t P, const uint64_t *v_int, const uint64_t *v_fra
     return MB_OK;
 }
 
-// The first point of largest |h| of each base point's grid.
+// The first point of largest |h| of each base point's grid; a NaN ranks above every number (numpy.argmax).
 struct HitBest {
     double h;
     int64_t m;
 };
 __global__ void __launch_bounds__(128) hit_best_kernel(const double *h, int n_m, HitBest *best) {
-    __shared__ double sv[4];
+    __shared__ long long sv[4];
     __shared__ int si[4];
     const double *row = h + (int64_t)blockIdx.x * n_m;
-    double bv = -1.0;
+    // |h| as its bits: ordered as the values are, one NaN above infinity
+    auto key = [](double x) { return x != x ? 0x7ff8000000000000ll : __double_as_longlong(fabs(x)); };
+    long long bv = -1;
     int bi = n_m;
-    for (int m = threadIdx.x; m < n_m; m += 128)
-        if (fabs(row[m]) > bv) {
-            bv = fabs(row[m]);
+    for (int m = threadIdx.x; m < n_m; m += 128) {
+        const long long v = key(row[m]);
+        if (v > bv) {
+            bv = v;
             bi = m;
         }
-    auto take = [&](double v, int i) {
+    }
+    auto take = [&](long long v, int i) {
         if (v > bv || (v == bv && i < bi)) {
             bv = v;
             bi = i;
         }
     };
     for (int o = 16; o > 0; o >>= 1) {
-        const double v = __shfl_xor_sync(0xffffffffu, bv, o);
+        const long long v = __shfl_xor_sync(0xffffffffu, bv, o);
         take(v, __shfl_xor_sync(0xffffffffu, bi, o));
     }
     if ((threadIdx.x & 31) == 0) {
@@ -388,7 +392,6 @@ __global__ void __launch_bounds__(128) hit_best_kernel(const double *h, int n_m,
     __syncthreads();
     if (threadIdx.x == 0) {
         for (int w = 1; w < 4; ++w) take(sv[w], si[w]);
-        if (bi >= n_m) bi = 0;
         best[blockIdx.x] = HitBest{row[bi], bi};
     }
 }
@@ -570,7 +573,7 @@ extern "C" int mb_hit_polish(mb_table *h, int64_t P, const uint64_t *v_int, cons
             if (keep_h[s]) out_h[p] = best[i].h;
             centre[p] = c;
             out_dy[p] = (double)c * 0x1p-64;
-            if (std::fabs(best[i].h) >= threshold[s]) alive[kept++] = p;
+            if (threshold[s] == -INFINITY || std::fabs(best[i].h) >= threshold[s]) alive[kept++] = p;
         }
         alive.resize(kept);
     }

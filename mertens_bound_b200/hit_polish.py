@@ -74,7 +74,9 @@ def polish_hits(table: k2.ZeroTable, points: np.ndarray, k: float = 3e-9, thresh
     steps = np.array([divmod(_fixed(s[2]), 1 << 64) for s in STAGES], dtype=np.uint64)
     recentre = np.array([s[3] for s in STAGES], dtype=np.int32)
     keep_h = np.array([i != 3 for i in range(len(STAGES))], dtype=np.int32)   # stage 3 only moves the centre
-    limit = np.array([-np.inf if t is None else t for t in (thr[:3] + [None] * len(STAGES))[:len(STAGES)]])
+    # None is -inf in the library, which keeps a NaN |h| too; a caller's own -inf does not
+    thr = (thr[:3] + [None] * len(STAGES))[:len(STAGES)]
+    limit = np.array([-np.inf if t is None else max(-np.finfo(float).max, t) if t == t else t for t in thr])
     check(lib().mb_hit_polish(table.handle, n, ptr(vi), ptr(vf), float(k), len(STAGES), ptr(zeros), ptr(m_half),
                               ptr(steps), ptr(recentre), ptr(keep_h), ptr(limit), ptr(res.h), ptr(res.dy),
                               ptr(res.stage)))
