@@ -61,7 +61,11 @@ def points_from_x(x) -> np.ndarray:
 
 
 def polish_hits(table: k2.ZeroTable, points: np.ndarray, k: float = 3e-9, thresholds=None) -> HitResult:
-    """Run the staged polish for every hit (points: (n, 2) u64 v_int, v_frac)."""
+    """Run the staged polish for every hit (points: (n, 2) u64 v_int, v_frac).
+
+    thresholds: of the first three stages, None where every hit goes on.  A shorter list is an IndexError if a hit
+    passes its last entry.
+    """
     thr = [s[4] for s in STAGES[:3]] if thresholds is None else list(thresholds)
     n = len(points)
     res = HitResult(np.zeros(n), np.zeros(n), np.zeros(n, dtype=np.int64))
@@ -69,17 +73,26 @@ def polish_hits(table: k2.ZeroTable, points: np.ndarray, k: float = 3e-9, thresh
         return res
     pts = np.ascontiguousarray(points, dtype=np.uint64)
     vi, vf = np.ascontiguousarray(pts[:, 0]), np.ascontiguousarray(pts[:, 1])
-    zeros = np.array([table.n if s[0] is None else s[0] for s in STAGES], dtype=np.int64)
-    m_half = np.array([s[1] for s in STAGES], dtype=np.int64)
-    steps = np.array([divmod(_fixed(s[2]), 1 << 64) for s in STAGES], dtype=np.uint64)
-    recentre = np.array([s[3] for s in STAGES], dtype=np.int32)
-    keep_h = np.array([i != 3 for i in range(len(STAGES))], dtype=np.int32)   # stage 3 only moves the centre
+    stages = STAGES if len(thr) >= 3 else STAGES[:len(thr)]
+    if not stages:
+        raise IndexError("polish_hits: no threshold for the first stage")
+    S = len(stages)
+    zeros = np.array([table.n if s[0] is None else s[0] for s in stages], dtype=np.int64)
+    m_half = np.array([s[1] for s in stages], dtype=np.int64)
+    steps = np.array([divmod(_fixed(s[2]), 1 << 64) for s in stages], dtype=np.uint64)
+    recentre = np.array([s[3] for s in stages], dtype=np.int32)
+    keep_h = np.array([i != 3 for i in range(S)], dtype=np.int32)   # stage 3 only moves the centre
     # None is -inf in the library, which keeps a NaN |h| too; a caller's own -inf does not
-    thr = (thr[:3] + [None] * len(STAGES))[:len(STAGES)]
+    thr = (thr[:3] + [None] * S)[:S]
     limit = np.array([-np.inf if t is None else max(-np.finfo(float).max, t) if t == t else t for t in thr])
-    check(lib().mb_hit_polish(table.handle, n, ptr(vi), ptr(vf), float(k), len(STAGES), ptr(zeros), ptr(m_half),
-                              ptr(steps), ptr(recentre), ptr(keep_h), ptr(limit), ptr(res.h), ptr(res.dy),
-                              ptr(res.stage)))
+    check(lib().mb_hit_polish(table.handle, n, ptr(vi), ptr(vf), float(k), S, ptr(zeros), ptr(m_half), ptr(steps),
+                              ptr(recentre), ptr(keep_h), ptr(limit), ptr(res.h), ptr(res.dy), ptr(res.stage)))
+    if S < 3:
+        on = res.stage == S - 1
+        if thr[-1] is not None:
+            on &= np.abs(res.h) >= thr[-1]
+        if on.any():
+            raise IndexError(f"polish_hits: no threshold for stage {S}")
     return res
 
 

@@ -1,4 +1,5 @@
-"""Thresholds of the staged hit polish where |h| is not a number."""
+"""Thresholds of the staged hit polish at their edges: lists shorter than the three stages that have one, and |h| that is
+not a number."""
 import math
 
 import numpy as np
@@ -11,6 +12,22 @@ pytestmark = pytest.mark.gpu
 
 def _points(P):
     return hit_polish.points_from_x(synth.leaves_x(P, 7))
+
+
+def test_short_threshold_lists(gpu):
+    data = synth.make_table(3000, seed=43)
+    pts = _points(5)
+    with k2.ZeroTable.from_data(data) as t:
+        full = hit_polish.polish_hits(t, pts, thresholds=(None, math.inf, None))
+        for thr in ((), (None,), (0.0,), (None, None), (0.0, -math.inf)):       # a hit needs the missing entry
+            with pytest.raises(IndexError):
+                hit_polish.polish_hits(t, pts, thresholds=thr)
+        dead = hit_polish.polish_hits(t, pts, thresholds=(math.inf,))           # none does
+        assert np.all(dead.stage == 0) and np.all(dead.h != 0.0)
+        dead = hit_polish.polish_hits(t, pts, thresholds=(None, math.inf))
+        for f in ("h", "dy", "stage"):
+            assert np.array_equal(getattr(dead, f), getattr(full, f))
+        assert len(hit_polish.polish_hits(t, pts[:0], thresholds=()).h) == 0
 
 
 def test_overflowing_sums(gpu):
