@@ -86,6 +86,13 @@ MB_DEV int32_t screen_phase(const CandRegs &c, const ZScreenS &z) {
     return (int32_t)light_phase32(c, z.b0, z.b1, z.gi, z.b0s, z.c1s, z.gis, z.b1s, z.psi32);
 }
 
+template <class Z>
+MB_DEV void screen_sincos(const CandRegs &c, const Z &z, float &sn, float &cs) {
+    const float th = (float)screen_phase(c, z) * 1.4629180792671596e-09f;       // 2pi 2^-32
+    sn = __sinf(th);
+    cs = __cosf(th);
+}
+
 // The seven sums of a leaf by parity: S_0 = e[0], S_{+-m} = e[m] -+ o[m - 1]
 // (cos(theta + m D) = cos theta cos m D - sin theta sin m D), so a term is seven FMAs.
 struct ScreenSums {
@@ -95,8 +102,8 @@ struct ScreenSums {
     }
     template <class Z>
     MB_DEV void add(const CandRegs &c, const Z &z) {
-        const float th = (float)screen_phase(c, z) * 1.4629180792671596e-09f;   // 2pi 2^-32
-        const float sn = __sinf(th), cs = __cosf(th);
+        float sn, cs;
+        screen_sincos(c, z, sn, cs);
         e[0] = fmaf(z.a, cs, e[0]);
 #pragma unroll
         for (int m = 0; m < 3; ++m) {
@@ -116,7 +123,9 @@ struct ScreenSums {
 // zero's record (four 16-byte broadcasts) serves LPT terms: with one leaf per thread those reads were half of the
 // time (2^20 leaves: 155 us; now 78).  Survivors are listed in shared memory with their sums, and the later
 // stages run over the list: a leaf per thread while a quarter of the tile or more is alive, eight lanes
-// per leaf below that, so a few survivors neither hold whole warps nor run a long serial loop.
+// per leaf below that, so a few survivors neither hold whole warps nor run a long serial loop: eight zeros' sines
+// and cosines at a time, one lane's each, then seven lanes add them in zero order, one sum each.  Every way adds a
+// leaf's terms in the same order, so its scores do not depend on the leaves beside it.
 template <int LPT, class Z>
 __global__ void __launch_bounds__(SCREEN_THREADS, LPT == 1 ? 4 : 2)
 screen_kernel(TabView t, int n_zeros, double k, uint64_t step_int, uint64_t step_frac, CandView c, ScreenArgs sa,
@@ -128,6 +137,7 @@ screen_kernel(TabView t, int n_zeros, double k, uint64_t step_int, uint64_t step
     float *sc = sums + 7 * LEAVES;                                                        // [n_stages][LEAVES]
     uint16_t *list = reinterpret_cast<uint16_t *>(sc + sa.n_stages * LEAVES);             // [2][LEAVES]
     __shared__ int n_list[2];
+    __shared__ __align__(16) float trig[SCREEN_THREADS / 32][2][32];     // cosines, sines of a warp's four leaves
     for (int j = threadIdx.x; j < n_zeros; j += SCREEN_THREADS) {
         Z r;
         screen_limbs(t, j, r);
@@ -243,25 +253,38 @@ screen_kernel(TabView t, int n_zeros, double k, uint64_t step_int, uint64_t step
                     const bool live = q < n;
                     const int l = in[live ? q : q0];
                     const CandRegs cr = cand_regs(c, p0 + l, true);
-                    ScreenSums x;
-                    x.clear();
-                    for (int j = j0 + (lane & 7); j < j1; j += 8) x.add(cr, zs[j]);
+                    // lanes 0..3: e[m], 4..6: o[m - 4], 7: none (it adds a copy of the sixth)
+                    const int m = min(lane & 7, 6);
+                    float x = sums[m * LEAVES + l];
+                    const float *coef = m == 0 ? &zs->a : (m < 4 ? zs->cm + m - 1 : zs->sm + m - 4);
+                    const float *val = &trig[warp][m < 4 ? 0 : 1][lane & 24];
+                    constexpr int stride = sizeof(Z) / sizeof(float);
+                    for (int j = j0; j < j1; j += 8) {
+                        float sn, cs;
+                        screen_sincos(cr, zs[min(j + (lane & 7), j1 - 1)], sn, cs);
+                        __syncwarp();                // the values before are read
+                        trig[warp][0][lane] = cs;
+                        trig[warp][1][lane] = sn;
+                        __syncwarp();
+                        if (j + 8 <= j1) {
+                            const float4 u = reinterpret_cast<const float4 *>(val)[0];
+                            const float4 w = reinterpret_cast<const float4 *>(val)[1];
+                            const float v[8] = {u.x, u.y, u.z, u.w, w.x, w.y, w.z, w.w};
+                            float a[8];
 #pragma unroll
-                    for (int o = 4; o > 0; o >>= 1) {
+                            for (int i = 0; i < 8; ++i) a[i] = coef[(j + i) * stride];
 #pragma unroll
-                        for (int m = 0; m < 4; ++m) x.e[m] += __shfl_xor_sync(0xffffffffu, x.e[m], o);
-#pragma unroll
-                        for (int m = 0; m < 3; ++m) x.o[m] += __shfl_xor_sync(0xffffffffu, x.o[m], o);
+                            for (int i = 0; i < 8; ++i) x = fmaf(a[i], v[i], x);
+                        } else {
+                            for (int i = 0; i < j1 - j; ++i) x = fmaf(coef[(j + i) * stride], val[i], x);
+                        }
                     }
-                    if (live && (lane & 7) == 0) {
-                        ScreenSums y;
-                        resume(l, y);
+                    ScreenSums y;
 #pragma unroll
-                        for (int m = 0; m < 4; ++m) y.e[m] += x.e[m];
+                    for (int i = 0; i < 4; ++i) y.e[i] = __shfl_sync(0xffffffffu, x, (lane & 24) + i);
 #pragma unroll
-                        for (int m = 0; m < 3; ++m) y.o[m] += x.o[m];
-                        finish(l, s, y);
-                    }
+                    for (int i = 0; i < 3; ++i) y.o[i] = __shfl_sync(0xffffffffu, x, (lane & 24) + 4 + i);
+                    if (live && (lane & 7) == 0) finish(l, s, y);
                 }
             }
         }
