@@ -122,10 +122,12 @@ struct ScreenSums {
 // One CTA slot each: an equal share of the leaves, in tiles of LPT x 256.  The first stage runs LPT leaves per thread, so that a
 // zero's record (four 16-byte broadcasts) serves LPT terms: with one leaf per thread those reads were half of the
 // time (2^20 leaves: 155 us; now 78).  Survivors are listed in shared memory with their sums, and the later
-// stages run over the list: a leaf per thread while a quarter of the tile or more is alive, eight lanes
-// per leaf below that, so a few survivors neither hold whole warps nor run a long serial loop: eight zeros' sines
-// and cosines at a time, one lane's each, then seven lanes add them in zero order, one sum each.  Every way adds a
-// leaf's terms in the same order, so its scores do not depend on the leaves beside it.
+// stages run over the list: a leaf per thread while there are 64 or more (two warps: with a quarter of a
+// 1,024-leaf tile as the limit, 200,000 leaves of which a fifth goes on took 105 us, more than one leaf per thread
+// throughout, 95; now 40), eight lanes per leaf below that, so a few survivors neither hold whole warps nor run a
+// long serial loop: eight zeros' sines and cosines at a time, one lane's each, then seven lanes add them in zero
+// order, one sum each.  Every way adds a leaf's terms in the same order, so its scores do not depend on the leaves
+// beside it.
 template <int LPT, class Z>
 __global__ void __launch_bounds__(SCREEN_THREADS, LPT == 1 ? 4 : 2)
 screen_kernel(TabView t, int n_zeros, double k, uint64_t step_int, uint64_t step_frac, CandView c, ScreenArgs sa,
@@ -238,7 +240,7 @@ screen_kernel(TabView t, int n_zeros, double k, uint64_t step_int, uint64_t step
                 if (threadIdx.x == 0) n_list[s & 1] = 0;
                 __syncthreads();
             }
-            if (4 * n >= LEAVES) {
+            if (n >= SCREEN_THREADS / 4) {
                 for (int q = threadIdx.x; q < n; q += SCREEN_THREADS) {
                     const int l = in[q];
                     const CandRegs cr = cand_regs(c, p0 + l, true);
