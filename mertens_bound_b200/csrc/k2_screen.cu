@@ -124,10 +124,10 @@ struct ScreenSums {
 // time (2^20 leaves: 155 us; now 78).  Survivors are listed in shared memory with their sums, and the later
 // stages run over the list: a leaf per thread while there are 64 or more (two warps: with a quarter of a
 // 1,024-leaf tile as the limit, 200,000 leaves of which a fifth goes on took 105 us, more than one leaf per thread
-// throughout, 95; now 40), eight lanes per leaf below that, so a few survivors neither hold whole warps nor run a
-// long serial loop: eight zeros' sines and cosines at a time, one lane's each, then seven lanes add them in zero
-// order, one sum each.  Every way adds a leaf's terms in the same order, so its scores do not depend on the leaves
-// beside it.
+// throughout, 95; now 40), eight lanes per leaf below that and a warp per leaf from eight leaves down, so a few
+// survivors neither hold whole warps nor run a long serial loop: as many zeros' sines and cosines at a time, one
+// lane's each, then seven lanes add them in zero order, one sum each.  Every way adds a leaf's terms in the same
+// order, so its scores do not depend on the leaves beside it.
 template <int LPT, class Z>
 __global__ void __launch_bounds__(SCREEN_THREADS, LPT == 1 ? 4 : 2)
 screen_kernel(TabView t, int n_zeros, double k, uint64_t step_int, uint64_t step_frac, CandView c, ScreenArgs sa,
@@ -229,6 +229,48 @@ screen_kernel(TabView t, int n_zeros, double k, uint64_t step_int, uint64_t step
             else if (n_leaves > SCREEN_THREADS) first(std::integral_constant<int, 2>());
             else first(std::integral_constant<int, 1>());
         }
+        // the list's n leaves with L lanes each
+        auto by_lanes = [&](auto lanes, int n, const uint16_t *in, int s, int j0, int j1) {
+            constexpr int L = decltype(lanes)::value, stride = sizeof(Z) / sizeof(float);
+            const int g0 = lane & ~(L - 1);              // the leaf's first lane
+            const int m = min(lane - g0, 6);             // 0..3: e[m], 4..6: o[m - 4]; lanes above add a copy
+            const float *coef = m == 0 ? &zs->a : (m < 4 ? zs->cm + m - 1 : zs->sm + m - 4);
+            const float *val = &trig[warp][m < 4 ? 0 : 1][g0];
+            for (int q0 = warp * (32 / L); q0 < n; q0 += SCREEN_THREADS / L) {
+                const int q = q0 + g0 / L;
+                const bool live = q < n;
+                const int l = in[live ? q : q0];
+                const CandRegs cr = cand_regs(c, p0 + l, true);
+                float x = sums[m * LEAVES + l];
+                for (int j = j0; j < j1; j += L) {
+                    float sn, cs;
+                    screen_sincos(cr, zs[min(j + lane - g0, j1 - 1)], sn, cs);
+                    __syncwarp();                        // the values before are read
+                    trig[warp][0][lane] = cs;
+                    trig[warp][1][lane] = sn;
+                    __syncwarp();
+                    const int nz = min(L, j1 - j);
+                    int i = 0;
+                    for (; i + 8 <= nz; i += 8) {
+                        const float4 u = reinterpret_cast<const float4 *>(val + i)[0];
+                        const float4 w = reinterpret_cast<const float4 *>(val + i)[1];
+                        const float v[8] = {u.x, u.y, u.z, u.w, w.x, w.y, w.z, w.w};
+                        float a[8];
+#pragma unroll
+                        for (int b = 0; b < 8; ++b) a[b] = coef[(j + i + b) * stride];
+#pragma unroll
+                        for (int b = 0; b < 8; ++b) x = fmaf(a[b], v[b], x);
+                    }
+                    for (; i < nz; ++i) x = fmaf(coef[(j + i) * stride], val[i], x);
+                }
+                ScreenSums y;
+#pragma unroll
+                for (int i = 0; i < 4; ++i) y.e[i] = __shfl_sync(0xffffffffu, x, g0 + i);
+#pragma unroll
+                for (int i = 0; i < 3; ++i) y.o[i] = __shfl_sync(0xffffffffu, x, g0 + 4 + i);
+                if (live && lane == g0) finish(l, s, y);
+            }
+        };
         for (int s = 1; s < sa.n_stages; ++s) {
             __syncthreads();                         // the list of stage s - 1 is complete
             const int n = n_list[(s - 1) & 1];
@@ -249,45 +291,10 @@ screen_kernel(TabView t, int n_zeros, double k, uint64_t step_int, uint64_t step
                     for (int j = j0; j < j1; ++j) x.add(cr, zs[j]);
                     finish(l, s, x);
                 }
+            } else if (n > SCREEN_THREADS / 32) {
+                by_lanes(std::integral_constant<int, 8>(), n, in, s, j0, j1);
             } else {
-                for (int q0 = warp * 4; q0 < n; q0 += SCREEN_THREADS / 8) {
-                    const int q = q0 + (lane >> 3);
-                    const bool live = q < n;
-                    const int l = in[live ? q : q0];
-                    const CandRegs cr = cand_regs(c, p0 + l, true);
-                    // lanes 0..3: e[m], 4..6: o[m - 4], 7: none (it adds a copy of the sixth)
-                    const int m = min(lane & 7, 6);
-                    float x = sums[m * LEAVES + l];
-                    const float *coef = m == 0 ? &zs->a : (m < 4 ? zs->cm + m - 1 : zs->sm + m - 4);
-                    const float *val = &trig[warp][m < 4 ? 0 : 1][lane & 24];
-                    constexpr int stride = sizeof(Z) / sizeof(float);
-                    for (int j = j0; j < j1; j += 8) {
-                        float sn, cs;
-                        screen_sincos(cr, zs[min(j + (lane & 7), j1 - 1)], sn, cs);
-                        __syncwarp();                // the values before are read
-                        trig[warp][0][lane] = cs;
-                        trig[warp][1][lane] = sn;
-                        __syncwarp();
-                        if (j + 8 <= j1) {
-                            const float4 u = reinterpret_cast<const float4 *>(val)[0];
-                            const float4 w = reinterpret_cast<const float4 *>(val)[1];
-                            const float v[8] = {u.x, u.y, u.z, u.w, w.x, w.y, w.z, w.w};
-                            float a[8];
-#pragma unroll
-                            for (int i = 0; i < 8; ++i) a[i] = coef[(j + i) * stride];
-#pragma unroll
-                            for (int i = 0; i < 8; ++i) x = fmaf(a[i], v[i], x);
-                        } else {
-                            for (int i = 0; i < j1 - j; ++i) x = fmaf(coef[(j + i) * stride], val[i], x);
-                        }
-                    }
-                    ScreenSums y;
-#pragma unroll
-                    for (int i = 0; i < 4; ++i) y.e[i] = __shfl_sync(0xffffffffu, x, (lane & 24) + i);
-#pragma unroll
-                    for (int i = 0; i < 3; ++i) y.o[i] = __shfl_sync(0xffffffffu, x, (lane & 24) + 4 + i);
-                    if (live && (lane & 7) == 0) finish(l, s, y);
-                }
+                by_lanes(std::integral_constant<int, 32>(), n, in, s, j0, j1);
             }
         }
     }
