@@ -1037,7 +1037,7 @@ int set_smem(K kern, int bytes) {
 
 }  // namespace
 
-// Warps sharing a peak group's zeros in the scans and power sums: as many as keep the CTA's peak slots full,
+// Warps sharing a peak group's zeros in the scans: as many as keep the CTA's peak slots full,
 // and two at least with 16 peaks a warp, unless there are peaks for eight full CTAs (fewer, larger items would
 // not balance).
 static int cell_nzw(int64_t P, int peaks) {
@@ -1149,16 +1149,12 @@ int launch_moments_weights(const Table &t, const Cells &c, const uint64_t *vi, c
     }
 }
 
-// Chunks so that every CTA slot gets about eight items, each at least 256 zeros on average.
-int taylor_chunks(const Table &t, int64_t P, int64_t n, int *n_chunk) {
-    int slots = 148;
-    MB_TRY(sm_count(t, &slots));
-    using Sh = CellShape<CELL_POWERS, 1, 17>;
-    slots *= Sh::ctas;
-    const int ppc = Sh::peaks / cell_nzw(P, Sh::peaks);
-    const int64_t n_pt = std::max<int64_t>(1, (P + ppc - 1) / ppc);
-    *n_chunk = (int)std::max<int64_t>(1, std::min<int64_t>((8 * (int64_t)slots + n_pt - 1) / n_pt, n / 256));
-    return MB_OK;
+// Chunks of 256 zeros on average, at most two per CTA slot, and one per SM where they hold 64 zeros.  Their number
+// depends on the zeros alone and one warp adds a chunk's zeros, so a peak's sums keep their bits whatever the peaks
+// beside it.  That costs calls of few peaks, whose CTAs have idle warps: one peak on 100,000 zeros 75 -> 88 us with
+// eight warps to a chunk's zeros where there are 8 peaks, but two for all calls cost 1,024 peaks 490 -> 524.
+int taylor_chunks(int64_t n) {
+    return (int)std::max<int64_t>({1, std::min<int64_t>(592, n / 256), std::min<int64_t>(148, n / 64)});
 }
 
 size_t taylor_work_bytes(int64_t P, int n_chunk) {
@@ -1175,8 +1171,7 @@ int launch_taylor_grid(const Table &t, const uint64_t *vi, const uint64_t *vf, c
     MB_CUDA(cudaGetLastError());
     const Cells c{n_chunk, n_chunk, 1, j0, j1, nullptr};
     const CellWeights cw{{w}};
-    MB_TRY((launch_moments<CELL_POWERS, 1, 17>(t, c, vi, vf, delta, nullptr, P, cw, 0.0,
-                                              cell_nzw(P, CellShape<CELL_POWERS, 1, 17>::peaks), S, s)));
+    MB_TRY((launch_moments<CELL_POWERS, 1, 17>(t, c, vi, vf, delta, nullptr, P, cw, 0.0, 1, S, s)));
     taylor_grid_kernel<<<(unsigned)P, TAY_THREADS, 0, s>>>(S, n_chunk, grid, n_grid, h_unpol, h_pol, ddy_pol);
     MB_CUDA(cudaGetLastError());
     return MB_OK;

@@ -68,11 +68,12 @@ int launch_moments_weights(const Table &t, const Cells &c, const uint64_t *vi, c
                            const double *delta, const int *sel, int64_t P, int nw, const CellWeights &w,
                            double *out, cudaStream_t s);
 
-// The Taylor polish's grid stage on P peaks: power sums of w C u^m, u = gamma 1e-4, over n_chunk equal
-// chunks of the zeros [0, n), then h(ddy) = sum_m (-1)^m / (2m)! z^{2m} sum w Re C u^{2m}
+// The Taylor polish's grid stage on P peaks: power sums of w C u^m, u = gamma 1e-4, over taylor_chunks(n)
+// chunks of the zeros [0, n) (edges n (c / n_chunk)^1.5: the first ones are the shortest, and may be empty), then h(ddy) = sum_m (-1)^m / (2m)! z^{2m} sum w Re C u^{2m}
 // - sum_m (-1)^m / (2m+1)! z^{2m+1} sum w Im C u^{2m+1}, z = ddy 1e4, on the grid: h_unpol = h(0), h_pol and
 // ddy_pol its first grid point of largest |h|.  work: taylor_work_bytes(P, n_chunk).
-int taylor_chunks(const Table &t, int64_t P, int64_t n, int *n_chunk);
+// The results of a peak have the same bits whatever P is.
+int taylor_chunks(int64_t n);
 size_t taylor_work_bytes(int64_t P, int n_chunk);
 int launch_taylor_grid(const Table &t, const uint64_t *vi, const uint64_t *vf, const double *delta, int64_t P,
                        int64_t n, int n_chunk, const double *w, const double *grid, int n_grid, void *work,

@@ -516,8 +516,7 @@ extern "C" int mb_fast_polish_exact(mb_table *h, int64_t P, const uint64_t *v_in
     MB_TRY(stage_exact(t, P, v_int, v_frac, delta, ddy_grid, n_grid, nsel, s));
     const ABExact src{view(t), s.vi, s.vf, s.delta};
     const double *d_w = t.d_weights[weight_slot];
-    int n_chunk = 1;
-    MB_TRY(taylor_chunks(t, P, n_zeros, &n_chunk));
+    const int n_chunk = taylor_chunks(n_zeros);
     const int64_t pc = std::max<int64_t>(
         1, std::min<int64_t>(P, (int64_t)(POLISH_MOMENT_BYTES / taylor_work_bytes(1, n_chunk))));
     MB_TRY(t.work.ensure(taylor_work_bytes(pc, n_chunk)));
