@@ -977,9 +977,14 @@ taylor_grid_kernel(const double *S, int n_chunk, const double *grid, int n_grid,
     const int64_t p = blockIdx.x;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     if (lane < 24) {
-        double x = 0.0;
-        for (int c = warp; c < n_chunk; c += 4) x += S[(p * n_chunk + c) * 24 + lane];
-        part[warp][lane] = x;
+        double x[8];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) x[i] = 0.0;
+        for (int c = warp; c < n_chunk; c += 32)
+#pragma unroll
+            for (int i = 0; i < 8; ++i)
+                if (c + 4 * i < n_chunk) x[i] += S[(p * n_chunk + c + 4 * i) * 24 + lane];
+        part[warp][lane] = ((x[0] + x[1]) + (x[2] + x[3])) + ((x[4] + x[5]) + (x[6] + x[7]));
     }
     __syncthreads();
     if (threadIdx.x < 24) mom[lane] = (part[0][lane] + part[1][lane]) + (part[2][lane] + part[3][lane]);
