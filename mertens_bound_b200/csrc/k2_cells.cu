@@ -542,10 +542,16 @@ constexpr int CPOL_LD = 2 * CELL_D1 + 1;       // row of staged moments: an odd 
 constexpr int CPOL_CELLS = 1200;               // cells that fit: 221 KB
 __host__ __device__ constexpr int cpol_threads(bool staged) { return staged ? 512 : 256; }
 
+// The part of a point's delta below 2^-64, which its fixed-point fold (fold_delta) dropped: at most 2^-65, an angle of
+// up to 3.5e-14 at gamma = 1.3e6.
+MB_DEV double delta_rest(double delta) {
+    const double fixed = delta * 0x1p64;
+    return (fixed - rint(fixed)) * 0x1p-64;
+}
+
 // The series at one offset: F0 = E Q0 and, with DERIV, F1 = E Q1, F2 = E Q2, where E = e^{2 pi i G_c d} and
 // Q0 = sum M_n (i y)^n / n!, Q1, Q2 its first and second derivative in i y (y = kappa d).
-// The rotation's offset is d + rho, rho the part of the point's delta below 2^-64 that its fixed-point fold
-// dropped (at most 2^-65; in the series it is far below rounding).
+// The rotation's offset is d + rho, rho = delta_rest of the point's delta (in the series it is far below rounding).
 struct CellSeries {
     double d, rho, e[CELL_D1];
     MB_DEV CellSeries(double d_, double rho_, double kappa) : d(d_), rho(rho_) {
@@ -638,7 +644,7 @@ cell_polish_kernel(Cells cells, const double *M, CellPolishArgs a, const double 
     const double H = (double)cells.half * 0x1p-16, kappa = 6.283185307179586 * H;
     const int64_t point = a.sel ? a.sel[p] : p;
     const int64_t o = (int64_t)w * a.out_stride + point;
-    const double fixed = (delta ? delta[point] : 0.0) * 0x1p64, rho = (fixed - rint(fixed)) * 0x1p-64;
+    const double rho = delta ? delta_rest(delta[point]) : 0.0;
 
     // N sums over the CTA, every thread gets them (warp partials in warp order)
     auto block_sums = [&](auto &x) {
@@ -678,7 +684,7 @@ cell_polish_kernel(Cells cells, const double *M, CellPolishArgs a, const double 
         for (int c = threadIdx.x; c < cells.n; c += THREADS) {
             const double *m = m0 + c * LD;
             const double g = 6.283185307179586 * (double)cells.ctr[c] * 0x1p-16, g2 = g * g;
-            x[0] += m[0];
+            x[0] += fma(-g * rho, m[CELL_D1], m[0]);             // the rotation by g rho to first order
             x[1] += g2 * g2 * (m[0] * m[0] + m[CELL_D1] * m[CELL_D1]);
         }
         block_sums(x);
@@ -964,8 +970,8 @@ constexpr int TAY_THREADS = 128;
 // One CTA per peak: the chunks' power sums added in a fixed order (four chunk strides, then those
 // four), then the grid points; ties of |h| go to the smaller index.
 __global__ void __launch_bounds__(TAY_THREADS)
-taylor_grid_kernel(const double *S, int n_chunk, const double *grid, int n_grid, double *h_unpol, double *h_pol,
-                   double *ddy_pol) {
+taylor_grid_kernel(const double *S, int n_chunk, const double *delta, const double *grid, int n_grid, double *h_unpol,
+                   double *h_pol, double *ddy_pol) {
     __shared__ double part[4][24], mom[24];
     __shared__ double best_v[TAY_THREADS / 32], best_h[TAY_THREADS / 32];
     __shared__ int best_i[TAY_THREADS / 32];
@@ -989,10 +995,11 @@ taylor_grid_kernel(const double *S, int n_chunk, const double *grid, int n_grid,
     __syncthreads();
     if (threadIdx.x < 24) mom[lane] = (part[0][lane] + part[1][lane]) + (part[2][lane] + part[3][lane]);
     __syncthreads();
+    const double rho = delta ? delta_rest(delta[p]) : 0.0, h0 = fma(-rho * 1.0e4, mom[16], mom[0]);
     double bv = -1.0, hv = 0.0;
     int bi = n_grid;
     for (int g = threadIdx.x; g < n_grid; g += TAY_THREADS) {
-        const double z = grid[g] * 1.0e4, z2 = z * z;
+        const double z = (grid[g] + rho) * 1.0e4, z2 = z * z;
         double hc = 0.0, hs = 0.0, pw = 1.0;
 #pragma unroll
         for (int m = 0; m < 9; ++m) {
@@ -1026,9 +1033,9 @@ taylor_grid_kernel(const double *S, int n_chunk, const double *grid, int n_grid,
     __syncthreads();
     if (threadIdx.x == 0) {
         for (int w = 1; w < TAY_THREADS / 32; ++w) take(best_v[w], best_i[w], best_h[w]);
-        h_unpol[p] = mom[0];
+        h_unpol[p] = h0;
         ddy_pol[p] = bi < n_grid ? grid[bi] : 0.0;
-        h_pol[p] = bi < n_grid ? hv : mom[0];
+        h_pol[p] = bi < n_grid ? hv : h0;
     }
 }
 
@@ -1177,7 +1184,7 @@ int launch_taylor_grid(const Table &t, const uint64_t *vi, const uint64_t *vf, c
     const Cells c{n_chunk, n_chunk, 1, j0, j1, nullptr};
     const CellWeights cw{{w}};
     MB_TRY((launch_moments<CELL_POWERS, 1, 17>(t, c, vi, vf, delta, nullptr, P, cw, 0.0, 1, S, s)));
-    taylor_grid_kernel<<<(unsigned)P, TAY_THREADS, 0, s>>>(S, n_chunk, grid, n_grid, h_unpol, h_pol, ddy_pol);
+    taylor_grid_kernel<<<(unsigned)P, TAY_THREADS, 0, s>>>(S, n_chunk, delta, grid, n_grid, h_unpol, h_pol, ddy_pol);
     MB_CUDA(cudaGetLastError());
     return MB_OK;
 }
