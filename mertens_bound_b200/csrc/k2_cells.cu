@@ -546,7 +546,7 @@ __host__ __device__ constexpr int cpol_threads(bool staged) { return staged ? 51
 // up to 3.5e-14 at gamma = 1.3e6.
 MB_DEV double delta_rest(double delta) {
     const double fixed = delta * 0x1p64;
-    return (fixed - rint(fixed)) * 0x1p-64;
+    return (fixed - round(fixed)) * 0x1p-64;                     // ties away from zero, as fold_delta rounds
 }
 
 // The series at one offset: F0 = E Q0 and, with DERIV, F1 = E Q1, F2 = E Q2, where E = e^{2 pi i G_c d} and

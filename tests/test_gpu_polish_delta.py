@@ -16,10 +16,12 @@ pytestmark = pytest.mark.gpu
 
 def _deltas(kind, P, rng):
     sign = rng.choice([-1.0, 1.0], P)
+    if kind == "tie":                                           # odd multiples of 2^-65: the rounding is a tie
+        return sign * (2.0 * rng.integers(2**51, 2**52, P) + 1.0) * 2.0**-65
     return sign * rng.uniform(1e-6, 1e-5, P)                    # last bits at 2^-72: any rest
 
 
-@pytest.mark.parametrize("kind", ["rest"])
+@pytest.mark.parametrize("kind", ["rest", "tie"])
 def test_rest_of_delta(gpu, small_table, kind):
     rng = np.random.default_rng(91)
     gam = 5.0e6 + np.cumsum(rng.uniform(0.2, 0.72, 3000))
