@@ -363,9 +363,10 @@ int mb_polish_peaks_exact(mb_table *t, int64_t P, const uint64_t *v_int, const u
  * weight vector): each candidate's terms are formed once and summed into moments over cells of zeros
  * under up to five vectors at a time, and the polishes run on the moments; a peak whose Newton path
  * amplifies rounding is polished over the zeros instead.  Device workspace of the table, at most
- * 0.6 GiB, kept between calls.  A grid too wide for the cells (grid_half_width above ~0.1) builds the
- * exact (A, B) of up to 65,535 peaks at a time in a buffer of at most 4 GiB and at most half of the
- * device's free memory, allocated for the call and freed before it returns. */
+ * 0.6 GiB, kept between calls.  A grid so wide that its cells hold few zeros (grid_half_width above
+ * 0.02 on 600,000 zeros) builds the exact (A, B) of up to 65,535 peaks at a time in a buffer of at most
+ * 4 GiB and at most half of the device's free memory, allocated for the call and freed before it
+ * returns. */
 int mb_polish_peaks_weights(mb_table *t, int64_t P, const uint64_t *v_int, const uint64_t *v_frac,
                             const double *delta, int64_t n_zeros, int n_weights, const int *weight_slots,
                             double grid_half_width, int grid_steps, double *out_h_unpol, double *out_h_pol,
@@ -374,7 +375,7 @@ int mb_fast_polish_exact(mb_table *t, int64_t P, const uint64_t *v_int, const ui
                          const double *delta, int64_t n_zeros, int weight_slot, const double *ddy_grid,
                          int64_t n_grid, int top, double *out_h_unpol, double *out_h_pol, double *out_ddy_pol);
 /* The (peak, weight) pairs that the table's last such call polished over the zeros after their cell
- * moments, because their Newton path amplifies rounding (0 where it used no moments). */
+ * moments, because their Newton path amplifies rounding; -1 where it polished all over the zeros. */
 int mb_table_polish_redone(const mb_table *t, int64_t *n_out);
 
 /* ---- compatibility with the reference's libpath1_eval.so ---------------------------------

@@ -539,7 +539,6 @@ constexpr int cscan_smem() {
 // ------------------------------------------------------------------ polishes on moments
 
 constexpr int CPOL_LD = 2 * CELL_D1 + 1;       // row of staged moments: an odd stride has no bank conflicts
-constexpr int CPOL_CELLS = 1200;               // cells that fit: 221 KB
 __host__ __device__ constexpr int cpol_threads(bool staged) { return staged ? 512 : 256; }
 
 // The part of a point's delta below 2^-64, which its fixed-point fold (fold_delta) dropped: at most 2^-65, an angle of

@@ -107,6 +107,8 @@ struct CellPolishArgs {
     const int *sel;            // POLISH_TOPK: point and output index of each peak, else null
     double *h_unpol, *h_pol, *ddy_pol;
 };
+// Cells whose moments of one peak fit shared memory (221 KB): the polish then reads them from there.
+constexpr int CPOL_CELLS = 1200;
 // Device bytes of the second pass's list for P x nw peaks (its terms are in t.redo).
 size_t cell_polish_bytes(int64_t P, int nw);
 // vi, vf, delta: the points (as for launch_moments_weights); w: the weights; work: cell_polish_bytes.  Waits

@@ -76,7 +76,7 @@ struct Table {
     // buffer must not overlap on the GPU.
     DevBuf io, work;
     DevBuf redo;                      // the second pass of polishes on cell moments (k2_cells.cu)
-    int64_t polish_redone = 0;        // (peak, weight) pairs the last polish took there
+    int64_t polish_redone = 0;        // (peak, weight) pairs the last polish took there; -1: no moments
     int n_plans = 0;                  // live plans on this table (it cannot be destroyed under them)
 
     int64_t count_below(double T) const;

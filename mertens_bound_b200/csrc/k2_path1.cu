@@ -100,7 +100,7 @@ int stage_exact(Table &t, int64_t P, const uint64_t *vi, const uint64_t *vf, con
                 const double *grid, int64_t n_grid, int top, ExactStage &s) {
     const size_t need = 6 * ((size_t)P * 8 + 256) + ((size_t)n_grid * 8 + 256) + ((size_t)top * 4 + 256) + 256;
     MB_TRY(t.io.ensure(need));
-    t.polish_redone = 0;
+    t.polish_redone = -1;
     char *p = (char *)t.io.p;
     s.vi = carve<uint64_t>(p, P);
     s.vf = carve<uint64_t>(p, P);
@@ -153,15 +153,28 @@ int fetch_outputs(cudaStream_t st, int64_t P, const double *hu, const double *hp
 
 constexpr size_t POLISH_MOMENT_BYTES = (size_t)256 << 20;
 
-// Plans the cells of a polish whose offsets stay within R of the peaks: true where they hold four zeros or
-// more on average (fewer cells than that make an evaluation on moments cheaper than one over the zeros:
-// ~110 FP64 operations per cell against ~60 per zero and pass).  At least 592 cells (two items per CTA
-// slot) where they hold 64 zeros: few peaks then still fill the GPU; the split depends on the zeros and
-// R alone, so a peak's results do not depend on the others in the call.
-bool plan_polish(const Table &t, int64_t n, int64_t split, double R, CellPlan &cp) {
+// Plans the cells of a polish whose offsets stay within R of the peaks: true where the polish on moments is not
+// slower than the loops over the zeros.  At least 592 cells (two items per CTA slot) where they hold 64 zeros: few
+// peaks then still fill the GPU.  The split and the choice depend on the zeros, R and the loop alone, so a
+// peak's results do not depend on the others in the call, nor on the number of weight vectors.
+//   Up to CPOL_CELLS cells (their moments fit shared memory) four zeros a cell are enough.
+//   Above that a polish costs ~cells per peak and start, and 1 / cells of the peaks fit a pass of
+// POLISH_MOMENT_BYTES, whose moment pass costs ~n however few they are: together ~cells^2 / n of the loops' cost, for
+// five vectors (POLISH_EVAL_FAST) more than for one.  Measured, in ms (256 peaks x 5 vectors unless given):
+//   EVAL_FAST 600,000 zeros, 19,900 cells 23.1 against 29.2, 29,800 cells 43.7 against 29.4, 78,000 cells 242 against
+//             29; 2,325,572 zeros, 34,000 cells 79 against 122, 66,000 cells 237 against 120; 20,000 zeros, one peak and
+//             vector, 2,300 cells 0.29 against 0.28, 3,600 cells 0.44 against 0.28
+//   SINGLE    one peak: 20,000 zeros, 1,400 cells 0.55 against 0.72, 3,600 cells 1.5 against 0.74; 600,000 zeros,
+//             29,800 cells 11.2 against 16.5, 78,000 cells 28.0 against 15.8
+//   TOPK      25 peaks: 100,000 zeros, 2,000 cells 0.21 against 0.29, 5,700 cells 0.31 against 0.29
+bool plan_polish(const Table &t, int64_t n, int64_t split, double R, int mode, CellPlan &cp) {
     if (n < 1 || !std::isfinite(R)) return false;
-    return plan_cells(t, n, split, R, CELL_D1, std::min<int64_t>(n / 64, 592), cp) &&
-           (int64_t)cp.cells() <= std::max<int64_t>(64, n / 4);
+    if (!plan_cells(t, n, split, R, CELL_D1, std::min<int64_t>(n / 64, 592), cp)) return false;
+    const int64_t c = cp.cells();
+    if (c <= std::max<int64_t>(64, std::min<int64_t>(n / 4, CPOL_CELLS))) return true;
+    const double zeros = mode == POLISH_EVAL_FAST ? 8 : (mode == POLISH_SINGLE ? 13 : 18);
+    const double square = mode == POLISH_EVAL_FAST ? 700 : 2500;
+    return (double)c * std::max(zeros, (double)c / square) <= (double)n;
 }
 
 // Polishes the P peaks of stage s (or its P selected ones, a.sel) over the zeros [0, n) under the weight
@@ -180,6 +193,7 @@ int polish_on_cells(Table &t, const ExactStage &s, int64_t P, int64_t n, int n_w
     Cells cells;
     MB_TRY(build_cells(t, cp, cbuf, cells, t.stream));
     const CellPolishArgs all = a;
+    t.polish_redone = 0;
     for (int64_t p0 = 0; p0 < P; p0 += chunk)
         for (int w0 = 0; w0 < n_weights; w0 += CELL_MAX_W) {
             const int64_t np = std::min(chunk, P - p0);
@@ -365,7 +379,7 @@ extern "C" int mb_polish_single_exact(mb_table *h, int64_t P, const uint64_t *v_
     ExactStage s;
     MB_TRY(stage_exact(t, P, v_int, v_frac, delta, grid.data(), (int64_t)grid.size(), 0, s));
     CellPlan cp;
-    if (plan_polish(t, n_zeros, 0, single_reach(grid_hw, grid_steps), cp)) {
+    if (plan_polish(t, n_zeros, 0, single_reach(grid_hw, grid_steps), POLISH_SINGLE, cp)) {
         MB_TRY(polish_on_cells(t, s, P, n_zeros, 1, &weight_slot, cp,
                                CellPolishArgs{POLISH_SINGLE, P, 1, P, s.grid, (int)grid.size(), 0.0, nullptr, s.hu, s.hp, s.dp}));
         return fetch_outputs(t.stream, P, s.hu, s.hp, s.dp, out_h_unpol, out_h_pol, out_ddy_pol);
@@ -393,7 +407,7 @@ extern "C" int mb_polish_peaks_exact(mb_table *h, int64_t P, const uint64_t *v_i
     ExactStage s;
     MB_TRY(stage_exact(t, P, v_int, v_frac, delta, nullptr, 0, 0, s));
     CellPlan cp;
-    if (plan_polish(t, n_zeros, 4096, eval_fast_reach(grid_half_width, grid_steps), cp)) {
+    if (plan_polish(t, n_zeros, 4096, eval_fast_reach(grid_half_width, grid_steps), POLISH_EVAL_FAST, cp)) {
         MB_TRY(polish_on_cells(t, s, P, n_zeros, 1, &weight_slot, cp,
                                CellPolishArgs{POLISH_EVAL_FAST, P, 1, P, nullptr, grid_steps, grid_half_width, nullptr,
                                               s.hu, s.hp, s.dp}));
@@ -436,7 +450,7 @@ extern "C" int mb_polish_peaks_weights(mb_table *h, int64_t P, const uint64_t *v
     MB_TRY(device_guard(t.device));
     ExactStage s;
     CellPlan cp;
-    if (plan_polish(t, n_zeros, 4096, eval_fast_reach(grid_half_width, grid_steps), cp)) {
+    if (plan_polish(t, n_zeros, 4096, eval_fast_reach(grid_half_width, grid_steps), POLISH_EVAL_FAST, cp)) {
         const size_t ob = (size_t)n_weights * P;
         MB_TRY(stage_exact(t, P, v_int, v_frac, delta, nullptr, (int64_t)(3 * ob), 0, s));
         double *hu = s.grid, *hp = hu + ob, *dp = hp + ob;       // outputs in the stage's grid array
@@ -531,7 +545,7 @@ extern "C" int mb_fast_polish_exact(mb_table *h, int64_t P, const uint64_t *v_in
     double reach = 4 * 1e-5;
     for (int64_t i = 0; i < n_grid; ++i) reach = std::max(reach, std::fabs(ddy_grid[i]) + 4 * 1e-5);
     CellPlan cp;
-    if (plan_polish(t, n_zeros, 0, reach, cp)) {
+    if (plan_polish(t, n_zeros, 0, reach, POLISH_TOPK, cp)) {
         MB_TRY(polish_on_cells(t, s, nsel, n_zeros, 1, &weight_slot, cp,
                                CellPolishArgs{POLISH_TOPK, nsel, 1, P, nullptr, 0, 0.0, s.sel, s.hu, s.hp, s.dp}));
         return fetch_outputs(t.stream, P, s.hu, s.hp, s.dp, out_h_unpol, out_h_pol, out_ddy_pol);
