@@ -362,8 +362,9 @@ int mb_polish_peaks_exact(mb_table *t, int64_t P, const uint64_t *v_int, const u
  * (search/eval_tech1_600k.py:216-273: compute_peak_AB once, then polish_peaks_with_weights per
  * weight vector): each candidate's terms are formed once and summed into moments over cells of zeros
  * under up to five vectors at a time, and the polishes run on the moments; a peak whose Newton path
- * amplifies rounding is polished over the zeros instead.  Device workspace of the table, at most
- * 0.6 GiB, kept between calls.  A grid so wide that its cells hold few zeros (grid_half_width above
+ * amplifies rounding is polished over the zeros instead.  Device workspace of the table, kept between
+ * calls: at most 0.4 GiB of moments and, once such a peak has come up, 0.4 GiB for these (20 bytes per
+ * zero where that is more).  A grid so wide that its cells hold few zeros (grid_half_width above
  * 0.02 on 600,000 zeros) builds the exact (A, B) of up to 65,535 peaks at a time in a buffer of at most
  * 4 GiB and at most half of the device's free memory, allocated for the call and freed before it
  * returns. */

@@ -171,6 +171,8 @@ bool plan_polish(const Table &t, int64_t n, int64_t split, double R, int mode, C
     if (n < 1 || !std::isfinite(R)) return false;
     if (!plan_cells(t, n, split, R, CELL_D1, std::min<int64_t>(n / 64, 592), cp)) return false;
     const int64_t c = cp.cells();
+    // one peak's moments under a full set of vectors stay within the workspace
+    if (c * (2 * CELL_D1 * 8 * CELL_MAX_W) > (int64_t)POLISH_MOMENT_BYTES) return false;
     if (c <= std::max<int64_t>(64, std::min<int64_t>(n / 4, CPOL_CELLS))) return true;
     const double zeros = mode == POLISH_EVAL_FAST ? 8 : (mode == POLISH_SINGLE ? 13 : 18);
     const double square = mode == POLISH_EVAL_FAST ? 700 : 2500;
