@@ -675,20 +675,24 @@ cell_polish_kernel(Cells cells, const double *M, CellPolishArgs a, const double 
         block_sums(x);
         return x[0];
     };
-    // h(0), and sqrt(sum gamma^4 |M_c0|^2): 2^-53 |d| times it is the size of the error that rounding
-    // gamma_j d leaves in h'(d)
+    // h(0); sqrt(sum gamma^4 |M_c0|^2): 2^-53 |d| times it is the size of the error that rounding
+    // gamma_j d leaves in h'(d); and sum |Re M_c0| + |Im M_c0|, times POLISH_TIE the distance at which two |h| may be
+    // told apart one way here and the other way by the loops over the zeros (shared: a register more spills)
+    __shared__ double tie;
     double h0, noise;
     {
-        double x[2] = {0.0, 0.0};
+        double x[3] = {0.0, 0.0, 0.0};
         for (int c = threadIdx.x; c < cells.n; c += THREADS) {
             const double *m = m0 + c * LD;
             const double g = 6.283185307179586 * (double)cells.ctr[c] * 0x1p-16, g2 = g * g;
             x[0] += fma(-g * rho, m[CELL_D1], m[0]);             // the rotation by g rho to first order
             x[1] += g2 * g2 * (m[0] * m[0] + m[CELL_D1] * m[CELL_D1]);
+            x[2] += fabs(m[0]) + fabs(m[CELL_D1]);
         }
         block_sums(x);
         h0 = x[0];
         noise = 0x1p-53 * sqrt(x[1]);
+        if (threadIdx.x == 0) tie = POLISH_TIE * x[2];
     }
     // Newton on h' = 0 from d (the loop of polish_newton): with g = 2 pi G_c,
     //   h'  = -(g Im F0 + kappa Im F1),   h'' = -(g^2 Re F0 + 2 g kappa Re F1 + kappa^2 Re F2),
@@ -782,6 +786,7 @@ cell_polish_kernel(Cells cells, const double *M, CellPolishArgs a, const double 
         const double d = newton(start[s], sens);
         const double h = value(d);
         if (!(sens <= worst)) worst = sens;
+        if (fabs(fabs(h) - fabs(hp)) <= tie && fabs(d - dp) > R::tol) worst = INFINITY;
         if (polish_keep<MODE>(h, hp)) {
             hp = h;
             dp = d;

@@ -95,7 +95,10 @@ int launch_cell_scan(const Table &t, const Cells &c, int d1, const double *M, in
 // vector without decay).  Each path carries an estimate of that error, and a peak whose offset could
 // differ by more than POLISH_SENSITIVE of the step clamp from the loops over the zeros is polished
 // again by those loops themselves (the same bits), spread over the GPU.
+// So is a peak where two offsets farther apart than the loop's last step have |h| closer than the two ways' roundings
+// (POLISH_TIE of the cells' amplitude): two starts that end near one maximum, the second not fully converged.
 constexpr double POLISH_SENSITIVE = 1e-10;
+constexpr double POLISH_TIE = 2e-15;
 struct CellPolishArgs {
     int mode;                  // PolishMode
     int64_t P;

@@ -98,3 +98,21 @@ def test_second_pass_of_several_weights(gpu):
             one += redone(t)
             assert all(np.array_equal(x[i], y) for x, y in zip(got, want))
         assert one == total
+
+
+@pytest.mark.parametrize("steps", [10, 40])
+def test_starts_that_end_near_one_maximum(gpu, steps):
+    """The single-peak loop's two starts can end within rounding of the same |h| at offsets 1e-13 to 1e-11 apart; which one
+    is kept then follows from the loops' own rounding, so the second pass decides.  The offsets of all peaks agree with
+    the matrix form's to twice the loop's last step, 1e-14."""
+    data = synth.make_table(20_000, seed=96)
+    w = np.exp(-3e-9 * data.gamma**2)
+    c = synth.make_candidates(1024, seed=97)
+    with k2.ZeroTable.from_data(data) as t:
+        got = path1.polish_single_exact(t, c, t.add_weights(w), None, 2.5e-4, steps)
+        n = redone(t)
+        A, B = path1.compute_exact_AB(t, c)
+    want = path1.polish_single_peak(A, B, data.gamma, w, data.n, 2.5e-4, steps)
+    assert 4 <= n <= 100
+    np.testing.assert_allclose(got[2], want[2], rtol=0, atol=2e-14)
+    np.testing.assert_allclose(got[1], want[1], rtol=0, atol=1e-14)
