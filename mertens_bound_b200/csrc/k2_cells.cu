@@ -1252,10 +1252,16 @@ static int polish_mode(Table &t, const Cells &c, const double *M, CellPolishArgs
     if (count == 0) return MB_OK;
     t.polish_redone += count;
     RedoBuf rb;
-    rb.batch = redo_batch(count, n);
-    const size_t bn = (size_t)rb.batch * n;
-    MB_TRY(t.redo.ensure((2 * rb.batch * sizeof(RedoState) + 256) + (2 * rb.batch * REDO_GROUPS * sizeof(double2) + 256) +
-                         2 * (rb.batch * 8 + 256) + (bn * sizeof(double2) + 256)));
+    size_t bn = 0;
+    bool room = false;
+    for (rb.batch = redo_batch(count, n);; rb.batch /= 2) {
+        bn = (size_t)rb.batch * n;
+        MB_TRY(t.redo.ensure((2 * rb.batch * sizeof(RedoState) + 256) +
+                             (2 * rb.batch * REDO_GROUPS * sizeof(double2) + 256) + 2 * (rb.batch * 8 + 256) +
+                             (bn * sizeof(double2) + 256), &room));
+        if (room) break;
+        if (rb.batch == 1) return NO_ROOM;
+    }
     q = (char *)t.redo.p;
     rb.state = carve<RedoState>(q, 2 * (size_t)rb.batch);
     rb.slot = carve<double2>(q, 2 * (size_t)rb.batch * REDO_GROUPS);

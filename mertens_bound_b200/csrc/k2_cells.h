@@ -115,7 +115,7 @@ constexpr int CPOL_CELLS = 1200;
 // Device bytes of the second pass's list for P x nw peaks (its terms are in t.redo).
 size_t cell_polish_bytes(int64_t P, int nw);
 // vi, vf, delta: the points (as for launch_moments_weights); w: the weights; work: cell_polish_bytes.  Waits
-// for the stream once, for the number of peaks to polish again.
+// for the stream once, for the number of peaks to polish again.  NO_ROOM: not even one of these peaks' terms fit.
 int launch_cell_polish(Table &t, const Cells &c, const double *M, const CellPolishArgs &a, const uint64_t *vi,
                        const uint64_t *vf, const double *delta, int64_t n, const CellWeights &w, void *work,
                        cudaStream_t s);

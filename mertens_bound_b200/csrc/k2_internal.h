@@ -37,6 +37,9 @@ const char *last_error();
         }                                                                                   \
     } while (0)
 
+// Status of a path whose workspace the device has no room for: its caller takes another one.
+constexpr int NO_ROOM = 1;
+
 #define MB_TRY(call)              \
     do {                          \
         int s_ = (call);          \
@@ -44,11 +47,12 @@ const char *last_error();
     } while (0)
 
 // Grow-only device buffer.  ensure() synchronises the device before it frees a smaller
-// buffer, so work still in flight on any stream never sees its memory released.
+// buffer, so work still in flight on any stream never sees its memory released.  Where the device
+// has no room for `need` it is an error, or with room != null MB_OK and *room = false.
 struct DevBuf {
     void *p = nullptr;
     size_t bytes = 0;
-    int ensure(size_t need);
+    int ensure(size_t need, bool *room = nullptr);
     void release();
 };
 

@@ -181,13 +181,16 @@ bool plan_polish(const Table &t, int64_t n, int64_t split, double R, int mode, C
 
 // Polishes the P peaks of stage s (or its P selected ones, a.sel) over the zeros [0, n) under the weight
 // slots, outputs a.h_unpol etc. on the device: per chunk of peaks and up to CELL_MAX_W vectors, one moment
-// pass over the zeros and the polish on the moments.
+// pass over the zeros and the polish on the moments.  NO_ROOM (outputs partly written): the device has no room
+// for the moments or the second pass, and the caller takes the loops over the zeros.
 int polish_on_cells(Table &t, const ExactStage &s, int64_t P, int64_t n, int n_weights, const int *slots,
                     const CellPlan &cp, CellPolishArgs a) {
     const size_t cb = cells_bytes(cp), one = (size_t)cp.cells() * 2 * CELL_D1 * 8;     // per (peak, weight)
     const int wmax = std::min(n_weights, CELL_MAX_W);
     const int64_t chunk = std::max<int64_t>(1, std::min<int64_t>(P, (int64_t)(POLISH_MOMENT_BYTES / (one * wmax))));
-    MB_TRY(t.work.ensure((cb + 256) + ((size_t)chunk * wmax * one + 256) + cell_polish_bytes(chunk, wmax)));
+    bool room;
+    MB_TRY(t.work.ensure((cb + 256) + ((size_t)chunk * wmax * one + 256) + cell_polish_bytes(chunk, wmax), &room));
+    if (!room) return NO_ROOM;
     char *q = (char *)t.work.p;
     void *cbuf = carve<char>(q, cb);
     double *M = carve<double>(q, (size_t)chunk * wmax * (one / 8));
@@ -382,9 +385,12 @@ extern "C" int mb_polish_single_exact(mb_table *h, int64_t P, const uint64_t *v_
     MB_TRY(stage_exact(t, P, v_int, v_frac, delta, grid.data(), (int64_t)grid.size(), 0, s));
     CellPlan cp;
     if (plan_polish(t, n_zeros, 0, single_reach(grid_hw, grid_steps), POLISH_SINGLE, cp)) {
-        MB_TRY(polish_on_cells(t, s, P, n_zeros, 1, &weight_slot, cp,
-                               CellPolishArgs{POLISH_SINGLE, P, 1, P, s.grid, (int)grid.size(), 0.0, nullptr, s.hu, s.hp, s.dp}));
-        return fetch_outputs(t.stream, P, s.hu, s.hp, s.dp, out_h_unpol, out_h_pol, out_ddy_pol);
+        const int st = polish_on_cells(t, s, P, n_zeros, 1, &weight_slot, cp,
+                                       CellPolishArgs{POLISH_SINGLE, P, 1, P, s.grid, (int)grid.size(), 0.0, nullptr, s.hu,
+                                                      s.hp, s.dp});
+        if (st == MB_OK) return fetch_outputs(t.stream, P, s.hu, s.hp, s.dp, out_h_unpol, out_h_pol, out_ddy_pol);
+        if (st != NO_ROOM) return st;
+        t.polish_redone = -1;
     }
     PolishArgs a{n_zeros, t.d_gamma, t.d_weights[weight_slot], s.grid, (int)grid.size(), 0.0, nullptr, s.hu, s.hp, s.dp};
     peak_polish_kernel<ABExact, POLISH_SINGLE><<<(unsigned)(P * POLISH_CLUSTER), POLISH_THREADS, 0, t.stream>>>(
@@ -410,10 +416,12 @@ extern "C" int mb_polish_peaks_exact(mb_table *h, int64_t P, const uint64_t *v_i
     MB_TRY(stage_exact(t, P, v_int, v_frac, delta, nullptr, 0, 0, s));
     CellPlan cp;
     if (plan_polish(t, n_zeros, 4096, eval_fast_reach(grid_half_width, grid_steps), POLISH_EVAL_FAST, cp)) {
-        MB_TRY(polish_on_cells(t, s, P, n_zeros, 1, &weight_slot, cp,
-                               CellPolishArgs{POLISH_EVAL_FAST, P, 1, P, nullptr, grid_steps, grid_half_width, nullptr,
-                                              s.hu, s.hp, s.dp}));
-        return fetch_outputs(t.stream, P, s.hu, s.hp, s.dp, out_h_unpol, out_h_pol, out_ddy_pol);
+        const int st = polish_on_cells(t, s, P, n_zeros, 1, &weight_slot, cp,
+                                       CellPolishArgs{POLISH_EVAL_FAST, P, 1, P, nullptr, grid_steps, grid_half_width,
+                                                      nullptr, s.hu, s.hp, s.dp});
+        if (st == MB_OK) return fetch_outputs(t.stream, P, s.hu, s.hp, s.dp, out_h_unpol, out_h_pol, out_ddy_pol);
+        if (st != NO_ROOM) return st;
+        t.polish_redone = -1;
     }
     PolishArgs a{n_zeros, t.d_gamma, t.d_weights[weight_slot], nullptr, grid_steps, grid_half_width, nullptr,
                  s.hu, s.hp, s.dp};
@@ -456,10 +464,11 @@ extern "C" int mb_polish_peaks_weights(mb_table *h, int64_t P, const uint64_t *v
         const size_t ob = (size_t)n_weights * P;
         MB_TRY(stage_exact(t, P, v_int, v_frac, delta, nullptr, (int64_t)(3 * ob), 0, s));
         double *hu = s.grid, *hp = hu + ob, *dp = hp + ob;       // outputs in the stage's grid array
-        MB_TRY(polish_on_cells(t, s, P, n_zeros, n_weights, weight_slots, cp,
-                               CellPolishArgs{POLISH_EVAL_FAST, P, n_weights, P, nullptr, grid_steps, grid_half_width,
-                                              nullptr, hu, hp, dp}));
-        return fetch_outputs(t.stream, (int64_t)ob, hu, hp, dp, out_h_unpol, out_h_pol, out_ddy_pol);
+        const int st = polish_on_cells(t, s, P, n_zeros, n_weights, weight_slots, cp,
+                                       CellPolishArgs{POLISH_EVAL_FAST, P, n_weights, P, nullptr, grid_steps,
+                                                      grid_half_width, nullptr, hu, hp, dp});
+        if (st == MB_OK) return fetch_outputs(t.stream, (int64_t)ob, hu, hp, dp, out_h_unpol, out_h_pol, out_ddy_pol);
+        if (st != NO_ROOM) return st;
     }
     MB_TRY(stage_exact(t, P, v_int, v_frac, delta, nullptr, 0, 0, s));
     // the matrices take at most AB_BUDGET bytes and at most half of the device's free memory
@@ -533,12 +542,20 @@ extern "C" int mb_fast_polish_exact(mb_table *h, int64_t P, const uint64_t *v_in
     const ABExact src{view(t), s.vi, s.vf, s.delta};
     const double *d_w = t.d_weights[weight_slot];
     const int n_chunk = taylor_chunks(n_zeros);
-    const int64_t pc = std::max<int64_t>(
-        1, std::min<int64_t>(P, (int64_t)(POLISH_MOMENT_BYTES / taylor_work_bytes(1, n_chunk))));
-    MB_TRY(t.work.ensure(taylor_work_bytes(pc, n_chunk)));
-    for (int64_t p0 = 0; p0 < P; p0 += pc)
-        MB_TRY(launch_taylor_grid(t, s.vi + p0, s.vf + p0, s.delta + p0, std::min(pc, P - p0), n_zeros, n_chunk, d_w,
-                                  s.grid, (int)n_grid, t.work.p, s.hu + p0, s.hp + p0, s.dp + p0, t.stream));
+    auto grid_stage = [&]() -> int {
+        int64_t pc = std::max<int64_t>(
+            1, std::min<int64_t>(P, (int64_t)(POLISH_MOMENT_BYTES / taylor_work_bytes(1, n_chunk))));
+        for (bool room = false; !room;) {                // fewer peaks a pass where memory is short
+            MB_TRY(t.work.ensure(taylor_work_bytes(pc, n_chunk), pc > 1 ? &room : nullptr));
+            if (pc == 1) break;
+            if (!room) pc = (pc + 1) / 2;
+        }
+        for (int64_t p0 = 0; p0 < P; p0 += pc)
+            MB_TRY(launch_taylor_grid(t, s.vi + p0, s.vf + p0, s.delta + p0, std::min(pc, P - p0), n_zeros, n_chunk,
+                                      d_w, s.grid, (int)n_grid, t.work.p, s.hu + p0, s.hp + p0, s.dp + p0, t.stream));
+        return MB_OK;
+    };
+    MB_TRY(grid_stage());
     if (nsel == 0) return fetch_outputs(t.stream, P, s.hu, s.hp, s.dp, out_h_unpol, out_h_pol, out_ddy_pol);
     MB_CUDA(cudaMemcpyAsync(out_h_pol, s.hp, P * 8, cudaMemcpyDeviceToHost, t.stream));
     MB_CUDA(cudaStreamSynchronize(t.stream));
@@ -548,9 +565,12 @@ extern "C" int mb_fast_polish_exact(mb_table *h, int64_t P, const uint64_t *v_in
     for (int64_t i = 0; i < n_grid; ++i) reach = std::max(reach, std::fabs(ddy_grid[i]) + 4 * 1e-5);
     CellPlan cp;
     if (plan_polish(t, n_zeros, 0, reach, POLISH_TOPK, cp)) {
-        MB_TRY(polish_on_cells(t, s, nsel, n_zeros, 1, &weight_slot, cp,
-                               CellPolishArgs{POLISH_TOPK, nsel, 1, P, nullptr, 0, 0.0, s.sel, s.hu, s.hp, s.dp}));
-        return fetch_outputs(t.stream, P, s.hu, s.hp, s.dp, out_h_unpol, out_h_pol, out_ddy_pol);
+        const int st = polish_on_cells(t, s, nsel, n_zeros, 1, &weight_slot, cp,
+                                       CellPolishArgs{POLISH_TOPK, nsel, 1, P, nullptr, 0, 0.0, s.sel, s.hu, s.hp, s.dp});
+        if (st == MB_OK) return fetch_outputs(t.stream, P, s.hu, s.hp, s.dp, out_h_unpol, out_h_pol, out_ddy_pol);
+        if (st != NO_ROOM) return st;
+        t.polish_redone = -1;
+        MB_TRY(grid_stage());                            // the starts again: the cells' polish writes over them
     }
     PolishArgs a{n_zeros, t.d_gamma, d_w, nullptr, 0, 0.0, s.sel, s.hu, s.hp, s.dp};
     peak_polish_kernel<ABExact, POLISH_TOPK><<<(unsigned)(nsel * POLISH_CLUSTER), POLISH_THREADS, 0, t.stream>>>(src, a);

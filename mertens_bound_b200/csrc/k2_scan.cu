@@ -318,7 +318,8 @@ bool scan_in_range(int64_t P, const uint64_t *vi, const uint64_t *vf, u128 step,
     return true;
 }
 
-// The scan of P base points on cell moments; take(p0, np, d_h) queues what is done with the results of the
+// The scan of P base points on cell moments (NO_ROOM, with nothing queued, where the device has no room for
+// them); take(p0, np, d_h) queues what is done with the results of the
 // base points [p0, p0 + np) (device, np x n_m) on t.stream.
 template <typename Take>
 int scan_cells(Table &t, int64_t P, const uint64_t *v_int, const uint64_t *v_frac, double k, uint64_t step_int,
@@ -326,8 +327,10 @@ int scan_cells(Table &t, int64_t P, const uint64_t *v_int, const uint64_t *v_fra
     const u128 step = (u128)step_int << 64 | step_frac;
     const int64_t per = sp.chunk * sp.NB;
     const size_t pb = (size_t)per * 8, cb = cells_bytes(sp.cp);
-    MB_TRY(t.io.ensure(2 * (pb + 256) + cb + 256 + (size_t)sp.chunk * n_m * 8 + 256));
-    MB_TRY(t.work.ensure((size_t)per * sp.cp.cells() * 2 * sp.d1 * 8));
+    bool room;
+    MB_TRY(t.io.ensure(2 * (pb + 256) + cb + 256 + (size_t)sp.chunk * n_m * 8 + 256, &room));
+    if (room) MB_TRY(t.work.ensure((size_t)per * sp.cp.cells() * 2 * sp.d1 * 8, &room));
+    if (!room) return NO_ROOM;
     char *q = (char *)t.io.p;
     uint64_t *d_v = carve<uint64_t>(q, 2 * per);
     void *cbuf = carve<char>(q, cb);
@@ -431,10 +434,13 @@ extern "C" int mb_grid_scan(mb_table *h, int64_t P, const uint64_t *v_int, const
     const int64_t grid_points = (n_m + SCAN_THREADS * SCAN_MPT - 1) / (SCAN_THREADS * SCAN_MPT) * (SCAN_THREADS * SCAN_MPT);
     if (plan_scan(t, P, n_use, n_m, step_int, step_frac, GRID_CYCLES, grid_points, sp) &&
         scan_in_range(P, v_int, v_frac, (u128)step_int << 64 | step_frac, m0, (int64_t)sp.NB * sp.Bp))
-        {
-        MB_TRY(scan_cells(t, P, v_int, v_frac, k, step_int, step_frac, m0, n_m, sp, ToHost{out_h, n_m, t.stream}));
-        MB_CUDA(cudaStreamSynchronize(t.stream));
-        return MB_OK;
+    {
+        const int st = scan_cells(t, P, v_int, v_frac, k, step_int, step_frac, m0, n_m, sp, ToHost{out_h, n_m, t.stream});
+        if (st != MB_OK && st != NO_ROOM) return st;
+        if (st == MB_OK) {
+            MB_CUDA(cudaStreamSynchronize(t.stream));
+            return MB_OK;
+        }
     }
     const size_t cb = (size_t)P * 8, hb = (size_t)P * n_m * 8;
     int sms = 148;
@@ -476,8 +482,10 @@ static int hit_scan(Table &t, int64_t P, const uint64_t *v_int, const uint64_t *
                     uint64_t step_int, uint64_t step_frac, int64_t m0, int64_t n_m, Take take) {
     ScanPlan sp;
     if (plan_scan(t, P, n_use, n_m, step_int, step_frac, HIT_CYCLES, (n_m + HIT_MB - 1) / HIT_MB * HIT_MB, sp) &&
-        scan_in_range(P, v_int, v_frac, (u128)step_int << 64 | step_frac, m0, (int64_t)sp.NB * sp.Bp))
-        return scan_cells(t, P, v_int, v_frac, k, step_int, step_frac, m0, n_m, sp, take);
+        scan_in_range(P, v_int, v_frac, (u128)step_int << 64 | step_frac, m0, (int64_t)sp.NB * sp.Bp)) {
+        const int st = scan_cells(t, P, v_int, v_frac, k, step_int, step_frac, m0, n_m, sp, take);
+        if (st != NO_ROOM) return st;
+    }
     const size_t cb = (size_t)P * 8, hb = (size_t)P * n_m * 8;
     MB_TRY(t.io.ensure(2 * cb + hb + 256));
     char *base = (char *)t.io.p;

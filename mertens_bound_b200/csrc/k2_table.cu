@@ -35,7 +35,8 @@ int64_t Table::count_below(double T) const {
     return (int64_t)(std::lower_bound(h_gamma.begin(), h_gamma.end(), T) - h_gamma.begin());
 }
 
-int DevBuf::ensure(size_t need) {
+int DevBuf::ensure(size_t need, bool *room) {
+    if (room) *room = true;
     if (need <= bytes) return MB_OK;
     if (p) {
         MB_CUDA(cudaDeviceSynchronize());
@@ -44,7 +45,19 @@ int DevBuf::ensure(size_t need) {
         bytes = 0;
     }
     size_t want = std::max(need + need / 4, (size_t)1 << 20);
-    MB_CUDA(cudaMalloc(&p, want));
+    cudaError_t e = cudaMalloc(&p, want);
+    if (e == cudaErrorMemoryAllocation) {
+        cudaGetLastError();                     // else the next launch's check would report it
+        want = need;
+        e = cudaMalloc(&p, want);
+    }
+    if (e == cudaErrorMemoryAllocation) cudaGetLastError();
+    if (e != cudaSuccess) p = nullptr;
+    if (e == cudaErrorMemoryAllocation && room) {
+        *room = false;
+        return MB_OK;
+    }
+    MB_CUDA(e);
     bytes = want;
     return MB_OK;
 }
