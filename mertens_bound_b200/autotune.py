@@ -12,7 +12,8 @@ The search space is the plan-wide tile configuration (mb_plan_configure) under e
 Every configuration is timed on the device (median of `reps` runs, synthetic candidates) and the
 fastest one is applied.  Results are cached per (GPU name, workload class) in a JSON file
 ($MB_AUTOTUNE_CACHE, default ~/.cache/mertens_k2/autotune.json); a workload class buckets the
-candidate count, the zero counts and the heavy-tier fraction on a log scale.
+candidate count, the zero counts and the heavy-tier fraction on a log scale, under the work-item rule in
+force (RULE).
 """
 from __future__ import annotations
 
@@ -25,6 +26,10 @@ from . import k2
 
 SPACE = [(cpt, shift, scale) for cpt in (2, 3, 4) for shift in (0, 1) for scale in (0.5, 1.0, 2.0)]
 SCHEDULES = (0, 1, 2, 3)
+# The rule that turns a configuration into work items (build_items in csrc/k2_plan.cu) and the kernels that run them; raised
+# when either changes, so a choice timed under another one is not applied.  1: light chunks of a fixed share of the terms;
+# 2: light chunks sized by the CTA slots, heavy groups of at most 32 candidates one per lane.
+RULE = 2
 _lock = threading.Lock()
 
 
@@ -51,6 +56,7 @@ def workload_key(plan: k2.Plan) -> str:
         f"P{round(math.log2(max(plan.P, 1)))}",
         f"N{round(math.log2(max(max(n_T), 1)))}",
         f"H{round(10 * heavy / terms)}",
+        f"R{RULE}",
     ]
     return "|".join(parts)
 
