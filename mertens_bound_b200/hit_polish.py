@@ -18,6 +18,7 @@ best points found on the device); hits are x = floor(y 2^30) as in the reference
 """
 from __future__ import annotations
 
+import functools
 from dataclasses import dataclass
 from fractions import Fraction
 
@@ -44,6 +45,7 @@ class HitResult:
     stage: np.ndarray      # last stage run per hit (0..4)
 
 
+@functools.lru_cache(maxsize=64)
 def _fixed(step: float) -> int:
     """64.64 fixed point of a positive double (exact for the stage steps' binary values)."""
     q = Fraction(step)
