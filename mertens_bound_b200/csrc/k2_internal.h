@@ -76,10 +76,11 @@ struct Table {
     cudaStream_t side = nullptr;      // second stream: heavy tier beside the light tier
     cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
     // grow-only scratch owned by the table: `io` stages candidates and results of host-pointer
-    // calls, `work` holds per-chunk partial sums and moments.  Calls on one table that use the same
-    // buffer must not overlap on the GPU.
-    DevBuf io, work;
-    DevBuf redo;                      // the second pass of polishes on cell moments (k2_cells.cu)
+    // calls, `work` holds per-chunk partial sums, also those of mb_k2_plain_dev on the caller's stream;
+    // `moments` the cell moments of scans and polishes and `redo` these polishes' second pass, which
+    // must not disturb such a call in flight.  Calls on one table that use the same buffer must not
+    // overlap on the GPU.
+    DevBuf io, work, moments, redo;
     int64_t polish_redone = 0;        // (peak, weight) pairs the last polish took there; -1: no moments
     int n_plans = 0;                  // live plans on this table (it cannot be destroyed under them)
 

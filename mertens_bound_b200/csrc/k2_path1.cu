@@ -189,9 +189,9 @@ int polish_on_cells(Table &t, const ExactStage &s, int64_t P, int64_t n, int n_w
     const int wmax = std::min(n_weights, CELL_MAX_W);
     const int64_t chunk = std::max<int64_t>(1, std::min<int64_t>(P, (int64_t)(POLISH_MOMENT_BYTES / (one * wmax))));
     bool room;
-    MB_TRY(t.work.ensure((cb + 256) + ((size_t)chunk * wmax * one + 256) + cell_polish_bytes(chunk, wmax), &room));
+    MB_TRY(t.moments.ensure((cb + 256) + ((size_t)chunk * wmax * one + 256) + cell_polish_bytes(chunk, wmax), &room));
     if (!room) return NO_ROOM;
-    char *q = (char *)t.work.p;
+    char *q = (char *)t.moments.p;
     void *cbuf = carve<char>(q, cb);
     double *M = carve<double>(q, (size_t)chunk * wmax * (one / 8));
     void *work = q;
@@ -546,13 +546,13 @@ extern "C" int mb_fast_polish_exact(mb_table *h, int64_t P, const uint64_t *v_in
         int64_t pc = std::max<int64_t>(
             1, std::min<int64_t>(P, (int64_t)(POLISH_MOMENT_BYTES / taylor_work_bytes(1, n_chunk))));
         for (bool room = false; !room;) {                // fewer peaks a pass where memory is short
-            MB_TRY(t.work.ensure(taylor_work_bytes(pc, n_chunk), pc > 1 ? &room : nullptr));
+            MB_TRY(t.moments.ensure(taylor_work_bytes(pc, n_chunk), pc > 1 ? &room : nullptr));
             if (pc == 1) break;
             if (!room) pc = (pc + 1) / 2;
         }
         for (int64_t p0 = 0; p0 < P; p0 += pc)
             MB_TRY(launch_taylor_grid(t, s.vi + p0, s.vf + p0, s.delta + p0, std::min(pc, P - p0), n_zeros, n_chunk,
-                                      d_w, s.grid, (int)n_grid, t.work.p, s.hu + p0, s.hp + p0, s.dp + p0, t.stream));
+                                      d_w, s.grid, (int)n_grid, t.moments.p, s.hu + p0, s.hp + p0, s.dp + p0, t.stream));
         return MB_OK;
     };
     MB_TRY(grid_stage());

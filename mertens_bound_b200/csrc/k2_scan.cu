@@ -329,13 +329,13 @@ int scan_cells(Table &t, int64_t P, const uint64_t *v_int, const uint64_t *v_fra
     const size_t pb = (size_t)per * 8, cb = cells_bytes(sp.cp);
     bool room;
     MB_TRY(t.io.ensure(2 * (pb + 256) + cb + 256 + (size_t)sp.chunk * n_m * 8 + 256, &room));
-    if (room) MB_TRY(t.work.ensure((size_t)per * sp.cp.cells() * 2 * sp.d1 * 8, &room));
+    if (room) MB_TRY(t.moments.ensure((size_t)per * sp.cp.cells() * 2 * sp.d1 * 8, &room));
     if (!room) return NO_ROOM;
     char *q = (char *)t.io.p;
     uint64_t *d_v = carve<uint64_t>(q, 2 * per);
     void *cbuf = carve<char>(q, cb);
     double *d_h = carve<double>(q, sp.chunk * n_m);
-    double *M = (double *)t.work.p;
+    double *M = (double *)t.moments.p;
     Cells cells;
     MB_TRY(build_cells(t, sp.cp, cbuf, cells, t.stream));
     std::vector<uint64_t> pts(2 * per);

@@ -93,6 +93,7 @@ static void free_table(Table &t) {
     cudaFree(t.d_psi);
     t.io.release();
     t.work.release();
+    t.moments.release();
     t.redo.release();
     for (double *w : t.d_weights) cudaFree(w);
     if (t.ev_fork) cudaEventDestroy(t.ev_fork);
