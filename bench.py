@@ -45,10 +45,10 @@ WORKLOAD = ("search_scoring: all 466,659 synthetic zeros below T0=3e5, 4,096 can
 # `bench.py --profile-case search` (dram__bytes_read.sum + dram__bytes_write.sum), and the
 # executed thread instructions per zero-term of each kernel from the same capture
 # (smsp__inst_executed.sum x 32 / zero-terms): the issue-slot side figure beside the pipe roofline.
-LIGHT_DRAM_BYTES = {2: 16468736, 3: 16439040, 4: 16438784}
-HEAVY_DRAM_BYTES = 2891008
-TIERS_DRAM_BYTES = 27556096          # k2_tiers_kernel<4> (both tiers in one launch)
-LIGHT_INST_PER_TERM = {2: 19.32, 3: 19.86, 4: 16.56}
+LIGHT_DRAM_BYTES = {2: 16518144, 3: 16473856, 4: 16438784}
+HEAVY_DRAM_BYTES = 2971648
+TIERS_DRAM_BYTES = 33348096          # k2_tiers_kernel<4> (both tiers in one launch)
+LIGHT_INST_PER_TERM = {2: 19.35, 3: 19.89, 4: 16.56}
 HEAVY_INST_PER_TERM = 34.93
 # Algorithmic operations per zero-term on each tier's binding pipe:
 #   light tier, XU (MUFU) pipe: one sine and one cosine of the reduced phase;

@@ -343,17 +343,18 @@ int mb_fast_polish_batch(int64_t n_peaks, int64_t n_zeros, const double *A, cons
                          const double *w, const double *ddy_grid, int64_t n_grid, int top, double *out_h_unpol,
                          double *out_h_pol, double *out_ddy_pol);
 
-/* The two polishes with (A_j, B_j) of peak p computed on the fly at y = v_p + delta_p as in
- * mb_exact_AB (no P x N matrices), over the table's first n_zeros zeros, gamma = the table's
- * FP64 gamma and w = a weight vector registered by mb_table_add_weights. */
+/* The two polishes of peak p at y = v_p + delta_p from the exact phase, as on the (A, B) of mb_exact_AB
+ * (no P x N matrices), over the table's first n_zeros zeros, gamma = the table's FP64 gamma and w = a
+ * weight vector registered by mb_table_add_weights.  They run on moments over cells of zeros (the same
+ * values within FP64 rounding) or, where the offsets reach too far for cells or memory is short, over
+ * the zeros; device workspace as mb_polish_peaks_weights. */
 int mb_polish_single_exact(mb_table *t, int64_t P, const uint64_t *v_int, const uint64_t *v_frac,
                            const double *delta, int64_t n_zeros, int weight_slot, double grid_hw, int grid_steps,
                            double *out_h_unpol, double *out_h_pol, double *out_ddy_pol);
 /* polish_peaks_with_weights (search/path1_eval_fast.cpp:58-143: h0; grid of 2 grid_steps + 1
  * shifts over the first min(n, 4096) zeros; <= 6 Newton steps, clamp 1e-4) for every candidate,
- * with (A_j, B_j) computed on the fly as in mb_exact_AB instead of read from P x N matrices:
- * the search drivers' compute_peak_AB + polish per weight vector (search/eval_tech1_600k.py:216-273)
- * without the matrices. */
+ * from the exact phase, as the two above: the search drivers' compute_peak_AB + polish per weight
+ * vector (search/eval_tech1_600k.py:216-273) without the matrices. */
 int mb_polish_peaks_exact(mb_table *t, int64_t P, const uint64_t *v_int, const uint64_t *v_frac,
                           const double *delta, int64_t n_zeros, int weight_slot, double grid_half_width,
                           int grid_steps, double *out_h_unpol, double *out_h_pol, double *out_ddy_pol);

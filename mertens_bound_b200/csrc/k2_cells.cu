@@ -173,8 +173,9 @@ struct CellTile {
 
 // One item = one cell x Sh::peaks / nzw peaks.  Warp w serves 8 MP peaks from 8 MP (w / nzw) and the
 // 4-zero steps congruent to w mod nzw; with nzw > 1 the warps' sums are added in warp order.
-// Bound: the FP64 pipe, 16 cycles per mma and scheduler, 2 mma per step and 8 columns, beside ~24 for
-// the phasor (60 instructions).  The next tile's zeros are loaded before the current one is summed and
+// Bound: instruction issue and the FP64 pipe together: an mma is 256 FMAs, 16 cycles of a scheduler's FP64 lanes, 2 of
+// them per step and 8 columns, beside the phasor's 60 instructions, and little of the one hides the other (256
+// points x 600,000 zeros with 8 terms: 620 us, where the FP64 operations alone need 290).  The next tile's zeros are loaded before the current one is summed and
 // staged after it, into the other half of a double buffer, across items too: one barrier per tile.
 template <int KIND, int W, int D1>
 __global__ void __launch_bounds__(CELL_THREADS, (CellShape<KIND, W, D1>::ctas))
@@ -971,8 +972,9 @@ __global__ void redo_keep_kernel(RedoBuf rb, CellPolishArgs a, int m, int start,
 
 constexpr int TAY_THREADS = 128;
 
-// One CTA per peak: the chunks' power sums added in a fixed order (four chunk strides, then those
-// four), then the grid points; ties of |h| go to the smaller index.
+// One CTA per peak: the chunks' power sums added in a fixed order (32 running sums over every 32nd chunk, then these
+// pairwise: longer chains of sums near the total would round more than the loops over the zeros), then the grid
+// points; ties of |h| go to the smaller index.
 __global__ void __launch_bounds__(TAY_THREADS)
 taylor_grid_kernel(const double *S, int n_chunk, const double *delta, const double *grid, int n_grid, double *h_unpol,
                    double *h_pol, double *ddy_pol) {

@@ -6,8 +6,8 @@
 //   h(d) = Re sum_c e^{2 pi i G_c d} sum_n M_cn (i kappa d)^n / n!,   kappa = 2 pi H,
 //   M_cn = sum_{j in c} w_j C_j x_j^n.
 // Every zero enters the moments once, whatever the number of offsets; with |kappa d| <= X the
-// series cut after D1 terms is within X^D1 / D1! per unit of amplitude, and (X, D1) below keep that
-// at or under the rounding of an FP64 sine.
+// series cut after D1 terms is within X^D1 / D1! per unit of amplitude: 1 to 9 units of 2^-53 at the worst for the
+// (X, D1) below, and less than one on average over a cell (the mean of |x|^D1 is 1 / (D1 + 1)).
 #pragma once
 #include <cstdint>
 #include <cuda_runtime.h>
@@ -18,7 +18,7 @@ namespace mb {
 
 // |kappa d| bound for D1 series terms: X^D1 / D1! (the first dropped term, per unit amplitude)
 //   D1 = 8,  X = 0.05: 9.7e-16    D1 = 16, X = 0.68: 1.0e-16    D1 = 11, X = 0.2: 5.1e-16
-// (largest over the cell; the mean of |x|^D1 over a cell is 1 / (D1 + 1)).
+// at the cell's edge and the farthest offset.
 constexpr double cell_x(int d1) { return d1 == 8 ? 0.05 : (d1 == 11 ? 0.2 : 0.68); }
 
 int cell_peaks(int64_t P, int d1);      // points of one CTA of launch_moments_gauss

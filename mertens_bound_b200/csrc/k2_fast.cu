@@ -122,8 +122,8 @@ MB_DEV void light_tile(const void *tile_v, int nt, int zl, int ZL, const CandReg
 }
 
 // The heavy tier's (cos, sin) table is k2_phasor.cuh's: 256 entries in eight interleaved copies, read without
-// bank conflicts.  (One copy of 2048 entries cost 9.4 shared-memory cycles per warp and term, more than the
-// term's 17 FP64 operations take on their pipe; this one costs 4.2 and two more operations.)  An entry is
+// bank conflicts.  (One copy of 2048 entries cost about nine shared-memory cycles per warp and term; this one costs
+// four and two more FP64 operations: the tier alone 608 -> 548 us.)  An entry is
 // rotated by d 2^-49 turn, |d| <= 2^40 (0.0123 rad); with a = 2 pi 2^-49:
 //   sin(a d)     = d (a - a^3 d^2 / 6 + a^5 d^4 / 120)    (truncation 8.4e-18)
 //   cos(a d) - 1 = d^2 (-a^2 / 2 + a^4 d^2 / 24)          (truncation 4.7e-15)
@@ -445,8 +445,8 @@ k2_tiers_kernel(TabView t, CandView c, const FastItem *items, int n_items, int n
 // REDUCE_CANDS candidates per CTA, REDUCE_LANES chunk lanes each: lane r of candidate q sums the chunks
 // r, r + REDUCE_LANES, ... (the eight lanes of one chunk read 192 consecutive bytes), then the lanes are
 // added pairwise through shared memory (deterministic: the order depends only on the chunk count).
-// Latency bound: a thousand candidates have ~460 chunks, so eight lanes per candidate took 31-49 us there
-// (15 rounds of loads); 32 lanes take 16 us, and 4,096 x 286 chunks 10 instead of 20 us.
+// Latency bound: with eight lanes per candidate 1,001 x 600,000 (some 1,700 chunks) took 49 us, 32 lanes take 25;
+// 4,096 x 466,659 (some 500 chunks) 20 and 12 us.
 constexpr int REDUCE_LANES = 32, REDUCE_CANDS = 8;
 __global__ void __launch_bounds__(REDUCE_LANES *REDUCE_CANDS)
 fast_reduce_kernel(const FastGroup *groups, int n_groups, const double *partial, int64_t P, double *val, double *dd,

@@ -2,13 +2,15 @@
 //   compute_exact_mpfr_AB   (:71-91)   -> mb_exact_AB: A_j, B_j = 2 c_j e^{i gamma_j y} from the exact
 //                                         128-bit phase (the reference rounds a 256-bit mpfr product)
 //   polish_single_peak      (:94-147)  -> mb_polish_single_peak (A/B rows) and
-//                                         mb_polish_single_exact (A/B computed on the fly)
+//                                         mb_polish_single_exact (exact phase)
 //   fast_polish_batch_blas  (:150-221) -> mb_fast_polish_batch (A/B rows) and
-//                                         mb_fast_polish_exact (A/B computed on the fly)
+//                                         mb_fast_polish_exact (exact phase)
 // and, for the search drivers' polish_peaks_with_weights (search/path1_eval_fast.cpp:58-143, whose
-// A/B form is in k2_compat.cu), mb_polish_peaks_exact with (A, B) computed on the fly.
-// The *_exact forms read the table and the peaks' 64.64 fixed-point v (+ delta) and never form the
-// P x N matrices, so they are bound by the phase and sincos work, not by 16 B/term of HBM traffic.
+// A/B form is in k2_compat.cu), mb_polish_peaks_exact and mb_polish_peaks_weights.
+// The exact-phase forms read the table and the peaks' 64.64 fixed-point v (+ delta).  They polish on moments
+// over cells of zeros (k2_cells.h), which visit each zero once per peak; where the offsets reach too far for
+// cells, or memory is short, over the zeros with (A, B) computed on the fly, or, under several weight
+// vectors, from matrices built chunk by chunk.
 #include <algorithm>
 #include <cmath>
 #include <cstring>
@@ -431,10 +433,11 @@ extern "C" int mb_polish_peaks_exact(mb_table *h, int64_t P, const uint64_t *v_i
     return fetch_outputs(t.stream, P, s.hu, s.hp, s.dp, out_h_unpol, out_h_pol, out_ddy_pol);
 }
 
-// polish_peaks_with_weights under several weight vectors: the exact (A, B) of a chunk of peaks is
-// written once to HBM (the reference's P x N matrices, search/eval_tech1_600k.py:216-273, with the
-// exact phase of mb_exact_AB) and every weight's polish reads it, instead of recomputing each term's
-// 128-bit phase and sine/cosine in every pass.  Chunks keep the matrices within AB_BUDGET bytes.
+// polish_peaks_with_weights under several weight vectors, where the cells do not serve: the exact (A, B)
+// of a chunk of peaks is written once to HBM (the reference's P x N matrices,
+// search/eval_tech1_600k.py:216-273, with the exact phase of mb_exact_AB) and every weight's polish reads
+// it, instead of recomputing each term's 128-bit phase and sine/cosine in every pass.  Chunks keep the
+// matrices within AB_BUDGET bytes.
 constexpr size_t AB_BUDGET = (size_t)4 << 30;
 
 extern "C" int mb_polish_peaks_weights(mb_table *h, int64_t P, const uint64_t *v_int, const uint64_t *v_frac,

@@ -7,8 +7,8 @@ namespace mb {
 
 // (cos, sin)(2 pi q / 256) in eight interleaved copies: entry q of copy c sits in the c-th
 // 16-byte bank group, and lane l reads copy l mod 8, so a warp's 32 random entries are read in the
-// four shared-memory cycles of a conflict-free 512-byte access (4.2 cycles measured, 9.4 for one
-// copy of a 2048-entry table).
+// four shared-memory cycles of a conflict-free 512-byte access (one copy of a 2048-entry table: about nine, for
+// the random entries' bank conflicts).
 constexpr int PH_TAB = 256;
 constexpr int PH_COPIES = 8;
 constexpr int PH_BYTES = PH_TAB * PH_COPIES * (int)sizeof(double2);

@@ -263,7 +263,7 @@ constexpr int64_t SCAN_MAX_POINTS = 65535;                  // block points per 
 // Chooses the block count and the series length with the smallest estimated work; false when the direct
 // kernel is the cheaper one (c_old: its warp cycles per 32 (point, zero) pairs): few points per base,
 // or a step so large that a block's cells hold less than a few zeros each.  The estimates are warp cycles
-// of one scheduler: a moment step (32 pairs) ~120 for the phasors + 20 per mma, the staging ~20 per zero and
+// of one scheduler, fitted to the kernels' measured times: a moment step (32 pairs) ~120 for the phasors + 20 per mma, the staging ~20 per zero and
 // CTA, 32 points of the evaluation 3.6 per FP64 operation, 2 D1 + 15 of them per cell.
 bool plan_scan(const Table &t, int64_t P, int64_t n_use, int64_t n_m, uint64_t step_int, uint64_t step_frac,
                double c_old, int64_t old_points, ScanPlan &best) {

@@ -6,8 +6,8 @@ Matrix forms (same arguments and results as the reference functions):
     h0, h, ddy = polish_single_peak(A[i], B[i], gamma, w)       # :94-147 (also 2-D: every row)
     h_unpol, h_pol, ddy_pol = fast_polish_batch(A, B, gamma, w) # fast_polish_batch_blas, :150-221
 
-Fused forms, which compute (A_j, B_j) on the fly from the exact phase of each peak's v (+ delta)
-and never form the P x N matrices:
+Fused forms, which work from the exact phase of each peak's v (+ delta) instead of P x N matrices: on
+moments over cells of zeros, taken in one pass, or over the zeros where a grid reaches too far for cells:
 
     slot = table.add_weights(w)
     h0, h, ddy = polish_single_exact(table, cands, slot, n_zeros)
@@ -95,7 +95,7 @@ def fast_polish_batch(A_mat, B_mat, gamma_vec, w_vec, ddy_grid=None, top: int = 
 
 def polish_single_exact(table, cands, weight_slot: int, n_zeros: int | None = None, grid_hw: float = 4e-5,
                         grid_steps: int = 40):
-    """polish_single_peak for every candidate, (A, B) computed on the fly."""
+    """polish_single_peak for every candidate, from the exact phase."""
     vi, vf, d = _cands(cands)
     P = vi.shape[0]
     n = table.n if n_zeros is None else int(n_zeros)
@@ -106,7 +106,7 @@ def polish_single_exact(table, cands, weight_slot: int, n_zeros: int | None = No
 
 
 def fast_polish_exact(table, cands, weight_slot: int, n_zeros: int | None = None, ddy_grid=None, top: int = 25):
-    """fast_polish_batch for every candidate, (A, B) computed on the fly."""
+    """fast_polish_batch for every candidate, from the exact phase."""
     vi, vf, d = _cands(cands)
     P = vi.shape[0]
     n = table.n if n_zeros is None else int(n_zeros)
@@ -119,8 +119,8 @@ def fast_polish_exact(table, cands, weight_slot: int, n_zeros: int | None = None
 
 def polish_peaks_exact(table, cands, weight_slot: int, n_zeros: int | None = None,
                        grid_half_width: float = 2.5e-4, grid_steps: int = 40):
-    """polish_peaks_with_weights (search/path1_eval_fast.cpp:58-143) for every candidate, (A, B)
-    computed on the fly; the defaults are the search drivers' settings (eval_tech1_600k.py:262)."""
+    """polish_peaks_with_weights (search/path1_eval_fast.cpp:58-143) for every candidate, from the exact
+    phase; the defaults are the search drivers' settings (eval_tech1_600k.py:262)."""
     vi, vf, d = _cands(cands)
     P = vi.shape[0]
     n = table.n if n_zeros is None else int(n_zeros)
@@ -133,8 +133,8 @@ def polish_peaks_exact(table, cands, weight_slot: int, n_zeros: int | None = Non
 def polish_peaks_weights(table, cands, weight_slots, n_zeros: int | None = None,
                          grid_half_width: float = 2.5e-4, grid_steps: int = 40):
     """polish_peaks_exact under several registered weight vectors at once: (h_unpol, h_pol,
-    ddy_pol), each of shape (len(weight_slots), P).  The exact (A, B) is built once in device
-    memory and read by every weight's polish (search/eval_tech1_600k.py:216-273)."""
+    ddy_pol), each of shape (len(weight_slots), P), each row that of the single-vector call
+    (search/eval_tech1_600k.py:216-273)."""
     vi, vf, d = _cands(cands)
     P = vi.shape[0]
     n = table.n if n_zeros is None else int(n_zeros)

@@ -4,8 +4,8 @@ search/eval_tech1_600k.py:216-273 (and eval_tech2_hdrop_600k.py, eval_sub35_cand
 their candidates by compute_peak_AB over all N zeros followed by one polish_peaks_with_weights per
 weight vector (grid_half_width 2.5e-4, 40 steps): the P x N A/B matrices are built once and read
 five times.  Here each weight vector is registered with the table once and all polishes are one
-mb_polish_peaks_weights call, which writes the exact-phase (A_j, B_j) of the candidates to device
-memory once and runs every weight's polish from it:
+mb_polish_peaks_weights call: the zeros' cell moments of every candidate under all vectors in one pass
+from the exact phase, grid and Newton on them, and no matrices:
 
     table = k2.ZeroTable.from_data(data)
     slots = register(table, reference_weights(data.gamma))   # once per table
