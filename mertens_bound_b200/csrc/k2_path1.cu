@@ -153,6 +153,18 @@ int fetch_outputs(cudaStream_t st, int64_t P, const double *hu, const double *hp
 
 // ------------------------------------------------------------------ polishes on cell moments
 
+// Whether v + delta stays in [0, 2^64) at every peak: the moments are taken at that sum as a 64.64 number, which
+// would wrap (the loops over the zeros keep delta apart).
+bool sums_in_range(int64_t P, const uint64_t *vi, const uint64_t *vf, const double *delta) {
+    typedef unsigned __int128 u128;
+    if (!delta) return true;
+    for (int64_t p = 0; p < P; ++p) {
+        const u128 v = (u128)vi[p] << 64 | vf[p], d = (u128)std::round(std::fabs(delta[p]) * 0x1p64);
+        if (delta[p] < 0.0 ? v < d : v + d < v) return false;
+    }
+    return true;
+}
+
 constexpr size_t POLISH_MOMENT_BYTES = (size_t)256 << 20;
 
 // Plans the cells of a polish whose offsets stay within R of the peaks: true where the polish on moments is not
@@ -386,7 +398,8 @@ extern "C" int mb_polish_single_exact(mb_table *h, int64_t P, const uint64_t *v_
     ExactStage s;
     MB_TRY(stage_exact(t, P, v_int, v_frac, delta, grid.data(), (int64_t)grid.size(), 0, s));
     CellPlan cp;
-    if (plan_polish(t, n_zeros, 0, single_reach(grid_hw, grid_steps), POLISH_SINGLE, cp)) {
+    if (sums_in_range(P, v_int, v_frac, delta) &&
+        plan_polish(t, n_zeros, 0, single_reach(grid_hw, grid_steps), POLISH_SINGLE, cp)) {
         const int st = polish_on_cells(t, s, P, n_zeros, 1, &weight_slot, cp,
                                        CellPolishArgs{POLISH_SINGLE, P, 1, P, s.grid, (int)grid.size(), 0.0, nullptr, s.hu,
                                                       s.hp, s.dp});
@@ -417,7 +430,8 @@ extern "C" int mb_polish_peaks_exact(mb_table *h, int64_t P, const uint64_t *v_i
     ExactStage s;
     MB_TRY(stage_exact(t, P, v_int, v_frac, delta, nullptr, 0, 0, s));
     CellPlan cp;
-    if (plan_polish(t, n_zeros, 4096, eval_fast_reach(grid_half_width, grid_steps), POLISH_EVAL_FAST, cp)) {
+    if (sums_in_range(P, v_int, v_frac, delta) &&
+        plan_polish(t, n_zeros, 4096, eval_fast_reach(grid_half_width, grid_steps), POLISH_EVAL_FAST, cp)) {
         const int st = polish_on_cells(t, s, P, n_zeros, 1, &weight_slot, cp,
                                        CellPolishArgs{POLISH_EVAL_FAST, P, 1, P, nullptr, grid_steps, grid_half_width,
                                                       nullptr, s.hu, s.hp, s.dp});
@@ -463,7 +477,8 @@ extern "C" int mb_polish_peaks_weights(mb_table *h, int64_t P, const uint64_t *v
     MB_TRY(device_guard(t.device));
     ExactStage s;
     CellPlan cp;
-    if (plan_polish(t, n_zeros, 4096, eval_fast_reach(grid_half_width, grid_steps), POLISH_EVAL_FAST, cp)) {
+    if (sums_in_range(P, v_int, v_frac, delta) &&
+        plan_polish(t, n_zeros, 4096, eval_fast_reach(grid_half_width, grid_steps), POLISH_EVAL_FAST, cp)) {
         const size_t ob = (size_t)n_weights * P;
         MB_TRY(stage_exact(t, P, v_int, v_frac, delta, nullptr, (int64_t)(3 * ob), 0, s));
         double *hu = s.grid, *hp = hu + ob, *dp = hp + ob;       // outputs in the stage's grid array
@@ -545,7 +560,14 @@ extern "C" int mb_fast_polish_exact(mb_table *h, int64_t P, const uint64_t *v_in
     const ABExact src{view(t), s.vi, s.vf, s.delta};
     const double *d_w = t.d_weights[weight_slot];
     const int n_chunk = taylor_chunks(n_zeros);
+    const bool fold = sums_in_range(P, v_int, v_frac, delta);
     auto grid_stage = [&]() -> int {
+        if (!fold) {
+            const MomentArgs m{n_zeros, t.d_gamma, d_w, s.grid, (int)n_grid, s.hu, s.hp, s.dp};
+            taylor_moments_kernel<ABExact><<<(unsigned)(P * POLISH_CLUSTER), POLISH_THREADS, 0, t.stream>>>(src, m);
+            MB_CUDA(cudaGetLastError());
+            return MB_OK;
+        }
         int64_t pc = std::max<int64_t>(
             1, std::min<int64_t>(P, (int64_t)(POLISH_MOMENT_BYTES / taylor_work_bytes(1, n_chunk))));
         for (bool room = false; !room;) {                // fewer peaks a pass where memory is short
@@ -567,7 +589,7 @@ extern "C" int mb_fast_polish_exact(mb_table *h, int64_t P, const uint64_t *v_in
     double reach = 4 * 1e-5;
     for (int64_t i = 0; i < n_grid; ++i) reach = std::max(reach, std::fabs(ddy_grid[i]) + 4 * 1e-5);
     CellPlan cp;
-    if (plan_polish(t, n_zeros, 0, reach, POLISH_TOPK, cp)) {
+    if (fold && plan_polish(t, n_zeros, 0, reach, POLISH_TOPK, cp)) {
         const int st = polish_on_cells(t, s, nsel, n_zeros, 1, &weight_slot, cp,
                                        CellPolishArgs{POLISH_TOPK, nsel, 1, P, nullptr, 0, 0.0, s.sel, s.hu, s.hp, s.dp});
         if (st == MB_OK) return fetch_outputs(t.stream, P, s.hu, s.hp, s.dp, out_h_unpol, out_h_pol, out_ddy_pol);

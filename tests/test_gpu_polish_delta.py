@@ -41,3 +41,27 @@ def test_rest_of_delta(gpu, small_table, kind):
                     path1.fast_polish_exact(t, c, s, None, ddy_grid=np.zeros(1), top=c.n)):
             assert np.max(np.abs(got[0] - want)) <= tol
             assert np.max(np.abs(got[1] - want)) <= tol
+
+
+@pytest.mark.parametrize("end", ["low", "high"])
+def test_sum_outside_the_fixed_point_range(gpu, small_table, end):
+    """v + delta below 0 or at 2^64 and above: as on the exact (A, B) of that sum, and for the peaks beside it too."""
+    from mertens_bound_b200 import compat
+    data = small_table.truncate(3000)
+    c = synth.make_candidates(20, seed=93)
+    c.delta[:] = np.random.default_rng(93).uniform(-1e-4, 1e-4, c.n)
+    c.v_int[:3] = 0 if end == "low" else 2**64 - 1
+    c.v_frac[:3] = np.array([12345, 2**40, 2**62] if end == "low" else [2**64 - 2, 2**64 - 2**40, 2**63], np.uint64)
+    c.delta[:3] = np.array([-1e-4, -0.7, -60000.0]) * (1 if end == "low" else -1)
+    w = np.exp(-3e-9 * data.gamma**2)
+    with k2.ZeroTable.from_data(data) as t:
+        s = t.add_weights(w)
+        A, B = path1.compute_exact_AB(t, c)
+        one, many = path1.polish_peaks_exact(t, c, s), path1.polish_peaks_weights(t, c, [s, s])
+        single, fast = path1.polish_single_exact(t, c, s), path1.fast_polish_exact(t, c, s, top=c.n)
+    peaks = compat.polish_peaks_with_weights(A, B, data.gamma, w, 2.5e-4, 40)
+    for got, want in ((one, peaks), ([x[1] for x in many], peaks),
+                      (single, path1.polish_single_peak(A, B, data.gamma, w)),
+                      (fast, path1.fast_polish_batch(A, B, data.gamma, w, top=c.n))):
+        for g, x, tol in zip(got, want, (3e-13, 3e-11, 1e-12)):
+            np.testing.assert_allclose(g, x, rtol=0, atol=tol)
