@@ -1102,6 +1102,9 @@ bool plan_cells(const Table &t, int64_t n, int64_t split, double R, int d1, int6
     int64_t half = (int64_t)std::min(want, 1e12);
     const int64_t lo = (int64_t)std::floor(t.h_gamma[0] / two_pi * 65536.0) - 2;
     const int64_t hi = (int64_t)std::ceil(t.h_gamma[n - 1] / two_pi * 65536.0) + 2;
+    // no wider than the zeros: with gamma far below the cells' centre, Newton's sums, formed about the centre,
+    // would cancel
+    half = std::min(half, std::max<int64_t>(2, (hi - lo + 1) / 2));
     if (min_cells > 1) half = std::min(half, std::max<int64_t>(2, (hi - lo) / (2 * min_cells)));
     out.half = half;
     auto group = [&](int q, int64_t a, int64_t b) {
