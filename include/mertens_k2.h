@@ -346,8 +346,8 @@ int mb_fast_polish_batch(int64_t n_peaks, int64_t n_zeros, const double *A, cons
 /* The two polishes of peak p at y = v_p + delta_p from the exact phase, as on the (A, B) of mb_exact_AB
  * (no P x N matrices), over the table's first n_zeros zeros, gamma = the table's FP64 gamma and w = a
  * weight vector registered by mb_table_add_weights.  They run on moments over cells of zeros (the same
- * values within FP64 rounding) or, where the offsets reach too far for cells or memory is short, over
- * the zeros; device workspace as mb_polish_peaks_weights. */
+ * values within FP64 rounding) or, where the offsets reach too far for cells, v + delta leaves
+ * [0, 2^64) or memory is short, over the zeros; device workspace as mb_polish_peaks_weights. */
 int mb_polish_single_exact(mb_table *t, int64_t P, const uint64_t *v_int, const uint64_t *v_frac,
                            const double *delta, int64_t n_zeros, int weight_slot, double grid_hw, int grid_steps,
                            double *out_h_unpol, double *out_h_pol, double *out_ddy_pol);
