@@ -169,7 +169,9 @@ constexpr size_t POLISH_MOMENT_BYTES = (size_t)256 << 20;
 
 // Plans the cells of a polish whose offsets stay within R of the peaks: true where the polish on moments is not
 // slower than the loops over the zeros.  At least 592 cells (two items per CTA slot) where they hold 64 zeros: few
-// peaks then still fill the GPU.  The split and the choice depend on the zeros, R and the loop alone, so a
+// peaks then still fill the GPU.  Twice as many, and 32 zeros, for POLISH_TOPK, whose offsets converge: shorter
+// running sums in the moments, without which its ddy are three times as far off as the loops' (6.9e-20 against
+// 2.4e-20 rms on 87,292 zeros, now 1.9e-20).  The split and the choice depend on the zeros, R and the loop alone, so a
 // peak's results do not depend on the others in the call, nor on the number of weight vectors.
 //   Up to CPOL_CELLS cells (their moments fit shared memory) four zeros a cell are enough.
 //   Above that a polish costs ~cells per peak and start, and 1 / cells of the peaks fit a pass of
@@ -183,7 +185,8 @@ constexpr size_t POLISH_MOMENT_BYTES = (size_t)256 << 20;
 //   TOPK      25 peaks: 100,000 zeros, 2,000 cells 0.21 against 0.29, 5,700 cells 0.31 against 0.29
 bool plan_polish(const Table &t, int64_t n, int64_t split, double R, int mode, CellPlan &cp) {
     if (n < 1 || !std::isfinite(R)) return false;
-    if (!plan_cells(t, n, split, R, CELL_D1, std::min<int64_t>(n / 64, 592), cp)) return false;
+    const int64_t few = mode == POLISH_TOPK ? std::min<int64_t>(n / 32, 1184) : std::min<int64_t>(n / 64, 592);
+    if (!plan_cells(t, n, split, R, CELL_D1, few, cp)) return false;
     const int64_t c = cp.cells();
     // one peak's moments under a full set of vectors stay within the workspace
     if (c * (2 * CELL_D1 * 8 * CELL_MAX_W) > (int64_t)POLISH_MOMENT_BYTES) return false;
