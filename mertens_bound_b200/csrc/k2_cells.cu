@@ -992,10 +992,14 @@ taylor_grid_kernel(const double *S, int n_chunk, const double *delta, const doub
         double x[8];
 #pragma unroll
         for (int i = 0; i < 8; ++i) x[i] = 0.0;
-        for (int c = warp; c < n_chunk; c += 32)
+        const double *s = S + p * n_chunk * 24 + lane;
+        int c = warp;
+        for (; c + 28 < n_chunk; c += 32)
 #pragma unroll
-            for (int i = 0; i < 8; ++i)
-                if (c + 4 * i < n_chunk) x[i] += S[(p * n_chunk + c + 4 * i) * 24 + lane];
+            for (int i = 0; i < 8; ++i) x[i] += s[(c + 4 * i) * 24];
+#pragma unroll
+        for (int i = 0; i < 8; ++i)
+            if (c + 4 * i < n_chunk) x[i] += s[(c + 4 * i) * 24];
         part[warp][lane] = ((x[0] + x[1]) + (x[2] + x[3])) + ((x[4] + x[5]) + (x[6] + x[7]));
     }
     __syncthreads();
