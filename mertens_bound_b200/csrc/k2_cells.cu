@@ -1174,12 +1174,12 @@ int launch_moments_weights(const Table &t, const Cells &c, const uint64_t *vi, c
     }
 }
 
-// Chunks of 256 zeros on average, at most two per CTA slot, and one per SM where they hold 64 zeros.  Their number
+// Chunks of 336 zeros on average, at most two per CTA slot, and one per SM where they hold 64 zeros.  Their number
 // depends on the zeros alone and one warp adds a chunk's zeros, so a peak's sums keep their bits whatever the peaks
 // beside it.  That costs calls of few peaks, whose CTAs have idle warps: one peak on 100,000 zeros 75 -> 88 us with
 // eight warps to a chunk's zeros where there are 8 peaks, but two for all calls cost 1,024 peaks 490 -> 524.
 int taylor_chunks(int64_t n) {
-    return (int)std::max<int64_t>({1, std::min<int64_t>(592, n / 256), std::min<int64_t>(148, n / 64)});
+    return (int)std::max<int64_t>({1, std::min<int64_t>(592, n / 336), std::min<int64_t>(148, n / 64)});
 }
 
 size_t taylor_work_bytes(int64_t P, int n_chunk) {
